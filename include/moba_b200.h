@@ -247,6 +247,23 @@ int moba_b200_bwd(const moba_b200_problem* p, const void* q, const void* k, cons
                   float* delta, void* dq_part, void* dkv_scratch, void* dq, void* dk, void* dv,
                   void* stream);
 
+/* The whole op in one call each way: what moba_forward (src/moba/kernels/moba_fwd.py:783-835)
+ * and the autograd pair (src/moba/kernels/attention.py:53-132) of the reference do in one Python
+ * call each. They run the stages above back to back on one stream, without a query window.
+ *   moba_b200_op_workspace  sizes of the three buffers the caller provides, functions of the
+ *                           problem record alone: `keep` holds the index and the log-sum-exps
+ *                           from a forward to its backward (an inference call may drop it
+ *                           afterwards), the other two only live during their call
+ *   moba_b200_op_forward    out, and (want_lse != 0) the log-sum-exp, which goes into `keep`
+ *   moba_b200_op_backward   dq, dk, dv from the `keep` of that forward, same problem record
+ * All three workspaces must be 256-byte aligned. The layout inside them is private. */
+int moba_b200_op_workspace(const moba_b200_problem* p, size_t* keep_bytes, size_t* forward_bytes, size_t* backward_bytes);
+int moba_b200_op_forward(const moba_b200_problem* p, const void* q, const void* k, const void* v,
+                         const int32_t* cu_seqlens, void* keep_ws, void* forward_ws, void* out, int want_lse, void* stream);
+int moba_b200_op_backward(const moba_b200_problem* p, const void* q, const void* k, const void* v, const void* out,
+                          const void* dout, const int32_t* cu_seqlens, const void* keep_ws, void* backward_ws,
+                          void* dq, void* dk, void* dv, void* stream);
+
 /* Packed (variable-length) batches, the step either side of the op. A "row" is
  * one token's H*D elements (row_bytes, a multiple of 16), contiguous in the
  * token-major layout.

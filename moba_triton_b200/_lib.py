@@ -29,6 +29,7 @@ EXPORTS = (
     "moba_b200_pack_index", "moba_b200_pack_rows", "moba_b200_unpack_rows", "moba_b200_seq_meta",
     "moba_b200_chunk_tiles", "moba_b200_work_items_per_row", "moba_b200_dkv_scratch_bytes",
     "moba_b200_launch_plan",
+    "moba_b200_op_workspace", "moba_b200_op_forward", "moba_b200_op_backward",
 )
 
 
@@ -84,6 +85,10 @@ def load():
     lib.moba_b200_fwd.argtypes = [P, vp, vp, vp, I, vp, vp, vp, vp]
     lib.moba_b200_merge.argtypes = [P, vp, vp, vp, vp, vp]
     lib.moba_b200_bwd.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, I, vp, vp, vp, vp, vp, vp, vp, vp]
+    SZ = POINTER(c_size_t)
+    lib.moba_b200_op_workspace.argtypes = [P, SZ, SZ, SZ]
+    lib.moba_b200_op_forward.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, c_int, vp]
+    lib.moba_b200_op_backward.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.moba_b200_pack_index.argtypes = [vp, c_int, c_int, c_int, vp, vp, vp, vp, vp]
     lib.moba_b200_pack_rows.argtypes = [vp, vp, vp, vp, c_int, c_int, c_size_t, vp]
     lib.moba_b200_unpack_rows.argtypes = [vp, vp, vp, c_int, c_int, c_size_t, vp]
@@ -115,6 +120,20 @@ def call(name: str, device, what: str, *args) -> None:
     stream appended as the last argument; raises on a failure status."""
     with torch.cuda.device(device):
         check(getattr(load(), name)(*args, stream_ptr(device)), what)
+
+
+def call_op(name: str, device_index: int, what: str, *args) -> None:
+    """`call` for the whole-op entry points: device number and plain addresses, and no device
+    switch when the device is current already (what is left of the host's share of a short
+    sequence)."""
+    fn = getattr(_lib or load(), name)
+    if torch.cuda.current_device() == device_index:
+        rc = fn(*args, torch._C._cuda_getCurrentRawStream(device_index))
+    else:
+        with torch.cuda.device(device_index):
+            rc = fn(*args, torch._C._cuda_getCurrentRawStream(device_index))
+    if rc < 0:
+        check(rc, what)
 
 
 def device_status(device=None) -> int:

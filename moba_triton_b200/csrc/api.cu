@@ -48,9 +48,31 @@ KernelTimer::~KernelTimer() {
   g_timed.push_back(TimedLaunch{name_, start_, stop});
 }
 
+int raise_smem_limit(SmemLimit& done, const void* kernel, size_t bytes) {
+  if (bytes <= 48 * 1024) return MOBA_B200_OK;
+  int dev = 0;
+  MOBA_CUDA_OK(cudaGetDevice(&dev));
+  int* have = dev >= 0 && dev < 64 ? &done.bytes[dev] : nullptr;      // racing callers set the same limit twice, harmlessly
+  if (have != nullptr && __atomic_load_n(have, __ATOMIC_RELAXED) >= (int)bytes) return MOBA_B200_OK;
+  MOBA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (have != nullptr) __atomic_store_n(have, (int)bytes, __ATOMIC_RELAXED);
+  return MOBA_B200_OK;
+}
+
+int sm_count() {
+  static int table[64] = {0};
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return sms;
+  const int known = __atomic_load_n(&table[dev], __ATOMIC_RELAXED);
+  if (known > 0) return known;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  __atomic_store_n(&table[dev], sms, __ATOMIC_RELAXED);
+  return sms;
+}
+
 static bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 
-static int check_problem(const moba_b200_problem* p) {
+int check_problem(const moba_b200_problem* p) {
   if (p == nullptr) { set_error("problem is NULL"); return MOBA_B200_EINVAL; }
   if (p->dtype < MOBA_B200_F32 || p->dtype > MOBA_B200_F16) {
     set_error("unknown dtype code %d", p->dtype); return MOBA_B200_EINVAL;
@@ -97,12 +119,12 @@ static int check_problem(const moba_b200_problem* p) {
   return MOBA_B200_OK;
 }
 
-static int need(const void* ptr, const char* name) {
+int need(const void* ptr, const char* name) {
   if (ptr == nullptr) { set_error("%s is NULL", name); return MOBA_B200_EINVAL; }
   return MOBA_B200_OK;
 }
 
-static int pick(const moba_b200_problem& p, bool fast_ok, const char* stage) {
+int pick(const moba_b200_problem& p, bool fast_ok, const char* stage) {
   if (p.path == MOBA_B200_PATH_PORTABLE) return MOBA_B200_PATH_PORTABLE;
   if (p.path == MOBA_B200_PATH_TCGEN05) {
     if (!fast_ok) { set_error("%s: tcgen05 kernels do not cover this shape/dtype", stage); return MOBA_B200_EUNSUPPORTED; }
@@ -114,8 +136,6 @@ static int pick(const moba_b200_problem& p, bool fast_ok, const char* stage) {
 }  // namespace moba
 
 using namespace moba;
-
-#define MOBA_TRY(expr) do { int rc__ = (expr); if (rc__ != MOBA_B200_OK) return rc__; } while (0)
 
 extern "C" {
 
@@ -225,7 +245,7 @@ int moba_b200_pool(const moba_b200_problem* p, const void* k, const int32_t* cu_
   MOBA_TRY(check_problem(p));
   MOBA_TRY(need(k, "k")); MOBA_TRY(need(kbar, "kbar"));
   if (p->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
-  return launch_pool(*p, k, cu_seqlens, kbar, (cudaStream_t)stream);
+  return launch_pool(*p, k, cu_seqlens, kbar, nullptr, (cudaStream_t)stream);
 }
 
 int moba_b200_gate(const moba_b200_problem* p, const void* q, const void* kbar,
@@ -236,8 +256,8 @@ int moba_b200_gate(const moba_b200_problem* p, const void* q, const void* kbar,
   const int path = pick(*p, gate_sm100_supported(*p), "gate");
   if (path < 0) return path;
   if (path == MOBA_B200_PATH_TCGEN05)
-    return launch_gate_sm100(*p, q, kbar, cu_seqlens, block_idx, (cudaStream_t)stream);
-  return launch_gate_portable(*p, q, kbar, cu_seqlens, block_idx, (cudaStream_t)stream);
+    return launch_gate_sm100(*p, q, kbar, cu_seqlens, block_idx, nullptr, (cudaStream_t)stream);
+  return launch_gate_portable(*p, q, kbar, cu_seqlens, block_idx, nullptr, (cudaStream_t)stream);
 }
 
 int moba_b200_transpose(const moba_b200_problem* p, const int32_t* block_idx,
@@ -253,7 +273,7 @@ int moba_b200_transpose(const moba_b200_problem* p, const int32_t* block_idx,
   MOBA_TRY(need(scratch, "scratch"));
   if (p->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
   return launch_transpose(*p, block_idx, cu_seqlens, col_nnz, col_offsets, order, row_indices,
-                          head_indices, slot_of_pair, work_items, scratch, scratch_bytes, (cudaStream_t)stream);
+                          head_indices, slot_of_pair, nullptr, work_items, scratch, scratch_bytes, (cudaStream_t)stream);
 }
 
 int moba_b200_transpose_noalloc(const moba_b200_problem* p, const int32_t* block_idx,

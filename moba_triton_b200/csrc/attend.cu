@@ -14,6 +14,8 @@
 namespace moba {
 
 __global__ void fill_kernel(float* __restrict__ dst, size_t n, float value) {
+  pdl_trigger();
+  pdl_wait();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = value;
 }
@@ -22,8 +24,7 @@ int launch_fill_lse(const moba_b200_problem& p, float* part_lse, cudaStream_t st
   KernelTimer timer__("fill_kernel", st);
   const size_t n = (size_t)p.batch * p.q_heads * window_rows(p) * p.slots;
   const int blocks = (int)((n + 1023) / 1024 < 148 * 8 ? (n + 1023) / 1024 : 148 * 8);
-  fill_kernel<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(part_lse, n, -INFINITY);
-  MOBA_LAUNCH_OK("fill_kernel");
+  MOBA_CUDA_OK(launch_chained(fill_kernel, blocks > 0 ? blocks : 1, 256, 0, st, part_lse, n, -INFINITY));
   return MOBA_B200_OK;
 }
 
@@ -40,6 +41,7 @@ __global__ void __launch_bounds__(256)
 fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                     moba_b200_index ix, const int32_t* __restrict__ cu, TP* __restrict__ part_o,
                     float* __restrict__ part_lse, moba_b200_problem p) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int d = p.head_dim, bs = p.block_size, nb = p.num_blocks;
   const int kstride = d + 1;
@@ -75,9 +77,7 @@ fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float scale = rsqrtf((float)d) * kLog2e;
-  const int32_t* rows_i = ix.row_indices + (size_t)kv_row * ix.capacity + lo;
-  const int32_t* heads_i = ix.head_indices + (size_t)kv_row * ix.capacity + lo;
-  const int32_t* slots_i = ix.slot_of_pair + (size_t)kv_row * ix.capacity + lo;
+  const size_t list0 = (size_t)kv_row * ix.capacity + lo;
   float* qw = Qs + warp * kFwdRows * d;
   float* pw = Ps + warp * kFwdRows * bs;
   const int key_iters = (bs + 31) / 32;
@@ -87,9 +87,9 @@ fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
 #pragma unroll
     for (int r = 0; r < kFwdRows; ++r) {
       const bool live = e0 + r < n;
-      row[r] = live ? rows_i[e0 + r] : -1;
-      head[r] = live ? heads_i[e0 + r] : 0;
-      slot[r] = live ? slots_i[e0 + r] : 0;
+      PairEntry pe{-1, 0, 0};
+      if (live) pe = load_pair(ix, list0 + e0 + r);
+      row[r] = pe.row; head[r] = pe.head; slot[r] = pe.slot;
       for (int c = lane; c < d; c += 32)
         qw[r * d + c] = live ? Elem<T>::to_f(q[((b * p.tokens + row[r]) * p.q_heads + head[r]) * (size_t)d + c]) : 0.f;
     }
@@ -196,16 +196,15 @@ int launch_fwd_portable(const moba_b200_problem& p, const void* q, const void* k
   dim3 grid(p.num_blocks, p.n_seq * p.kv_heads);
 #define MOBA_FWD(T, TP)                                                                        \
   do {                                                                                         \
-    MOBA_CUDA_OK(cudaFuncSetAttribute(fwd_portable_kernel<T, TP>,                              \
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    fwd_portable_kernel<T, TP><<<grid, 256, smem, st>>>((const T*)q, (const T*)k, (const T*)v, \
-                                                        ix, cu, (TP*)part_o, part_lse, p);     \
+    static SmemLimit limit;                                                                    \
+    if (int rc = raise_smem_limit(limit, (const void*)fwd_portable_kernel<T, TP>, smem)) return rc; \
+    MOBA_CUDA_OK(launch_chained(fwd_portable_kernel<T, TP>, grid, 256, smem, st, (const T*)q, (const T*)k, (const T*)v, \
+                                ix, cu, (TP*)part_o, part_lse, p));                           \
   } while (0)
   if (p.dtype == MOBA_B200_F32) MOBA_FWD(float, float);
   else if (p.dtype == MOBA_B200_BF16) { if (p.part_f32) MOBA_FWD(__nv_bfloat16, float); else MOBA_FWD(__nv_bfloat16, __nv_bfloat16); }
   else { if (p.part_f32) MOBA_FWD(__half, float); else MOBA_FWD(__half, __half); }
 #undef MOBA_FWD
-  MOBA_LAUNCH_OK("fwd_portable_kernel");
   return MOBA_B200_OK;
 }
 
@@ -219,6 +218,8 @@ __global__ void __launch_bounds__(256)
 merge_kernel(const TP* __restrict__ part_o, const float* __restrict__ part_lse,
              TO* __restrict__ out, float* __restrict__ lse_out, int tokens,
              int q_heads, int d, int slots, int win_begin, int win_rows) {
+  pdl_trigger();
+  pdl_wait();
   // grid (row groups of one (batch entry, head), heads, batch): no division anywhere (generic
   // 64-bit divisions cost this streaming kernel more instructions than its sums)
   constexpr int EPV = 16 / sizeof(TP);
@@ -286,14 +287,12 @@ int launch_merge(const moba_b200_problem& p, const void* part_o, const float* pa
   if (threads == 0 || p.batch == 0) return MOBA_B200_OK;
   const dim3 blocks((unsigned)((threads + 255) / 256), (unsigned)p.q_heads, (unsigned)p.batch);
 #define MOBA_MERGE(TP, TO)                                                                      \
-  merge_kernel<TP, TO><<<blocks, 256, 0, st>>>((const TP*)part_o, part_lse, (TO*)out, lse,      \
-                                               p.tokens, p.q_heads, p.head_dim, p.slots,        \
-                                               p.win_begin, window_rows(p))
+  MOBA_CUDA_OK(launch_chained(merge_kernel<TP, TO>, blocks, 256, 0, st, (const TP*)part_o, part_lse, (TO*)out, lse, \
+                              p.tokens, p.q_heads, p.head_dim, p.slots, p.win_begin, window_rows(p)))
   if (p.dtype == MOBA_B200_F32) MOBA_MERGE(float, float);
   else if (p.dtype == MOBA_B200_BF16) { if (pf32) MOBA_MERGE(float, __nv_bfloat16); else MOBA_MERGE(__nv_bfloat16, __nv_bfloat16); }
   else { if (pf32) MOBA_MERGE(float, __half); else MOBA_MERGE(__half, __half); }
 #undef MOBA_MERGE
-  MOBA_LAUNCH_OK("merge_kernel");
   return MOBA_B200_OK;
 }
 

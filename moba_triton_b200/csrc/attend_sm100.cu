@@ -204,6 +204,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem = bars->tmem_base;
 
   const float cs = rsqrtf((float)D) * kLog2e;
@@ -255,9 +256,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       const int e = (int)(k.t - k.t0) * kTile + r;
       row = head = slot = 0;
       if (r < kTile && e < k.c.n) {
-        const size_t o = (size_t)k.c.kv_row * ix.capacity + k.c.lo + e;
-        row = ld_nc_pinned(ix.row_indices + o); head = ld_nc_pinned(ix.head_indices + o);
-        slot = ld_nc_pinned(ix.slot_of_pair + o);
+        const PairEntry pe = load_pair_pinned(ix, (size_t)k.c.kv_row * ix.capacity + k.c.lo + e);
+        row = pe.row; head = pe.head; slot = pe.slot;
       }
     };
     // Copies the 128 query rows of tile k.t into its stage. `n_gather` alternates the row
@@ -596,7 +596,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       const int item = item_of(round);
       Column c;
       if (round * G >= n_items || item >= n_items || !load_column(c, item, ix, p, cu, n_kv_rows)) return;
-      if (lane < 3) {
+      if (packed_pairs(ix)) {
+        if (lane == 0)
+          l2_prefetch_i32(ix.row_indices, 2 * ((size_t)c.kv_row * ix.capacity + c.lo), 2 * c.n, 2 * index_elems);
+      } else if (lane < 3) {
         const int32_t* arr = lane == 0 ? ix.row_indices : (lane == 1 ? ix.head_indices : ix.slot_of_pair);
         l2_prefetch_i32(arr, (size_t)c.kv_row * ix.capacity + c.lo, c.n, index_elems);
       }
@@ -695,14 +698,12 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
                const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse, int n_items,
                unsigned* err, cudaStream_t st) {
   auto kern = fwd_sm100_kernel<D, T, TP>;
-  MOBA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<D>::kSmem));
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  static SmemLimit limit;
+  if (int rc = raise_smem_limit(limit, (const void*)kern, FwdCfg<D>::kSmem)) return rc;
+  const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
-  kern<<<grid, FwdCfg<D>::kThreads, FwdCfg<D>::kSmem, st>>>(km, vm, (const T*)q, ix, cu, (TP*)part_o, part_lse, p,
-                                                             n_items, err);
-  MOBA_LAUNCH_OK("fwd_sm100_kernel");
+  MOBA_CUDA_OK(launch_chained(kern, grid, FwdCfg<D>::kThreads, FwdCfg<D>::kSmem, st, km, vm, (const T*)q, ix, cu,
+                              (TP*)part_o, part_lse, p, n_items, err));
   return MOBA_B200_OK;
 }
 

@@ -24,6 +24,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 delta_kernel(const T* __restrict__ out, const T* __restrict__ dout, float* __restrict__ delta,
              unsigned rows_per_batch, int tokens, int q_heads, int d, unsigned long long heads_recip, int heads_shift) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int EPV = 16 / sizeof(T);
   const int tpr = d / EPV;                        // threads per row: power of two, <= 32
   const unsigned gid = blockIdx.x * 256u + threadIdx.x;
@@ -70,13 +72,12 @@ int launch_delta(const moba_b200_problem& p, const void* out, const void* dout, 
   const unsigned long long recip = ((1ull << shift) + p.q_heads - 1) / p.q_heads;
   const dim3 grid((unsigned)((rows_per_batch * tpr + 255) / 256), (unsigned)p.batch);
 #define MOBA_DELTA(T) \
-  delta_kernel<T><<<grid, 256, 0, st>>>((const T*)out, (const T*)dout, delta, (unsigned)rows_per_batch, p.tokens, \
-                                        p.q_heads, p.head_dim, recip, shift)
+  MOBA_CUDA_OK(launch_chained(delta_kernel<T>, grid, 256, 0, st, (const T*)out, (const T*)dout, delta, (unsigned)rows_per_batch, \
+                              p.tokens, p.q_heads, p.head_dim, recip, shift))
   if (p.dtype == MOBA_B200_F32) MOBA_DELTA(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_DELTA(__nv_bfloat16);
   else MOBA_DELTA(__half);
 #undef MOBA_DELTA
-  MOBA_LAUNCH_OK("delta_kernel");
   return MOBA_B200_OK;
 }
 
@@ -100,6 +101,7 @@ bwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
                     const float* __restrict__ delta, moba_b200_index ix,
                     const int32_t* __restrict__ cu, T* __restrict__ dq_part, T* __restrict__ dk,
                     T* __restrict__ dv, moba_b200_problem p) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int d = p.head_dim, bs = p.block_size, nb = p.num_blocks;
   const int kstride = d + Pad<T>::value;
@@ -141,9 +143,7 @@ bwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float softmax_scale = rsqrtf((float)d);
   const float scale2 = softmax_scale * kLog2e;
-  const int32_t* rows_i = ix.row_indices + (size_t)kv_row * ix.capacity + lo;
-  const int32_t* heads_i = ix.head_indices + (size_t)kv_row * ix.capacity + lo;
-  const int32_t* slots_i = ix.slot_of_pair + (size_t)kv_row * ix.capacity + lo;
+  const size_t list0 = (size_t)kv_row * ix.capacity + lo;
   const int key_iters = (bs + 31) / 32;
   // phase-2 ownership: column dcol, keys jbase + i * jstep
   const int dcol = threadIdx.x % d;
@@ -153,9 +153,9 @@ bwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
     // ---- phase 1 ----
     const int e = e0 + warp;
     const bool live = e < n;
-    const int row = live ? rows_i[e] : -1;
-    const int head = live ? heads_i[e] : 0;
-    const int slot = live ? slots_i[e] : 0;
+    PairEntry pe{-1, 0, 0};
+    if (live) pe = load_pair(ix, list0 + e);
+    const int row = pe.row, head = pe.head, slot = pe.slot;
     float lse_r = 0.f, delta_r = 0.f;
     if (live) {
       const size_t qrow = (b * p.q_heads + head) * p.tokens + row;
@@ -250,16 +250,15 @@ int launch_bwd_portable(const moba_b200_problem& p, const void* q, const void* k
   dim3 grid(p.num_blocks, p.n_seq * p.kv_heads);
 #define MOBA_BWD(T)                                                                            \
   do {                                                                                         \
-    MOBA_CUDA_OK(cudaFuncSetAttribute(bwd_portable_kernel<T>,                                  \
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    bwd_portable_kernel<T><<<grid, 256, smem, st>>>((const T*)q, (const T*)k, (const T*)v,     \
-        (const T*)dout, lse, delta, ix, cu, (T*)dq_part, (T*)dk, (T*)dv, p);                   \
+    static SmemLimit limit;                                                                    \
+    if (int rc = raise_smem_limit(limit, (const void*)bwd_portable_kernel<T>, smem)) return rc; \
+    MOBA_CUDA_OK(launch_chained(bwd_portable_kernel<T>, grid, 256, smem, st, (const T*)q, (const T*)k, (const T*)v, \
+        (const T*)dout, lse, delta, ix, cu, (T*)dq_part, (T*)dk, (T*)dv, p));                 \
   } while (0)
   if (p.dtype == MOBA_B200_F32) MOBA_BWD(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_BWD(__nv_bfloat16);
   else MOBA_BWD(__half);
 #undef MOBA_BWD
-  MOBA_LAUNCH_OK("bwd_portable_kernel");
   return MOBA_B200_OK;
 }
 
@@ -272,6 +271,8 @@ __global__ void __launch_bounds__(256)
 dq_reduce_kernel(const T* __restrict__ dq_part, const float* __restrict__ part_lse,
                  T* __restrict__ dq, int tokens, int q_heads, int d, int slots,
                  int win_begin, int win_rows) {
+  pdl_trigger();
+  pdl_wait();
   // grid (row groups of one (batch entry, head), heads, batch): no division anywhere
   constexpr int EPV = 16 / sizeof(T);
   const unsigned tpr = (unsigned)(d / EPV);       // threads per row, a power of two
@@ -325,13 +326,12 @@ int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const floa
   if (threads == 0 || p.batch == 0) return MOBA_B200_OK;
   const dim3 blocks((unsigned)((threads + 255) / 256), (unsigned)p.q_heads, (unsigned)p.batch);
 #define MOBA_DQR(T) \
-  dq_reduce_kernel<T><<<blocks, 256, 0, st>>>((const T*)dq_part, part_lse, (T*)dq, p.tokens, p.q_heads, p.head_dim, p.slots, \
-                                              p.win_begin, window_rows(p))
+  MOBA_CUDA_OK(launch_chained(dq_reduce_kernel<T>, blocks, 256, 0, st, (const T*)dq_part, part_lse, (T*)dq, p.tokens, p.q_heads, \
+                              p.head_dim, p.slots, p.win_begin, window_rows(p)))
   if (p.dtype == MOBA_B200_F32) MOBA_DQR(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_DQR(__nv_bfloat16);
   else MOBA_DQR(__half);
 #undef MOBA_DQR
-  MOBA_LAUNCH_OK("dq_reduce_kernel");
   return MOBA_B200_OK;
 }
 

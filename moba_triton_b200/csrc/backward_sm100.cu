@@ -175,6 +175,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem = bars->tmem_base;
   // At head_dim 64 TMEM has room for dQ columns of their own; at 128 dQ lands on S.
   constexpr uint32_t cS = 0, cDP = 128, cDV = 256, cDK = 256 + D, cDQ = Cfg::kOwnStage ? 256 + 2 * D : 0;
@@ -464,6 +465,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         Column c;
         if (round * (int)gridDim.x >= n_items || item >= n_items || !load_column(c, item, ix, p, cu, n_kv_rows)) return;
         const size_t lo = (size_t)c.kv_row * ix.capacity + c.lo;
+        if (packed_pairs(ix)) {
+          l2_prefetch_i32(ix.row_indices, 2 * lo, 2 * c.n, 2 * index_elems);
+          return;
+        }
         l2_prefetch_i32(ix.row_indices, lo, c.n, index_elems);
         l2_prefetch_i32(ix.head_indices, lo, c.n, index_elems);
         l2_prefetch_i32(ix.slot_of_pair, lo, c.n, index_elems);
@@ -526,22 +531,20 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         fence_proxy_async();
         mbar_arrive_warp(&bars->v_fix);
       }
-      const int32_t* rows_i = ix.row_indices + (size_t)c.kv_row * ix.capacity + c.lo;
-      const int32_t* heads_i = ix.head_indices + (size_t)c.kv_row * ix.capacity + c.lo;
-      const int32_t* slots_i = ix.slot_of_pair + (size_t)c.kv_row * ix.capacity + c.lo;
-      int n_row = 0, n_head = 0, n_slot = 0;               // index entry of the next tile, fetched ahead
-      if (pt < c.n) { n_row = rows_i[pt]; n_head = heads_i[pt]; n_slot = slots_i[pt]; }
+      const size_t list0 = (size_t)c.kv_row * ix.capacity + c.lo;
+      PairEntry nx{0, 0, 0};                               // index entry of the next tile, fetched ahead
+      if (pt < c.n) nx = load_pair_pinned(ix, list0 + pt);
       for (int i = 0; i < nt; ++i, ++t) {
         const uint32_t st = t % NST, us = t / NST;
         const int e = i * kTile + pt;
         long long off = -1;
         int4 mt = make_int4(-1, 0, 0, 0);
         if (e < c.n) {
-          off = (long long)(((c.b * p.tokens + n_row) * p.q_heads + n_head) * (size_t)D);
-          const size_t qr = (c.b * p.q_heads + n_head) * p.tokens + n_row;
-          mt = make_int4(n_row, (n_head << 8) | n_slot, __float_as_int(lse[qr]), __float_as_int(delta[qr]));
+          off = (long long)(((c.b * p.tokens + nx.row) * p.q_heads + nx.head) * (size_t)D);
+          const size_t qr = (c.b * p.q_heads + nx.head) * p.tokens + nx.row;
+          mt = make_int4(nx.row, (nx.head << 8) | nx.slot, __float_as_int(lse[qr]), __float_as_int(delta[qr]));
         }
-        if (e + kTile < c.n) { n_row = rows_i[e + kTile]; n_head = heads_i[e + kTile]; n_slot = slots_i[e + kTile]; }
+        if (e + kTile < c.n) nx = load_pair_pinned(ix, list0 + e + kTile);
         if (us >= 1) mbar_wait(&bars->qd_empty[st], (us - 1) & 1, wc, 13);
         TRACE(error_word, t, 0);
         bars->meta[st][pt] = mt;
@@ -567,7 +570,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           // the L2 now (the index entry has arrived while this tile's copies were issued), so
           // that those copies find them there instead of in DRAM. With two stages the copies
           // run a tile ahead anyway and the extra requests only cost (0.72 -> 0.73 ms at D=64).
-          const size_t nxt = ((c.b * p.tokens + n_row) * p.q_heads + n_head) * (size_t)D;
+          const size_t nxt = ((c.b * p.tokens + nx.row) * p.q_heads + nx.head) * (size_t)D;
 #pragma unroll
           for (int line = 0; line < D * 2 / 128; ++line) {
             l2_prefetch_line(q + nxt + line * 64);
@@ -610,6 +613,8 @@ dkv_reduce_kernel(const float* __restrict__ dkv_scratch, moba_b200_index ix, con
                   T* __restrict__ dk, T* __restrict__ dv, moba_b200_problem p, int ctas_per_row) {
   __shared__ int4 found[256];
   __shared__ int n_found;
+  pdl_trigger();
+  pdl_wait();
   const int kv_row = blockIdx.x / ctas_per_row;
   const int j = (blockIdx.x % ctas_per_row) * 256 + threadIdx.x;
   if (threadIdx.x == 0) n_found = 0;
@@ -675,18 +680,19 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
                const void* dout, const float* lse, const float* delta, const moba_b200_index& ix,
                const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int n_items, unsigned* err,
                cudaStream_t st) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
   {
     KernelTimer timer__("bwd_sm100_kernel", st);
     auto kern = bwd_sm100_kernel<D, T>;
-    MOBA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdCfg<D>::kSmem));
-    kern<<<grid, kThreads, BwdCfg<D>::kSmem, st>>>(km, vm, (const T*)q, (const T*)dout, lse, delta, ix, cu,
-                                                    (T*)dq_part, dkv_scratch, (T*)dk, (T*)dv, p, n_items, err);
-    MOBA_LAUNCH_OK("bwd_sm100_kernel");
+    static SmemLimit limit;
+    if (int rc = raise_smem_limit(limit, (const void*)kern, BwdCfg<D>::kSmem)) return rc;
+    MOBA_CUDA_OK(launch_chained(kern, grid, kThreads, BwdCfg<D>::kSmem, st, km, vm, (const T*)q, (const T*)dout, lse, delta,
+                                ix, cu, (T*)dq_part, dkv_scratch, (T*)dk, (T*)dv, p, n_items, err));
   }
+  // No column can be long enough to be cut: nothing to sum.
+  const long long longest = ((long long)(p.q_heads / p.kv_heads) * (p.win_rows > 0 ? p.win_rows : p.max_seqlen) + kTile - 1) / kTile;
+  if (longest <= ix.chunk_tiles) return MOBA_B200_OK;
   KernelTimer timer__("dkv_reduce_kernel", st);
   const int ctas_per_row = (ix.items_per_row + 255) / 256;
   // z: the 2 x 128 x D sums of a column in parts of at least 1024 float4; fewer parts when the
@@ -696,9 +702,8 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
   slices = slices < 1 ? 1 : (slices > kReduceSlices ? kReduceSlices : slices);
   int parts = 4096 / (x_ctas * slices);
   parts = parts < 1 ? 1 : (parts > D / 16 ? D / 16 : parts);
-  dkv_reduce_kernel<D, T><<<dim3(x_ctas, slices, parts), 256, 0, st>>>(
-      dkv_scratch, ix, cu, (T*)dk, (T*)dv, p, ctas_per_row);
-  MOBA_LAUNCH_OK("dkv_reduce_kernel");
+  MOBA_CUDA_OK(launch_chained(dkv_reduce_kernel<D, T>, dim3(x_ctas, slices, parts), 256, 0, st, (const float*)dkv_scratch, ix, cu,
+                              (T*)dk, (T*)dv, p, ctas_per_row));
   return MOBA_B200_OK;
 }
 

@@ -27,6 +27,8 @@ void set_error(const char* fmt, ...);
     }                                                                             \
   } while (0)
 
+#define MOBA_TRY(expr) do { int rc__ = (expr); if (rc__ != MOBA_B200_OK) return rc__; } while (0)
+
 // Counts every kernel launch of the library and, when profiling is switched on
 // through moba_b200_profile_enable(), brackets it with CUDA events on its stream.
 struct KernelTimer {
@@ -46,6 +48,36 @@ struct KernelTimer {
       return MOBA_B200_ECUDA;                                                     \
     }                                                                             \
   } while (0)
+
+// ---- programmatic dependent launch ----------------------------------------
+// The op is a chain of kernels, each reading what the one before wrote. Every kernel of the
+// chain is launched with programmatic stream serialisation: it may be scheduled while its
+// predecessor still runs, does its private set-up, and then waits (pdl_wait, executed by every
+// thread before the first global access) until the predecessor has completed and its writes are
+// visible. Completion of a kernel implies completion of everything before it, because it waited
+// too. A launch then costs the chain about a microsecond instead of three, which is most of the
+// time of a short sequence.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream be scheduled as soon as every CTA of this one got here.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                         Args&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Raises a kernel's dynamic shared-memory limit once per device. `done` is the caller's static
+// table (one entry per device), so that repeated launches cost a comparison.
+struct SmemLimit { int bytes[64] = {0}; };
+int raise_smem_limit(SmemLimit& done, const void* kernel, size_t bytes);
+int sm_count();                              // SMs of the current device (cached)
 
 // ---- element types -------------------------------------------------------
 template <typename T> struct Elem;
@@ -154,6 +186,38 @@ static inline size_t sched_dkv_scratch_bytes(const moba_b200_problem& p) {
   return (size_t)sched_part_slots(p) * 2 * 128 * p.head_dim * sizeof(float);
 }
 
+// One pair of a column's list. Inside the whole-op entry points, where no caller looks at the
+// index, the pairs are packed into eight bytes {query position, query head << 8 | slot}, so that
+// building and reading the list moves one word per pair: `row_indices` then points at those and
+// `head_indices` is NULL.
+struct PairEntry { int row, head, slot; };
+__host__ __device__ __forceinline__ bool packed_pairs(const moba_b200_index& ix) { return ix.head_indices == nullptr; }
+__device__ __forceinline__ PairEntry load_pair(const moba_b200_index& ix, size_t at) {
+  PairEntry e;
+  if (packed_pairs(ix)) {
+    const int2 v = __ldg(reinterpret_cast<const int2*>(ix.row_indices) + at);
+    e.row = v.x; e.head = v.y >> 8; e.slot = v.y & 0xff;
+  } else {
+    e.row = __ldg(ix.row_indices + at); e.head = __ldg(ix.head_indices + at); e.slot = __ldg(ix.slot_of_pair + at);
+  }
+  return e;
+}
+// The same with loads the compiler may not move: a plain load may be sunk to its first use,
+// which defeats fetching an entry a tile ahead.
+__device__ __forceinline__ PairEntry load_pair_pinned(const moba_b200_index& ix, size_t at) {
+  PairEntry e;
+  if (packed_pairs(ix)) {
+    int a, b;
+    asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "l"(reinterpret_cast<const int2*>(ix.row_indices) + at));
+    e.row = a; e.head = b >> 8; e.slot = b & 0xff;
+  } else {
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(e.row) : "l"(ix.row_indices + at));
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(e.head) : "l"(ix.head_indices + at));
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(e.slot) : "l"(ix.slot_of_pair + at));
+  }
+  return e;
+}
+
 // One work item as the kernels see it.
 struct WorkItem {
   int blk;        // block (column) of the (sequence, kv head) row
@@ -175,19 +239,24 @@ __device__ __forceinline__ bool load_work_item(WorkItem& w, const moba_b200_inde
 }
 
 // ---- stage launchers (defined one per .cu file) -----------------------------
-int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar,
+int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell,
                 cudaStream_t st);
+// `lse_fill` (may be NULL): the partial log-sum-exps, set to -inf where a slot names no block.
 int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* kbar,
-                         const int32_t* cu, int32_t* block_idx, cudaStream_t st);
+                         const int32_t* cu, int32_t* block_idx, float* lse_fill, cudaStream_t st);
 int launch_gate_sm100(const moba_b200_problem& p, const void* q, const void* kbar,
-                      const int32_t* cu, int32_t* block_idx, cudaStream_t st);
+                      const int32_t* cu, int32_t* block_idx, float* lse_fill, cudaStream_t st);
 bool gate_sm100_supported(const moba_b200_problem& p);
 
 size_t transpose_scratch_bytes(const moba_b200_problem& p);
 int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                      int32_t* col_nnz, int32_t* col_offsets, int32_t* order, int32_t* rows,
-                     int32_t* heads, int32_t* slots, int32_t* work_items, void* scratch, size_t scratch_bytes,
+                     int32_t* heads, int32_t* slots, int2* entries, int32_t* work_items, void* scratch, size_t scratch_bytes,
                      cudaStream_t st);
+bool transpose_small_supported(const moba_b200_problem& p);
+int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu, int32_t* col_nnz,
+                           int32_t* col_offsets, int32_t* order, int2* entries, int32_t* work_items, int32_t* slot_counter,
+                           cudaStream_t st);
 
 int launch_transpose_noalloc(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                              int32_t* col_nnz, int32_t* col_offsets, int32_t* order, int32_t* rows,
@@ -217,6 +286,11 @@ int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, c
 bool bwd_sm100_supported(const moba_b200_problem& p);
 int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const float* part_lse,
                      void* dq, cudaStream_t st);
+
+// ---- argument checks and kernel-family selection, shared by the entry points (api.cu) ----
+int check_problem(const moba_b200_problem* p);
+int need(const void* ptr, const char* name);
+int pick(const moba_b200_problem& p, bool fast_ok, const char* stage);
 
 int launch_pack_index(const void* mask, int mask_bytes, int batch, int seq_len, int32_t* dest, int32_t* lengths,
                       int32_t* cu, int32_t* meta, cudaStream_t st);

@@ -23,7 +23,10 @@ namespace moba {
 template <typename T>
 __global__ void __launch_bounds__(128)
 pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restrict__ kbar,
-            int packed, int tokens, int hkv, int d, int bs, int nb) {
+            int packed, int tokens, int hkv, int d, int bs, int nb, int* __restrict__ zero_cell) {
+  pdl_trigger();
+  pdl_wait();
+  if (zero_cell != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_cell = 0;
   constexpr int EPV = 16 / sizeof(T);            // elements per 16-byte vector
   const int blk = (int)(blockIdx.x % nb), kv_row = (int)(blockIdx.x / nb);
   const int seq = kv_row / hkv, h = kv_row % hkv;
@@ -82,7 +85,8 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
   }
 }
 
-int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar,
+// `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from.
+int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell,
                 cudaStream_t st) {
   KernelTimer timer__("pool_kernel", st);
   const int epv = 16 / (int)dtype_size(p.dtype);
@@ -93,14 +97,13 @@ int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, vo
   const long long ctas = (long long)p.num_blocks * p.n_seq * p.kv_heads;
   if (ctas > 0x7fffffffLL) { set_error("pool: %lld blocks exceed the grid limit", ctas); return MOBA_B200_EUNSUPPORTED; }
   const unsigned grid = (unsigned)ctas;
-#define MOBA_POOL(T)                                                                   \
-  pool_kernel<T><<<grid, 128, 0, st>>>((const T*)k, cu, (T*)kbar, p.packed, p.tokens,  \
-                                       p.kv_heads, p.head_dim, p.block_size, p.num_blocks)
+#define MOBA_POOL(T)                                                                                   \
+  MOBA_CUDA_OK(launch_chained(pool_kernel<T>, grid, 128, 0, st, (const T*)k, cu, (T*)kbar, p.packed, p.tokens, \
+                              p.kv_heads, p.head_dim, p.block_size, p.num_blocks, zero_cell))
   if (p.dtype == MOBA_B200_F32) MOBA_POOL(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_POOL(__nv_bfloat16);
   else MOBA_POOL(__half);
 #undef MOBA_POOL
-  MOBA_LAUNCH_OK("pool_kernel");
   return MOBA_B200_OK;
 }
 
@@ -147,7 +150,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
                      const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx,
-                     moba_b200_problem p) {
+                     float* __restrict__ lse_fill, moba_b200_problem p) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int d = p.head_dim, take = p.take, slots = p.slots;
   double* qs = reinterpret_cast<double*>(smem_raw);                       // [32][d]
@@ -251,7 +255,8 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
     const int own = row / p.block_size;
     const int* li = lidx + lrow * take;
     const size_t b = p.packed ? 0 : (size_t)seq;
-    int32_t* out = block_idx + ((b * p.q_heads + hq) * p.tokens + sp.bos + row) * (size_t)slots;
+    const size_t out_at = ((b * p.q_heads + hq) * p.tokens + sp.bos + row) * (size_t)slots;
+    int32_t* out = block_idx + out_at;
     const int n_items = take + (p.always_current ? 1 : 0);
     int kept = 0;
     for (int e = lane; e < n_items; e += 32) {
@@ -267,12 +272,15 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
-    for (int e = kept + lane; e < slots; e += 32) out[e] = -1;
+    for (int e = kept + lane; e < slots; e += 32) {
+      out[e] = -1;
+      if (lse_fill != nullptr) lse_fill[out_at + e] = -INFINITY;
+    }
   }
 }
 
 int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* kbar,
-                         const int32_t* cu, int32_t* block_idx, cudaStream_t st) {
+                         const int32_t* cu, int32_t* block_idx, float* lse_fill, cudaStream_t st) {
   KernelTimer timer__("gate_portable_kernel", st);
   const int d = p.head_dim;
   const size_t smem = sizeof(double) * (kGateRows * d + kGateChunk * (d + 1)) +
@@ -288,15 +296,14 @@ int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* 
   dim3 grid((p.max_seqlen + kGateRows - 1) / kGateRows, p.n_seq * p.q_heads);
 #define MOBA_GATE(T)                                                                          \
   do {                                                                                        \
-    MOBA_CUDA_OK(cudaFuncSetAttribute(gate_portable_kernel<T>,                                \
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    gate_portable_kernel<T><<<grid, 128, smem, st>>>((const T*)q, (const T*)kbar, cu, block_idx, p); \
+    static SmemLimit limit;                                                                   \
+    if (int rc = raise_smem_limit(limit, (const void*)gate_portable_kernel<T>, smem)) return rc; \
+    MOBA_CUDA_OK(launch_chained(gate_portable_kernel<T>, grid, 128, smem, st, (const T*)q, (const T*)kbar, cu, block_idx, lse_fill, p)); \
   } while (0)
   if (p.dtype == MOBA_B200_F32) MOBA_GATE(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_GATE(__nv_bfloat16);
   else MOBA_GATE(__half);
 #undef MOBA_GATE
-  MOBA_LAUNCH_OK("gate_portable_kernel");
   return MOBA_B200_OK;
 }
 

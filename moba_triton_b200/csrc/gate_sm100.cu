@@ -167,8 +167,8 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
 template <int D, typename T, int L>
 __global__ void __launch_bounds__(kThreads, 2)
 gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kb_map,
-                  const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx, moba_b200_problem p,
-                  int n_tiles, int n_units, unsigned* error_word) {
+                  const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx, float* __restrict__ lse_fill,
+                  moba_b200_problem p, int n_tiles, int n_units, unsigned* error_word) {
   using Cfg = GateCfg<D>;
   constexpr int CAP = Cfg::kCap, STEP = Cfg::kStep;
   extern __shared__ unsigned char smem_dyn[];
@@ -205,6 +205,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem = bars->tmem_base;
 
   // Every role walks the same units and counts the same steps: a unit of n chunks takes 2 n
@@ -343,7 +344,8 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           kept += ok ? 1 : 0;
         }
         const size_t b = p.packed ? 0 : (size_t)u.seq;
-        int32_t* dst = block_idx + ((b * p.q_heads + u.hq) * p.tokens + u.bos + u.row0 + r) * (size_t)p.slots;
+        const size_t dst_at = ((b * p.q_heads + u.hq) * p.tokens + u.bos + u.row0 + r) * (size_t)p.slots;
+        int32_t* dst = block_idx + dst_at;
 #pragma unroll
         for (int e = 0; e < L; ++e) {                           // rank by id: position in the output
           if (ids[e] == kEmpty) continue;
@@ -353,7 +355,10 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           dst[rank] = ids[e];
         }
         if (p.always_current) dst[kept++] = u.tile;             // the own block is past every candidate
-        for (int e = kept; e < p.slots; ++e) dst[e] = -1;
+        for (int e = kept; e < p.slots; ++e) {
+          dst[e] = -1;
+          if (lse_fill != nullptr) lse_fill[dst_at + e] = -INFINITY;   // the slot's partial will not be written
+        }
       }
       // Warpgroup 0 reads the exchange area (its own buffer) before it appends to it again;
       // warpgroup 1 writes there only behind the first barrier of the next unit.
@@ -445,17 +450,16 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 
 template <int D, typename T, int L>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& qm, const CUtensorMap& km, const int32_t* cu,
-               int32_t* block_idx, unsigned* err, cudaStream_t st) {
+               int32_t* block_idx, float* lse_fill, unsigned* err, cudaStream_t st) {
   auto kern = gate_sm100_kernel<D, T, L>;
-  MOBA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GateCfg<D>::kSmem));
+  static SmemLimit limit;
+  if (int rc = raise_smem_limit(limit, (const void*)kern, GateCfg<D>::kSmem)) return rc;
   const int n_tiles = (p.max_seqlen + kTile - 1) / kTile;
   const long long n_units = (long long)n_tiles * p.n_seq * p.q_heads;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const int grid = (int)(n_units < 2LL * sms ? n_units : 2LL * sms);
-  kern<<<grid, kThreads, GateCfg<D>::kSmem, st>>>(qm, km, cu, block_idx, p, n_tiles, (int)n_units, err);
-  MOBA_LAUNCH_OK("gate_sm100_kernel");
+  MOBA_CUDA_OK(launch_chained(kern, grid, kThreads, GateCfg<D>::kSmem, st, qm, km, cu, block_idx, lse_fill, p, n_tiles,
+                              (int)n_units, err));
   return MOBA_B200_OK;
 }
 
@@ -472,7 +476,7 @@ bool gate_sm100_supported(const moba_b200_problem& p) {
 int encode_kbar_map_impl(CUtensorMap* out, const void* base, uint64_t kv_rows, uint64_t nb, uint64_t dim);
 
 int launch_gate_sm100(const moba_b200_problem& p, const void* q, const void* kbar, const int32_t* cu,
-                      int32_t* block_idx, cudaStream_t st) {
+                      int32_t* block_idx, float* lse_fill, cudaStream_t st) {
   KernelTimer timer__("gate_sm100_kernel", st);
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("gate: no device error word"); return MOBA_B200_ECUDA; }
@@ -482,8 +486,8 @@ int launch_gate_sm100(const moba_b200_problem& p, const void* q, const void* kba
   rc = encode_kbar_map_impl(&km, kbar, (uint64_t)p.n_seq * p.kv_heads, p.num_blocks, p.head_dim);
   if (rc) return rc;
   const bool bf = p.dtype == MOBA_B200_BF16;
-#define GO(D, T) return (p.take <= 7) ? launch_one<D, T, 7>(p, qm, km, cu, block_idx, err, st) \
-                                      : launch_one<D, T, 8>(p, qm, km, cu, block_idx, err, st)
+#define GO(D, T) return (p.take <= 7) ? launch_one<D, T, 7>(p, qm, km, cu, block_idx, lse_fill, err, st) \
+                                      : launch_one<D, T, 8>(p, qm, km, cu, block_idx, lse_fill, err, st)
   if (p.head_dim == 64) { if (bf) GO(64, __nv_bfloat16); else GO(64, __half); }
   if (bf) GO(128, __nv_bfloat16); else GO(128, __half);
 #undef GO

@@ -1,0 +1,175 @@
+// The whole op in two calls: moba_b200_op_forward (pool, gate, transpose, attention, merge) and
+// moba_b200_op_backward (delta, dK/dV and dQ partials, reductions), each into one caller-owned
+// workspace. They run the stages' kernels; what they save is what lies between the stages: a
+// dozen allocations and as many foreign calls per pass on the host (300 of the 360 us of a
+// thousand-token training step, 100 of the 150 us of an 8 192-token forward), the passes that
+// only the separate entry points need (the fill of the partial log-sum-exps, the public form of
+// the index) and, for short rows, four of the transpose's five launches.
+#include "common.cuh"
+#include "sm100.cuh"
+
+namespace moba {
+namespace {
+
+constexpr size_t kAlign = 256;
+inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
+
+// The cut of the work items. The policy of the scheduler has a floor of eight tiles, which is
+// right when the rows fill the GPU; a problem of at most four tiles per SM is all tail, and
+// finer items spread it over the SMs (their dK/dV partials then fit the L2). The size depends on
+// the length of a row only, so that running the KV heads of such a problem in several passes
+// cuts them the same way and gives the same bits.
+moba_b200_problem with_cut(const moba_b200_problem& p0) {
+  moba_b200_problem p = p0;
+  if (p.chunk_tiles > 0) return p;
+  p.chunk_tiles = sched_chunk_tiles(p);
+  const long long tiles = (sched_pairs_bound(p) + 127) / 128;
+  const long long row_tiles = ((long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots + 127) / 128;
+  if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = row_tiles <= 128 ? 2 : 4;
+  return p;
+}
+
+// Byte offsets of the buffers inside the caller's workspaces.
+struct Layout {
+  size_t col_nnz, col_offsets, order, items, entries, part_lse, lse, keep_bytes;      // kept for the backward
+  size_t kbar, block_idx, counter, transpose_scratch, part_o, fwd_bytes;              // forward only
+  size_t delta, dq_part, dkv, bwd_bytes;                                              // backward only
+};
+Layout layout_of(const moba_b200_problem& p) {
+  Layout l;
+  const size_t rows = (size_t)p.n_seq * p.kv_heads, nb = p.num_blocks;
+  const size_t pairs = (size_t)p.batch * p.q_heads * p.tokens * p.slots;
+  const size_t capacity = (size_t)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
+  size_t at = 0;
+  auto take = [&](size_t bytes) { const size_t o = at; at = up(at + bytes); return o; };
+  l.col_nnz = take(rows * nb * 4);
+  l.col_offsets = take(rows * (nb + 1) * 4);
+  l.order = take(rows * nb * 4);
+  l.items = take(rows * (size_t)sched_items_per_row(p) * 16);
+  l.entries = take(rows * capacity * 8);
+  l.part_lse = take(pairs * 4);
+  l.lse = take((size_t)p.batch * p.q_heads * p.tokens * 4);
+  l.keep_bytes = at;
+  at = 0;
+  const size_t part_size = p.part_f32 ? 4 : dtype_size(p.dtype);
+  l.kbar = take(rows * nb * p.head_dim * dtype_size(p.dtype));
+  l.block_idx = take(pairs * 4);
+  l.counter = take(16);
+  l.transpose_scratch = take(transpose_small_supported(p) ? 16 : transpose_scratch_bytes(p));
+  l.part_o = take(pairs * p.head_dim * part_size);
+  l.fwd_bytes = at;
+  at = 0;
+  l.delta = take((size_t)p.batch * p.q_heads * p.tokens * 4);
+  l.dq_part = take(pairs * p.head_dim * dtype_size(p.dtype));
+  l.dkv = take(sched_dkv_scratch_bytes(p));
+  l.bwd_bytes = at;
+  return l;
+}
+
+moba_b200_index index_in(const moba_b200_problem& p, const Layout& l, unsigned char* keep) {
+  moba_b200_index ix = {};
+  ix.col_nnz = reinterpret_cast<int32_t*>(keep + l.col_nnz);
+  ix.col_offsets = reinterpret_cast<int32_t*>(keep + l.col_offsets);
+  ix.order = reinterpret_cast<int32_t*>(keep + l.order);
+  ix.capacity = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
+  ix.work_items = reinterpret_cast<int32_t*>(keep + l.items);
+  ix.items_per_row = (int)sched_items_per_row(p);
+  ix.chunk_tiles = sched_chunk_tiles(p);
+  ix.row_indices = reinterpret_cast<int32_t*>(keep + l.entries);   // packed pairs
+  return ix;
+}
+
+int check_op(const moba_b200_problem* p) {
+  MOBA_TRY(check_problem(p));
+  if (p->win_rows > 0) { set_error("the whole-op entry points take no query window"); return MOBA_B200_EUNSUPPORTED; }
+  if (p->q_heads >= 1 << 23) { set_error("%d query heads do not fit a packed index entry", p->q_heads); return MOBA_B200_EUNSUPPORTED; }
+  if (sched_items_per_row(*p) > 0x7fffffffLL || sched_part_slots(*p) > 0x7fffffffLL) {
+    set_error("chunk_tiles %d cuts the problem into too many work items", sched_chunk_tiles(*p));
+    return MOBA_B200_EUNSUPPORTED;
+  }
+  return MOBA_B200_OK;
+}
+
+}  // namespace
+}  // namespace moba
+
+using namespace moba;
+
+extern "C" {
+
+int moba_b200_op_workspace(const moba_b200_problem* p0, size_t* keep_bytes, size_t* forward_bytes, size_t* backward_bytes) {
+  MOBA_TRY(check_op(p0));
+  const Layout l = layout_of(with_cut(*p0));
+  if (keep_bytes) *keep_bytes = l.keep_bytes;
+  if (forward_bytes) *forward_bytes = l.fwd_bytes;
+  if (backward_bytes) *backward_bytes = l.bwd_bytes;
+  return MOBA_B200_OK;
+}
+
+int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void* k, const void* v,
+                         const int32_t* cu_seqlens, void* keep_ws, void* forward_ws, void* out, int want_lse, void* stream) {
+  MOBA_TRY(check_op(p0));
+  MOBA_TRY(need(q, "q")); MOBA_TRY(need(k, "k")); MOBA_TRY(need(v, "v")); MOBA_TRY(need(out, "out"));
+  MOBA_TRY(need(keep_ws, "keep_ws")); MOBA_TRY(need(forward_ws, "forward_ws"));
+  if (p0->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
+  const moba_b200_problem p = with_cut(*p0);
+  const int gate_path = pick(p, gate_sm100_supported(p), "gate"), fwd_path = pick(p, fwd_sm100_supported(p), "forward");
+  if (gate_path < 0) return gate_path;
+  if (fwd_path < 0) return fwd_path;
+  cudaStream_t st = (cudaStream_t)stream;
+  const Layout l = layout_of(p);
+  unsigned char* keep = static_cast<unsigned char*>(keep_ws);
+  unsigned char* tmp = static_cast<unsigned char*>(forward_ws);
+  const moba_b200_index ix = index_in(p, l, keep);
+  void* kbar = tmp + l.kbar;
+  int32_t* block_idx = reinterpret_cast<int32_t*>(tmp + l.block_idx);
+  float* part_lse = reinterpret_cast<float*>(keep + l.part_lse);
+  void* part_o = tmp + l.part_o;
+  int32_t* counter = reinterpret_cast<int32_t*>(tmp + l.counter);
+  int32_t* col_nnz = const_cast<int32_t*>(ix.col_nnz);
+  int32_t* col_offsets = const_cast<int32_t*>(ix.col_offsets);
+  int32_t* items = const_cast<int32_t*>(ix.work_items);
+  MOBA_TRY(launch_pool(p, k, cu_seqlens, kbar, counter, st));
+  if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(p, q, kbar, cu_seqlens, block_idx, part_lse, st));
+  else MOBA_TRY(launch_gate_portable(p, q, kbar, cu_seqlens, block_idx, part_lse, st));
+  int2* entries = reinterpret_cast<int2*>(const_cast<int32_t*>(ix.row_indices));
+  int32_t* order = const_cast<int32_t*>(ix.order);
+  if (transpose_small_supported(p))
+    MOBA_TRY(launch_transpose_small(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, entries, items, counter, st));
+  else
+    MOBA_TRY(launch_transpose(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, nullptr, nullptr, nullptr, entries, items,
+                              tmp + l.transpose_scratch, transpose_scratch_bytes(p), st));
+  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu_seqlens, part_o, part_lse, st));
+  else MOBA_TRY(launch_fwd_portable(p, q, k, v, ix, cu_seqlens, part_o, part_lse, st));
+  return launch_merge(p, part_o, part_lse, out, want_lse ? reinterpret_cast<float*>(keep + l.lse) : nullptr, st);
+}
+
+int moba_b200_op_backward(const moba_b200_problem* p0, const void* q, const void* k, const void* v, const void* out,
+                          const void* dout, const int32_t* cu_seqlens, const void* keep_ws, void* backward_ws,
+                          void* dq, void* dk, void* dv, void* stream) {
+  MOBA_TRY(check_op(p0));
+  MOBA_TRY(need(q, "q")); MOBA_TRY(need(k, "k")); MOBA_TRY(need(v, "v")); MOBA_TRY(need(out, "out"));
+  MOBA_TRY(need(dout, "dout")); MOBA_TRY(need(dq, "dq")); MOBA_TRY(need(dk, "dk")); MOBA_TRY(need(dv, "dv"));
+  MOBA_TRY(need(keep_ws, "keep_ws")); MOBA_TRY(need(backward_ws, "backward_ws"));
+  if (p0->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
+  const moba_b200_problem p = with_cut(*p0);
+  const int path = pick(p, bwd_sm100_supported(p), "backward");
+  if (path < 0) return path;
+  cudaStream_t st = (cudaStream_t)stream;
+  const Layout l = layout_of(p);
+  unsigned char* keep = const_cast<unsigned char*>(static_cast<const unsigned char*>(keep_ws));
+  unsigned char* tmp = static_cast<unsigned char*>(backward_ws);
+  const moba_b200_index ix = index_in(p, l, keep);
+  const float* part_lse = reinterpret_cast<const float*>(keep + l.part_lse);
+  const float* lse = reinterpret_cast<const float*>(keep + l.lse);
+  float* delta = reinterpret_cast<float*>(tmp + l.delta);
+  void* dq_part = tmp + l.dq_part;
+  MOBA_TRY(launch_delta(p, out, dout, delta, st));
+  if (path == MOBA_B200_PATH_TCGEN05)
+    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, st));
+  else
+    MOBA_TRY(launch_bwd_portable(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, dk, dv, st));
+  return launch_dq_reduce(p, dq_part, part_lse, dq, st);
+}
+
+}  // extern "C"

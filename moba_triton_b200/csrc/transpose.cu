@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(256)
 count_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu,
              int32_t* __restrict__ tile_counts, int32_t* __restrict__ slot_counter, moba_b200_problem p, int R, int C) {
   extern __shared__ int hist[];
+  pdl_trigger();
+  pdl_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) *slot_counter = 0;     // claimed from by work_items_kernel, two launches on
   const int chunk = blockIdx.x % C, y = blockIdx.x / C;
   const int seq = y / p.q_heads, hq = y % p.q_heads;
@@ -86,6 +88,8 @@ count_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ 
 __global__ void __launch_bounds__(128)
 colscan_kernel(const int32_t* __restrict__ cu, int32_t* __restrict__ tile_counts,
                int32_t* __restrict__ col_nnz, moba_b200_problem p, int R, int C, int ctas_per_row) {
+  pdl_trigger();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = (int)(blockIdx.x % ctas_per_row) * 4 + warp;
   const int kv_row = (int)(blockIdx.x / ctas_per_row);       // (sequence, kv head)
@@ -129,6 +133,8 @@ __global__ void __launch_bounds__(1024)
 offsets_order_kernel(const int32_t* __restrict__ col_nnz, int32_t* __restrict__ col_offsets,
                      int32_t* __restrict__ order, int nb) {
   extern __shared__ int cnt[];              // [nb]
+  pdl_trigger();
+  pdl_wait();
   __shared__ int warp_sums[32];
   __shared__ int carry_s;
   const int32_t* nnz = col_nnz + (size_t)blockIdx.x * nb;
@@ -196,18 +202,16 @@ offsets_order_kernel(const int32_t* __restrict__ col_nnz, int32_t* __restrict__ 
 // the order of the list. A row with more than kMaxCut cut columns keeps its columns' pieces
 // side by side, in column order (it has items enough for the order not to matter).
 constexpr int kMaxCut = 2048;
-__global__ void __launch_bounds__(1024)
-work_items_kernel(const int32_t* __restrict__ col_nnz, const int32_t* __restrict__ order, int4* __restrict__ items,
-                  int32_t* __restrict__ slot_counter, int nb, int items_per_row, int tc, int slot_cap,
-                  unsigned* error_word) {
+// The row's work items, by all 1024 threads of a CTA. `nnz` and `ord` are the row's column
+// totals and dispatch order (global or shared memory), `out` its stretch of the item table.
+template <int MAXCUT>
+__device__ void write_work_items(const int32_t* nnz, const int32_t* ord, int4* out, int32_t* slot_counter, int nb,
+                                 int items_per_row, int tc, int slot_cap, unsigned* error_word) {
   __shared__ long long warp_sums[32];
   __shared__ long long carry_s;
   __shared__ int base_s;
-  __shared__ int rem_s[kMaxCut], rank_s[kMaxCut], sorted_s[kMaxCut], slot_s[kMaxCut];
+  __shared__ int rem_s[MAXCUT], rank_s[MAXCUT], sorted_s[MAXCUT], slot_s[MAXCUT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int32_t* nnz = col_nnz + (size_t)blockIdx.x * nb;
-  const int32_t* ord = order + (size_t)blockIdx.x * nb;
-  int4* out = items + (size_t)blockIdx.x * items_per_row;
   auto tiles_of = [&](int r) { return (nnz[ord[r]] + 127) / 128; };
   auto chunks_of = [&](int r, int& blk, int& tiles) {
     blk = ord[r];
@@ -260,7 +264,7 @@ work_items_kernel(const int32_t* __restrict__ col_nnz, const int32_t* __restrict
     else atomicOr(error_word, 2u);
   };
 
-  if (n_cut <= kMaxCut) {
+  if (n_cut <= MAXCUT) {
     const int n_full = row_slots - n_cut;                   // pieces of exactly tc tiles: they lead the list
     // the cut columns: full pieces in column order, the last piece's size and slot for later
     for (int r0 = 0; r0 < n_cut; r0 += 1024) {
@@ -339,19 +343,34 @@ work_items_kernel(const int32_t* __restrict__ col_nnz, const int32_t* __restrict
   for (int j = used + threadIdx.x; j < items_per_row; j += 1024) out[j] = make_int4(0, 0, 0, -2);   // padding
 }
 
+__global__ void __launch_bounds__(1024)
+work_items_kernel(const int32_t* __restrict__ col_nnz, const int32_t* __restrict__ order, int4* __restrict__ items,
+                  int32_t* __restrict__ slot_counter, int nb, int items_per_row, int tc, int slot_cap,
+                  unsigned* error_word) {
+  pdl_trigger();
+  pdl_wait();
+  write_work_items<kMaxCut>(col_nnz + (size_t)blockIdx.x * nb, order + (size_t)blockIdx.x * nb,
+                            items + (size_t)blockIdx.x * items_per_row, slot_counter, nb, items_per_row, tc, slot_cap,
+                            error_word);
+}
+
 // One CTA of W warps per (row chunk, sequence, query head). The walk of a run is one
 // dependent chain per warp (match, cursor, store), so the chunk is cut into W runs that are
 // walked side by side: a histogram per run and a scan over the runs (both in shared memory)
 // turn the chunk's cursors into cursors per run. The order inside a column stays
 // (query head, row): runs are consecutive rows and keep the chunk's order.
-template <int W>
+// PACKED: one eight-byte entry per pair instead of three words in three arrays. The stores are
+// scattered, so their number is what this kernel costs.
+template <int W, bool PACKED>
 __global__ void __launch_bounds__(32 * W)
 scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu,
                const int32_t* __restrict__ tile_prefix, const int32_t* __restrict__ col_offsets,
                int32_t* __restrict__ rows_out, int32_t* __restrict__ heads_out,
-               int32_t* __restrict__ slots_out, moba_b200_problem p, int R, int C,
+               int32_t* __restrict__ slots_out, int2* __restrict__ entries_out, moba_b200_problem p, int R, int C,
                long long capacity) {
   extern __shared__ int cursor_all[];                        // [W][nb_lim]
+  pdl_trigger();
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int chunk = blockIdx.x % C, y = blockIdx.x / C;
   const int seq = y / p.q_heads, hq = y % p.q_heads;
@@ -396,6 +415,7 @@ scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict_
   int32_t* ro = rows_out + kv_row * capacity;
   int32_t* ho = heads_out + kv_row * capacity;
   int32_t* so = slots_out + kv_row * capacity;
+  int2* eo = entries_out + kv_row * capacity;
   const unsigned lt = (1u << lane) - 1u;
   const int first_row = sp.bos + row0 + r_lo;
   // The entries are fetched a batch of kBatch steps ahead: one memory latency per batch
@@ -431,9 +451,14 @@ scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict_
       if (valid) {
         const long long dst = base + __popc(same & lt);
         if (dst < capacity) {
-          ro[dst] = first_row + e / p.slots;
-          ho[dst] = hq;
-          so[dst] = e % p.slots;
+          const int row = (int)((unsigned)e / (unsigned)p.slots), slot = e - row * p.slots;
+          if constexpr (PACKED) {
+            eo[dst] = make_int2(first_row + row, (hq << 8) | slot);
+          } else {
+            ro[dst] = first_row + row;
+            ho[dst] = hq;
+            so[dst] = slot;
+          }
         }
       }
     }
@@ -452,23 +477,23 @@ void transpose_plan(const moba_b200_problem& p, int* chunk_rows, int* chunks, in
   *chunk_rows = g.chunk_rows; *chunks = g.chunks; *scatter_warps = scatter_warps_for(p);
 }
 
-template <int W>
+template <int W, bool PACKED>
 static int launch_scatter(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                           const int32_t* tiles, const int32_t* col_offsets, int32_t* rows, int32_t* heads,
-                          int32_t* slots, const TransposeGeom& g, long long capacity, cudaStream_t st) {
+                          int32_t* slots, int2* entries, const TransposeGeom& g, long long capacity, cudaStream_t st) {
   const size_t smem = (size_t)W * p.num_blocks * sizeof(int);
-  if (smem > 48 * 1024)
-    MOBA_CUDA_OK(cudaFuncSetAttribute(scatter_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static SmemLimit limit;
+  if (int rc = raise_smem_limit(limit, (const void*)scatter_kernel<W, PACKED>, smem)) return rc;
   const long long ctas = (long long)g.chunks * p.n_seq * p.q_heads;
-  scatter_kernel<W><<<(unsigned)ctas, 32 * W, smem, st>>>(block_idx, cu, tiles, col_offsets, rows, heads, slots, p,
-                                                           g.chunk_rows, g.chunks, capacity);
-  MOBA_LAUNCH_OK("scatter_kernel");
+  MOBA_CUDA_OK(launch_chained(scatter_kernel<W, PACKED>, (unsigned)ctas, 32 * W, smem, st, block_idx, cu, tiles, col_offsets,
+                              rows, heads, slots, entries, p, g.chunk_rows, g.chunks, capacity));
   return MOBA_B200_OK;
 }
 
+// `entries` non-null: packed pairs, and rows / heads / slots are not written.
 int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                      int32_t* col_nnz, int32_t* col_offsets, int32_t* order, int32_t* rows,
-                     int32_t* heads, int32_t* slots, int32_t* work_items, void* scratch, size_t scratch_bytes,
+                     int32_t* heads, int32_t* slots, int2* entries, int32_t* work_items, void* scratch, size_t scratch_bytes,
                      cudaStream_t st) {
   const TransposeGeom g = transpose_geom(p);
   if (scratch_bytes < transpose_scratch_bytes(p)) {
@@ -492,37 +517,212 @@ int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const
     set_error("transpose: chunk_tiles %d cuts the problem into too many work items", sched_chunk_tiles(p));
     return MOBA_B200_EUNSUPPORTED;
   }
+  unsigned* err = device_error_word();
+  if (err == nullptr) { set_error("transpose: no device error word"); return MOBA_B200_ECUDA; }
   const int group = p.q_heads / p.kv_heads;
   const long long capacity = (long long)group * (p.win_rows > 0 ? p.win_rows : p.max_seqlen) * p.slots;
-  if (hist_bytes > 48 * 1024) {
-    MOBA_CUDA_OK(cudaFuncSetAttribute(count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes));
-    MOBA_CUDA_OK(cudaFuncSetAttribute(offsets_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes));
-  }
+  static SmemLimit count_limit, order_limit;
+  if (int rc = raise_smem_limit(count_limit, (const void*)count_kernel, hist_bytes)) return rc;
+  if (int rc = raise_smem_limit(order_limit, (const void*)offsets_order_kernel, hist_bytes)) return rc;
   { KernelTimer t__("count_kernel", st);
-  count_kernel<<<(unsigned)row_ctas, 256, hist_bytes, st>>>(block_idx, cu, tiles, slot_counter, p, g.chunk_rows, g.chunks);
-  MOBA_LAUNCH_OK("count_kernel"); }
+  MOBA_CUDA_OK(launch_chained(count_kernel, (unsigned)row_ctas, 256, hist_bytes, st, block_idx, cu, tiles, slot_counter, p,
+                              g.chunk_rows, g.chunks)); }
   { KernelTimer t__("colscan_kernel", st);
   const unsigned per_row = (unsigned)((p.num_blocks + 3) / 4);
-  colscan_kernel<<<per_row * (unsigned)(p.n_seq * p.kv_heads), 128, 0, st>>>(cu, tiles, col_nnz, p, g.chunk_rows, g.chunks, (int)per_row);
-  MOBA_LAUNCH_OK("colscan_kernel"); }
+  MOBA_CUDA_OK(launch_chained(colscan_kernel, per_row * (unsigned)(p.n_seq * p.kv_heads), 128, 0, st, cu, tiles, col_nnz, p,
+                              g.chunk_rows, g.chunks, (int)per_row)); }
   { KernelTimer t__("offsets_order_kernel", st);
-  offsets_order_kernel<<<dim3(p.n_seq * p.kv_heads, (p.num_blocks + 127) / 128), 1024, hist_bytes, st>>>(
-      col_nnz, col_offsets, order, p.num_blocks);
-  MOBA_LAUNCH_OK("offsets_order_kernel"); }
+  MOBA_CUDA_OK(launch_chained(offsets_order_kernel, dim3(p.n_seq * p.kv_heads, (p.num_blocks + 127) / 128), 1024, hist_bytes, st,
+                              (const int32_t*)col_nnz, col_offsets, order, p.num_blocks)); }
   if (work_items != nullptr) {
     KernelTimer t__("work_items_kernel", st);
-    unsigned* err = device_error_word();
-    if (err == nullptr) { set_error("transpose: no device error word"); return MOBA_B200_ECUDA; }
-    work_items_kernel<<<p.n_seq * p.kv_heads, 1024, 0, st>>>(col_nnz, order, reinterpret_cast<int4*>(work_items), slot_counter,
-                                                            p.num_blocks, (int)sched_items_per_row(p), sched_chunk_tiles(p),
-                                                            (int)sched_part_slots(p), err);
-    MOBA_LAUNCH_OK("work_items_kernel");
+    MOBA_CUDA_OK(launch_chained(work_items_kernel, p.n_seq * p.kv_heads, 1024, 0, st, (const int32_t*)col_nnz, (const int32_t*)order,
+                                reinterpret_cast<int4*>(work_items), slot_counter, p.num_blocks, (int)sched_items_per_row(p),
+                                sched_chunk_tiles(p), (int)sched_part_slots(p), err));
   }
-  { KernelTimer t__("scatter_kernel", st);
+  KernelTimer t__("scatter_kernel", st);
   const int w = scatter_warps_for(p);
-  if (w == 8) return launch_scatter<8>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, g, capacity, st);
-  if (w == 4) return launch_scatter<4>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, g, capacity, st);
-  return launch_scatter<1>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, g, capacity, st); }
+#define MOBA_SCATTER(W) \
+  return entries != nullptr ? launch_scatter<W, true>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, entries, g, capacity, st) \
+                            : launch_scatter<W, false>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, entries, g, capacity, st)
+  if (w == 8) MOBA_SCATTER(8);
+  if (w == 4) MOBA_SCATTER(4);
+  MOBA_SCATTER(1);
+#undef MOBA_SCATTER
+}
+
+// ---------------------------------------------------------------------------
+// Short rows: the five passes in one launch, one cluster of CTAs per (sequence, kv head).
+//
+// The cluster's warps cut the row's queries, in (query head, position) order, into consecutive
+// runs. A histogram per warp, a scan over the warps of a CTA and one exchange of column totals
+// over distributed shared memory give every warp its own cursors; the walk that follows is the
+// one of scatter_kernel, so the order inside a column is the same. The last CTA of the cluster
+// also ranks the columns and writes the work items. What bounds it is latency: two reads of the
+// selections (the second from the L2), two cluster barriers and the walk.
+// Lines: up to kSmallBlocks columns, because one CTA ranks them all against one another, and up
+// to kSmallPairs pairs per row and cluster; a longer row leaves too much to one cluster.
+// ---------------------------------------------------------------------------
+constexpr int kSmallBlocks = 512;
+constexpr int kSmallCluster = 8;
+constexpr long long kSmallPairs = 1 << 17;
+constexpr int kSmallThreads = 1024, kSmallWarps = kSmallThreads / 32;
+
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int ld_cluster_i32(const int* mine, uint32_t rank) {
+  uint32_t local = sm100::smem_u32(mine), remote;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 1)
+transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu, int32_t* __restrict__ col_nnz,
+                       int32_t* __restrict__ col_offsets, int32_t* __restrict__ order, int2* __restrict__ entries, int4* __restrict__ items,
+                       int32_t* __restrict__ slot_counter, moba_b200_problem p, long long capacity, int items_per_row,
+                       int tc, int slot_cap, unsigned* error_word) {
+  extern __shared__ int cursor_all[];                        // [warps][nb]
+  __shared__ int totals[kSmallBlocks];                       // this CTA's pairs per column (read by its peers)
+  __shared__ int nnz_s[kSmallBlocks], base_s[kSmallBlocks], ord_s[kSmallBlocks];
+  __shared__ int warp_sums[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nb = p.num_blocks;
+  const uint32_t rank = cluster_rank();
+  for (int i = threadIdx.x; i < kSmallWarps * nb; i += kSmallThreads) cursor_all[i] = 0;
+  pdl_trigger();
+  pdl_wait();
+  const int kv_row = (int)(blockIdx.x / kSmallCluster);
+  const int seq = kv_row / p.kv_heads, kvh = kv_row % p.kv_heads;
+  const int group = p.q_heads / p.kv_heads;
+  const SeqSpan sp = seq_span(cu, p.packed, seq, p.tokens);
+  const unsigned slots = (unsigned)p.slots;
+  // this warp's run of queries, in (head, position) order
+  const long long total_q = (long long)group * sp.len;
+  const int per_warp = (int)((total_q + kSmallCluster * kSmallWarps - 1) / (kSmallCluster * kSmallWarps));
+  const long long q_lo = min(total_q, (long long)((int)rank * kSmallWarps + warp) * per_warp), q_hi = min(total_q, q_lo + per_warp);
+  const int n = (int)(q_hi - q_lo) * (int)slots;
+  int g0 = 0, r0 = (int)q_lo;                                // head and position of the run's first query
+  if (sp.len > 0) { g0 = (int)(q_lo / sp.len); r0 = (int)(q_lo - (long long)g0 * sp.len); }
+  const size_t head0 = (p.packed ? 0 : (size_t)seq * p.q_heads) + (size_t)kvh * group;
+  // entry e of the run: query, slot and where its block id is
+  auto entry = [&](int e, int& g, int& row, int& slot) -> const int32_t* {
+    const unsigned qi = (unsigned)e / slots;
+    slot = (int)((unsigned)e - qi * slots);
+    row = r0 + (int)qi; g = g0;
+    while (row >= sp.len) { row -= sp.len; ++g; }
+    return block_idx + ((head0 + g) * p.tokens + sp.bos + row) * (size_t)slots + slot;
+  };
+  int* cursor = cursor_all + warp * nb;
+  __syncthreads();
+  for (int e = lane; e < n; e += 32) {
+    int g, row, slot;
+    const int blk = __ldg(entry(e, g, row, slot));
+    if (blk >= 0 && blk < nb) atomicAdd(&cursor[blk], 1);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nb; i += kSmallThreads) {
+    int at = 0;
+#pragma unroll 8
+    for (int w = 0; w < kSmallWarps; ++w) {
+      const int t = cursor_all[w * nb + i];
+      cursor_all[w * nb + i] = at;
+      at += t;
+    }
+    totals[i] = at;
+  }
+  cluster_barrier();
+  // column i: its pairs in the CTAs before this one, and in all of them
+  int mine = 0, before = 0;
+  const int col = threadIdx.x;                               // nb <= kSmallBlocks < threads
+  if (col < nb) {
+#pragma unroll
+    for (int c = 0; c < kSmallCluster; ++c) {
+      const int t = ld_cluster_i32(&totals[col], (uint32_t)c);
+      mine += t;
+      before += c < (int)rank ? t : 0;
+    }
+    nnz_s[col] = mine;
+  }
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  int off = incl - mine;
+  for (int w = 0; w < warp; ++w) off += warp_sums[w];        // (warps beyond the columns add nothing to later ones)
+  if (col < nb) base_s[col] = off + before;
+  if (rank == kSmallCluster - 1) {
+    if (col < nb) {
+      col_nnz[(size_t)kv_row * nb + col] = mine;
+      col_offsets[(size_t)kv_row * (nb + 1) + col] = off;
+      if (col == nb - 1) col_offsets[(size_t)kv_row * (nb + 1) + nb] = off + mine;
+      int rk = 0;                                            // stable descending rank
+      for (int j = 0; j < nb; ++j) { const int o = nnz_s[j]; rk += (o > mine || (o == mine && j < col)) ? 1 : 0; }
+      ord_s[rk] = col;
+      order[(size_t)kv_row * nb + rk] = col;
+    }
+  }
+  cluster_barrier();                                         // totals have been read; base_s and ord_s are complete
+
+  int2* eo = entries + (size_t)kv_row * capacity;
+  const unsigned lt = (1u << lane) - 1u;
+  for (int e0 = 0; e0 < n; e0 += 32) {
+    const int e = e0 + lane;
+    int g = 0, row = 0, slot = 0, blk = -1;
+    if (e < n) blk = __ldg(entry(e, g, row, slot));
+    const bool valid = blk >= 0 && blk < nb;
+    const unsigned same = __match_any_sync(0xffffffffu, valid ? blk : (0x40000000 + lane));
+    int base = 0;
+    if (valid) base = cursor[blk];
+    __syncwarp();
+    if (valid && (same & lt) == 0) cursor[blk] = base + __popc(same);
+    __syncwarp();
+    if (valid) {
+      const long long dst = (long long)base_s[blk] + base + __popc(same & lt);
+      if (dst < capacity) eo[dst] = make_int2(sp.bos + row, ((kvh * group + g) << 8) | slot);
+    }
+  }
+  if (rank == kSmallCluster - 1)
+    write_work_items<kSmallBlocks>(nnz_s, ord_s, items + (size_t)kv_row * items_per_row, slot_counter, nb, items_per_row, tc,
+                                   slot_cap, error_word);
+}
+
+bool transpose_small_supported(const moba_b200_problem& p) {
+  const long long row_pairs = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
+  return p.num_blocks <= kSmallBlocks && row_pairs <= kSmallPairs && p.win_rows == 0 &&
+         (long long)p.n_seq * p.kv_heads * kSmallCluster < 0x7fffffffLL;
+}
+
+// `slot_counter` must hold zero.
+int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu, int32_t* col_nnz,
+                           int32_t* col_offsets, int32_t* order, int2* entries, int32_t* work_items, int32_t* slot_counter,
+                           cudaStream_t st) {
+  KernelTimer t__("transpose_small_kernel", st);
+  unsigned* err = device_error_word();
+  if (err == nullptr) { set_error("transpose: no device error word"); return MOBA_B200_ECUDA; }
+  const size_t smem = (size_t)kSmallWarps * p.num_blocks * sizeof(int);
+  static SmemLimit limit;
+  if (int rc = raise_smem_limit(limit, (const void*)transpose_small_kernel, smem)) return rc;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = kSmallCluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.n_seq * p.kv_heads * kSmallCluster)); cfg.blockDim = dim3(kSmallThreads);
+  cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;
+  const long long capacity = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
+  MOBA_CUDA_OK(cudaLaunchKernelEx(&cfg, transpose_small_kernel, block_idx, cu, col_nnz, col_offsets, order, entries,
+                                  reinterpret_cast<int4*>(work_items), slot_counter, p, capacity, (int)sched_items_per_row(p),
+                                  sched_chunk_tiles(p), (int)sched_part_slots(p), err));
+  return MOBA_B200_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -576,7 +776,7 @@ int launch_transpose_noalloc(const moba_b200_problem& p, const int32_t* block_id
   // Nothing in the array has to be cleared by the caller: the count pass writes every entry
   // the scan pass reads and resets the slot counter, so the previous call's contents are
   // simply overwritten.
-  return launch_transpose(p, block_idx, cu, col_nnz, col_offsets, order, rows, heads, slots, work_items, scratch,
+  return launch_transpose(p, block_idx, cu, col_nnz, col_offsets, order, rows, heads, slots, nullptr, work_items, scratch,
                           kStaticScratchBytes, st);
 }
 

@@ -7,6 +7,7 @@ log2-sum-exp, `part_lse`. The merged output and the global log-sum-exp are the
 same quantities. `combine_partials` still accepts the reference's triple.
 """
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -49,6 +50,62 @@ def _validate(q, k, v, cfg: MoBAConfig, cu_seqlens=None, max_seqlen=None) -> Non
         raise ValueError(
             f"block_size {cfg.block_size} below the tl.dot minimum of {MIN_BLOCK_SIZE} "
             "(wording kept from the reference; it is this engine's minimum block too)")
+
+
+class _OpPlan:
+    """What a whole-op call needs beside its tensors: the problem record and the sizes of its
+    workspaces. Functions of shapes, dtype and configuration only, kept between calls."""
+    __slots__ = ("problem", "keep_bytes", "forward_bytes", "backward_bytes")
+
+    def __init__(self, problem):
+        self.problem = problem
+        sizes = [ctypes.c_size_t() for _ in range(3)]
+        _lib.check(_lib.load().moba_b200_op_workspace(problem, *(ctypes.byref(x) for x in sizes)), "moba_attention")
+        self.keep_bytes, self.forward_bytes, self.backward_bytes = (x.value for x in sizes)
+
+
+_PLANS = {}
+_MAX_PLANS = 512
+
+
+def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, partials_dtype=None) -> "_OpPlan":
+    """Validates a call and returns its plan; a call like an earlier one skips both."""
+    on_gpu = q.is_cuda and k.is_cuda and v.is_cuda and (cu_seqlens is None or cu_seqlens.is_cuda)
+    key = (q.shape, k.shape, v.shape, q.dtype, k.dtype, v.dtype, cfg, causal, max_seqlen, partials_dtype,
+           None if cu_seqlens is None else (cu_seqlens.shape, cu_seqlens.dtype),
+           _lib._force_path[0], _lib._chunk_tiles[0])
+    try:
+        plan = _PLANS.get(key) if on_gpu else None
+    except TypeError:                                        # a foreign configuration object that cannot be hashed
+        key = None
+        plan = None
+    if plan is not None:
+        return plan
+    _validate(q, k, v, cfg, cu_seqlens, max_seqlen)
+    _lib.require_cuda(q, k, v, cu_seqlens)
+    if partials_dtype not in (None, q.dtype, torch.float32):
+        raise ValueError(f"partials_dtype must be {q.dtype} or float32, got {partials_dtype}")
+    part_f32 = partials_dtype == torch.float32 and q.dtype != torch.float32
+    plan = _OpPlan(_lib.make_problem(tuple(q.shape), k.shape[2], q.dtype, cfg, cu_seqlens, max_seqlen, causal=causal,
+                                     part_f32=part_f32))
+    if key is not None:
+        if len(_PLANS) >= _MAX_PLANS:
+            _PLANS.clear()
+        _PLANS[key] = plan
+    return plan
+
+
+def op_forward(plan: "_OpPlan", q, k, v, cu_seqlens, want_lse: bool):
+    """pool, gate, transpose, attention and merge in one call; returns (out, keep), where `keep`
+    is the workspace a backward of this forward needs."""
+    out = torch.empty_like(q)
+    dev = q.device
+    keep = torch.empty((plan.keep_bytes,), device=dev, dtype=torch.uint8)
+    scratch = torch.empty((plan.forward_bytes,), device=dev, dtype=torch.uint8)
+    _lib.call_op("moba_b200_op_forward", dev.index, "moba_forward", plan.problem, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                 None if cu_seqlens is None else cu_seqlens.data_ptr(), keep.data_ptr(), scratch.data_ptr(), out.data_ptr(),
+                 want_lse)
+    return out, keep
 
 
 def _problem(q, k, cfg, index: CSCIndex, causal=True, part_f32=False):
@@ -227,12 +284,11 @@ def moba_forward(q, k, v, cfg: MoBAConfig, index: Optional[CSCIndex] = None, cau
                                                    partials_dtype=partials_dtype, partials=partials)
                 out[:, :, h0 * group:h1 * group] = merge_partials(part_lse, part_o, q.dtype)
             return out
-    if index is not None:
-        cu_seqlens, max_seqlen = index.cu_seqlens, index.max_seqlen
-    _validate(q, k, v, cfg, cu_seqlens, max_seqlen)
-    _lib.require_cuda(q, k, v, cu_seqlens)
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     if index is None:
-        index = build_csc_fused(q, k, cfg, cu_seqlens=cu_seqlens, max_seqlen=max_seqlen)
+        plan = op_plan(q, k, v, cfg, causal, cu_seqlens, max_seqlen, partials_dtype)
+        return op_forward(plan, q.contiguous(), k.contiguous(), v.contiguous(), cu_seqlens, False)[0]
+    _validate(q, k, v, cfg, index.cu_seqlens, index.max_seqlen)
+    _lib.require_cuda(q, k, v, index.cu_seqlens)
+    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
     part_lse, part_o = attend_partials(q, k, v, cfg, index, causal=causal, partials_dtype=partials_dtype)
     return merge_partials(part_lse, part_o, q.dtype)

@@ -1,0 +1,48 @@
+"""The whole-op entry points (`moba_b200_op_forward` / `_op_backward`, what `moba_attention` and
+`moba_forward` call when no index is given) against the staged ones with an explicit index: same
+selections, so O and dQ are the same bits; dK/dV may be cut into other work items and are compared
+within the engine's tolerance. Sizes lie on both sides of the line between the one-launch
+transpose and the five-pass one, and of the finer cut of small problems."""
+
+import pytest
+import torch
+
+import moba_triton_b200 as moba
+
+from conftest import make_qkv
+from helpers import max_abs_error
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # B, S, Hq, Hkv, D, block, top_k, dtype, cu_seqlens
+    (1, 100, 2, 1, 64, 128, 3, torch.bfloat16, None),            # one short block
+    (1, 1000, 4, 2, 64, 128, 4, torch.bfloat16, None),
+    (3, 900, 2, 2, 128, 128, 8, torch.float16, None),            # batch rows end inside a block
+    (1, 16384, 1, 1, 64, 128, 8, torch.bfloat16, None),          # the last row length of the one-launch transpose
+    (1, 16512, 1, 1, 64, 128, 8, torch.bfloat16, None),          # the first beyond it
+    (1, 8192, 2, 2, 64, 16, 2, torch.bfloat16, None),            # 512 columns
+    (1, 8208, 2, 2, 64, 16, 2, torch.bfloat16, None),            # 513
+    (1, 1500, 4, 2, 64, 128, 4, torch.bfloat16, [0, 1, 130, 700, 1500]),
+    (1, 700, 2, 2, 64, 32, 5, torch.float32, [0, 333, 700]),
+]
+
+
+@pytest.mark.parametrize("b,s,hq,hkv,d,bs,top_k,dtype,cu", CASES, ids=[f"s{c[1]}-h{c[2]}kv{c[3]}-blk{c[5]}" for c in CASES])
+def test_whole_op_equals_the_staged_calls(b, s, hq, hkv, d, bs, top_k, dtype, cu, device):
+    cfg = moba.MoBAConfig(bs, top_k, dtype=dtype)
+    q, k, v, do = (t.to(device) for t in make_qkv((b, s, hq, d), hkv, dtype=dtype, seed=61, with_do=True))
+    kw = {} if cu is None else dict(cu_seqlens=torch.tensor(cu, dtype=torch.int32, device=device),
+                                    max_seqlen=max(y - x for x, y in zip(cu[:-1], cu[1:])))
+    index = moba.build_csc_fused(q, k, cfg, **kw)
+    got = []
+    for args in (dict(index=index), kw):
+        leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        out = moba.moba_attention(*leaves, cfg, **args)
+        out.backward(do)
+        got.append([out.detach()] + [t.grad for t in leaves])
+    staged, whole = got
+    assert torch.equal(whole[0], staged[0]) and torch.equal(whole[1], staged[1])
+    for a, w in zip(whole[2:], staged[2:]):
+        assert max_abs_error(a, w) <= (1e-5 if dtype == torch.float32 else 2e-2)
+    assert torch.equal(moba.moba_forward(q, k, v, cfg, **kw), staged[0])
