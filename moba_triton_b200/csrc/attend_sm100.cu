@@ -252,13 +252,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       }
     };
     // This thread's index entry (row r of tile k.t): query position, head, slot.
-    auto load_entry = [&](const Cur& k, int& row, int& head, int& slot) {
+    auto load_entry = [&](const Cur& k, RawPair& raw) {
       const int e = (int)(k.t - k.t0) * kTile + r;
-      row = head = slot = 0;
-      if (r < kTile && e < k.c.n) {
-        const PairEntry pe = load_pair_pinned(ix, (size_t)k.c.kv_row * ix.capacity + k.c.lo + e);
-        row = pe.row; head = pe.head; slot = pe.slot;
-      }
+      raw = RawPair{0, 0, 0};
+      if (r < kTile && e < k.c.n) raw = fetch_pair(ix, (size_t)k.c.kv_row * ix.capacity + k.c.lo + e);
     };
     // Copies the 128 query rows of tile k.t into its stage. `n_gather` alternates the row
     // table, so one barrier per gather is enough (the table of gather g is rewritten by
@@ -318,16 +315,17 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
     };
 
     Cur pf{0u, 0u, (uint32_t)wg, 0, false, Column{}};
-    int n_row = 0, n_head = 0, n_slot = 0;
+    RawPair raw{0, 0, 0};                             // the next tile's entry
     bool more = locate(pf, true) == 1;
-    if (more) load_entry(pf, n_row, n_head, n_slot);
+    if (more) load_entry(pf, raw);
     if (is_mover) {
       // ---- movers: copy the rows of this warpgroup's tiles in, a tile ahead of the softmax
       // warps, and the staged output rows of the tile before out ----
       for (uint32_t j = 0;; ++j) {
         const bool have_tile = more;
         if (have_tile) {
-          gather(pf, n_row, n_head);
+          const PairEntry ge = pair_of(ix, raw);
+          gather(pf, ge.row, ge.head);
           cp_async_wait<0>();
           fence_proxy_async();
           mbar_arrive_warp(&bars->q_full[wg]);
@@ -340,7 +338,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         if (!have_tile) break;
         pf.t += NB;
         more = locate(pf, true) == 1;
-        if (more) load_entry(pf, n_row, n_head, n_slot);
+        if (more) load_entry(pf, raw);
       }
     } else {
     bool gathered = false;
@@ -348,7 +346,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
     while (more) {
       const Cur cur = pf;
       const Column& c = cur.c;
-      const int row = n_row, head = n_head, slot = n_slot;
+      const PairEntry ce = pair_of(ix, raw);
+      const int row = ce.row, head = ce.head, slot = ce.slot;
       const uint32_t u = cur.t / NB;                   // how often this buffer has been used before
       const bool live = (int)(cur.t - cur.t0) * kTile + r < c.n;
       if (!Cfg::kMovers && !gathered) {                // first tile, or its descriptor came late
@@ -371,7 +370,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       // the first pass over the scores; its rows are copied while the second pass runs.
       pf.t += NB;
       const int nxt = locate(pf, false);
-      if (nxt == 1) load_entry(pf, n_row, n_head, n_slot);
+      if (nxt == 1) load_entry(pf, raw);
       PHASE_ADD(wc, 11, ph);                           // s_full wait, next tile located
       TRACE(error_word, cur.t, 1);
 
@@ -397,7 +396,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
 
       PHASE_ADD(wc, 12, ph);                           // first pass (row maximum)
       TRACE(error_word, cur.t, 2);
-      if (!Cfg::kMovers && nxt == 1) gather(pf, n_row, n_head);
+      if (!Cfg::kMovers && nxt == 1) { const PairEntry ge = pair_of(ix, raw); gather(pf, ge.row, ge.head); }
       PHASE_ADD(wc, 13, ph);                           // copies of the next tile issued
       TRACE(error_word, cur.t, 3);
 
@@ -494,7 +493,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       if (nxt == 1) { gathered = true; continue; }
       if (nxt == 0) break;
       more = locate(pf, true) == 1;                    // the descriptor was not there in time
-      if (more) load_entry(pf, n_row, n_head, n_slot);
+      if (more) load_entry(pf, raw);
       gathered = false;
     }
     }

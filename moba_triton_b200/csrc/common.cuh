@@ -153,7 +153,7 @@ struct TensorCorePlan {
 };
 constexpr TensorCorePlan kTensorCorePlans[2] = {
     {64, 4, 4, 2, 2, 16, 8},
-    {128, 2, 2, 1, 1, 7, 4},
+    {128, 2, 2, 1, 2, 7, 4},
 };
 constexpr const TensorCorePlan& tensor_core_plan(int head_dim) { return kTensorCorePlans[head_dim == 64 ? 0 : 1]; }
 
@@ -202,20 +202,23 @@ __device__ __forceinline__ PairEntry load_pair(const moba_b200_index& ix, size_t
   }
   return e;
 }
-// The same with loads the compiler may not move: a plain load may be sunk to its first use,
-// which defeats fetching an entry a tile ahead.
-__device__ __forceinline__ PairEntry load_pair_pinned(const moba_b200_index& ix, size_t at) {
-  PairEntry e;
+// Fetching an entry a tile ahead: the loads may not be moved (a plain load may be sunk to its
+// first use), and nothing looks at the words before `pair_of` (unpacking them at once would wait
+// for the load: a memory latency per tile, which had cost the attention kernels 3 to 8 %).
+struct RawPair { int a, b, c; };
+__device__ __forceinline__ RawPair fetch_pair(const moba_b200_index& ix, size_t at) {
+  RawPair r{0, 0, 0};
   if (packed_pairs(ix)) {
-    int a, b;
-    asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "l"(reinterpret_cast<const int2*>(ix.row_indices) + at));
-    e.row = a; e.head = b >> 8; e.slot = b & 0xff;
+    asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];" : "=r"(r.a), "=r"(r.b) : "l"(reinterpret_cast<const int2*>(ix.row_indices) + at));
   } else {
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(e.row) : "l"(ix.row_indices + at));
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(e.head) : "l"(ix.head_indices + at));
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(e.slot) : "l"(ix.slot_of_pair + at));
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.a) : "l"(ix.row_indices + at));
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.b) : "l"(ix.head_indices + at));
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.c) : "l"(ix.slot_of_pair + at));
   }
-  return e;
+  return r;
+}
+__device__ __forceinline__ PairEntry pair_of(const moba_b200_index& ix, const RawPair& r) {
+  return packed_pairs(ix) ? PairEntry{r.a, r.b >> 8, r.b & 0xff} : PairEntry{r.a, r.b, r.c};
 }
 
 // One work item as the kernels see it.

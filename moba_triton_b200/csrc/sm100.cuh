@@ -57,6 +57,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Whether the phase has completed, without waiting (try_wait may suspend the thread).
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 struct WaitCtx {
   volatile int* abort;        // shared-memory flag of the CTA
   unsigned* error_word;       // global
@@ -247,6 +260,12 @@ __device__ __forceinline__ void tma_load_3d(void* dst_smem, const CUtensorMap* m
       : "memory");
 }
 
+// Asks the L2 for a tile; nothing waits for it.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* m, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+
 // Four rows of a 2-D tensor (map with a box of one row) -> four consecutive 128-byte rows
 // of a swizzled tile. Rows outside the tensor read as zeros.
 __device__ __forceinline__ void tma_gather4(void* dst_smem, const CUtensorMap* m, uint64_t* bar, int col,
@@ -256,6 +275,16 @@ __device__ __forceinline__ void tma_gather4(void* dst_smem, const CUtensorMap* m
       "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1),
         "r"(r2), "r"(r3)
+      : "memory");
+}
+
+__device__ __forceinline__ void tma_gather4_hint(void* dst_smem, const CUtensorMap* m, uint64_t* bar, int col,
+                                                 int r0, int r1, int r2, int r3, uint64_t pol) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
+      ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1),
+        "r"(r2), "r"(r3), "l"(pol)
       : "memory");
 }
 
