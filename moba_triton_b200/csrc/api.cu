@@ -245,7 +245,7 @@ int moba_b200_pool(const moba_b200_problem* p, const void* k, const int32_t* cu_
   MOBA_TRY(check_problem(p));
   MOBA_TRY(need(k, "k")); MOBA_TRY(need(kbar, "kbar"));
   if (p->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
-  return launch_pool(*p, k, cu_seqlens, kbar, nullptr, (cudaStream_t)stream);
+  return launch_pool(*p, k, cu_seqlens, kbar, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int moba_b200_gate(const moba_b200_problem* p, const void* q, const void* kbar,
@@ -273,7 +273,7 @@ int moba_b200_transpose(const moba_b200_problem* p, const int32_t* block_idx,
   MOBA_TRY(need(scratch, "scratch"));
   if (p->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
   return launch_transpose(*p, block_idx, cu_seqlens, col_nnz, col_offsets, order, row_indices,
-                          head_indices, slot_of_pair, nullptr, work_items, scratch, scratch_bytes, (cudaStream_t)stream);
+                          head_indices, slot_of_pair, nullptr, 0, work_items, scratch, scratch_bytes, (cudaStream_t)stream);
 }
 
 int moba_b200_transpose_noalloc(const moba_b200_problem* p, const int32_t* block_idx,
@@ -318,7 +318,7 @@ int moba_b200_fwd(const moba_b200_problem* p, const void* q, const void* k, cons
   cudaStream_t st = (cudaStream_t)stream;
   MOBA_TRY(launch_fill_lse(*p, part_lse, st));
   if (path == MOBA_B200_PATH_TCGEN05)
-    return launch_fwd_sm100(*p, q, k, v, *index, cu_seqlens, part_o, part_lse, st);
+    return launch_fwd_sm100(*p, q, k, v, *index, cu_seqlens, part_o, part_lse, kBlockKeys, st);
   return launch_fwd_portable(*p, q, k, v, *index, cu_seqlens, part_o, part_lse, st);
 }
 
@@ -346,7 +346,7 @@ int moba_b200_bwd(const moba_b200_problem* p, const void* q, const void* k, cons
   MOBA_TRY(launch_delta(*p, out, dout, delta, st));
   if (path == MOBA_B200_PATH_TCGEN05)
     MOBA_TRY(launch_bwd_sm100(*p, q, k, v, dout, lse, delta, *index, cu_seqlens, dq_part,
-                              static_cast<float*>(dkv_scratch), dk, dv, st));
+                              static_cast<float*>(dkv_scratch), dk, dv, kBlockKeys, st));
   else
     MOBA_TRY(launch_bwd_portable(*p, q, k, v, dout, lse, delta, *index, cu_seqlens, dq_part, dk, dv, st));
   return launch_dq_reduce(*p, dq_part, part_lse, dq, st);

@@ -87,7 +87,7 @@ fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
 #pragma unroll
     for (int r = 0; r < kFwdRows; ++r) {
       const bool live = e0 + r < n;
-      PairEntry pe{-1, 0, 0};
+      PairEntry pe{-1, 0, 0, 0};
       if (live) pe = load_pair(ix, list0 + e0 + r);
       row[r] = pe.row; head[r] = pe.head; slot[r] = pe.slot;
       for (int c = lane; c < d; c += 32)

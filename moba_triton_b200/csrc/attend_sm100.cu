@@ -156,7 +156,7 @@ template <int D, typename T, typename TP>
 __global__ void __launch_bounds__(FwdCfg<D>::kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                  const T* __restrict__ q, moba_b200_index ix, const int32_t* __restrict__ cu,
-                 TP* __restrict__ part_o, float* __restrict__ part_lse, moba_b200_problem p, int n_items,
+                 TP* __restrict__ part_o, float* __restrict__ part_lse, moba_b200_problem p, int part_keys, int n_items,
                  unsigned* error_word) {
   using Cfg = FwdCfg<D>;
   constexpr int NQ = Cfg::kQStages, NB = Cfg::kBufs, NKV = Cfg::kKvBufs;
@@ -358,11 +358,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       }
       PHASE_ADD(wc, 10, ph);                           // late gather
       TRACE(error_word, cur.t, 0);
-      int jmax = c.keys - 1;
+      // keys [jmin, jmax] of the column: those of the pair's block, up to the query itself
+      const int jmin = ce.part * part_keys;
+      int jmax = min(c.keys, jmin + part_keys) - 1;
       if (p.causal && live && (row - c.bos) / kTile == c.blk) jmax = min(jmax, row - c.key0);
       // Away from the diagonal block and the ragged ends every row keeps all 128 keys; such
       // a warp runs without the per-element comparison.
-      const bool all_open = __all_sync(0xffffffffu, jmax >= kTile - 1);
+      const bool all_open = __all_sync(0xffffffffu, jmin == 0 && jmax >= kTile - 1);
 
       const bool s_ok = mbar_wait(&bars->s_full[wg], u & 1, wc, 2);
       tc_fence_after();
@@ -387,7 +389,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         } else {
 #pragma unroll
           for (int k = 0; k < 32; ++k) {
-            const float s = (ch * 32 + k <= jmax) ? __uint_as_float(v[k]) : -INFINITY;
+            const float s = (ch * 32 + k >= jmin && ch * 32 + k <= jmax) ? __uint_as_float(v[k]) : -INFINITY;
             mx4[k & 3] = fmaxf(mx4[k & 3], s);
           }
         }
@@ -415,7 +417,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               const float x = ex2(fmaf(__uint_as_float(v[g * 8 + k]), cs, -m2));
-              if constexpr (decltype(masked)::value) pe[k] = (ch * 32 + g * 8 + k <= jmax) ? x : 0.f;
+              if constexpr (decltype(masked)::value) pe[k] = (ch * 32 + g * 8 + k >= jmin && ch * 32 + g * 8 + k <= jmax) ? x : 0.f;
               else pe[k] = x;
               l4[k & 3] += pe[k];
             }
@@ -694,7 +696,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
 
 template <int D, typename T, typename TP>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensorMap& vm, const void* q,
-               const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse, int n_items,
+               const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse, int part_keys, int n_items,
                unsigned* err, cudaStream_t st) {
   auto kern = fwd_sm100_kernel<D, T, TP>;
   static SmemLimit limit;
@@ -702,7 +704,7 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
   const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
   MOBA_CUDA_OK(launch_chained(kern, grid, FwdCfg<D>::kThreads, FwdCfg<D>::kSmem, st, km, vm, (const T*)q, ix, cu,
-                              (TP*)part_o, part_lse, p, n_items, err));
+                              (TP*)part_o, part_lse, p, part_keys, n_items, err));
   return MOBA_B200_OK;
 }
 
@@ -716,7 +718,7 @@ bool fwd_sm100_supported(const moba_b200_problem& p) {
 
 int launch_fwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse,
-                     cudaStream_t st) {
+                     int part_keys, cudaStream_t st) {
   KernelTimer timer__("fwd_sm100_kernel", st);
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("forward: no device error word"); return MOBA_B200_ECUDA; }
@@ -734,7 +736,7 @@ int launch_fwd_sm100(const moba_b200_problem& p, const void* q, const void* k, c
   if (n_items_ll > 0x7fffffffLL) { set_error("forward: too many work items"); return MOBA_B200_EUNSUPPORTED; }
   const int n_items = (int)n_items_ll;
   const bool bf = p.dtype == MOBA_B200_BF16;
-#define GO(D, T, TP) return launch_one<D, T, TP>(p, km, vm, q, ix, cu, part_o, part_lse, n_items, err, st)
+#define GO(D, T, TP) return launch_one<D, T, TP>(p, km, vm, q, ix, cu, part_o, part_lse, part_keys, n_items, err, st)
   if (p.head_dim == 64) {
     if (bf) { if (p.part_f32) GO(64, __nv_bfloat16, float); else GO(64, __nv_bfloat16, __nv_bfloat16); }
     else { if (p.part_f32) GO(64, __half, float); else GO(64, __half, __half); }

@@ -153,7 +153,7 @@ bwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
     // ---- phase 1 ----
     const int e = e0 + warp;
     const bool live = e < n;
-    PairEntry pe{-1, 0, 0};
+    PairEntry pe{-1, 0, 0, 0};
     if (live) pe = load_pair(ix, list0 + e);
     const int row = pe.row, head = pe.head, slot = pe.slot;
     float lse_r = 0.f, delta_r = 0.f;

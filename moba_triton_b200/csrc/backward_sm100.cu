@@ -209,7 +209,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
                  const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap g_map, const float* __restrict__ lse,
                  const float* __restrict__ delta, moba_b200_index ix, const int32_t* __restrict__ cu,
                  T* __restrict__ dq_part, float* __restrict__ dkv_scratch, T* __restrict__ dk, T* __restrict__ dv,
-                 moba_b200_problem p, int n_items, unsigned* error_word) {
+                 moba_b200_problem p, int part_keys, int n_items, unsigned* error_word) {
   using Cfg = BwdCfg<D>;
   constexpr int NST = Cfg::kStages, NKV = Cfg::kKvBufs, NS = Cfg::kSBufs;
   constexpr uint32_t cS = Cfg::cS, cDP = Cfg::cDP, cDV = Cfg::cDV, cDK = Cfg::cDK;
@@ -297,6 +297,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         // and as such ordered alike when read as half-precision numbers.
         const bool masked = c.keys < kTile || bars->masked[st][wq] != 0;
         const uint32_t key2 = r < c.keys ? (uint32_t)r * 0x10001u : 0x7bff7bffu;   // past the end: after every `last`
+        const uint32_t part_mask = (uint32_t)(~(part_keys - 1) & 0xffff) * 0x10001u;   // key -> first key of its block
         auto apply_mask = [&](uint32_t (&w)[8], const uint16_t* last) {
           const uint4 a = *reinterpret_cast<const uint4*>(last), b4 = *reinterpret_cast<const uint4*>(last + 8);
           const uint32_t l[8] = {a.x, a.y, a.z, a.w, b4.x, b4.y, b4.z, b4.w};
@@ -305,6 +306,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             uint32_t m;
             asm("set.le.u32.f16x2 %0, %1, %2;" : "=r"(m) : "r"(key2), "r"(l[k]));
             w[k] &= m;
+            if (part_keys < kTile) {                   // a finer block: not before its first key either
+              const uint32_t first2 = l[k] & part_mask;
+              asm("set.le.u32.f16x2 %0, %1, %2;" : "=r"(m) : "r"(first2), "r"(key2));
+              w[k] &= m;
+            }
           }
         };
         // ---- P = exp2(S c - lse), kept in registers for dS ----
@@ -710,8 +716,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             const size_t qr = (b * p.q_heads + me.head) * p.tokens + me.row;
             l = ld_nc_pinned_f(lse + qr);
             dl = ld_nc_pinned_f(delta + qr);
-            const int own = me.row - c.key0;                 // position of the query relative to the block's first key
-            if (p.causal && own < kTile) last = (uint32_t)own;
+            last = (uint32_t)((me.part + 1) * part_keys - 1);
+            const int own = me.row - c.key0;                 // the query's own place, if it lies in the column
+            if (p.causal && own >= 0 && own < (int)last) last = (uint32_t)own;
           }
           if (e + kTile < c.n) nx = fetch_pair(ix, list0 + e + kTile);
           int rows[4];                                       // the four rows lane gathers (lanes 0..7)
@@ -735,7 +742,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           mt.neg_lse[pt] = -l;
           mt.delta[pt] = dl;
           mt.last[pt] = (uint16_t)last;
-          const bool any = __any_sync(0xffffffffu, last != kTile - 1);
+          const bool any = __any_sync(0xffffffffu, last != kTile - 1) || part_keys < kTile;
           if (lane == 0) bars->masked[st][gw] = any ? 1 : 0;
           __syncwarp();
           if (lane == 0) mbar_expect_tx(&bars->q_full[st], 32 * D * 2);     // releases the row data, too
@@ -841,7 +848,7 @@ dkv_reduce_kernel(const float* __restrict__ dkv_scratch, moba_b200_index ix, con
 template <int D, typename T>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensorMap& vm, const CUtensorMap& qm,
                const CUtensorMap& gm, const float* lse, const float* delta, const moba_b200_index& ix,
-               const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int n_items, unsigned* err,
+               const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, int n_items, unsigned* err,
                cudaStream_t st) {
   const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
@@ -851,10 +858,11 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
     static SmemLimit limit;
     if (int rc = raise_smem_limit(limit, (const void*)kern, BwdCfg<D>::kSmem)) return rc;
     MOBA_CUDA_OK(launch_chained(kern, grid, kThreads, BwdCfg<D>::kSmem, st, km, vm, qm, gm, lse, delta,
-                                ix, cu, (T*)dq_part, dkv_scratch, (T*)dk, (T*)dv, p, n_items, err));
+                                ix, cu, (T*)dq_part, dkv_scratch, (T*)dk, (T*)dv, p, part_keys, n_items, err));
   }
   // No column can be long enough to be cut: nothing to sum.
-  const long long longest = ((long long)(p.q_heads / p.kv_heads) * (p.win_rows > 0 ? p.win_rows : p.max_seqlen) + kTile - 1) / kTile;
+  // (a query lists a column once per block in it)
+  const long long longest = ((long long)(p.q_heads / p.kv_heads) * window_rows_of_seq(p) * (kTile / part_keys) + kTile - 1) / kTile;
   if (longest <= ix.chunk_tiles) return MOBA_B200_OK;
   KernelTimer timer__("dkv_reduce_kernel", st);
   const int ctas_per_row = (ix.items_per_row + 255) / 256;
@@ -879,7 +887,7 @@ bool bwd_sm100_supported(const moba_b200_problem& p) {
 
 int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const void* dout, const float* lse, const float* delta, const moba_b200_index& ix,
-                     const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, cudaStream_t st) {
+                     const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, cudaStream_t st) {
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("backward: no device error word"); return MOBA_B200_ECUDA; }
   CUtensorMap km, vm;
@@ -903,11 +911,11 @@ int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, c
   const int n_items = (int)n_items_ll;
   const bool bf = p.dtype == MOBA_B200_BF16;
   if (p.head_dim == 64) {
-    if (bf) return launch_one<64, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, n_items, err, st);
-    return launch_one<64, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, n_items, err, st);
+    if (bf) return launch_one<64, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
+    return launch_one<64, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
   }
-  if (bf) return launch_one<128, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, n_items, err, st);
-  return launch_one<128, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, n_items, err, st);
+  if (bf) return launch_one<128, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
+  return launch_one<128, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
 }
 
 }  // namespace moba

@@ -136,6 +136,8 @@ __host__ __device__ inline bool gate_candidate(const moba_b200_problem& p, int b
 // output, then exist for one window at a time). Row (b, head, row) of part_o / part_lse /
 // dq_part:
 __host__ __device__ inline int window_rows(const moba_b200_problem& p) { return p.win_rows > 0 ? p.win_rows : p.tokens; }
+// rows of a sequence that a call can list: a bound of a column's pairs per query head
+static inline int window_rows_of_seq(const moba_b200_problem& p) { return p.win_rows > 0 ? p.win_rows : p.max_seqlen; }
 __device__ __forceinline__ size_t part_row(const moba_b200_problem& p, size_t b, int head, int row) {
   return (b * p.q_heads + head) * (size_t)window_rows(p) + (size_t)(row - p.win_begin);
 }
@@ -158,6 +160,8 @@ constexpr TensorCorePlan kTensorCorePlans[2] = {
 constexpr const TensorCorePlan& tensor_core_plan(int head_dim) { return kTensorCorePlans[head_dim == 64 ? 0 : 1]; }
 
 void transpose_plan(const moba_b200_problem& p, int* chunk_rows, int* chunks, int* scatter_warps);
+
+constexpr int kBlockKeys = 128;              // keys of a column of the tensor-core kernels
 
 // ---- scheduling: columns are dispatched as work items of at most chunk_tiles tiles ----
 // Sizes are fixed functions of the problem record, so that the caller can allocate the
@@ -187,17 +191,21 @@ static inline size_t sched_dkv_scratch_bytes(const moba_b200_problem& p) {
 }
 
 // One pair of a column's list. Inside the whole-op entry points, where no caller looks at the
-// index, the pairs are packed into eight bytes {query position, query head << 8 | slot}, so that
-// building and reading the list moves one word per pair: `row_indices` then points at those and
-// `head_indices` is NULL.
-struct PairEntry { int row, head, slot; };
+// index, the pairs are packed into eight bytes {query position, query head << 12 | part << 8 |
+// slot}, so that building and reading the list moves one word per pair: `row_indices` then points
+// at those and `head_indices` is NULL.
+// `part`: with blocks finer than 128 keys the tensor-core kernels work on columns of 128 keys,
+// each of 128 / block_size blocks, and a pair names the block of its column it is for.
+struct PairEntry { int row, head, slot, part; };
+__host__ __device__ __forceinline__ int pack_pair(int head, int part, int slot) { return (head << 12) | (part << 8) | slot; }
 __host__ __device__ __forceinline__ bool packed_pairs(const moba_b200_index& ix) { return ix.head_indices == nullptr; }
 __device__ __forceinline__ PairEntry load_pair(const moba_b200_index& ix, size_t at) {
   PairEntry e;
   if (packed_pairs(ix)) {
     const int2 v = __ldg(reinterpret_cast<const int2*>(ix.row_indices) + at);
-    e.row = v.x; e.head = v.y >> 8; e.slot = v.y & 0xff;
+    e.row = v.x; e.head = v.y >> 12; e.part = (v.y >> 8) & 15; e.slot = v.y & 0xff;
   } else {
+    e.part = 0;
     e.row = __ldg(ix.row_indices + at); e.head = __ldg(ix.head_indices + at); e.slot = __ldg(ix.slot_of_pair + at);
   }
   return e;
@@ -218,7 +226,7 @@ __device__ __forceinline__ RawPair fetch_pair(const moba_b200_index& ix, size_t 
   return r;
 }
 __device__ __forceinline__ PairEntry pair_of(const moba_b200_index& ix, const RawPair& r) {
-  return packed_pairs(ix) ? PairEntry{r.a, r.b >> 8, r.b & 0xff} : PairEntry{r.a, r.b, r.c};
+  return packed_pairs(ix) ? PairEntry{r.a, r.b >> 12, r.b & 0xff, (r.b >> 8) & 15} : PairEntry{r.a, r.b, r.c, 0};
 }
 
 // One work item as the kernels see it.
@@ -242,7 +250,7 @@ __device__ __forceinline__ bool load_work_item(WorkItem& w, const moba_b200_inde
 }
 
 // ---- stage launchers (defined one per .cu file) -----------------------------
-int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell,
+int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell, float* norms,
                 cudaStream_t st);
 // `lse_fill` (may be NULL): the partial log-sum-exps, set to -inf where a slot names no block.
 int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* kbar,
@@ -250,16 +258,20 @@ int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* 
 int launch_gate_sm100(const moba_b200_problem& p, const void* q, const void* kbar,
                       const int32_t* cu, int32_t* block_idx, float* lse_fill, cudaStream_t st);
 bool gate_sm100_supported(const moba_b200_problem& p);
+// The exact gate on tensor cores: selections of the portable (float64) gate, for 16-bit inputs.
+int launch_gate_exact_sm100(const moba_b200_problem& p, const void* q, const void* kbar, const float* norms, const int32_t* cu,
+                            int32_t* block_idx, float* lse_fill, cudaStream_t st);
+bool gate_exact_sm100_supported(const moba_b200_problem& p);
 
 size_t transpose_scratch_bytes(const moba_b200_problem& p);
 int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                      int32_t* col_nnz, int32_t* col_offsets, int32_t* order, int32_t* rows,
-                     int32_t* heads, int32_t* slots, int2* entries, int32_t* work_items, void* scratch, size_t scratch_bytes,
-                     cudaStream_t st);
+                     int32_t* heads, int32_t* slots, int2* entries, int part_shift, int32_t* work_items, void* scratch,
+                     size_t scratch_bytes, cudaStream_t st);
 bool transpose_small_supported(const moba_b200_problem& p);
 int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu, int32_t* col_nnz,
-                           int32_t* col_offsets, int32_t* order, int2* entries, int32_t* work_items, int32_t* slot_counter,
-                           cudaStream_t st);
+                           int32_t* col_offsets, int32_t* order, int2* entries, int part_shift, int32_t* work_items,
+                           int32_t* slot_counter, cudaStream_t st);
 
 int launch_transpose_noalloc(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                              int32_t* col_nnz, int32_t* col_offsets, int32_t* order, int32_t* rows,
@@ -271,7 +283,7 @@ int launch_fwd_portable(const moba_b200_problem& p, const void* q, const void* k
                         float* part_lse, cudaStream_t st);
 int launch_fwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const moba_b200_index& ix, const int32_t* cu, void* part_o,
-                     float* part_lse, cudaStream_t st);
+                     float* part_lse, int part_keys, cudaStream_t st);
 bool fwd_sm100_supported(const moba_b200_problem& p);
 int launch_merge(const moba_b200_problem& p, const void* part_o, const float* part_lse,
                  void* out, float* lse, cudaStream_t st);
@@ -285,7 +297,7 @@ int launch_bwd_portable(const moba_b200_problem& p, const void* q, const void* k
 int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const void* dout, const float* lse, const float* delta,
                      const moba_b200_index& ix, const int32_t* cu, void* dq_part, float* dkv_scratch,
-                     void* dk, void* dv, cudaStream_t st);
+                     void* dk, void* dv, int part_keys, cudaStream_t st);
 bool bwd_sm100_supported(const moba_b200_problem& p);
 int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const float* part_lse,
                      void* dq, cudaStream_t st);

@@ -23,7 +23,7 @@ namespace moba {
 template <typename T>
 __global__ void __launch_bounds__(128)
 pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restrict__ kbar,
-            int packed, int tokens, int hkv, int d, int bs, int nb, int* __restrict__ zero_cell) {
+            int packed, int tokens, int hkv, int d, int bs, int nb, int* __restrict__ zero_cell, float* __restrict__ norms) {
   pdl_trigger();
   pdl_wait();
   if (zero_cell != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_cell = 0;
@@ -40,6 +40,7 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
   if (lo >= sp.len) {                            // padded slot of a short packed sequence
     if (threadIdx.x < d) dst[threadIdx.x] = Elem<T>::from_f(0.f);
     for (int i = threadIdx.x + 128; i < d; i += 128) dst[i] = Elem<T>::from_f(0.f);
+    if (norms != nullptr && threadIdx.x == 0) norms[(size_t)kv_row * nb + blk] = 0.f;
     return;
   }
   const int hi = min(lo + bs, sp.len);
@@ -77,16 +78,28 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
   for (int e = 0; e < EPV; ++e) red[threadIdx.x * EPV + e] = acc[e];
   __syncthreads();
   const float occ = (float)(hi - lo);
+  float square = 0.f;
   for (int i = threadIdx.x; i < d; i += 128) {
     double s = 0.0;
     for (int g = 0; g < groups; ++g) s += red[g * d + i];       // thread g * vpr + i / EPV, element i % EPV
     const float total = Elem<T>::round_f((float)s);
-    dst[i] = Elem<T>::from_f(__fdiv_rn(total, occ));
+    const T mean = Elem<T>::from_f(__fdiv_rn(total, occ));
+    dst[i] = mean;
+    square = fmaf(Elem<T>::to_f(mean), Elem<T>::to_f(mean), square);
   }
+  if (norms == nullptr) return;
+  // the block mean's length, for the error bound of the exact gate
+  __shared__ float part[4];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) square += __shfl_xor_sync(0xffffffffu, square, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = square;
+  __syncthreads();
+  if (threadIdx.x == 0) norms[(size_t)kv_row * nb + blk] = sqrtf(part[0] + part[1] + part[2] + part[3]);
 }
 
-// `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from.
-int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell,
+// `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from; `norms`
+// (may be NULL): the length of every block mean, [n_seq, Hkv, num_blocks].
+int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell, float* norms,
                 cudaStream_t st) {
   KernelTimer timer__("pool_kernel", st);
   const int epv = 16 / (int)dtype_size(p.dtype);
@@ -99,7 +112,7 @@ int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, vo
   const unsigned grid = (unsigned)ctas;
 #define MOBA_POOL(T)                                                                                   \
   MOBA_CUDA_OK(launch_chained(pool_kernel<T>, grid, 128, 0, st, (const T*)k, cu, (T*)kbar, p.packed, p.tokens, \
-                              p.kv_heads, p.head_dim, p.block_size, p.num_blocks, zero_cell))
+                              p.kv_heads, p.head_dim, p.block_size, p.num_blocks, zero_cell, norms))
   if (p.dtype == MOBA_B200_F32) MOBA_POOL(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_POOL(__nv_bfloat16);
   else MOBA_POOL(__half);

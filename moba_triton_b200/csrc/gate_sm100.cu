@@ -26,6 +26,13 @@
 // At the end of a unit the two warpgroups' lists are merged and each thread emits
 // its ids plus the own block, ascending, -1 padded.
 //
+// EXACT: the same kernel where the portable gate used to run (other block sizes that divide 128,
+// more than eight ranked blocks): its selections are those of exact scores, bit for bit. The
+// tensor-core sum is off by at most `err` (a bound from the lengths of the query and of the block
+// means), so the entry test is loosened by err, and a candidate whose rounding to the input dtype
+// depends on that error is scored again in float64 by its whole warp before it is ranked: about
+// one candidate in forty. With blocks finer than the tile a row's candidates end at its own block.
+//
 // Scores are float32 tensor-core sums rounded to the input dtype; the portable
 // gate rounds the exact sum. The two differ only when a float32 partial sum
 // straddles a rounding boundary of the input dtype.
@@ -128,6 +135,7 @@ __device__ __forceinline__ int unit_of(int round) {
 
 struct Unit {
   int tile, seq, hq, row0, n_chunks, bos, len;
+  int own_lo, own_hi;       // own blocks of the tile's first and last row (equal when a block is a tile)
   int n_lo, c_hi0;          // chunks [0, n_lo) and [c_hi0, ...) of the Kbar row are visited
   int n_first;              // chunks the bounding pass scores before the ranking pass scores all
   // chunk of the Kbar row that step `s` of a pass scores
@@ -149,13 +157,15 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
   const SeqSpan sp = seq_span(cu, p.packed, u.seq, p.tokens);
   u.bos = sp.bos; u.len = sp.len;
   u.row0 = u.tile * kTile;
+  u.own_lo = u.row0 / p.block_size;
+  u.own_hi = min(u.row0 + kTile - 1, sp.len - 1) / p.block_size;
   // Candidates are blocks [0, tile); with a candidate window only [0, sinks) and
   // [tile - window, tile), so only the chunks that hold some of those are scored.
-  const int total = (p.take > 0) ? (u.tile + kTile - 1) / kTile : 0;
+  const int total = (p.take > 0) ? (u.own_hi + kTile - 1) / kTile : 0;
   if (p.gate_window <= 0) {
     u.n_lo = total; u.c_hi0 = total;
   } else {
-    const int recent0 = max(0, u.tile - p.gate_window);         // first block of the recent window
+    const int recent0 = max(0, u.own_lo - p.gate_window);         // first block of the recent window
     u.n_lo = min(total, (min(p.gate_sinks, recent0) + kTile - 1) / kTile);
     u.c_hi0 = max(u.n_lo, recent0 / kTile);
   }
@@ -164,11 +174,25 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
   return u.row0 < sp.len;
 }
 
-template <int D, typename T, int L>
+// Exact score of one (query, block) pair by a whole warp: the products of two 16-bit numbers and
+// their float64 sum carry no error, the result is rounded to float32 as everywhere in the gate.
+template <int D, typename T>
+__device__ __forceinline__ float exact_score(const T* q_row, const T* kbar_row, int lane) {
+  double acc = 0.0;
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i)
+    acc = fma((double)Elem<T>::to_f(q_row[i * 32 + lane]), (double)Elem<T>::to_f(kbar_row[i * 32 + lane]), acc);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return (float)acc;
+}
+
+template <int D, typename T, int L, bool EXACT>
 __global__ void __launch_bounds__(kThreads, 2)
 gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kb_map,
                   const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx, float* __restrict__ lse_fill,
-                  moba_b200_problem p, int n_tiles, int n_units, unsigned* error_word) {
+                  moba_b200_problem p, int n_tiles, int n_units, unsigned* error_word,
+                  const T* __restrict__ q, const T* __restrict__ kbar, const float* __restrict__ norms, int n_norms) {
   using Cfg = GateCfg<D>;
   constexpr int CAP = Cfg::kCap, STEP = Cfg::kStep;
   extern __shared__ unsigned char smem_dyn[];
@@ -207,6 +231,17 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
   tc_fence_after();
   pdl_wait();
   const uint32_t tmem = bars->tmem_base;
+  float longest_mean = 0.f;                                     // EXACT: of all block means
+  if constexpr (EXACT) {
+    __shared__ float longest[10];
+    for (int i = threadIdx.x; i < n_norms; i += kThreads) longest_mean = fmaxf(longest_mean, norms[i]);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) longest_mean = fmaxf(longest_mean, __shfl_xor_sync(0xffffffffu, longest_mean, o));
+    if (lane == 0) longest[warp] = longest_mean;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 10; ++w) longest_mean = fmaxf(longest_mean, longest[w]);
+  }
 
   // Every role walks the same units and counts the same steps: a unit of n chunks takes 2 n
   // steps (chunk `step mod n`), `gc` is the number of steps of all earlier units of this CTA,
@@ -231,27 +266,59 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
       if (ui >= n_units) continue;
       Unit u;
       if (!load_unit(u, ui, p, cu, n_tiles)) continue;
+      constexpr int NM = L <= 8 ? 8 : 16;                       // column subsets of the bounding pass: at least L
+      const int own = EXACT ? min(u.row0 + r, u.len - 1) / p.block_size : u.tile;
+      float err = 0.f;                                          // EXACT: bound of |tensor-core sum - exact score|
+      const T* q_row = nullptr;
+      if constexpr (EXACT) {
+        // D / 16 accumulation steps of 17 addends, each cut at 2^-23 of the largest: D 17/16 2^-23
+        // of a quantity that |q| |kbar| bounds; doubled.
+        q_row = q + ((size_t)(p.packed ? u.bos : (size_t)u.seq * p.tokens) + min(u.row0 + r, u.len - 1)) * ((size_t)p.q_heads * D) + (size_t)u.hq * D;
+        float square = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < D / 8; ++i) {
+          const uint4 raw = *reinterpret_cast<const uint4*>(q_row + i * 8);
+          const T* x = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) square = fmaf(Elem<T>::to_f(x[e]), Elem<T>::to_f(x[e]), square);
+        }
+        err = sqrtf(square) * longest_mean * (float)D * (17.f / 8.f) * 1.1920929e-7f;
+      }
       uint32_t best[L];
 #pragma unroll
       for (int e = 0; e < L; ++e) best[e] = 0u;                 // 0 sorts below every real key
-      float mx[8];                                              // first pass: maxima of 8 column subsets
+      float mx[NM];                                             // first pass: maxima of 8 (16) column subsets
 #pragma unroll
-      for (int e = 0; e < 8; ++e) mx[e] = -INFINITY;
+      for (int e = 0; e < NM; ++e) mx[e] = -INFINITY;
       float bar = -INFINITY;                                    // a score must exceed this to be appended
       uint32_t wa = buf0;                                       // address of the next free slot
       auto flush = [&]() {                                      // whole warp: empty the buffers into the lists
         PHASE_CLOCK(fl);
         while (__any_sync(0xffffffffu, wa != buf0)) {
           uint32_t key = 0u;
-          if (wa != buf0) {
+          uint32_t sx = 0, sy = 0;
+          const bool popped = wa != buf0;
+          if (popped) {
             wa -= kSlot;
-            uint32_t sx, sy;
             asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(sx), "=r"(sy) : "r"(wa));
-            key = make_key<T>(__uint_as_float(sx), sy);
           }
+          if constexpr (EXACT) {                                // does the rounding depend on the sum's error?
+            const float s = __uint_as_float(sx);
+            unsigned unsure = __ballot_sync(0xffffffffu, popped && round16<T>(s - err) != round16<T>(s + err));
+            while (unsure) {
+              const int who = __ffs((int)unsure) - 1;
+              unsure &= unsure - 1;
+              const uint32_t blk = __shfl_sync(0xffffffffu, sy, who);
+              const T* qr = reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(q_row), who));
+              const size_t kv_row = (size_t)u.seq * p.kv_heads + u.hq / group;
+              const float exact = exact_score<D, T>(qr, kbar + (kv_row * p.num_blocks + blk) * (size_t)D, lane);
+              if (lane == who) sx = __float_as_uint(exact);
+            }
+          }
+          if (popped) key = make_key<T>(__uint_as_float(sx), sy);
           list_offer<L>(best, key);
         }
-        bar = fmaxf(bar, entry_bar<T>(best[L - 1]));
+        bar = fmaxf(bar, entry_bar<T>(best[L - 1]) - err);
         PHASE_ADD(wc, 4, fl);                                   // flushes (also counted in their phase)
       };
       PHASE_ADD(wc, 1, ph);                                     // unit set-up
@@ -263,11 +330,11 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           // The L-th largest of the eight subset maxima: at least L candidates reach it.
           float lo1 = INFINITY, lo2 = INFINITY;                 // smallest and second smallest
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
+          for (int e = 0; e < NM; ++e) {
             lo2 = fminf(lo2, fmaxf(lo1, mx[e]));
             lo1 = fminf(lo1, mx[e]);
           }
-          bar = one_step_below<T>(L >= 8 ? lo1 : lo2);
+          bar = one_step_below<T>((L >= 8 ? lo1 : lo2) - err) - err;
         }
         const bool s_ok = mbar_wait(&bars->s_full[st], (gidx >> 1) & 1u, wc, 9);
         tc_fence_after();
@@ -282,18 +349,18 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           if (h == 1) { tc_fence_before(); mbar_arrive_warp(&bars->s_free[st]); }   // the scores are in registers
           // which of these 32 blocks are candidates of the tile: all, none, or some
           const int g0 = c0 + h * 32;
-          const bool none = g0 >= u.tile || (p.gate_window > 0 && g0 >= p.gate_sinks && g0 + 32 <= u.tile - p.gate_window);
+          const bool none = g0 >= u.own_hi || (p.gate_window > 0 && g0 >= p.gate_sinks && g0 + 32 <= u.own_lo - p.gate_window);
           if (!run || none) continue;
-          const bool all = g0 + 32 <= u.tile &&
-                           (p.gate_window <= 0 || g0 + 32 <= p.gate_sinks || g0 >= u.tile - p.gate_window);
+          const bool all = g0 + 32 <= u.own_lo &&
+                           (p.gate_window <= 0 || g0 + 32 <= p.gate_sinks || g0 >= u.own_hi - p.gate_window);
           if (!all) {
 #pragma unroll
             for (int k = 0; k < 32; ++k)
-              if (!gate_candidate(p, g0 + k, u.tile)) v[k] = 0xff800000u;   // -inf: never passes
+              if (!gate_candidate(p, g0 + k, own)) v[k] = 0xff800000u;   // -inf: never passes
           }
           if (!second) {
 #pragma unroll
-            for (int k = 0; k < 32; ++k) mx[k & 7] = fmaxf(mx[k & 7], __uint_as_float(v[k]));
+            for (int k = 0; k < 32; ++k) mx[k & (NM - 1)] = fmaxf(mx[k & (NM - 1)], __uint_as_float(v[k]));
             continue;
           }
           const uint32_t col0 = (uint32_t)(c0 + h * 32);
@@ -354,7 +421,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           for (int f = 0; f < L; ++f) rank += (ids[f] < ids[e]) ? 1 : 0;
           dst[rank] = ids[e];
         }
-        if (p.always_current) dst[kept++] = u.tile;             // the own block is past every candidate
+        if (p.always_current) dst[kept++] = own;                // the own block is past every candidate
         for (int e = kept; e < p.slots; ++e) {
           dst[e] = -1;
           if (lse_fill != nullptr) lse_fill[dst_at + e] = -INFINITY;   // the slot's partial will not be written
@@ -448,10 +515,11 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 }
 
 
-template <int D, typename T, int L>
+template <int D, typename T, int L, bool EXACT>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& qm, const CUtensorMap& km, const int32_t* cu,
-               int32_t* block_idx, float* lse_fill, unsigned* err, cudaStream_t st) {
-  auto kern = gate_sm100_kernel<D, T, L>;
+               int32_t* block_idx, float* lse_fill, unsigned* err, const void* q, const void* kbar, const float* norms,
+               cudaStream_t st) {
+  auto kern = gate_sm100_kernel<D, T, L, EXACT>;
   static SmemLimit limit;
   if (int rc = raise_smem_limit(limit, (const void*)kern, GateCfg<D>::kSmem)) return rc;
   const int n_tiles = (p.max_seqlen + kTile - 1) / kTile;
@@ -459,7 +527,7 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& qm, const CUtensor
   const int sms = sm_count();
   const int grid = (int)(n_units < 2LL * sms ? n_units : 2LL * sms);
   MOBA_CUDA_OK(launch_chained(kern, grid, kThreads, GateCfg<D>::kSmem, st, qm, km, cu, block_idx, lse_fill, p, n_tiles,
-                              (int)n_units, err));
+                              (int)n_units, err, (const T*)q, (const T*)kbar, norms, p.n_seq * p.kv_heads * p.num_blocks));
   return MOBA_B200_OK;
 }
 
@@ -486,8 +554,38 @@ int launch_gate_sm100(const moba_b200_problem& p, const void* q, const void* kba
   rc = encode_kbar_map_impl(&km, kbar, (uint64_t)p.n_seq * p.kv_heads, p.num_blocks, p.head_dim);
   if (rc) return rc;
   const bool bf = p.dtype == MOBA_B200_BF16;
-#define GO(D, T) return (p.take <= 7) ? launch_one<D, T, 7>(p, qm, km, cu, block_idx, lse_fill, err, st) \
-                                      : launch_one<D, T, 8>(p, qm, km, cu, block_idx, lse_fill, err, st)
+#define GO(D, T) return (p.take <= 7) ? launch_one<D, T, 7, false>(p, qm, km, cu, block_idx, lse_fill, err, q, kbar, nullptr, st) \
+                                      : launch_one<D, T, 8, false>(p, qm, km, cu, block_idx, lse_fill, err, q, kbar, nullptr, st)
+  if (p.head_dim == 64) { if (bf) GO(64, __nv_bfloat16); else GO(64, __half); }
+  if (bf) GO(128, __nv_bfloat16); else GO(128, __half);
+#undef GO
+}
+
+// Block sizes that divide the tile of 128 queries; as many ranked blocks as the per-thread buffers
+// can exchange; a candidate window keeps the portable kernel.
+bool gate_exact_sm100_supported(const moba_b200_problem& p) {
+  return (p.dtype == MOBA_B200_BF16 || p.dtype == MOBA_B200_F16) && p.block_size >= 16 && kTile % p.block_size == 0 &&
+         (p.head_dim == 64 || p.head_dim == 128) && p.take <= (p.head_dim == 64 ? 16 : 12) && p.gate_window == 0 &&
+         p.num_blocks <= 0xFFFF && (long long)p.batch * p.tokens < 0x7fffffffLL &&
+         (long long)p.n_seq * p.kv_heads * p.num_blocks < 0x7fffffffLL &&
+         (long long)((p.max_seqlen + 127) / 128) * p.n_seq * p.q_heads < 0x7fffffffLL;
+}
+
+int launch_gate_exact_sm100(const moba_b200_problem& p, const void* q, const void* kbar, const float* norms, const int32_t* cu,
+                            int32_t* block_idx, float* lse_fill, cudaStream_t st) {
+  KernelTimer timer__("gate_exact_sm100_kernel", st);
+  unsigned* err = device_error_word();
+  if (err == nullptr) { set_error("gate: no device error word"); return MOBA_B200_ECUDA; }
+  CUtensorMap qm, km;
+  int rc = encode_rows_map(&qm, q, (uint64_t)p.batch * p.tokens, p.q_heads, p.head_dim, 128);
+  if (rc) return rc;
+  rc = encode_kbar_map_impl(&km, kbar, (uint64_t)p.n_seq * p.kv_heads, p.num_blocks, p.head_dim);
+  if (rc) return rc;
+  const bool bf = p.dtype == MOBA_B200_BF16;
+#define GO(D, T)                                                                                                      \
+  return p.take <= 8    ? launch_one<D, T, 8, true>(p, qm, km, cu, block_idx, lse_fill, err, q, kbar, norms, st)     \
+         : p.take <= 12 ? launch_one<D, T, 12, true>(p, qm, km, cu, block_idx, lse_fill, err, q, kbar, norms, st)    \
+                        : launch_one<D, T, D == 64 ? 16 : 12, true>(p, qm, km, cu, block_idx, lse_fill, err, q, kbar, norms, st)
   if (p.head_dim == 64) { if (bf) GO(64, __nv_bfloat16); else GO(64, __half); }
   if (bf) GO(128, __nv_bfloat16); else GO(128, __half);
 #undef GO

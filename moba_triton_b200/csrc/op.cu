@@ -29,13 +29,36 @@ moba_b200_problem with_cut(const moba_b200_problem& p0) {
   return p;
 }
 
+// Blocks of 16, 32 or 64 keys on the tensor-core kernels, whose columns are 128 keys: a column
+// then holds 128 / block_size blocks, its list the pairs of all of them, and the kernels mask a
+// pair to its own block. Half of the scores of a tile (three quarters, ...) are computed for
+// nothing, at many times the rate of the CUDA-core kernels that took these sizes before
+// (2 x 8192 tokens, 4 heads of 128, blocks of 64: forward 2.2 ms, backward 6.1 ms there). Only
+// where the library chooses the kernels: a caller who asks for a family gets it.
+struct Columns {
+  moba_b200_problem p;       // the problem in columns of the attention kernels
+  int part_keys, part_shift; // keys per block, log2 of the blocks per column
+};
+Columns columns_of(const moba_b200_problem& p) {
+  Columns c{p, kBlockKeys, 0};
+  if (p.path != MOBA_B200_PATH_AUTO || p.block_size >= kBlockKeys || kBlockKeys % p.block_size || p.gate_window != 0) return c;
+  moba_b200_problem w = p;
+  w.block_size = kBlockKeys;
+  w.num_blocks = (p.max_seqlen + kBlockKeys - 1) / kBlockKeys;
+  if (!fwd_sm100_supported(w) || !bwd_sm100_supported(w)) return c;
+  c.p = w;
+  c.part_keys = p.block_size;
+  while ((p.block_size << c.part_shift) < kBlockKeys) ++c.part_shift;
+  return c;
+}
+
 // Byte offsets of the buffers inside the caller's workspaces.
 struct Layout {
   size_t col_nnz, col_offsets, order, items, entries, part_lse, lse, keep_bytes;      // kept for the backward
-  size_t kbar, block_idx, counter, transpose_scratch, part_o, fwd_bytes;              // forward only
+  size_t kbar, norms, block_idx, counter, transpose_scratch, part_o, fwd_bytes;              // forward only
   size_t delta, dq_part, dkv, bwd_bytes;                                              // backward only
 };
-Layout layout_of(const moba_b200_problem& p) {
+Layout layout_of(const moba_b200_problem& gate, const moba_b200_problem& p) {
   Layout l;
   const size_t rows = (size_t)p.n_seq * p.kv_heads, nb = p.num_blocks;
   const size_t pairs = (size_t)p.batch * p.q_heads * p.tokens * p.slots;
@@ -52,7 +75,8 @@ Layout layout_of(const moba_b200_problem& p) {
   l.keep_bytes = at;
   at = 0;
   const size_t part_size = p.part_f32 ? 4 : dtype_size(p.dtype);
-  l.kbar = take(rows * nb * p.head_dim * dtype_size(p.dtype));
+  l.kbar = take(rows * gate.num_blocks * p.head_dim * dtype_size(p.dtype));
+  l.norms = take(rows * gate.num_blocks * 4);
   l.block_idx = take(pairs * 4);
   l.counter = take(16);
   l.transpose_scratch = take(transpose_small_supported(p) ? 16 : transpose_scratch_bytes(p));
@@ -82,7 +106,7 @@ moba_b200_index index_in(const moba_b200_problem& p, const Layout& l, unsigned c
 int check_op(const moba_b200_problem* p) {
   MOBA_TRY(check_problem(p));
   if (p->win_rows > 0) { set_error("the whole-op entry points take no query window"); return MOBA_B200_EUNSUPPORTED; }
-  if (p->q_heads >= 1 << 23) { set_error("%d query heads do not fit a packed index entry", p->q_heads); return MOBA_B200_EUNSUPPORTED; }
+  if (p->q_heads >= 1 << 19) { set_error("%d query heads do not fit a packed index entry", p->q_heads); return MOBA_B200_EUNSUPPORTED; }
   if (sched_items_per_row(*p) > 0x7fffffffLL || sched_part_slots(*p) > 0x7fffffffLL) {
     set_error("chunk_tiles %d cuts the problem into too many work items", sched_chunk_tiles(*p));
     return MOBA_B200_EUNSUPPORTED;
@@ -99,7 +123,8 @@ extern "C" {
 
 int moba_b200_op_workspace(const moba_b200_problem* p0, size_t* keep_bytes, size_t* forward_bytes, size_t* backward_bytes) {
   MOBA_TRY(check_op(p0));
-  const Layout l = layout_of(with_cut(*p0));
+  const moba_b200_problem gate = with_cut(*p0);
+  const Layout l = layout_of(gate, columns_of(gate).p);
   if (keep_bytes) *keep_bytes = l.keep_bytes;
   if (forward_bytes) *forward_bytes = l.fwd_bytes;
   if (backward_bytes) *backward_bytes = l.bwd_bytes;
@@ -112,12 +137,14 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   MOBA_TRY(need(q, "q")); MOBA_TRY(need(k, "k")); MOBA_TRY(need(v, "v")); MOBA_TRY(need(out, "out"));
   MOBA_TRY(need(keep_ws, "keep_ws")); MOBA_TRY(need(forward_ws, "forward_ws"));
   if (p0->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
-  const moba_b200_problem p = with_cut(*p0);
-  const int gate_path = pick(p, gate_sm100_supported(p), "gate"), fwd_path = pick(p, fwd_sm100_supported(p), "forward");
+  const moba_b200_problem gate = with_cut(*p0);
+  const Columns columns = columns_of(gate);
+  const moba_b200_problem& p = columns.p;
+  const int gate_path = pick(gate, gate_sm100_supported(gate), "gate"), fwd_path = pick(p, fwd_sm100_supported(p), "forward");
   if (gate_path < 0) return gate_path;
   if (fwd_path < 0) return fwd_path;
   cudaStream_t st = (cudaStream_t)stream;
-  const Layout l = layout_of(p);
+  const Layout l = layout_of(gate, p);
   unsigned char* keep = static_cast<unsigned char*>(keep_ws);
   unsigned char* tmp = static_cast<unsigned char*>(forward_ws);
   const moba_b200_index ix = index_in(p, l, keep);
@@ -129,17 +156,22 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   int32_t* col_nnz = const_cast<int32_t*>(ix.col_nnz);
   int32_t* col_offsets = const_cast<int32_t*>(ix.col_offsets);
   int32_t* items = const_cast<int32_t*>(ix.work_items);
-  MOBA_TRY(launch_pool(p, k, cu_seqlens, kbar, counter, st));
-  if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(p, q, kbar, cu_seqlens, block_idx, part_lse, st));
-  else MOBA_TRY(launch_gate_portable(p, q, kbar, cu_seqlens, block_idx, part_lse, st));
+  // Where the portable gate would run by the library's choice, its selections come from the exact
+  // tensor-core gate if that covers the problem.
+  const bool exact_gate = gate_path == MOBA_B200_PATH_PORTABLE && gate.path == MOBA_B200_PATH_AUTO && gate_exact_sm100_supported(gate);
+  float* norms = reinterpret_cast<float*>(tmp + l.norms);
+  MOBA_TRY(launch_pool(gate, k, cu_seqlens, kbar, counter, exact_gate ? norms : nullptr, st));
+  if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
+  else if (exact_gate) MOBA_TRY(launch_gate_exact_sm100(gate, q, kbar, norms, cu_seqlens, block_idx, part_lse, st));
+  else MOBA_TRY(launch_gate_portable(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
   int2* entries = reinterpret_cast<int2*>(const_cast<int32_t*>(ix.row_indices));
   int32_t* order = const_cast<int32_t*>(ix.order);
   if (transpose_small_supported(p))
-    MOBA_TRY(launch_transpose_small(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, entries, items, counter, st));
+    MOBA_TRY(launch_transpose_small(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, entries, columns.part_shift, items, counter, st));
   else
-    MOBA_TRY(launch_transpose(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, nullptr, nullptr, nullptr, entries, items,
+    MOBA_TRY(launch_transpose(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, nullptr, nullptr, nullptr, entries, columns.part_shift, items,
                               tmp + l.transpose_scratch, transpose_scratch_bytes(p), st));
-  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu_seqlens, part_o, part_lse, st));
+  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu_seqlens, part_o, part_lse, columns.part_keys, st));
   else MOBA_TRY(launch_fwd_portable(p, q, k, v, ix, cu_seqlens, part_o, part_lse, st));
   return launch_merge(p, part_o, part_lse, out, want_lse ? reinterpret_cast<float*>(keep + l.lse) : nullptr, st);
 }
@@ -152,11 +184,13 @@ int moba_b200_op_backward(const moba_b200_problem* p0, const void* q, const void
   MOBA_TRY(need(dout, "dout")); MOBA_TRY(need(dq, "dq")); MOBA_TRY(need(dk, "dk")); MOBA_TRY(need(dv, "dv"));
   MOBA_TRY(need(keep_ws, "keep_ws")); MOBA_TRY(need(backward_ws, "backward_ws"));
   if (p0->packed) MOBA_TRY(need(cu_seqlens, "cu_seqlens"));
-  const moba_b200_problem p = with_cut(*p0);
+  const moba_b200_problem gate = with_cut(*p0);
+  const Columns columns = columns_of(gate);
+  const moba_b200_problem& p = columns.p;
   const int path = pick(p, bwd_sm100_supported(p), "backward");
   if (path < 0) return path;
   cudaStream_t st = (cudaStream_t)stream;
-  const Layout l = layout_of(p);
+  const Layout l = layout_of(gate, p);
   unsigned char* keep = const_cast<unsigned char*>(static_cast<const unsigned char*>(keep_ws));
   unsigned char* tmp = static_cast<unsigned char*>(backward_ws);
   const moba_b200_index ix = index_in(p, l, keep);
@@ -166,7 +200,7 @@ int moba_b200_op_backward(const moba_b200_problem* p0, const void* q, const void
   void* dq_part = tmp + l.dq_part;
   MOBA_TRY(launch_delta(p, out, dout, delta, st));
   if (path == MOBA_B200_PATH_TCGEN05)
-    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, st));
+    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, columns.part_keys, st));
   else
     MOBA_TRY(launch_bwd_portable(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, dk, dv, st));
   return launch_dq_reduce(p, dq_part, part_lse, dq, st);

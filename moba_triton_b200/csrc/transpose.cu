@@ -54,7 +54,7 @@ __device__ __forceinline__ size_t block_idx_row(const moba_b200_problem& p, int 
 
 __global__ void __launch_bounds__(256)
 count_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu,
-             int32_t* __restrict__ tile_counts, int32_t* __restrict__ slot_counter, moba_b200_problem p, int R, int C) {
+             int32_t* __restrict__ tile_counts, int32_t* __restrict__ slot_counter, moba_b200_problem p, int part_shift, int R, int C) {
   extern __shared__ int hist[];
   pdl_trigger();
   pdl_wait();
@@ -73,7 +73,7 @@ count_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ 
   const int w_lo = max(0, p.win_begin - row0), w_hi = min(rows, (p.win_rows > 0 ? p.win_begin + p.win_rows : sp.len) - row0);
   const int n = max(w_lo, w_hi) * p.slots;
   for (int e = w_lo * p.slots + threadIdx.x; e < n; e += 256) {
-    const int blk = src[e];
+    const int blk = src[e] >> part_shift;
     if (blk >= 0 && blk < nb_lim) atomicAdd(&hist[blk], 1);
   }
   __syncthreads();
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(32 * W)
 scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu,
                const int32_t* __restrict__ tile_prefix, const int32_t* __restrict__ col_offsets,
                int32_t* __restrict__ rows_out, int32_t* __restrict__ heads_out,
-               int32_t* __restrict__ slots_out, int2* __restrict__ entries_out, moba_b200_problem p, int R, int C,
+               int32_t* __restrict__ slots_out, int2* __restrict__ entries_out, moba_b200_problem p, int part_shift, int R, int C,
                long long capacity) {
   extern __shared__ int cursor_all[];                        // [W][nb_lim]
   pdl_trigger();
@@ -397,7 +397,7 @@ scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict_
   for (int i = threadIdx.x; i < W * nb_lim; i += 32 * W) cursor_all[i] = 0;
   __syncthreads();
   for (int e = lane; e < n; e += 32) {
-    const int blk = src[e];
+    const int blk = src[e] >> part_shift;
     if (blk >= 0 && blk < nb_lim) atomicAdd(&cursor[blk], 1);
   }
   __syncthreads();
@@ -439,7 +439,7 @@ scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict_
     for (int j = 0; j < kBatch; ++j) {
       const int e = e0 + j * 32 + lane;
       if (e0 + j * 32 >= n) break;                         // warp-uniform
-      const int blk = cur[j];
+      const int blk = cur[j] >> part_shift;
       const bool valid = blk >= 0 && blk < nb_lim;
       const int key = valid ? blk : (0x40000000 + lane);
       const unsigned same = __match_any_sync(0xffffffffu, key);
@@ -453,7 +453,7 @@ scatter_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict_
         if (dst < capacity) {
           const int row = (int)((unsigned)e / (unsigned)p.slots), slot = e - row * p.slots;
           if constexpr (PACKED) {
-            eo[dst] = make_int2(first_row + row, (hq << 8) | slot);
+            eo[dst] = make_int2(first_row + row, pack_pair(hq, cur[j] & ((1 << part_shift) - 1), slot));
           } else {
             ro[dst] = first_row + row;
             ho[dst] = hq;
@@ -480,21 +480,22 @@ void transpose_plan(const moba_b200_problem& p, int* chunk_rows, int* chunks, in
 template <int W, bool PACKED>
 static int launch_scatter(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                           const int32_t* tiles, const int32_t* col_offsets, int32_t* rows, int32_t* heads,
-                          int32_t* slots, int2* entries, const TransposeGeom& g, long long capacity, cudaStream_t st) {
+                          int32_t* slots, int2* entries, int part_shift, const TransposeGeom& g, long long capacity, cudaStream_t st) {
   const size_t smem = (size_t)W * p.num_blocks * sizeof(int);
   static SmemLimit limit;
   if (int rc = raise_smem_limit(limit, (const void*)scatter_kernel<W, PACKED>, smem)) return rc;
   const long long ctas = (long long)g.chunks * p.n_seq * p.q_heads;
   MOBA_CUDA_OK(launch_chained(scatter_kernel<W, PACKED>, (unsigned)ctas, 32 * W, smem, st, block_idx, cu, tiles, col_offsets,
-                              rows, heads, slots, entries, p, g.chunk_rows, g.chunks, capacity));
+                              rows, heads, slots, entries, p, part_shift, g.chunk_rows, g.chunks, capacity));
   return MOBA_B200_OK;
 }
 
-// `entries` non-null: packed pairs, and rows / heads / slots are not written.
+// `entries` non-null: packed pairs, and rows / heads / slots are not written. `part_shift`: the
+// block ids are those of blocks 2^part_shift times finer than the columns of `p`.
 int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu,
                      int32_t* col_nnz, int32_t* col_offsets, int32_t* order, int32_t* rows,
-                     int32_t* heads, int32_t* slots, int2* entries, int32_t* work_items, void* scratch, size_t scratch_bytes,
-                     cudaStream_t st) {
+                     int32_t* heads, int32_t* slots, int2* entries, int part_shift, int32_t* work_items, void* scratch,
+                     size_t scratch_bytes, cudaStream_t st) {
   const TransposeGeom g = transpose_geom(p);
   if (scratch_bytes < transpose_scratch_bytes(p)) {
     set_error("transpose: scratch has %zu bytes, needs %zu", scratch_bytes,
@@ -525,7 +526,7 @@ int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const
   if (int rc = raise_smem_limit(count_limit, (const void*)count_kernel, hist_bytes)) return rc;
   if (int rc = raise_smem_limit(order_limit, (const void*)offsets_order_kernel, hist_bytes)) return rc;
   { KernelTimer t__("count_kernel", st);
-  MOBA_CUDA_OK(launch_chained(count_kernel, (unsigned)row_ctas, 256, hist_bytes, st, block_idx, cu, tiles, slot_counter, p,
+  MOBA_CUDA_OK(launch_chained(count_kernel, (unsigned)row_ctas, 256, hist_bytes, st, block_idx, cu, tiles, slot_counter, p, part_shift,
                               g.chunk_rows, g.chunks)); }
   { KernelTimer t__("colscan_kernel", st);
   const unsigned per_row = (unsigned)((p.num_blocks + 3) / 4);
@@ -543,8 +544,8 @@ int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const
   KernelTimer t__("scatter_kernel", st);
   const int w = scatter_warps_for(p);
 #define MOBA_SCATTER(W) \
-  return entries != nullptr ? launch_scatter<W, true>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, entries, g, capacity, st) \
-                            : launch_scatter<W, false>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, entries, g, capacity, st)
+  return entries != nullptr ? launch_scatter<W, true>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, entries, part_shift, g, capacity, st) \
+                            : launch_scatter<W, false>(p, block_idx, cu, tiles, col_offsets, rows, heads, slots, entries, part_shift, g, capacity, st)
   if (w == 8) MOBA_SCATTER(8);
   if (w == 4) MOBA_SCATTER(4);
   MOBA_SCATTER(1);
@@ -583,7 +584,7 @@ __device__ __forceinline__ int ld_cluster_i32(const int* mine, uint32_t rank) {
 __global__ void __launch_bounds__(kSmallThreads, 1)
 transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu, int32_t* __restrict__ col_nnz,
                        int32_t* __restrict__ col_offsets, int32_t* __restrict__ order, int2* __restrict__ entries, int4* __restrict__ items,
-                       int32_t* __restrict__ slot_counter, moba_b200_problem p, long long capacity, int items_per_row,
+                       int32_t* __restrict__ slot_counter, moba_b200_problem p, int part_shift, long long capacity, int items_per_row,
                        int tc, int slot_cap, unsigned* error_word) {
   extern __shared__ int cursor_all[];                        // [warps][nb]
   __shared__ int totals[kSmallBlocks];                       // this CTA's pairs per column (read by its peers)
@@ -620,7 +621,7 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
   __syncthreads();
   for (int e = lane; e < n; e += 32) {
     int g, row, slot;
-    const int blk = __ldg(entry(e, g, row, slot));
+    const int blk = __ldg(entry(e, g, row, slot)) >> part_shift;
     if (blk >= 0 && blk < nb) atomicAdd(&cursor[blk], 1);
   }
   __syncthreads();
@@ -675,8 +676,9 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
   const unsigned lt = (1u << lane) - 1u;
   for (int e0 = 0; e0 < n; e0 += 32) {
     const int e = e0 + lane;
-    int g = 0, row = 0, slot = 0, blk = -1;
-    if (e < n) blk = __ldg(entry(e, g, row, slot));
+    int g = 0, row = 0, slot = 0, id = -1;
+    if (e < n) id = __ldg(entry(e, g, row, slot));
+    const int blk = id >> part_shift;
     const bool valid = blk >= 0 && blk < nb;
     const unsigned same = __match_any_sync(0xffffffffu, valid ? blk : (0x40000000 + lane));
     int base = 0;
@@ -686,7 +688,7 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
     __syncwarp();
     if (valid) {
       const long long dst = (long long)base_s[blk] + base + __popc(same & lt);
-      if (dst < capacity) eo[dst] = make_int2(sp.bos + row, ((kvh * group + g) << 8) | slot);
+      if (dst < capacity) eo[dst] = make_int2(sp.bos + row, pack_pair(kvh * group + g, id & ((1 << part_shift) - 1), slot));
     }
   }
   if (rank == kSmallCluster - 1)
@@ -702,8 +704,8 @@ bool transpose_small_supported(const moba_b200_problem& p) {
 
 // `slot_counter` must hold zero.
 int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu, int32_t* col_nnz,
-                           int32_t* col_offsets, int32_t* order, int2* entries, int32_t* work_items, int32_t* slot_counter,
-                           cudaStream_t st) {
+                           int32_t* col_offsets, int32_t* order, int2* entries, int part_shift, int32_t* work_items,
+                           int32_t* slot_counter, cudaStream_t st) {
   KernelTimer t__("transpose_small_kernel", st);
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("transpose: no device error word"); return MOBA_B200_ECUDA; }
@@ -720,7 +722,7 @@ int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx,
   cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;
   const long long capacity = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
   MOBA_CUDA_OK(cudaLaunchKernelEx(&cfg, transpose_small_kernel, block_idx, cu, col_nnz, col_offsets, order, entries,
-                                  reinterpret_cast<int4*>(work_items), slot_counter, p, capacity, (int)sched_items_per_row(p),
+                                  reinterpret_cast<int4*>(work_items), slot_counter, p, part_shift, capacity, (int)sched_items_per_row(p),
                                   sched_chunk_tiles(p), (int)sched_part_slots(p), err));
   return MOBA_B200_OK;
 }
@@ -776,7 +778,7 @@ int launch_transpose_noalloc(const moba_b200_problem& p, const int32_t* block_id
   // Nothing in the array has to be cleared by the caller: the count pass writes every entry
   // the scan pass reads and resets the slot counter, so the previous call's contents are
   // simply overwritten.
-  return launch_transpose(p, block_idx, cu, col_nnz, col_offsets, order, rows, heads, slots, nullptr, work_items, scratch,
+  return launch_transpose(p, block_idx, cu, col_nnz, col_offsets, order, rows, heads, slots, nullptr, 0, work_items, scratch,
                           kStaticScratchBytes, st);
 }
 
