@@ -174,6 +174,190 @@ fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
   }
 }
 
+// ---------------------------------------------------------------------------
+// float32 attention, blocks of 64 to 128 keys, head_dim 64 or 128. One CTA per tile of 128 pairs
+// of a work item: S is a 128 x 128 x D product and O a 128 x D x 128 one, each thread holding 8 x 8
+// (8 x D/16) of them in registers and reading operands as 16-byte pieces, so that an FMA costs a
+// sixteenth of a shared-memory load; P takes the place of Q and K between the two. The sums run in
+// the order of the portable kernel (over the head dim, over the keys), in float32 FMAs. It is bound
+// by the FMA pipe: 16 400 clocks of a tile at head_dim 64, of 18 000 to 20 000. The portable kernel,
+// with one CTA per column, a load per FMA and as many as 32 tiles in one CTA, took 1.3 ms for
+// [1,4096,4,64].
+// ---------------------------------------------------------------------------
+constexpr int kF32Tile = 128;
+template <int D> struct F32Cfg {
+  static constexpr int kRow = D + 4;                        // floats per row of Q, K, V: rows of 16 lanes on different banks
+  static constexpr int kPRow = kF32Tile + 4;
+  static constexpr int kQk = 2 * kF32Tile * kRow;           // Q and K, then P
+  static constexpr int kFloats = (kQk > kF32Tile * kPRow ? kQk : kF32Tile * kPRow) + kF32Tile * kRow;
+  static constexpr int kSmem = kFloats * 4;
+};
+
+template <int D>
+__global__ void __launch_bounds__(256, D == 64 ? 2 : 1)
+fwd_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+               moba_b200_index ix, const int32_t* __restrict__ cu, float* __restrict__ part_o,
+               float* __restrict__ part_lse, moba_b200_problem p, int n_kv_rows) {
+  using Cfg = F32Cfg<D>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int row_s[kF32Tile], dst_s[kF32Tile];          // query position; row of the partial buffers (-1: none)
+  float* Qs = reinterpret_cast<float*>(smem_raw);           // [128][D + 4]
+  float* Ks = Qs + kF32Tile * Cfg::kRow;
+  float* Ps = Qs;                                           // [128][128 + 4]
+  float* Vs = Qs + Cfg::kFloats - kF32Tile * Cfg::kRow;
+  pdl_wait();
+  const int kv_row = (int)(blockIdx.x % n_kv_rows), seq = kv_row / p.kv_heads, kvh = kv_row % p.kv_heads;
+  WorkItem w;
+  if (!load_work_item(w, ix, ix.col_nnz + (size_t)kv_row * p.num_blocks, kv_row, (int)(blockIdx.x / n_kv_rows))) return;
+  const int n = min(kF32Tile, w.n - (int)blockIdx.y * kF32Tile);
+  const SeqSpan sp = seq_span(cu, p.packed, seq, p.tokens);
+  const size_t b = p.packed ? 0 : (size_t)seq;
+  const int key0 = sp.bos + w.blk * p.block_size;
+  const int keys = min(p.block_size, sp.bos + sp.len - key0);
+  if (n <= 0 || keys <= 0) return;
+  const size_t list0 = (size_t)kv_row * ix.capacity + ix.col_offsets[(size_t)kv_row * (p.num_blocks + 1) + w.blk] + w.first +
+                       (size_t)blockIdx.y * kF32Tile;
+  constexpr int CPR = D / 4;                                // 16-byte pieces per row
+  for (int i = threadIdx.x; i < kF32Tile * CPR; i += 256) {
+    const int j = i / CPR, c = (i % CPR) * 4;
+    float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+    if (j < keys) {
+      const size_t src = ((b * p.tokens + key0 + j) * p.kv_heads + kvh) * (size_t)D + c;
+      kv = __ldg(reinterpret_cast<const float4*>(k + src));
+      vv = __ldg(reinterpret_cast<const float4*>(v + src));
+    }
+    *reinterpret_cast<float4*>(Ks + j * Cfg::kRow + c) = kv;
+    *reinterpret_cast<float4*>(Vs + j * Cfg::kRow + c) = vv;
+  }
+  for (int i = threadIdx.x; i < kF32Tile * CPR; i += 256) {
+    const int j = i / CPR, c = (i % CPR) * 4;
+    float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
+    int row = -1, dst = -1;
+    if (j < n) {
+      const PairEntry e = load_pair(ix, list0 + j);
+      row = e.row;
+      dst = (int)(part_row(p, b, e.head, e.row) * (size_t)p.slots + e.slot);
+      qv = __ldg(reinterpret_cast<const float4*>(q + ((b * p.tokens + e.row) * p.q_heads + e.head) * (size_t)D + c));
+    }
+    if (c == 0) { row_s[j] = row; dst_s[j] = dst; }
+    *reinterpret_cast<float4*>(Qs + j * Cfg::kRow + c) = qv;
+  }
+  __syncthreads();
+
+  // thread (ty, tx): queries ty + 16 i, keys tx + 16 j
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float s[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[i][j] = 0.f;
+#pragma unroll 1
+  for (int c = 0; c < D; c += 4) {
+    float4 a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4*>(Qs + (ty + 16 * i) * Cfg::kRow + c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 bk = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * Cfg::kRow + c);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        s[i][j] = fmaf(a[i].x, bk.x, s[i][j]);
+        s[i][j] = fmaf(a[i].y, bk.y, s[i][j]);
+        s[i][j] = fmaf(a[i].z, bk.z, s[i][j]);
+        s[i][j] = fmaf(a[i].w, bk.w, s[i][j]);
+      }
+    }
+  }
+  __syncthreads();                                          // Q and K have been read
+  const float scale = rsqrtf((float)D) * kLog2e;
+  float l[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = row_s[ty + 16 * i];
+    const int last = p.causal ? min(keys - 1, row - key0) : keys - 1;       // a dead query (row -1) keeps nothing
+    float m = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      s[i][j] = (row >= 0 && tx + 16 * j <= last) ? s[i][j] * scale : -INFINITY;
+      m = fmaxf(m, s[i][j]);
+    }
+#pragma unroll
+    for (int o = 8; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float pe = s[i][j] == -INFINITY ? 0.f : exp2f(s[i][j] - m);
+      sum += pe;
+      Ps[(ty + 16 * i) * Cfg::kPRow + tx + 16 * j] = pe;
+    }
+#pragma unroll
+    for (int o = 8; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    l[i] = sum;
+    if (tx == 0 && row >= 0) part_lse[dst_s[ty + 16 * i]] = m + log2f(sum);
+  }
+  __syncthreads();
+
+  // thread (ty, tx): queries ty + 16 i, head-dim columns 4 tx + 64 h
+  constexpr int H = D / 64;
+  float4 o[8][H];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int h = 0; h < H; ++h) o[i][h] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int j = 0; j < kF32Tile; j += 4) {
+    float4 pr[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) pr[i] = *reinterpret_cast<const float4*>(Ps + (ty + 16 * i) * Cfg::kPRow + j);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const float4 vv = *reinterpret_cast<const float4*>(Vs + (j + u) * Cfg::kRow + h * 64 + tx * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float pe = u == 0 ? pr[i].x : u == 1 ? pr[i].y : u == 2 ? pr[i].z : pr[i].w;
+          o[i][h].x = fmaf(pe, vv.x, o[i][h].x);
+          o[i][h].y = fmaf(pe, vv.y, o[i][h].y);
+          o[i][h].z = fmaf(pe, vv.z, o[i][h].z);
+          o[i][h].w = fmaf(pe, vv.w, o[i][h].w);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int dst = dst_s[ty + 16 * i];
+    if (dst < 0) continue;
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+      *reinterpret_cast<float4*>(part_o + (size_t)dst * D + h * 64 + tx * 4) =
+          make_float4(o[i][h].x / l[i], o[i][h].y / l[i], o[i][h].z / l[i], o[i][h].w / l[i]);
+  }
+}
+
+template <int D>
+static int launch_fwd_f32(const moba_b200_problem& p, const void* q, const void* k, const void* v, const moba_b200_index& ix,
+                          const int32_t* cu, void* part_o, float* part_lse, cudaStream_t st) {
+  static SmemLimit limit;
+  if (int rc = raise_smem_limit(limit, (const void*)fwd_f32_kernel<D>, F32Cfg<D>::kSmem)) return rc;
+  const int n_kv_rows = p.n_seq * p.kv_heads;
+  const long long items = (long long)ix.items_per_row * n_kv_rows;
+  // no item has more tiles than the longest possible column
+  const long long longest = ((long long)(p.q_heads / p.kv_heads) * window_rows_of_seq(p) + kF32Tile - 1) / kF32Tile;
+  const long long tiles = longest < ix.chunk_tiles ? longest : ix.chunk_tiles;
+  if (items > 0x7fffffffLL || tiles > 65535) { set_error("float32 forward: %lld items of %lld tiles exceed the grid", items, tiles); return MOBA_B200_EUNSUPPORTED; }
+  MOBA_CUDA_OK(launch_chained(fwd_f32_kernel<D>, dim3((unsigned)items, (unsigned)tiles), 256, F32Cfg<D>::kSmem, st, (const float*)q,
+                              (const float*)k, (const float*)v, ix, cu, (float*)part_o, part_lse, p, n_kv_rows));
+  return MOBA_B200_OK;
+}
+// Pairs in one slot of the partial buffers are numbered in 31 bits; the index must carry work items.
+static bool fwd_f32_supported(const moba_b200_problem& p, const moba_b200_index& ix) {
+  return p.dtype == MOBA_B200_F32 && p.path == MOBA_B200_PATH_AUTO && p.block_size >= 64 && p.block_size <= kF32Tile &&
+         (p.head_dim == 64 || p.head_dim == 128) && ix.work_items != nullptr && ix.chunk_tiles > 0 && ix.chunk_tiles <= 65535 &&
+         (long long)p.batch * p.q_heads * window_rows(p) * p.slots < 0x7fffffffLL;
+}
+
 static size_t fwd_portable_smem(const moba_b200_problem& p) {
   const size_t d = p.head_dim, bs = p.block_size;
   return sizeof(float) * (bs * (d + 1) + bs * d + kFwdWarps * kFwdRows * (d + bs));
@@ -182,6 +366,11 @@ static size_t fwd_portable_smem(const moba_b200_problem& p) {
 int launch_fwd_portable(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                         const moba_b200_index& ix, const int32_t* cu, void* part_o,
                         float* part_lse, cudaStream_t st) {
+  if (fwd_f32_supported(p, ix)) {
+    KernelTimer timer__("fwd_f32_kernel", st);
+    return p.head_dim == 64 ? launch_fwd_f32<64>(p, q, k, v, ix, cu, part_o, part_lse, st)
+                            : launch_fwd_f32<128>(p, q, k, v, ix, cu, part_o, part_lse, st);
+  }
   KernelTimer timer__("fwd_portable_kernel", st);
   const size_t smem = fwd_portable_smem(p);
   if (smem > 220 * 1024) {
