@@ -343,13 +343,14 @@ int moba_b200_bwd(const moba_b200_problem* p, const void* q, const void* k, cons
   const int path = pick(*p, bwd_sm100_supported(*p), "backward");
   if (path < 0) return path;
   cudaStream_t st = (cudaStream_t)stream;
+  bool reduces = false;
   MOBA_TRY(launch_delta(*p, out, dout, delta, st));
   if (path == MOBA_B200_PATH_TCGEN05)
     MOBA_TRY(launch_bwd_sm100(*p, q, k, v, dout, lse, delta, *index, cu_seqlens, dq_part,
-                              static_cast<float*>(dkv_scratch), dk, dv, kBlockKeys, st));
+                              static_cast<float*>(dkv_scratch), dk, dv, kBlockKeys, &reduces, st));
   else
     MOBA_TRY(launch_bwd_portable(*p, q, k, v, dout, lse, delta, *index, cu_seqlens, dq_part, dk, dv, st));
-  return launch_dq_reduce(*p, dq_part, part_lse, dq, st);
+  return launch_dq_reduce(*p, dq_part, part_lse, dq, reduces, st);
 }
 
 int moba_b200_pack_index(const void* mask, int mask_elem_bytes, int batch, int seq_len, int32_t* dest,

@@ -270,16 +270,19 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 dq_reduce_kernel(const T* __restrict__ dq_part, const float* __restrict__ part_lse,
                  T* __restrict__ dq, int tokens, int q_heads, int d, int slots,
-                 int win_begin, int win_rows) {
+                 int win_begin, int win_rows, bool beside) {
+  // `beside`: the kernel before is the dK/dV reduction. It lets this one start when its own wait is
+  // over, i.e. when the partials are complete, and the two run side by side; this kernel waits for
+  // it at its end, so that whatever follows finds both done.
   pdl_trigger();
-  pdl_wait();
+  if (!beside) pdl_wait();
   // grid (row groups of one (batch entry, head), heads, batch): no division anywhere
   constexpr int EPV = 16 / sizeof(T);
   const unsigned tpr = (unsigned)(d / EPV);       // threads per row, a power of two
   const unsigned gid = blockIdx.x * 256u + threadIdx.x;
   const unsigned row = gid / tpr;                 // row of the window
   const int c = (int)(gid % tpr);
-  if (row >= (unsigned)win_rows) return;
+  if (row >= (unsigned)win_rows) { if (beside) pdl_wait(); return; }
   const size_t h = blockIdx.y, b = blockIdx.z;
   const size_t r = (b * q_heads + h) * win_rows + row;   // head-major row (b, h, s) of the partials
   float acc[EPV];
@@ -311,10 +314,11 @@ dq_reduce_kernel(const T* __restrict__ dq_part, const float* __restrict__ part_l
   for (int e = 0; e < EPV; ++e) packed_out[e] = Elem<T>::from_f(acc[e]);
   *reinterpret_cast<uint4*>(dq + ((b * tokens + s) * q_heads + h) * (size_t)d + c * EPV) =
       *reinterpret_cast<const uint4*>(packed_out);
+  if (beside) pdl_wait();
 }
 
 int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const float* part_lse,
-                     void* dq, cudaStream_t st) {
+                     void* dq, bool beside, cudaStream_t st) {
   KernelTimer timer__("dq_reduce_kernel", st);
   const int epv = 16 / (int)dtype_size(p.dtype);
   const int tpr = p.head_dim / epv;
@@ -327,7 +331,7 @@ int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const floa
   const dim3 blocks((unsigned)((threads + 255) / 256), (unsigned)p.q_heads, (unsigned)p.batch);
 #define MOBA_DQR(T) \
   MOBA_CUDA_OK(launch_chained(dq_reduce_kernel<T>, blocks, 256, 0, st, (const T*)dq_part, part_lse, (T*)dq, p.tokens, p.q_heads, \
-                              p.head_dim, p.slots, p.win_begin, window_rows(p)))
+                              p.head_dim, p.slots, p.win_begin, window_rows(p), beside))
   if (p.dtype == MOBA_B200_F32) MOBA_DQR(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_DQR(__nv_bfloat16);
   else MOBA_DQR(__half);

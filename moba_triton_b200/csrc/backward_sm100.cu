@@ -783,8 +783,8 @@ dkv_reduce_kernel(const float* __restrict__ dkv_scratch, moba_b200_index ix, con
                   T* __restrict__ dk, T* __restrict__ dv, moba_b200_problem p, int ctas_per_row) {
   __shared__ int4 found[256];
   __shared__ int n_found;
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();                                         // behind the wait: the dQ sums may start beside this kernel
   const int kv_row = blockIdx.x / ctas_per_row;
   const int j = (blockIdx.x % ctas_per_row) * 256 + threadIdx.x;
   if (threadIdx.x == 0) n_found = 0;
@@ -814,20 +814,32 @@ dkv_reduce_kernel(const float* __restrict__ dkv_scratch, moba_b200_index ix, con
     const int key0 = sp.bos + col.x * kTile;
     const int keys = min(kTile, sp.bos + sp.len - key0);
     constexpr int V4 = D / 4;                              // float4 per row
-    constexpr int kAhead = 4;                              // elements per thread in flight
+    constexpr int kAhead = 2, kDeep = 4;                   // elements per thread and partials of each in flight
     for (int i0 = (int)blockIdx.z * 256 * kAhead + threadIdx.x; i0 < 2 * kTile * V4; i0 += 256 * kAhead * (int)gridDim.z) {
       float4 acc[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int c = 0; c < n_chunks; ++c) {
+      for (int c0 = 0; c0 < n_chunks; c0 += kDeep) {       // loads first, then the sums in item order
+        float4 x[kDeep][kAhead];
 #pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-          const int i = i0 + u * 256;
-          const int which = i / (kTile * V4), row = (i / V4) % kTile, c4 = i % V4;
-          if (row >= keys) continue;
-          const float4 x = __ldcs(reinterpret_cast<const float4*>(
-              dkv_scratch + (((size_t)(col.w + c) * 2 + which) * kTile + row) * D) + c4);
-          acc[u].x += x.x; acc[u].y += x.y; acc[u].z += x.z; acc[u].w += x.w;
+        for (int d = 0; d < kDeep; ++d) {
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) {
+            const int i = i0 + u * 256;
+            const int which = i / (kTile * V4), row = (i / V4) % kTile, c4 = i % V4;
+            x[d][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row >= keys || which > 1 || c0 + d >= n_chunks) continue;
+            x[d][u] = __ldcs(reinterpret_cast<const float4*>(
+                dkv_scratch + (((size_t)(col.w + c0 + d) * 2 + which) * kTile + row) * D) + c4);
+          }
+        }
+#pragma unroll
+        for (int d = 0; d < kDeep; ++d) {
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) {
+            if (c0 + d >= n_chunks) continue;
+            acc[u].x += x[d][u].x; acc[u].y += x[d][u].y; acc[u].z += x[d][u].z; acc[u].w += x[d][u].w;
+          }
         }
       }
 #pragma unroll
@@ -848,7 +860,7 @@ dkv_reduce_kernel(const float* __restrict__ dkv_scratch, moba_b200_index ix, con
 template <int D, typename T>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensorMap& vm, const CUtensorMap& qm,
                const CUtensorMap& gm, const float* lse, const float* delta, const moba_b200_index& ix,
-               const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, int n_items, unsigned* err,
+               const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, bool* reduces, int n_items, unsigned* err,
                cudaStream_t st) {
   const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
@@ -864,6 +876,7 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
   // (a query lists a column once per block in it)
   const long long longest = ((long long)(p.q_heads / p.kv_heads) * window_rows_of_seq(p) * (kTile / part_keys) + kTile - 1) / kTile;
   if (longest <= ix.chunk_tiles) return MOBA_B200_OK;
+  *reduces = true;
   KernelTimer timer__("dkv_reduce_kernel", st);
   const int ctas_per_row = (ix.items_per_row + 255) / 256;
   // z: the 2 x 128 x D sums of a column in parts of at least 1024 float4; fewer parts when the
@@ -887,7 +900,9 @@ bool bwd_sm100_supported(const moba_b200_problem& p) {
 
 int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const void* dout, const float* lse, const float* delta, const moba_b200_index& ix,
-                     const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, cudaStream_t st) {
+                     const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, bool* reduces,
+                     cudaStream_t st) {
+  *reduces = false;
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("backward: no device error word"); return MOBA_B200_ECUDA; }
   CUtensorMap km, vm;
@@ -911,11 +926,11 @@ int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, c
   const int n_items = (int)n_items_ll;
   const bool bf = p.dtype == MOBA_B200_BF16;
   if (p.head_dim == 64) {
-    if (bf) return launch_one<64, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
-    return launch_one<64, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
+    if (bf) return launch_one<64, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
+    return launch_one<64, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
   }
-  if (bf) return launch_one<128, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
-  return launch_one<128, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, n_items, err, st);
+  if (bf) return launch_one<128, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
+  return launch_one<128, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
 }
 
 }  // namespace moba

@@ -297,10 +297,11 @@ int launch_bwd_portable(const moba_b200_problem& p, const void* q, const void* k
 int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const void* dout, const float* lse, const float* delta,
                      const moba_b200_index& ix, const int32_t* cu, void* dq_part, float* dkv_scratch,
-                     void* dk, void* dv, int part_keys, cudaStream_t st);
+                     void* dk, void* dv, int part_keys, bool* reduces, cudaStream_t st);
 bool bwd_sm100_supported(const moba_b200_problem& p);
+// `beside`: the kernel before is the dK/dV reduction, which this one does not depend on.
 int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const float* part_lse,
-                     void* dq, cudaStream_t st);
+                     void* dq, bool beside, cudaStream_t st);
 
 // ---- argument checks and kernel-family selection, shared by the entry points (api.cu) ----
 int check_problem(const moba_b200_problem* p);

@@ -15,10 +15,10 @@ constexpr size_t kAlign = 256;
 inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 
 // The cut of the work items. The policy of the scheduler has a floor of eight tiles, which is
-// right when the rows fill the GPU; a problem of at most four tiles per SM is all tail, and
-// finer items spread it over the SMs (their dK/dV partials then fit the L2). The size depends on
-// the length of a row only, so that running the KV heads of such a problem in several passes
-// cuts them the same way and gives the same bits.
+// right when the rows fill the GPU; a problem of at most sixteen tiles per SM is mostly tail, and
+// finer items spread it over the SMs (their dK/dV partials then fit the L2). Up to four tiles per
+// SM the size depends on the length of a row only, so that running the KV heads of such a problem
+// in several passes cuts them the same way and gives the same bits.
 moba_b200_problem with_cut(const moba_b200_problem& p0) {
   moba_b200_problem p = p0;
   if (p.chunk_tiles > 0) return p;
@@ -26,6 +26,7 @@ moba_b200_problem with_cut(const moba_b200_problem& p0) {
   const long long tiles = (sched_pairs_bound(p) + 127) / 128;
   const long long row_tiles = ((long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots + 127) / 128;
   if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = row_tiles <= 128 ? 2 : 4;
+  else if (tiles <= 16LL * kSchedSMs) p.chunk_tiles = 4;
   return p;
 }
 
@@ -198,12 +199,13 @@ int moba_b200_op_backward(const moba_b200_problem* p0, const void* q, const void
   const float* lse = reinterpret_cast<const float*>(keep + l.lse);
   float* delta = reinterpret_cast<float*>(tmp + l.delta);
   void* dq_part = tmp + l.dq_part;
+  bool reduces = false;
   MOBA_TRY(launch_delta(p, out, dout, delta, st));
   if (path == MOBA_B200_PATH_TCGEN05)
-    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, columns.part_keys, st));
+    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, columns.part_keys, &reduces, st));
   else
     MOBA_TRY(launch_bwd_portable(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, dk, dv, st));
-  return launch_dq_reduce(p, dq_part, part_lse, dq, st);
+  return launch_dq_reduce(p, dq_part, part_lse, dq, reduces, st);
 }
 
 }  // extern "C"

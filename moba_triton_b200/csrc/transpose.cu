@@ -204,13 +204,12 @@ offsets_order_kernel(const int32_t* __restrict__ col_nnz, int32_t* __restrict__ 
 constexpr int kMaxCut = 2048;
 // The row's work items, by all 1024 threads of a CTA. `nnz` and `ord` are the row's column
 // totals and dispatch order (global or shared memory), `out` its stretch of the item table.
-template <int MAXCUT>
 __device__ void write_work_items(const int32_t* nnz, const int32_t* ord, int4* out, int32_t* slot_counter, int nb,
                                  int items_per_row, int tc, int slot_cap, unsigned* error_word) {
   __shared__ long long warp_sums[32];
   __shared__ long long carry_s;
   __shared__ int base_s;
-  __shared__ int rem_s[MAXCUT], rank_s[MAXCUT], sorted_s[MAXCUT], slot_s[MAXCUT];
+  __shared__ int rem_s[kMaxCut], rank_s[kMaxCut], sorted_s[kMaxCut], slot_s[kMaxCut];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   auto tiles_of = [&](int r) { return (nnz[ord[r]] + 127) / 128; };
   auto chunks_of = [&](int r, int& blk, int& tiles) {
@@ -264,7 +263,7 @@ __device__ void write_work_items(const int32_t* nnz, const int32_t* ord, int4* o
     else atomicOr(error_word, 2u);
   };
 
-  if (n_cut <= MAXCUT) {
+  if (n_cut <= kMaxCut) {
     const int n_full = row_slots - n_cut;                   // pieces of exactly tc tiles: they lead the list
     // the cut columns: full pieces in column order, the last piece's size and slot for later
     for (int r0 = 0; r0 < n_cut; r0 += 1024) {
@@ -349,7 +348,7 @@ work_items_kernel(const int32_t* __restrict__ col_nnz, const int32_t* __restrict
                   unsigned* error_word) {
   pdl_trigger();
   pdl_wait();
-  write_work_items<kMaxCut>(col_nnz + (size_t)blockIdx.x * nb, order + (size_t)blockIdx.x * nb,
+  write_work_items(col_nnz + (size_t)blockIdx.x * nb, order + (size_t)blockIdx.x * nb,
                             items + (size_t)blockIdx.x * items_per_row, slot_counter, nb, items_per_row, tc, slot_cap,
                             error_word);
 }
@@ -556,11 +555,13 @@ int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const
 // Short rows: the five passes in one launch, one cluster of CTAs per (sequence, kv head).
 //
 // The cluster's warps cut the row's queries, in (query head, position) order, into consecutive
-// runs. A histogram per warp, a scan over the warps of a CTA and one exchange of column totals
-// over distributed shared memory give every warp its own cursors; the walk that follows is the
-// one of scatter_kernel, so the order inside a column is the same. The last CTA of the cluster
-// also ranks the columns and writes the work items. What bounds it is latency: two reads of the
-// selections (the second from the L2), two cluster barriers and the walk.
+// runs, and hold the block ids of their run in registers. A histogram per warp, a scan over the
+// warps of a CTA and one exchange of column totals over distributed shared memory give every warp
+// its own cursors; the walk that follows is the one of scatter_kernel, so the order inside a column
+// is the same. The last CTA of the cluster also writes the work items: the pieces of `tc` tiles
+// first, then the last piece of every column by size (the same balance as write_work_items, whose
+// block-wide passes cost this kernel a quarter of its time). What bounds it is latency: one read
+// of the selections, two cluster barriers and the walk.
 // Lines: up to kSmallBlocks columns, because one CTA ranks them all against one another, and up
 // to kSmallPairs pairs per row and cluster; a longer row leaves too much to one cluster.
 // ---------------------------------------------------------------------------
@@ -581,19 +582,23 @@ __device__ __forceinline__ int ld_cluster_i32(const int* mine, uint32_t rank) {
   return v;
 }
 
+// K: block ids per lane, an upper bound of the run's entries / 32
+template <int K>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu, int32_t* __restrict__ col_nnz,
                        int32_t* __restrict__ col_offsets, int32_t* __restrict__ order, int2* __restrict__ entries, int4* __restrict__ items,
-                       int32_t* __restrict__ slot_counter, moba_b200_problem p, int part_shift, long long capacity, int items_per_row,
-                       int tc, int slot_cap, unsigned* error_word) {
+                       int32_t* __restrict__ slot_counter, moba_b200_problem p, unsigned slots_recip, int part_shift, long long capacity,
+                       int items_per_row, int tc, int slot_cap, unsigned* error_word) {
   extern __shared__ int cursor_all[];                        // [warps][nb]
   __shared__ int totals[kSmallBlocks];                       // this CTA's pairs per column (read by its peers)
-  __shared__ int nnz_s[kSmallBlocks], base_s[kSmallBlocks], ord_s[kSmallBlocks];
-  __shared__ int warp_sums[32];
+  __shared__ int base_s[kSmallBlocks];
+  __shared__ int2 size_s[kSmallBlocks];                      // pairs of a column, tiles of its last piece
+  __shared__ int warp_sums[32], warp_pieces[32], slot_base;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = p.num_blocks;
   const uint32_t rank = cluster_rank();
   for (int i = threadIdx.x; i < kSmallWarps * nb; i += kSmallThreads) cursor_all[i] = 0;
+  __syncthreads();
   pdl_trigger();
   pdl_wait();
   const int kv_row = (int)(blockIdx.x / kSmallCluster);
@@ -602,36 +607,50 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
   const SeqSpan sp = seq_span(cu, p.packed, seq, p.tokens);
   const unsigned slots = (unsigned)p.slots;
   // this warp's run of queries, in (head, position) order
-  const long long total_q = (long long)group * sp.len;
-  const int per_warp = (int)((total_q + kSmallCluster * kSmallWarps - 1) / (kSmallCluster * kSmallWarps));
-  const long long q_lo = min(total_q, (long long)((int)rank * kSmallWarps + warp) * per_warp), q_hi = min(total_q, q_lo + per_warp);
-  const int n = (int)(q_hi - q_lo) * (int)slots;
+  const unsigned total_q = (unsigned)group * (unsigned)sp.len;
+  const unsigned per_warp = (total_q + kSmallCluster * kSmallWarps - 1) / (kSmallCluster * kSmallWarps);
+  const unsigned q_lo = min(total_q, (rank * kSmallWarps + warp) * per_warp), q_hi = min(total_q, q_lo + per_warp);
+  const int n = (int)((q_hi - q_lo) * slots);
   int g0 = 0, r0 = (int)q_lo;                                // head and position of the run's first query
-  if (sp.len > 0) { g0 = (int)(q_lo / sp.len); r0 = (int)(q_lo - (long long)g0 * sp.len); }
+  if (sp.len > 0) { g0 = (int)(q_lo / (unsigned)sp.len); r0 = (int)(q_lo - (unsigned)g0 * (unsigned)sp.len); }
   const size_t head0 = (p.packed ? 0 : (size_t)seq * p.q_heads) + (size_t)kvh * group;
-  // entry e of the run: query, slot and where its block id is
-  auto entry = [&](int e, int& g, int& row, int& slot) -> const int32_t* {
-    const unsigned qi = (unsigned)e / slots;
-    slot = (int)((unsigned)e - qi * slots);
+  // entry e of the run: its query (head of the group, position) and slot; e < 2^16
+  auto entry = [&](int e, int& g, int& row, int& slot) {
+    const unsigned qi = slots == 1 ? (unsigned)e : __umulhi((unsigned)e, slots_recip);
+    slot = e - (int)(qi * slots);
     row = r0 + (int)qi; g = g0;
     while (row >= sp.len) { row -= sp.len; ++g; }
-    return block_idx + ((head0 + g) * p.tokens + sp.bos + row) * (size_t)slots + slot;
   };
   int* cursor = cursor_all + warp * nb;
-  __syncthreads();
-  for (int e = lane; e < n; e += 32) {
-    int g, row, slot;
-    const int blk = __ldg(entry(e, g, row, slot)) >> part_shift;
+  int id[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int e = k * 32 + lane;
+    id[k] = -1;
+    if (e < n) {
+      int g, row, slot;
+      entry(e, g, row, slot);
+      id[k] = __ldg(block_idx + ((head0 + g) * p.tokens + sp.bos + row) * (size_t)slots + slot);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int blk = id[k] >> part_shift;
     if (blk >= 0 && blk < nb) atomicAdd(&cursor[blk], 1);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += kSmallThreads) {
     int at = 0;
-#pragma unroll 8
-    for (int w = 0; w < kSmallWarps; ++w) {
-      const int t = cursor_all[w * nb + i];
-      cursor_all[w * nb + i] = at;
-      at += t;
+#pragma unroll 1
+    for (int w0 = 0; w0 < kSmallWarps; w0 += 16) {
+      int c[16];
+#pragma unroll
+      for (int w = 0; w < 16; ++w) c[w] = cursor_all[(w0 + w) * nb + i];
+#pragma unroll
+      for (int w = 0; w < 16; ++w) {
+        cursor_all[(w0 + w) * nb + i] = at;
+        at += c[w];
+      }
     }
     totals[i] = at;
   }
@@ -640,45 +659,49 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
   int mine = 0, before = 0;
   const int col = threadIdx.x;                               // nb <= kSmallBlocks < threads
   if (col < nb) {
+    int t[kSmallCluster];
+#pragma unroll
+    for (int c = 0; c < kSmallCluster; ++c) t[c] = ld_cluster_i32(&totals[col], (uint32_t)c);
 #pragma unroll
     for (int c = 0; c < kSmallCluster; ++c) {
-      const int t = ld_cluster_i32(&totals[col], (uint32_t)c);
-      mine += t;
-      before += c < (int)rank ? t : 0;
+      mine += t[c];
+      before += c < (int)rank ? t[c] : 0;
     }
-    nnz_s[col] = mine;
   }
-  int incl = mine;
+  const int tiles = (mine + 127) / 128;
+  const int pieces = tiles <= tc ? 1 : (tiles + tc - 1) / tc;   // of the column; all but the last have tc tiles
+  const int last_tiles = tiles - (pieces - 1) * tc;
+  if (col < nb) size_s[col] = make_int2(mine, last_tiles);
+  // scans over the columns: pairs; full pieces (low half) and partial slots (high half)
+  int incl = mine, cuts = col < nb ? (pieces - 1) | ((pieces > 1 ? pieces : 0) << 16) : 0, cuts_incl = cuts;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
+    const int t = __shfl_up_sync(0xffffffffu, incl, o), u = __shfl_up_sync(0xffffffffu, cuts_incl, o);
+    if (lane >= o) { incl += t; cuts_incl += u; }
   }
-  if (lane == 31) warp_sums[warp] = incl;
+  if (lane == 31) { warp_sums[warp] = incl; warp_pieces[warp] = cuts_incl; }
   __syncthreads();
-  int off = incl - mine;
-  for (int w = 0; w < warp; ++w) off += warp_sums[w];        // (warps beyond the columns add nothing to later ones)
-  if (col < nb) base_s[col] = off + before;
-  if (rank == kSmallCluster - 1) {
-    if (col < nb) {
-      col_nnz[(size_t)kv_row * nb + col] = mine;
-      col_offsets[(size_t)kv_row * (nb + 1) + col] = off;
-      if (col == nb - 1) col_offsets[(size_t)kv_row * (nb + 1) + nb] = off + mine;
-      int rk = 0;                                            // stable descending rank
-      for (int j = 0; j < nb; ++j) { const int o = nnz_s[j]; rk += (o > mine || (o == mine && j < col)) ? 1 : 0; }
-      ord_s[rk] = col;
-      order[(size_t)kv_row * nb + rk] = col;
-    }
+  int off = incl - mine, cuts_before = cuts_incl - cuts, cuts_all = 0;
+  for (int w = 0; w * 32 < nb; ++w) {
+    if (w < warp) { off += warp_sums[w]; cuts_before += warp_pieces[w]; }
+    cuts_all += warp_pieces[w];
   }
-  cluster_barrier();                                         // totals have been read; base_s and ord_s are complete
+  if (col < nb) base_s[col] = off + before;
+  const bool lister = rank == kSmallCluster - 1;
+  if (lister && threadIdx.x == 0) {
+    const int need = (int)((unsigned)cuts_all >> 16);
+    const int base = need > 0 ? atomicAdd(slot_counter, need) : 0;
+    slot_base = base;
+    if (base + need > slot_cap || (cuts_all & 0xffff) + nb > items_per_row) atomicOr(error_word, 2u);   // sizes were promised by the host
+  }
+  cluster_barrier();                                         // totals have been read; base_s is complete
 
   int2* eo = entries + (size_t)kv_row * capacity;
   const unsigned lt = (1u << lane) - 1u;
-  for (int e0 = 0; e0 < n; e0 += 32) {
-    const int e = e0 + lane;
-    int g = 0, row = 0, slot = 0, id = -1;
-    if (e < n) id = __ldg(entry(e, g, row, slot));
-    const int blk = id >> part_shift;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k * 32 >= n) break;                                  // warp-uniform
+    const int blk = id[k] >> part_shift;
     const bool valid = blk >= 0 && blk < nb;
     const unsigned same = __match_any_sync(0xffffffffu, valid ? blk : (0x40000000 + lane));
     int base = 0;
@@ -687,18 +710,48 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
     if (valid && (same & lt) == 0) cursor[blk] = base + __popc(same);
     __syncwarp();
     if (valid) {
+      int g, row, slot;
+      entry(k * 32 + lane, g, row, slot);
       const long long dst = (long long)base_s[blk] + base + __popc(same & lt);
-      if (dst < capacity) eo[dst] = make_int2(sp.bos + row, pack_pair(kvh * group + g, id & ((1 << part_shift) - 1), slot));
+      if (dst < capacity) eo[dst] = make_int2(sp.bos + row, pack_pair(kvh * group + g, id[k] & ((1 << part_shift) - 1), slot));
     }
   }
-  if (rank == kSmallCluster - 1)
-    write_work_items<kSmallBlocks>(nnz_s, ord_s, items + (size_t)kv_row * items_per_row, slot_counter, nb, items_per_row, tc,
-                                   slot_cap, error_word);
+  if (!lister) return;
+  int4* out = items + (size_t)kv_row * items_per_row;
+  const int n_full = cuts_all & 0xffff;
+  if (col < nb) {
+    col_nnz[(size_t)kv_row * nb + col] = mine;
+    col_offsets[(size_t)kv_row * (nb + 1) + col] = off;
+    if (col == nb - 1) col_offsets[(size_t)kv_row * (nb + 1) + nb] = off + mine;
+    // stable descending ranks: of the column by pairs, of its last piece by tiles
+    int by_pairs = 0, by_piece = 0;
+    for (int j = 0; j < nb; ++j) {
+      const int2 o = size_s[j];
+      by_pairs += (o.x > mine || (o.x == mine && j < col)) ? 1 : 0;
+      by_piece += (o.y > last_tiles || (o.y == last_tiles && j < col)) ? 1 : 0;
+    }
+    order[(size_t)kv_row * nb + by_pairs] = col;
+    const int full0 = cuts_before & 0xffff, slot0 = slot_base + (int)((unsigned)cuts_before >> 16);
+    auto slot_or_none = [&](int i) { return pieces > 1 && slot0 + i < slot_cap ? slot0 + i : -1; };
+    for (int i = 0; i + 1 < pieces; ++i)
+      if (full0 + i < items_per_row) out[full0 + i] = make_int4(col, i * tc, tc, slot_or_none(i));
+    if (n_full + by_piece < items_per_row) out[n_full + by_piece] = make_int4(col, (pieces - 1) * tc, last_tiles, slot_or_none(pieces - 1));
+  }
+  for (int j = n_full + nb + threadIdx.x; j < items_per_row; j += kSmallThreads) out[j] = make_int4(0, 0, 0, -2);   // padding
+}
+
+// Entries of a warp's run: at most this many per lane.
+static inline int small_ids_per_lane(const moba_b200_problem& p) {
+  const long long total_q = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen;
+  const long long per_warp = (total_q + kSmallCluster * kSmallWarps - 1) / (kSmallCluster * kSmallWarps);
+  return (int)((per_warp * p.slots + 31) / 32);
 }
 
 bool transpose_small_supported(const moba_b200_problem& p) {
   const long long row_pairs = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
-  return p.num_blocks <= kSmallBlocks && row_pairs <= kSmallPairs && p.win_rows == 0 &&
+  return p.num_blocks <= kSmallBlocks && row_pairs <= kSmallPairs && p.win_rows == 0 && small_ids_per_lane(p) <= 20 &&
+         row_pairs / (128LL * sched_chunk_tiles(p)) < 16384 &&        // two piece counts share a word
+        
          (long long)p.n_seq * p.kv_heads * kSmallCluster < 0x7fffffffLL;
 }
 
@@ -710,8 +763,11 @@ int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx,
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("transpose: no device error word"); return MOBA_B200_ECUDA; }
   const size_t smem = (size_t)kSmallWarps * p.num_blocks * sizeof(int);
-  static SmemLimit limit;
-  if (int rc = raise_smem_limit(limit, (const void*)transpose_small_kernel, smem)) return rc;
+  const int k = small_ids_per_lane(p);
+  const int which = k <= 4 ? 0 : (k <= 8 ? 1 : 2);
+  auto kern = which == 0 ? transpose_small_kernel<4> : (which == 1 ? transpose_small_kernel<8> : transpose_small_kernel<20>);
+  static SmemLimit limit[3];
+  if (int rc = raise_smem_limit(limit[which], (const void*)kern, smem)) return rc;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -721,9 +777,10 @@ int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx,
   cfg.gridDim = dim3((unsigned)(p.n_seq * p.kv_heads * kSmallCluster)); cfg.blockDim = dim3(kSmallThreads);
   cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;
   const long long capacity = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
-  MOBA_CUDA_OK(cudaLaunchKernelEx(&cfg, transpose_small_kernel, block_idx, cu, col_nnz, col_offsets, order, entries,
-                                  reinterpret_cast<int4*>(work_items), slot_counter, p, part_shift, capacity, (int)sched_items_per_row(p),
-                                  sched_chunk_tiles(p), (int)sched_part_slots(p), err));
+  const unsigned recip = (unsigned)(((1ull << 32) + p.slots - 1) / p.slots);    // e / slots for e < 2^16 and slots > 1
+  MOBA_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, block_idx, cu, col_nnz, col_offsets, order, entries,
+                                  reinterpret_cast<int4*>(work_items), slot_counter, p, recip, part_shift, capacity,
+                                  (int)sched_items_per_row(p), sched_chunk_tiles(p), (int)sched_part_slots(p), err));
   return MOBA_B200_OK;
 }
 
