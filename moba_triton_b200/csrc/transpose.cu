@@ -751,7 +751,6 @@ bool transpose_small_supported(const moba_b200_problem& p) {
   const long long row_pairs = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
   return p.num_blocks <= kSmallBlocks && row_pairs <= kSmallPairs && p.win_rows == 0 && small_ids_per_lane(p) <= 20 &&
          row_pairs / (128LL * sched_chunk_tiles(p)) < 16384 &&        // two piece counts share a word
-        
          (long long)p.n_seq * p.kv_heads * kSmallCluster < 0x7fffffffLL;
 }
 
