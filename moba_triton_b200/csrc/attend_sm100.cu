@@ -121,11 +121,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 }
 
 // Work item `item` of the launch: the items of the (sequence, kv head) rows interleaved, each
-// row's in its dispatch order (heaviest first).
+// row's in its dispatch order (heaviest first); false for padding.
 __device__ __forceinline__ bool load_column(Column& c, int item, const moba_b200_index& ix,
                                             const moba_b200_problem& p, const int32_t* cu, int n_kv_rows) {
   c.kv_row = item % n_kv_rows;
-  c.n = 0; c.keys = 0;
   WorkItem w;
   if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, item / n_kv_rows)) return false;
   c.blk = w.blk;
@@ -565,13 +564,28 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           l2_prefetch_i32(arr, (size_t)c.kv_row * ix.capacity + c.lo, c.n, index_elems);
         }
       };
-      // The next item with pairs at or after `round` (its round is returned, -1 at the end).
-      auto find = [&](Column& c, int round) {
-        for (; round * G < n_items; ++round) {
-          const int item = round * G + ((round & 1) ? (G - 1 - (int)blockIdx.x) : (int)blockIdx.x);
-          if (item < n_items && load_column(c, item, ix, p, cu, n_kv_rows)) return round;
+      // The next item with pairs; false at the end. The lanes look at 32 items at once: most of a
+      // packed batch's list is padding (every row has room for the longest sequence's items), which
+      // walked one by one took 0.15 of 1.13 ms (16 sequences of 300 to 9000 tokens, 32 heads) and
+      // 0.85 of 4.9 ms (32 of 1024 to 32768, 16 heads).
+      Column mine;
+      unsigned found = 0;
+      int round0 = 0;
+      auto next = [&](Column& c) {
+        while (found == 0) {
+          if ((long long)round0 * G >= n_items) return false;
+          const int round = round0 + lane;
+          const long long item = (long long)round * G + ((round & 1) ? (G - 1 - (int)blockIdx.x) : (int)blockIdx.x);
+          found = __ballot_sync(0xffffffffu, item < n_items && load_column(mine, (int)item, ix, p, cu, n_kv_rows));
+          round0 += 32;
         }
-        return -1;
+        const int src = __ffs(found) - 1;
+        found &= found - 1;
+        c.kv_row = __shfl_sync(0xffffffffu, mine.kv_row, src); c.blk = __shfl_sync(0xffffffffu, mine.blk, src);
+        c.n = __shfl_sync(0xffffffffu, mine.n, src); c.lo = __shfl_sync(0xffffffffu, mine.lo, src);
+        c.key0 = __shfl_sync(0xffffffffu, mine.key0, src); c.keys = __shfl_sync(0xffffffffu, mine.keys, src);
+        c.bos = __shfl_sync(0xffffffffu, mine.bos, src); c.tok0 = __shfl_sync(0xffffffffu, mine.tok0, src);
+        return true;
       };
       auto publish = [&](const Column& c, uint32_t n) {
         if (n >= 8) mbar_wait(&bars->col_free[n & 7], ((n >> 3) - 1) & 1, wc, 6);
@@ -582,14 +596,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         }
       };
       Column c, c_next;
-      int round = find(c, 0);
-      if (round >= 0) { prefetch_entries(c); publish(c, 0); }
-      while (round >= 0) {
+      bool more = next(c);
+      if (more) { prefetch_entries(c); publish(c, 0); }
+      while (more) {
         // The gather warps run ahead of the MMAs: at the last tiles of an item they are at tiles of
         // the next one, so its descriptor (and, in the L2, its index entries) must be there before
         // this item's K and V are even loaded.
-        const int round_next = find(c_next, round + 1);
-        if (round_next >= 0) { prefetch_entries(c_next); publish(c_next, it_cnt + 1); }
+        more = next(c_next);
+        if (more) { prefetch_entries(c_next); publish(c_next, it_cnt + 1); }
         if (__any_sync(0xffffffffu, *wc.abort)) break;        // no new loads once a wait gave up
         const int kvh = c.kv_row % p.kv_heads;
         const int tok = c.tok0 + c.key0;
@@ -625,7 +639,6 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         }
         ++it_cnt;
         c = c_next;
-        round = round_next;
       }
       c.n = -1;                                                 // end of the stream
       publish(c, it_cnt);

@@ -97,14 +97,13 @@ template <int D> struct Bars {
 };
 static_assert(sizeof(Bars<64>) <= BwdCfg<64>::kBarBytes && sizeof(Bars<128>) <= BwdCfg<128>::kBarBytes, "barrier block outgrew its reservation");
 
-// The next item in dispatch order: the items of the (sequence, kv head) rows interleaved, each
-// row's in its own order (heaviest first).
+// Work item `item` of the launch: the items of the (sequence, kv head) rows interleaved, each
+// row's in its dispatch order (heaviest first); false for padding.
 __device__ __forceinline__ bool load_column(Column& c, int item, const moba_b200_index& ix,
                                             const moba_b200_problem& p, const int32_t* cu, int n_kv_rows) {
   c.kv_row = item % n_kv_rows;
-  c.n = 0; c.keys = 0; c.slot = -1;
   WorkItem w;
-  if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, item / n_kv_rows)) return false;   // padding
+  if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, item / n_kv_rows)) return false;
   const int seq = c.kv_row / p.kv_heads;
   const SeqSpan sp = seq_span(cu, p.packed, seq, p.tokens);
   c.blk = w.blk;
@@ -120,9 +119,9 @@ __device__ __forceinline__ bool load_column(Column& c, int item, const moba_b200
 
 // The work list is sorted longest first; CTAs take it in alternating direction
 // (0..G-1, G-1..0, ...) so that no CTA collects the largest column of every round.
-__device__ __forceinline__ int snake_item(int round) {
+__device__ __forceinline__ long long snake_item(int round) {
   const int g = (int)gridDim.x, c = (int)blockIdx.x;
-  return round * g + ((round & 1) ? (g - 1 - c) : c);
+  return (long long)round * g + ((round & 1) ? (g - 1 - c) : c);
 }
 
 __device__ __forceinline__ float ex2(float x) {
@@ -593,27 +592,44 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       __syncwarp();
     } else if (warp == kLoadWarp) {
       // ================= work-list walker and K/V TMA loader =================
-      if (lane == 0 && sound) {
+      // All 32 lanes walk the list, lane 0 publishes and issues the loads.
+      if (sound) {
         uint32_t it = 0, n_seen = 0;
         const uint64_t keep = l2_policy_evict_last();
         const size_t index_elems = (size_t)n_kv_rows * ix.capacity;
         auto publish = [&](const Column& c) {
           if (it >= 4) mbar_wait(&bars->col_free[it & 3], ((it >> 2) - 1) & 1, wc, 10);
-          bars->cols[it & 3] = c;
-          mbar_arrive(&bars->col_full[it & 3]);
+          __syncwarp();
+          if (lane == 0) {
+            bars->cols[it & 3] = c;
+            mbar_arrive(&bars->col_full[it & 3]);
+          }
           ++it;
         };
-        // the next item at or after `round` that has something to do
-        auto find = [&](Column& c, int round) -> int {
-          for (; round * (int)gridDim.x < n_items; ++round) {
-            const int item = snake_item(round);
-            if (item < n_items && load_column(c, item, ix, p, cu, n_kv_rows)) return round;
+        // The next item that has something to do; false at the end. The lanes look at 32 items at
+        // once: most of a packed batch's list is padding.
+        Column mine;
+        unsigned found = 0;
+        int round0 = 0;
+        auto next = [&](Column& c) {
+          while (found == 0) {
+            if ((long long)round0 * gridDim.x >= n_items) return false;
+            const long long item = snake_item(round0 + lane);
+            found = __ballot_sync(0xffffffffu, item < n_items && load_column(mine, (int)item, ix, p, cu, n_kv_rows));
+            round0 += 32;
           }
-          return -1;
+          const int src = __ffs(found) - 1;
+          found &= found - 1;
+          c.kv_row = __shfl_sync(0xffffffffu, mine.kv_row, src); c.blk = __shfl_sync(0xffffffffu, mine.blk, src);
+          c.n = __shfl_sync(0xffffffffu, mine.n, src); c.lo = __shfl_sync(0xffffffffu, mine.lo, src);
+          c.keys = __shfl_sync(0xffffffffu, mine.keys, src); c.key0 = __shfl_sync(0xffffffffu, mine.key0, src);
+          c.slot = __shfl_sync(0xffffffffu, mine.slot, src); c.tok0 = __shfl_sync(0xffffffffu, mine.tok0, src);
+          return true;
         };
         // The index entries of a column are read a tile at a time; asking the L2 for them, and for
         // its K and V blocks, a column ahead saves a DRAM round trip per tile and item.
         auto prefetch = [&](const Column& c) {
+          if (c.n <= 0 || lane != 0) return;
           const size_t lo = (size_t)c.kv_row * ix.capacity + c.lo;
           if (packed_pairs(ix)) {
             l2_prefetch_i32(ix.row_indices, 2 * lo, 2 * c.n, 2 * index_elems);
@@ -628,36 +644,41 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           }
         };
         Column c, c_next;
-        int round = find(c, 0);
-        if (round >= 0 && c.n > 0) prefetch(c);
-        while (round >= 0) {
+        bool more = next(c);
+        if (more) prefetch(c);
+        while (more) {
           publish(c);
-          const int round_next = find(c_next, round + 1);
-          if (round_next >= 0 && c_next.n > 0) prefetch(c_next);
-          if (*wc.abort) break;                            // no new loads once a wait gave up
+          more = next(c_next);
+          if (more) prefetch(c_next);
+          if (__any_sync(0xffffffffu, *wc.abort)) break;   // no new loads once a wait gave up
           if (c.n > 0) {
             const int kvh = c.kv_row % p.kv_heads, tok = c.tok0 + c.key0;
             const uint32_t kb = n_seen % NKV, ku = n_seen / NKV;
             if (ku >= 1) mbar_wait(&bars->v_free[kb], (ku - 1) & 1, wc, 11);
-            mbar_expect_tx(&bars->v_full[kb], Cfg::kOperand);
-            for (int s = 0; s < Cfg::kSubs; ++s)
-              tma_load_3d_hint(sV + kb * Cfg::kOperand + s * kSub, &v_map, &bars->v_full[kb], s * 64, kvh, tok, keep);
+            if (lane == 0) {
+              mbar_expect_tx(&bars->v_full[kb], Cfg::kOperand);
+              for (int s = 0; s < Cfg::kSubs; ++s)
+                tma_load_3d_hint(sV + kb * Cfg::kOperand + s * kSub, &v_map, &bars->v_full[kb], s * 64, kvh, tok, keep);
+            }
             if (ku >= 1) mbar_wait(&bars->k_free[kb], (ku - 1) & 1, wc, 12);
-            mbar_expect_tx(&bars->k_full[kb], Cfg::kOperand);
-            for (int s = 0; s < Cfg::kSubs; ++s)
-              tma_load_3d_hint(sK + kb * Cfg::kOperand + s * kSub, &k_map, &bars->k_full[kb], s * 64, kvh, tok, keep);
+            if (lane == 0) {
+              mbar_expect_tx(&bars->k_full[kb], Cfg::kOperand);
+              for (int s = 0; s < Cfg::kSubs; ++s)
+                tma_load_3d_hint(sK + kb * Cfg::kOperand + s * kSub, &k_map, &bars->k_full[kb], s * 64, kvh, tok, keep);
+            }
             ++n_seen;
           }
           c = c_next;
-          round = round_next;
         }
         c.n = -1;
         publish(c);
         // No load may be in flight into this CTA's shared memory when it exits.
-        for (uint32_t k = 1; k <= (uint32_t)NKV && k <= n_seen; ++k) {
-          const uint32_t n = n_seen - k;
-          mbar_wait_quiet(&bars->k_full[n % NKV], (n / NKV) & 1);
-          mbar_wait_quiet(&bars->v_full[n % NKV], (n / NKV) & 1);
+        if (lane == 0) {
+          for (uint32_t k = 1; k <= (uint32_t)NKV && k <= n_seen; ++k) {
+            const uint32_t n = n_seen - k;
+            mbar_wait_quiet(&bars->k_full[n % NKV], (n / NKV) & 1);
+            mbar_wait_quiet(&bars->v_full[n % NKV], (n / NKV) & 1);
+          }
         }
       }
       __syncwarp();
