@@ -11,14 +11,19 @@
 //   select (2 x 4 warps; warpgroup w takes columns [64 w, 64 w + 64) of every chunk)
 //          tcgen05.ld, one row per thread. The first two chunks of a unit are scored twice.
 //          The first pass only keeps, per row, the maxima of eight interleaved subsets
-//          of the scores (one max per score): the L-th largest of them is a score that
-//          at least L candidates reach, so nothing below it can be selected. The second
+//          of the scores (half an instruction per score): the L-th largest of the two
+//          warpgroups' sixteen is a score that at least L candidates reach, so nothing
+//          below it can be selected. The second
 //          pass tests every score against that bound with one compare and appends the
 //          few that pass, by predicated stores, to a small per-thread buffer in shared
 //          memory; the buffer is emptied into the row's sorted register list of L keys
 //          whenever some lane of the warp is about to run out of room, which also
 //          raises the bound to the score of the list's last entry (candidates arrive
-//          in ascending block order, so an equal score never wins). A key is the score
+//          in ascending block order, so an equal score never wins), and a step under it
+//          for the row's other half. (A bar from one half's maxima let one score in seven
+//          through at first, and emptying the buffers took most of the time: 131072 queries
+//          x 4 heads 0.244 ms, with the bar of both halves 0.215; exact, 12 of 512 blocks:
+//          0.50 and 0.30.) A key is the score
 //          rounded to the input dtype and made monotone in the high half and
 //          0xFFFF - block id in the low half, so "score descending, ties to the lower
 //          id" is plain integer order. Scoring two chunks twice costs tensor-core time the
@@ -64,7 +69,7 @@ template <int D> struct GateCfg {
   static constexpr int kCap = tensor_core_plan(D).gate_slots;
   static constexpr int kStep = tensor_core_plan(D).gate_step;
   static constexpr int kBufBytes = kCap * kTile * 8;                       // per warpgroup
-  static constexpr int kSmem = 3 * kOperand + 2 * kBufBytes + 1024 + 512;  // Q + two Kbar stages + buffers
+  static constexpr int kSmem = 3 * kOperand + 2 * kBufBytes + 1024 + 512 + 2 * kTile * 4;  // Q + two Kbar stages + buffers, bars
 };
 
 struct Bars {
@@ -82,6 +87,30 @@ __device__ __forceinline__ void list_offer(uint32_t (&t)[L], uint32_t x) {
     x = min(t[i], x);
     t[i] = hi;
   }
+}
+
+// Descending order by Batcher's odd-even merge sort; N a power of two.
+template <int N>
+__device__ __forceinline__ void sort_descending(float (&a)[N]) {
+#pragma unroll
+  for (int p = 1; p < N; p <<= 1)
+#pragma unroll
+    for (int k = p; k >= 1; k >>= 1)
+#pragma unroll
+      for (int j = k % p; j + k < N; j += 2 * k)
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+            const float x = a[i + j], y = a[i + j + k];
+            a[i + j] = fmaxf(x, y);
+            a[i + j + k] = fminf(x, y);
+          }
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 template <typename T> __device__ __forceinline__ uint32_t round16(float a);
@@ -116,14 +145,17 @@ __device__ __forceinline__ float entry_bar(uint32_t key) {
 }
 
 // The largest score that is certainly below every score whose rounding to T is at least
-// round_T(m): one step of T under round_T(m), widened back to float.
+// that of `key`: one step of T under it, widened back to float.
 template <typename T>
-__device__ __forceinline__ float one_step_below(float m) {
-  if (!(m > -INFINITY)) return -INFINITY;
-  const uint32_t key = make_key<T>(m, 0u);
+__device__ __forceinline__ float one_step_below_key(uint32_t key) {
   const uint32_t mono = key >> 16;
   if (mono == 0u) return -INFINITY;
   return entry_bar<T>(((mono - 1u) << 16) | 1u);
+}
+template <typename T>
+__device__ __forceinline__ float one_step_below(float m) {
+  if (!(m > -INFINITY)) return -INFINITY;
+  return one_step_below_key<T>(make_key<T>(m, 0u));
 }
 
 // Which unit a CTA takes in its `round`-th turn: heaviest units first, alternating
@@ -148,6 +180,9 @@ struct Unit {
 // one score in ten of a later chunk passes until the first flush raises it, and scoring a long
 // row of block means twice would cost more tensor-core time than the tighter bar saves.
 constexpr int kBoundChunks = 2;
+// So few candidates go through the buffers faster than through a pass of their own (16 sequences
+// of 300 to 9000 tokens, 32 heads: 0.31 ms with a bounding pass for every unit, 0.27 without).
+constexpr int kUnboundedBlocks = 32;
 __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_problem& p, const int32_t* cu,
                                           int n_tiles) {
   const int ny = p.n_seq * p.q_heads;
@@ -170,7 +205,7 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
     u.c_hi0 = max(u.n_lo, recent0 / kTile);
   }
   u.n_chunks = u.n_lo + (total - u.c_hi0);
-  u.n_first = min(u.n_chunks, kBoundChunks);
+  u.n_first = u.own_hi > kUnboundedBlocks ? min(u.n_chunks, kBoundChunks) : 0;
   return u.row0 < sp.len;
 }
 
@@ -200,7 +235,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
   unsigned char* sQ = smem;
   unsigned char* sKb = sQ + Cfg::kOperand;                    // two stages
   unsigned char* sBuf = sKb + 2 * Cfg::kOperand;              // two warpgroups' buffers
-  Bars* bars = reinterpret_cast<Bars*>(sBuf + 2 * Cfg::kBufBytes);
+  Bars* bars = reinterpret_cast<Bars*>(sBuf + 2 * Cfg::kBufBytes + 2 * kTile * 4);   // (bars of the rows' lists in between)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int group = p.q_heads / p.kv_heads;
@@ -259,6 +294,8 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     // warpgroup 0 only ever reads and overwrites words of its own.
     const uint32_t xk0 = smem_u32(sBuf) + (uint32_t)r * 8u;
     static_assert((L + 1) / 2 <= CAP, "a list fits the slots of one thread");
+    // The bar of this row's list in either warpgroup, for the other one.
+    const uint32_t bar_mine = smem_u32(sBuf + 2 * Cfg::kBufBytes) + (uint32_t)(wg * kTile + r) * 4u, bar_other = bar_mine ^ (kTile * 4u);
     uint32_t gc = 0;
     PHASE_CLOCK(ph);
     for (int round = 0; round * (int)gridDim.x < n_units; ++round) {
@@ -319,6 +356,9 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           list_offer<L>(best, key);
         }
         bar = fmaxf(bar, entry_bar<T>(best[L - 1]) - err);
+        // to the other warpgroup, whose blocks may be the lower ones: a step less, so that it
+        // does not drop an equal score
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(bar_mine), "f"(one_step_below_key<T>(best[L - 1]) - err) : "memory");
         PHASE_ADD(wc, 4, fl);                                   // flushes (also counted in their phase)
       };
       PHASE_ADD(wc, 1, ph);                                     // unit set-up
@@ -326,15 +366,36 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         const uint32_t gidx = gc + (uint32_t)step, st = gidx & 1u;
         const bool second = step >= u.n_first;
         const int c = u.chunk_of_step(step);
-        if (step == u.n_first) {
-          // The L-th largest of the eight subset maxima: at least L candidates reach it.
-          float lo1 = INFINITY, lo2 = INFINITY;                 // smallest and second smallest
+        const bool halves = u.own_hi > kTile / 2;               // both warpgroups have candidates
+        if (step == u.n_first && u.n_first > 0 && !halves) {
+          // The L-th largest of the subset maxima: at least L candidates reach it.
+          sort_descending<NM>(mx);
+          bar = one_step_below<T>(mx[L - 1] - err) - err;
+        } else if (step == u.n_first && u.n_first > 0) {
+          // The L-th largest of both warpgroups' subset maxima.
+          // Each leaves its maxima in the (empty) buffer of its thread, in descending order; of two
+          // descending lists a and b the L-th largest is the least of max(a[i], b[L - 1 - i]).
+          sort_descending<NM>(mx);
 #pragma unroll
-          for (int e = 0; e < NM; ++e) {
-            lo2 = fminf(lo2, fmaxf(lo1, mx[e]));
-            lo1 = fminf(lo1, mx[e]);
+          for (int e = 0; e < L; ++e)
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(buf0 + (uint32_t)(e >> 1) * kSlot + (uint32_t)(e & 1) * 4u), "f"(mx[e]) : "memory");
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(bar_mine), "f"(-INFINITY) : "memory");
+          asm volatile("bar.sync 3, 256;" ::: "memory");
+          const uint32_t other0 = smem_u32(sBuf + (wg ^ 1) * Cfg::kBufBytes) + (uint32_t)r * 8u;
+          float reached = INFINITY;
+#pragma unroll
+          for (int e = 0; e < L; ++e) {
+            float o;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(o) : "r"(other0 + (uint32_t)((L - 1 - e) >> 1) * kSlot + (uint32_t)((L - 1 - e) & 1) * 4u) : "memory");
+            reached = fminf(reached, fmaxf(mx[e], o));
           }
-          bar = one_step_below<T>((L >= 8 ? lo1 : lo2) - err) - err;
+          bar = one_step_below<T>(reached - err) - err;
+          asm volatile("bar.sync 3, 256;" ::: "memory");        // both have read: the buffers may be filled
+        }
+        if (second && halves) {
+          float o;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(o) : "r"(bar_other) : "memory");
+          bar = fmaxf(bar, o);
         }
         const bool s_ok = mbar_wait(&bars->s_full[st], (gidx >> 1) & 1u, wc, 9);
         tc_fence_after();
@@ -360,7 +421,9 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           }
           if (!second) {
 #pragma unroll
-            for (int k = 0; k < 32; ++k) mx[k & (NM - 1)] = fmaxf(mx[k & (NM - 1)], __uint_as_float(v[k]));
+            for (int k = 0; k < 32; k += 2 * NM)
+#pragma unroll
+              for (int e = 0; e < NM; ++e) mx[e] = max3(mx[e], __uint_as_float(v[k + e]), __uint_as_float(v[k + NM + e]));
             continue;
           }
           const uint32_t col0 = (uint32_t)(c0 + h * 32);
