@@ -74,3 +74,27 @@ def test_finer_blocks_with_the_other_options(flags, device):
     for staged, whole in zip(*got):
         assert torch.equal(torch.isnan(staged), torch.isnan(whole))          # no own block: the first rows select nothing
         assert max_abs_error(staged.nan_to_num(), whole.nan_to_num()) <= 2e-2
+
+
+@pytest.mark.parametrize("d,top_k", [(64, 8), (64, 3), (128, 9)])
+@pytest.mark.parametrize("blocks", [32, 33, 34, 64, 65, 66, 129, 258])
+def test_gate_at_its_bounds(blocks, d, top_k, device):
+    """Candidate counts around the lines between no bounding pass, one half's bar and both halves' bar.
+    Scores are whole numbers, exact in every precision; rounded to bfloat16 many of them tie."""
+    cfg = moba.MoBAConfig(128, top_k, dtype=torch.bfloat16)
+    s = (blocks - 1) * 128 + 5
+    g = torch.Generator().manual_seed(blocks)
+    q = torch.randint(-7, 8, (1, s, 2, d), generator=g).to(torch.bfloat16).to(device)
+    kbar = moba.pool_blocks(q[:, :, :1].contiguous(), cfg)
+    kbar = torch.randint(-7, 8, kbar.shape, generator=g).to(kbar.dtype).to(device)
+    got = moba.gate_select(q, kbar, cfg).reshape(2, s, -1)
+    scores = torch.einsum("shd,nd->hsn", q[0].double(), kbar.reshape(blocks, d).double()).to(torch.bfloat16).double()
+    own = torch.arange(s, device=device) // 128
+    ids = torch.arange(blocks, device=device)
+    key = scores * 1024 - ids                                # score descending, ties to the lower id
+    key[:, ids[None, :] >= own[:, None]] = -float("inf")
+    best = key.topk(min(top_k - 1, blocks), dim=-1)
+    want = torch.where(best.values > -float("inf"), best.indices, blocks)
+    want = torch.cat([want, own[None, :, None].expand(2, -1, 1)], -1).sort(-1).values
+    have = torch.where(got < 0, blocks, got.long()).sort(-1).values
+    assert torch.equal(have, want)
