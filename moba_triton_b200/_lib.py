@@ -55,6 +55,7 @@ class Plan(Structure):
 
 
 _lib = None
+_autograd = None
 
 
 def load():
@@ -101,6 +102,22 @@ def load():
         raise RuntimeError("libmoba_b200.so was built from a different ABI version; rebuild it")
     _lib = lib
     return lib
+
+
+def autograd():
+    """The extension module of the differentiable op (csrc/autograd.cpp), bound to the library's
+    entry points; raises if it has not been built."""
+    global _autograd
+    if _autograd is None:
+        if not os.path.exists(os.path.join(PKG, "_autograd.so")):
+            raise RuntimeError("_autograd.so is missing: build it with `python -m moba_triton_b200.build` "
+                               "(there is no fallback path)")
+        from moba_triton_b200 import _autograd as module
+        lib = load()
+        module.bind(*(ctypes.cast(fn, c_void_p).value for fn in (lib.moba_b200_op_forward, lib.moba_b200_op_backward,
+                                                                 lib.moba_b200_last_error)))
+        _autograd = module
+    return _autograd
 
 
 def check(rc: int, what: str) -> None:

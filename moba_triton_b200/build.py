@@ -1,23 +1,27 @@
-"""Builds libmoba_b200.so in-tree with nvcc for sm_100a.
+"""Builds libmoba_b200.so in-tree with nvcc for sm_100a, and the autograd node with the host compiler.
 
     python -m moba_triton_b200.build [--force] [--verbose]
 
 Every csrc/*.cu is compiled to an object (in parallel) and linked into
 `moba_triton_b200/libmoba_b200.so`. The library links the static CUDA runtime
 only; the driver entry points it needs (tensor-map encoding) are resolved at
-run time, so it loads on machines without a GPU driver.
+run time, so it loads on machines without a GPU driver. csrc/autograd.cpp becomes
+`moba_triton_b200/_autograd.so`, a torch extension module without device code.
 """
 
 import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libmoba_b200.so")
+AUTOGRAD_SRC = os.path.join(CSRC, "autograd.cpp")
+AUTOGRAD = os.path.join(PKG, "_autograd.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -39,8 +43,29 @@ def sources():
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
 
+def build_autograd(force: bool = False) -> str:
+    header = os.path.join(PKG, "..", "include", "moba_b200.h")
+    if not force and os.path.exists(AUTOGRAD) and os.path.getmtime(AUTOGRAD) >= max(map(os.path.getmtime, (AUTOGRAD_SRC, header))):
+        return AUTOGRAD
+    import torch
+    from torch.utils import cpp_extension
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    includes = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-DTORCH_EXTENSION_NAME=_autograd", *(f"-isystem{i}" for i in includes), AUTOGRAD_SRC, "-o", AUTOGRAD,
+           f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("build of _autograd.so failed")
+    return AUTOGRAD
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compiles what is out of date and returns the library path."""
+    build_autograd(force)
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest_dep():
         return LIB
     os.makedirs(OBJ, exist_ok=True)

@@ -83,6 +83,11 @@ class MoBAQueryChunkedFunction(torch.autograd.Function):
         return dq, dk32.to(k.dtype), dv32.to(v.dtype), None, None, None
 
 
+def _attention(q, k, v, cfg, causal, cu_seqlens, max_seqlen):
+    plan = op_plan(q, k, v, cfg, causal, cu_seqlens, max_seqlen)
+    return _lib.autograd().attention(q, k, v, plan.native, cu_seqlens)
+
+
 def _kv_head_passes(q, k, v, kv_heads_per_pass: int):
     """Slices of (q, k, v) that hold whole groups of query heads with their KV heads."""
     hkv = k.shape[2]
@@ -128,7 +133,9 @@ def moba_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cfg: MoBAC
         if kv_heads_per_pass < 1:
             raise ValueError(f"kv_heads_per_pass must be positive, got {kv_heads_per_pass}")
         if kv_heads_per_pass < k.shape[2]:
-            outs = [MoBAAttentionFunction.apply(qs, ks, vs, cfg, None, causal, cu_seqlens, max_seqlen)
+            outs = [_attention(qs, ks, vs, cfg, causal, cu_seqlens, max_seqlen)
                     for qs, ks, vs in _kv_head_passes(q, k, v, kv_heads_per_pass)]
             return torch.cat(outs, dim=2)
+    if index is None:
+        return _attention(q, k, v, cfg, causal, cu_seqlens, max_seqlen)
     return MoBAAttentionFunction.apply(q, k, v, cfg, index, causal, cu_seqlens, max_seqlen)

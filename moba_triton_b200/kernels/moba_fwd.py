@@ -55,13 +55,14 @@ def _validate(q, k, v, cfg: MoBAConfig, cu_seqlens=None, max_seqlen=None) -> Non
 class _OpPlan:
     """What a whole-op call needs beside its tensors: the problem record and the sizes of its
     workspaces. Functions of shapes, dtype and configuration only, kept between calls."""
-    __slots__ = ("problem", "keep_bytes", "forward_bytes", "backward_bytes")
+    __slots__ = ("problem", "keep_bytes", "forward_bytes", "backward_bytes", "native")
 
     def __init__(self, problem):
         self.problem = problem
         sizes = [ctypes.c_size_t() for _ in range(3)]
         _lib.check(_lib.load().moba_b200_op_workspace(problem, *(ctypes.byref(x) for x in sizes)), "moba_attention")
         self.keep_bytes, self.forward_bytes, self.backward_bytes = (x.value for x in sizes)
+        self.native = _lib.autograd().Plan(ctypes.addressof(problem), *(x.value for x in sizes))
 
 
 _PLANS = {}
