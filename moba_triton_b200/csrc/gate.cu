@@ -124,7 +124,7 @@ int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, vo
 // portable gate: grid (cdiv(max_seqlen, 32), n_seq * Hq), 128 threads.
 // Each warp owns 8 query rows; a lane scores one candidate block of the
 // current 32-block chunk for all 8 rows in float64, then the warp merges the
-// chunk into each row's running list (shared memory, `take` entries).
+// chunk into each row's running list (over its lanes; past 32 entries in shared memory).
 // ---------------------------------------------------------------------------
 constexpr int kGateRows = 32;
 constexpr int kGateChunk = 32;
@@ -159,7 +159,46 @@ __device__ __forceinline__ Cand warp_weakest(Cand c, int& slot) {
   return c;
 }
 
-template <typename T>
+// Score (descending) and block id (ascending) as one number; 0 for what cannot be selected.
+__device__ __forceinline__ unsigned long long rank_key(float s, int blk) {
+  if (!(s > -INFINITY)) return 0ull;
+  const unsigned u = __float_as_uint(s + 0.f);                   // one zero
+  return (unsigned long long)(u & 0x80000000u ? ~u : u | 0x80000000u) << 32 | (0xffffffffu - (unsigned)blk);
+}
+__device__ __forceinline__ unsigned long long exchange(unsigned long long x, int j, bool keep_larger) {
+  const unsigned long long o = __shfl_xor_sync(0xffffffffu, x, j);
+  return (x > o) == keep_larger ? x : o;
+}
+// Bitonic: the warp's 32 keys in descending order over the lanes.
+__device__ __forceinline__ unsigned long long sort_lanes(unsigned long long x, int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j >= 1; j >>= 1) x = exchange(x, j, ((lane & j) == 0) == ((lane & k) == 0));
+  return x;
+}
+// The 32 largest of two descending sequences, descending.
+__device__ __forceinline__ unsigned long long merge_sorted(unsigned long long a, unsigned long long b, int lane) {
+  b = __shfl_sync(0xffffffffu, b, 31 - lane);
+  unsigned long long x = a > b ? a : b;
+#pragma unroll
+  for (int j = 16; j >= 1; j >>= 1) x = exchange(x, j, (lane & j) == 0);
+  return x;
+}
+// best[r] for an r that the compiler does not know
+template <int N>
+__device__ __forceinline__ unsigned long long sorted_row(const unsigned long long (&best)[N], int r) {
+  unsigned long long x = best[0];
+#pragma unroll
+  for (int e = 1; e < N; ++e) if (r == e) x = best[e];
+  return x;
+}
+
+// SORTED: up to 32 ranked blocks. The row's list lies sorted over the lanes of its warp, and a chunk
+// of 32 candidates is sorted and merged into it in 21 exchanges; offering them one by one, a reduction
+// over the warp and two over the list each, was two thirds of the kernel ([1,4096,4,64] float32,
+// 7 of 32 blocks: 76 us, sorted 29).
+template <typename T, bool SORTED>
 __global__ void __launch_bounds__(128)
 gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
                      const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx,
@@ -199,8 +238,9 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
   const int horizon = min(last_row / p.block_size, n_cand);      // blocks < horizon can be candidates
   const T* kb = kbar + ((size_t)seq * p.kv_heads + hq / group) * p.num_blocks * (size_t)d;
   float thr[kRowsPerWarp];                                       // current entry bar per row
+  unsigned long long best[kRowsPerWarp];                         // SORTED: lane e holds the row's e-th best key, 0 = none
 #pragma unroll
-  for (int r = 0; r < kRowsPerWarp; ++r) thr[r] = -INFINITY;
+  for (int r = 0; r < kRowsPerWarp; ++r) { thr[r] = -INFINITY; best[r] = 0ull; }
 
   for (int c0 = 0; take > 0 && c0 < horizon; c0 += kGateChunk) {
     __syncthreads();
@@ -228,6 +268,12 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
       const int own = row / p.block_size;
       float s = Elem<T>::round_f((float)acc[r]);
       if (!(gate_candidate(p, blk, own) && blk < n_cand && row < sp.len)) s = -INFINITY;
+      if constexpr (SORTED) {
+        const unsigned long long key = rank_key(s, blk);
+        if (__any_sync(0xffffffffu, key > __shfl_sync(0xffffffffu, best[r], take - 1)))
+          best[r] = merge_sorted(best[r], sort_lanes(key, lane), lane);
+        continue;
+      }
       float* lv = lval + lrow * take;
       int* li = lidx + lrow * take;
       // offer the chunk's candidates in (score desc, id asc) order while they clear the bar
@@ -270,6 +316,24 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
     const size_t b = p.packed ? 0 : (size_t)seq;
     const size_t out_at = ((b * p.q_heads + hq) * p.tokens + sp.bos + row) * (size_t)slots;
     int32_t* out = block_idx + out_at;
+    if constexpr (SORTED) {
+      const unsigned long long key = sorted_row(best, r);
+      const bool have = lane < take && key != 0ull;
+      const int id = have ? (int)(0xffffffffu - (unsigned)key) : kEmptyIdx;
+      int rank = 0;
+      for (int f = 0; f < take; ++f) rank += __shfl_sync(0xffffffffu, id, f) < id ? 1 : 0;
+      int kept = __popc(__ballot_sync(0xffffffffu, have));
+      if (have) out[rank] = id;
+      if (p.always_current) {                                    // the own block is past every candidate
+        if (lane == 0) out[kept] = own;
+        ++kept;
+      }
+      for (int e = kept + lane; e < slots; e += 32) {
+        out[e] = -1;
+        if (lse_fill != nullptr) lse_fill[out_at + e] = -INFINITY;
+      }
+      continue;
+    }
     const int n_items = take + (p.always_current ? 1 : 0);
     int kept = 0;
     for (int e = lane; e < n_items; e += 32) {
@@ -307,15 +371,17 @@ int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* 
     return MOBA_B200_EUNSUPPORTED;
   }
   dim3 grid((p.max_seqlen + kGateRows - 1) / kGateRows, p.n_seq * p.q_heads);
-#define MOBA_GATE(T)                                                                          \
+#define MOBA_GATE(T, SORTED)                                                                  \
   do {                                                                                        \
     static SmemLimit limit;                                                                   \
-    if (int rc = raise_smem_limit(limit, (const void*)gate_portable_kernel<T>, smem)) return rc; \
-    MOBA_CUDA_OK(launch_chained(gate_portable_kernel<T>, grid, 128, smem, st, (const T*)q, (const T*)kbar, cu, block_idx, lse_fill, p)); \
+    if (int rc = raise_smem_limit(limit, (const void*)gate_portable_kernel<T, SORTED>, smem)) return rc; \
+    MOBA_CUDA_OK(launch_chained(gate_portable_kernel<T, SORTED>, grid, 128, smem, st, (const T*)q, (const T*)kbar, cu, block_idx, lse_fill, p)); \
   } while (0)
-  if (p.dtype == MOBA_B200_F32) MOBA_GATE(float);
-  else if (p.dtype == MOBA_B200_BF16) MOBA_GATE(__nv_bfloat16);
-  else MOBA_GATE(__half);
+#define MOBA_GATE_T(T) do { if (p.take <= 32) MOBA_GATE(T, true); else MOBA_GATE(T, false); } while (0)
+  if (p.dtype == MOBA_B200_F32) MOBA_GATE_T(float);
+  else if (p.dtype == MOBA_B200_BF16) MOBA_GATE_T(__nv_bfloat16);
+  else MOBA_GATE_T(__half);
+#undef MOBA_GATE_T
 #undef MOBA_GATE
   return MOBA_B200_OK;
 }

@@ -98,3 +98,25 @@ def test_gate_at_its_bounds(blocks, d, top_k, device):
     want = torch.cat([want, own[None, :, None].expand(2, -1, 1)], -1).sort(-1).values
     have = torch.where(got < 0, blocks, got.long()).sort(-1).values
     assert torch.equal(have, want)
+
+
+@pytest.mark.parametrize("top_k", [2, 9, 33, 34])
+@pytest.mark.parametrize("blocks", [20, 33, 34, 100])
+def test_portable_gate_lists(blocks, top_k, device):
+    """The list over a warp's lanes (up to 32 ranked blocks) and the one in shared memory, with ties."""
+    cfg = moba.MoBAConfig(16, top_k, dtype=torch.float32)
+    s = blocks * 16 - 3
+    g = torch.Generator().manual_seed(blocks)
+    q = torch.randint(-2, 3, (1, s, 2, 64), generator=g).float().to(device)
+    kbar = torch.randint(-2, 3, (1, 1, blocks, 64), generator=g).float().to(device)
+    got = moba.gate_select(q, kbar, cfg).reshape(2, s, -1)
+    scores = torch.einsum("shd,nd->hsn", q[0].double(), kbar.reshape(blocks, 64).double())
+    own = torch.arange(s, device=device) // 16
+    ids = torch.arange(blocks, device=device)
+    key = scores * 1024 - ids
+    key[:, ids[None, :] >= own[:, None]] = -float("inf")
+    best = key.topk(min(top_k - 1, blocks), dim=-1)
+    want = torch.where(best.values > -float("inf"), best.indices, blocks)
+    want = torch.cat([want, own[None, :, None].expand(2, -1, 1)], -1).sort(-1).values
+    have = torch.where(got < 0, blocks, got.long()).sort(-1).values[..., :want.shape[-1]]
+    assert torch.equal(have, want)
