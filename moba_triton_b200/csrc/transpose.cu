@@ -566,7 +566,7 @@ int launch_transpose(const moba_b200_problem& p, const int32_t* block_idx, const
 // to kSmallPairs pairs per row and cluster; a longer row leaves too much to one cluster.
 // ---------------------------------------------------------------------------
 constexpr int kSmallBlocks = 512;
-constexpr int kSmallCluster = 8;
+constexpr int kSmallCluster = 8, kWideCluster = 16;
 constexpr long long kSmallPairs = 1 << 17;
 constexpr int kSmallThreads = 1024, kSmallWarps = kSmallThreads / 32;
 
@@ -582,8 +582,8 @@ __device__ __forceinline__ int ld_cluster_i32(const int* mine, uint32_t rank) {
   return v;
 }
 
-// K: block ids per lane, an upper bound of the run's entries / 32
-template <int K>
+// K: block ids per lane, an upper bound of the run's entries / 32. C: CTAs of the cluster.
+template <int K, int C>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __restrict__ cu, int32_t* __restrict__ col_nnz,
                        int32_t* __restrict__ col_offsets, int32_t* __restrict__ order, int2* __restrict__ entries, int4* __restrict__ items,
@@ -601,14 +601,14 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
   __syncthreads();
   pdl_trigger();
   pdl_wait();
-  const int kv_row = (int)(blockIdx.x / kSmallCluster);
+  const int kv_row = (int)(blockIdx.x / C);
   const int seq = kv_row / p.kv_heads, kvh = kv_row % p.kv_heads;
   const int group = p.q_heads / p.kv_heads;
   const SeqSpan sp = seq_span(cu, p.packed, seq, p.tokens);
   const unsigned slots = (unsigned)p.slots;
   // this warp's run of queries, in (head, position) order
   const unsigned total_q = (unsigned)group * (unsigned)sp.len;
-  const unsigned per_warp = (total_q + kSmallCluster * kSmallWarps - 1) / (kSmallCluster * kSmallWarps);
+  const unsigned per_warp = (total_q + C * kSmallWarps - 1) / (C * kSmallWarps);
   const unsigned q_lo = min(total_q, (rank * kSmallWarps + warp) * per_warp), q_hi = min(total_q, q_lo + per_warp);
   const int n = (int)((q_hi - q_lo) * slots);
   int g0 = 0, r0 = (int)q_lo;                                // head and position of the run's first query
@@ -659,11 +659,11 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
   int mine = 0, before = 0;
   const int col = threadIdx.x;                               // nb <= kSmallBlocks < threads
   if (col < nb) {
-    int t[kSmallCluster];
+    int t[C];
 #pragma unroll
-    for (int c = 0; c < kSmallCluster; ++c) t[c] = ld_cluster_i32(&totals[col], (uint32_t)c);
+    for (int c = 0; c < C; ++c) t[c] = ld_cluster_i32(&totals[col], (uint32_t)c);
 #pragma unroll
-    for (int c = 0; c < kSmallCluster; ++c) {
+    for (int c = 0; c < C; ++c) {
       mine += t[c];
       before += c < (int)rank ? t[c] : 0;
     }
@@ -687,7 +687,7 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
     cuts_all += warp_pieces[w];
   }
   if (col < nb) base_s[col] = off + before;
-  const bool lister = rank == kSmallCluster - 1;
+  const bool lister = rank == C - 1;
   if (lister && threadIdx.x == 0) {
     const int need = (int)((unsigned)cuts_all >> 16);
     const int base = need > 0 ? atomicAdd(slot_counter, need) : 0;
@@ -741,9 +741,9 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
 }
 
 // Entries of a warp's run: at most this many per lane.
-static inline int small_ids_per_lane(const moba_b200_problem& p) {
+static inline int small_ids_per_lane(const moba_b200_problem& p, int cluster = kSmallCluster) {
   const long long total_q = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen;
-  const long long per_warp = (total_q + kSmallCluster * kSmallWarps - 1) / (kSmallCluster * kSmallWarps);
+  const long long per_warp = (total_q + cluster * kSmallWarps - 1) / (cluster * kSmallWarps);
   return (int)((per_warp * p.slots + 31) / 32);
 }
 
@@ -754,6 +754,34 @@ bool transpose_small_supported(const moba_b200_problem& p) {
          (long long)p.n_seq * p.kv_heads * kSmallCluster < 0x7fffffffLL;
 }
 
+// Whether the current device can hold a cluster of kWideCluster CTAs with the largest shared memory
+// they take here (more than eight is not portable). Asked once per device, which also allows it to
+// the kernels.
+static bool wide_clusters_fit() {
+  static int known[64];                                      // 0 unknown, 1 yes, -1 no; written alike by whoever asks first
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  if (__atomic_load_n(&known[dev], __ATOMIC_ACQUIRE) == 0) {
+    const auto kern = transpose_small_kernel<12, kWideCluster>;
+    const size_t smem = (size_t)kSmallWarps * kSmallBlocks * sizeof(int);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kWideCluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kWideCluster); cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = smem; cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                    cudaFuncSetAttribute(transpose_small_kernel<4, kWideCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(transpose_small_kernel<8, kWideCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1;
+    if (!ok) cudaGetLastError();
+    __atomic_store_n(&known[dev], ok ? 1 : -1, __ATOMIC_RELEASE);
+  }
+  return __atomic_load_n(&known[dev], __ATOMIC_ACQUIRE) > 0;
+}
+
 // `slot_counter` must hold zero.
 int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx, const int32_t* cu, int32_t* col_nnz,
                            int32_t* col_offsets, int32_t* order, int2* entries, int part_shift, int32_t* work_items,
@@ -762,18 +790,27 @@ int launch_transpose_small(const moba_b200_problem& p, const int32_t* block_idx,
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("transpose: no device error word"); return MOBA_B200_ECUDA; }
   const size_t smem = (size_t)kSmallWarps * p.num_blocks * sizeof(int);
-  const int k = small_ids_per_lane(p);
-  const int which = k <= 4 ? 0 : (k <= 8 ? 1 : 2);
-  auto kern = which == 0 ? transpose_small_kernel<4> : (which == 1 ? transpose_small_kernel<8> : transpose_small_kernel<20>);
-  static SmemLimit limit[3];
+  // A few rows: clusters of sixteen, if the device has room for one. The scattered stores, a line per
+  // entry, take about half of the kernel at 8192 keys a row: 4 rows 21.0 us with eight CTAs each, 16.8
+  // with sixteen. Eight rows are slower (20.6 and 23.0): a part of the chip holds one such cluster.
+  int cluster = kSmallCluster;
+  if (p.n_seq * p.kv_heads <= 4 && small_ids_per_lane(p) > 2 && wide_clusters_fit()) cluster = kWideCluster;
+  const bool wide = cluster == kWideCluster;
+  const int k = small_ids_per_lane(p, cluster);
+  const int which = (wide ? 3 : 0) + (k <= 4 ? 0 : (k <= 8 ? 1 : 2));
+  const decltype(&transpose_small_kernel<4, kSmallCluster>) kernels[6] = {
+      transpose_small_kernel<4, kSmallCluster>, transpose_small_kernel<8, kSmallCluster>, transpose_small_kernel<20, kSmallCluster>,
+      transpose_small_kernel<4, kWideCluster>, transpose_small_kernel<8, kWideCluster>, transpose_small_kernel<12, kWideCluster>};
+  auto kern = kernels[which];
+  static SmemLimit limit[6];
   if (int rc = raise_smem_limit(limit[which], (const void*)kern, smem)) return rc;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = kSmallCluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(p.n_seq * p.kv_heads * kSmallCluster)); cfg.blockDim = dim3(kSmallThreads);
+  cfg.gridDim = dim3((unsigned)(p.n_seq * p.kv_heads * cluster)); cfg.blockDim = dim3(kSmallThreads);
   cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;
   const long long capacity = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
   const unsigned recip = (unsigned)(((1ull << 32) + p.slots - 1) / p.slots);    // e / slots for e < 2^16 and slots > 1

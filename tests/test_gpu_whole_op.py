@@ -24,6 +24,8 @@ CASES = [
     (3, 900, 2, 2, 128, 128, 8, torch.float16, None),            # batch rows end inside a block
     (1, 16384, 1, 1, 64, 128, 8, torch.bfloat16, None),          # the last row length of the one-launch transpose
     (1, 16512, 1, 1, 64, 128, 8, torch.bfloat16, None),          # the first beyond it
+    (1, 13000, 1, 1, 64, 128, 10, torch.bfloat16, None),         # nine ids per lane of a cluster of sixteen
+    (1, 5000, 5, 5, 64, 128, 4, torch.bfloat16, None),           # five rows: clusters of eight
     (1, 8192, 2, 2, 64, 16, 2, torch.bfloat16, None),            # 512 columns
     (1, 8208, 2, 2, 64, 16, 2, torch.bfloat16, None),            # 513
     (1, 1500, 4, 2, 64, 128, 4, torch.bfloat16, [0, 1, 130, 700, 1500]),
