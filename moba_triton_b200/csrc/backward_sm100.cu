@@ -690,7 +690,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       // every tile on them and held up every other load and store of the SM meanwhile (it keeps
       // about 24 KB outstanding; a gather of 32 or 64 KB fills that for a memory latency or two).
       const int gw = warp - kGatherWarp0, pt = gw * 32 + lane;
-      const uint64_t keep = l2_policy_evict_last();
       const int n_rows = p.batch * p.tokens * p.q_heads;
       uint32_t t = 0, n_seen = 0;
       for (uint32_t it = 0; sound; ++it) {

@@ -57,19 +57,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Whether the phase has completed, without waiting (try_wait may suspend the thread).
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 struct WaitCtx {
   volatile int* abort;        // shared-memory flag of the CTA
   unsigned* error_word;       // global
@@ -158,25 +145,12 @@ __device__ __forceinline__ void mbar_wait_quiet(uint64_t* bar, uint32_t parity) 
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// generic-proxy writes (st.shared, cp.async) -> visible to the async proxy (TMA, tcgen05.mma)
+// generic-proxy writes (st.shared) -> visible to the async proxy (TMA, tcgen05.mma)
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// ---------------------------------------------------------------------------
-// cp.async (16-byte, zero-fill when src_bytes == 0)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// L2 eviction policies. Rows that are gathered again and again (Q, dO, K, V) are loaded
+// L2 eviction policies. Blocks that are loaded again and again (K, V) are loaded
 // "evict last"; the partial buffers, which are written once and read once by a later
 // kernel, are stored "evict first", so that their stream does not push the reused rows
 // out of the L2.
@@ -185,10 +159,6 @@ __device__ __forceinline__ uint64_t l2_policy_evict_last() {
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
-__device__ __forceinline__ void cp_async16_hint(uint32_t dst_smem, const void* src, uint32_t src_bytes, uint64_t pol) {
-  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;" ::"r"(dst_smem), "l"(src), "r"(src_bytes), "l"(pol)
-               : "memory");
-}
 __device__ __forceinline__ void st_global_stream16(void* dst, const uint4& w) {
   asm volatile("st.global.cs.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
 }
@@ -196,25 +166,9 @@ __device__ __forceinline__ void st_global_stream_f32(float* dst, float v) {
   asm volatile("st.global.cs.f32 [%0], %1;" ::"l"(dst), "f"(v) : "memory");
 }
 
-// Bulk copy shared -> global (both 16-byte aligned, size a multiple of 16) by the copy engine;
-// the issuing thread groups its copies and waits until they have read their source.
-__device__ __forceinline__ void bulk_store(void* dst, uint32_t src_smem, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_smem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-
 // Asks the L2 to fetch [p, p + bytes) (both multiples of 16); nothing waits for it.
 __device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-// Asks the L2 for the 128-byte line that holds `p` (an ordinary load-store-unit request: cheap
-// to issue, unlike the bulk form above, which goes through the copy engine one request at a time).
-__device__ __forceinline__ void l2_prefetch_line(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
 }
 // Prefetches elements [lo, lo + n) of an int32 array of `total` elements.
 __device__ __forceinline__ void l2_prefetch_i32(const int32_t* base, size_t lo, int n, size_t total) {
@@ -227,12 +181,6 @@ __device__ __forceinline__ void l2_prefetch_i32(const int32_t* base, size_t lo, 
 
 // A global load the compiler may not move: used to fetch index entries a tile or two before
 // they are needed (a plain load may be sunk to its first use, which defeats the prefetch).
-__device__ __forceinline__ int ld_nc_pinned(const int32_t* p) {
-  int v;
-  asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
-
 __device__ __forceinline__ float ld_nc_pinned_f(const float* p) {
   float v;
   asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
@@ -275,16 +223,6 @@ __device__ __forceinline__ void tma_gather4(void* dst_smem, const CUtensorMap* m
       "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
       ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1),
         "r"(r2), "r"(r3)
-      : "memory");
-}
-
-__device__ __forceinline__ void tma_gather4_hint(void* dst_smem, const CUtensorMap* m, uint64_t* bar, int col,
-                                                 int r0, int r1, int r2, int r3, uint64_t pol) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.L2::cache_hint "
-      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2], %8;"
-      ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(col), "r"(r0), "r"(r1),
-        "r"(r2), "r"(r3), "l"(pol)
       : "memory");
 }
 
