@@ -127,11 +127,12 @@ template <> __device__ __forceinline__ float widen16<__half>(uint32_t bits) {
 }
 
 // Score (rounded to T) and block id -> sortable key; never 0 for a real candidate
-// (the low half of a key is 0xFFFF - id with id <= 0xFFFE).
+// (the low half of a key is 0xFFFF - id with id <= 0xFFFE). The high half counts the steps of T from
+// zero, which both zeros are, with 0x8000 added.
 template <typename T>
 __device__ __forceinline__ uint32_t make_key(float score, uint32_t block) {
   const uint32_t b = round16<T>(score);
-  const uint32_t mono = (b & 0x8000u) ? (~b & 0xFFFFu) : (b | 0x8000u);
+  const uint32_t mono = (b & 0x8000u) ? 0x10000u - b : b + 0x8000u;
   return (mono << 16) | (0xFFFFu - block);
 }
 // The score a candidate has to exceed to get past `key` (the list's last entry):
@@ -140,7 +141,7 @@ template <typename T>
 __device__ __forceinline__ float entry_bar(uint32_t key) {
   if (key == 0u) return -INFINITY;
   const uint32_t mono = key >> 16;
-  const uint32_t b = (mono & 0x8000u) ? (mono & 0x7FFFu) : (~mono & 0xFFFFu);
+  const uint32_t b = (mono & 0x8000u) ? (mono & 0x7FFFu) : 0x10000u - mono;
   return widen16<T>(b);
 }
 
