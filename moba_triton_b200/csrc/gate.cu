@@ -78,23 +78,23 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
   for (int e = 0; e < EPV; ++e) red[threadIdx.x * EPV + e] = acc[e];
   __syncthreads();
   const float occ = (float)(hi - lo);
-  float square = 0.f;
+  double square = 0.0;                                          // in float64: no square leaves its range
   for (int i = threadIdx.x; i < d; i += 128) {
     double s = 0.0;
     for (int g = 0; g < groups; ++g) s += red[g * d + i];       // thread g * vpr + i / EPV, element i % EPV
     const float total = Elem<T>::round_f((float)s);
     const T mean = Elem<T>::from_f(__fdiv_rn(total, occ));
     dst[i] = mean;
-    square = fmaf(Elem<T>::to_f(mean), Elem<T>::to_f(mean), square);
+    square = fma((double)Elem<T>::to_f(mean), (double)Elem<T>::to_f(mean), square);
   }
   if (norms == nullptr) return;
   // the block mean's length, for the error bound of the exact gate
-  __shared__ float part[4];
+  __shared__ double part[4];
 #pragma unroll
   for (int o = 16; o; o >>= 1) square += __shfl_xor_sync(0xffffffffu, square, o);
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = square;
   __syncthreads();
-  if (threadIdx.x == 0) norms[(size_t)kv_row * nb + blk] = sqrtf(part[0] + part[1] + part[2] + part[3]);
+  if (threadIdx.x == 0) norms[(size_t)kv_row * nb + blk] = (float)sqrt(part[0] + part[1] + part[2] + part[3]);
 }
 
 // `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from; `norms`

@@ -33,10 +33,12 @@
 //
 // EXACT: the same kernel where the portable gate used to run (other block sizes that divide 128,
 // more than eight ranked blocks): its selections are those of exact scores, bit for bit. The
-// tensor-core sum is off by at most `err` (a bound from the lengths of the query and of the block
-// means), so the entry test is loosened by err, and a candidate whose rounding to the input dtype
-// depends on that error is scored again in float64 by its whole warp before it is ranked: about
-// one candidate in forty. With blocks finer than the tile a row's candidates end at its own block.
+// tensor-core sum is off by at most `err` (a bound from the lengths of the query and of the means of
+// the unit's candidates), so the entry test is loosened by err, and a candidate whose rounding to the
+// input dtype depends on that error is scored again in float64 by its whole warp before it is ranked:
+// about one buffered candidate in forty where scores are large against err, every one near zero. A
+// row without a finite bound (infinities, NaN, squares outside float32) has every candidate scored in
+// float64. With blocks finer than the tile a row's candidates end at its own block.
 //
 // Scores are float32 tensor-core sums rounded to the input dtype; the portable
 // gate rounds the exact sum. The two differ only when a float32 partial sum
@@ -223,12 +225,41 @@ __device__ __forceinline__ float exact_score(const T* q_row, const T* kbar_row, 
   return (float)acc;
 }
 
+// Bound of |tensor-core sum - exact score| for one query and the blocks [0, n_cand) of its KV row,
+// whose lengths are `norms`; the warp's lanes share the blocks. D / 16 accumulation steps of 17
+// addends, each cut at 2^-23 of the largest: D 17/16 2^-23 of a quantity that |q| |kbar| bounds;
+// doubled, and the smallest normal number for what is lost below it. Infinite where that cannot be
+// said: an infinity or NaN in the query, an infinity in a block mean, squares whose sum does not fit
+// float32. A NaN in a block mean needs no bound, its score is NaN either way; nor does a query of zeros.
+template <int D, typename T>
+__device__ __forceinline__ float score_error(const T* q_row, const float* norms, int n_cand, int lane) {
+  float longest = 0.f;
+#pragma unroll 4
+  for (int i = lane; i < n_cand; i += 32) longest = fmaxf(longest, __ldg(norms + i));
+#pragma unroll
+  for (int o = 16; o; o >>= 1) longest = fmaxf(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+  float square = 0.f;
+  uint32_t any = 0u;
+#pragma unroll 4
+  for (int i = 0; i < D / 8; ++i) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(q_row + i * 8);
+    any |= raw.x | raw.y | raw.z | raw.w;
+    const T* x = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) square = fmaf(Elem<T>::to_f(x[e]), Elem<T>::to_f(x[e]), square);
+  }
+  if ((any & 0x7fff7fffu) == 0u || longest == 0.f) return 0.f;
+  if (!(square >= 1e-30f && square <= 1e30f)) return INFINITY;
+  const float e = sqrtf(square) * longest * ((float)D * (17.f / 8.f) * 1.1920929e-7f);
+  return e < INFINITY ? e + 1.17549435e-38f : INFINITY;
+}
+
 template <int D, typename T, int L, bool EXACT>
 __global__ void __launch_bounds__(kThreads, 2)
 gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kb_map,
                   const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx, float* __restrict__ lse_fill,
                   moba_b200_problem p, int n_tiles, int n_units, unsigned* error_word,
-                  const T* __restrict__ q, const T* __restrict__ kbar, const float* __restrict__ norms, int n_norms) {
+                  const T* __restrict__ q, const T* __restrict__ kbar, const float* __restrict__ norms) {
   using Cfg = GateCfg<D>;
   constexpr int CAP = Cfg::kCap, STEP = Cfg::kStep;
   extern __shared__ unsigned char smem_dyn[];
@@ -267,21 +298,10 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
   tc_fence_after();
   pdl_wait();
   const uint32_t tmem = bars->tmem_base;
-  float longest_mean = 0.f;                                     // EXACT: of all block means
-  if constexpr (EXACT) {
-    __shared__ float longest[10];
-    for (int i = threadIdx.x; i < n_norms; i += kThreads) longest_mean = fmaxf(longest_mean, norms[i]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) longest_mean = fmaxf(longest_mean, __shfl_xor_sync(0xffffffffu, longest_mean, o));
-    if (lane == 0) longest[warp] = longest_mean;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < 10; ++w) longest_mean = fmaxf(longest_mean, longest[w]);
-  }
 
-  // Every role walks the same units and counts the same steps: a unit of n chunks takes 2 n
-  // steps (chunk `step mod n`), `gc` is the number of steps of all earlier units of this CTA,
-  // and a step uses Kbar stage and TMEM buffer (gc + step) & 1.
+  // Every role walks the same units and counts the same steps: a unit takes the steps of its
+  // bounding pass and one per chunk (Unit::steps), `gc` is the number of steps of all earlier units
+  // of this CTA, and a step uses Kbar stage and TMEM buffer (gc + step) & 1.
   if (warp < 8) {
     // ================================ select ================================
     const int wg = warp >> 2;
@@ -309,18 +329,8 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
       float err = 0.f;                                          // EXACT: bound of |tensor-core sum - exact score|
       const T* q_row = nullptr;
       if constexpr (EXACT) {
-        // D / 16 accumulation steps of 17 addends, each cut at 2^-23 of the largest: D 17/16 2^-23
-        // of a quantity that |q| |kbar| bounds; doubled.
         q_row = q + ((size_t)(p.packed ? u.bos : (size_t)u.seq * p.tokens) + min(u.row0 + r, u.len - 1)) * ((size_t)p.q_heads * D) + (size_t)u.hq * D;
-        float square = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < D / 8; ++i) {
-          const uint4 raw = *reinterpret_cast<const uint4*>(q_row + i * 8);
-          const T* x = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) square = fmaf(Elem<T>::to_f(x[e]), Elem<T>::to_f(x[e]), square);
-        }
-        err = sqrtf(square) * longest_mean * (float)D * (17.f / 8.f) * 1.1920929e-7f;
+        err = score_error<D, T>(q_row, norms + ((size_t)u.seq * p.kv_heads + u.hq / group) * p.num_blocks, u.own_hi, lane);
       }
       uint32_t best[L];
 #pragma unroll
@@ -342,7 +352,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           }
           if constexpr (EXACT) {                                // does the rounding depend on the sum's error?
             const float s = __uint_as_float(sx);
-            unsigned unsure = __ballot_sync(0xffffffffu, popped && round16<T>(s - err) != round16<T>(s + err));
+            unsigned unsure = __ballot_sync(0xffffffffu, popped && (err == INFINITY || round16<T>(s - err) != round16<T>(s + err)));
             while (unsure) {
               const int who = __ffs((int)unsure) - 1;
               unsure &= unsure - 1;
@@ -353,7 +363,8 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
               if (lane == who) sx = __float_as_uint(exact);
             }
           }
-          if (popped) key = make_key<T>(__uint_as_float(sx), sy);
+          // (a score taken again in float64 may be one that is never selected)
+          if (popped && (!EXACT || __uint_as_float(sx) > -INFINITY)) key = make_key<T>(__uint_as_float(sx), sy);
           list_offer<L>(best, key);
         }
         bar = fmaxf(bar, entry_bar<T>(best[L - 1]) - err);
@@ -413,6 +424,13 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           const int g0 = c0 + h * 32;
           const bool none = g0 >= u.own_hi || (p.gate_window > 0 && g0 >= p.gate_sinks && g0 + 32 <= u.own_lo - p.gate_window);
           if (!run || none) continue;
+          if constexpr (EXACT) {                                // no bound: every candidate is to be scored again
+            if (__any_sync(0xffffffffu, err == INFINITY)) {
+#pragma unroll
+              for (int k = 0; k < 32; ++k)
+                if (err == INFINITY) v[k] = 0x7f800000u;        // +inf passes the entry test
+            }
+          }
           const bool all = g0 + 32 <= u.own_lo &&
                            (p.gate_window <= 0 || g0 + 32 <= p.gate_sinks || g0 >= u.own_hi - p.gate_window);
           if (!all) {
@@ -591,7 +609,7 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& qm, const CUtensor
   const int sms = sm_count();
   const int grid = (int)(n_units < 2LL * sms ? n_units : 2LL * sms);
   MOBA_CUDA_OK(launch_chained(kern, grid, kThreads, GateCfg<D>::kSmem, st, qm, km, cu, block_idx, lse_fill, p, n_tiles,
-                              (int)n_units, err, (const T*)q, (const T*)kbar, norms, p.n_seq * p.kv_heads * p.num_blocks));
+                              (int)n_units, err, (const T*)q, (const T*)kbar, norms));
   return MOBA_B200_OK;
 }
 

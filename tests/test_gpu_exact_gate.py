@@ -1,4 +1,6 @@
-"""The tensor-core gates against float64 scores where floating-point details decide: signed zeros.
+"""The exact tensor-core gate against float64 scores where its rounding is decided by its error
+bound: scores a little off the middle between two values of the input type, hidden behind terms
+that cancel; signed zeros; infinities, NaN and numbers whose squares leave the range of float32.
 
 Keys are constant within a block, so the block means are the keys themselves. The gate runs inside
 the whole op only; which blocks it selected is read off the output, with one-hot values per block."""
@@ -52,6 +54,67 @@ def check(q, kb, cfg, unseen=()):
     for b in unseen:
         got[..., b] = want[..., b]
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("d,top_k", [(64, 4), (64, 12), (64, 17), (128, 9), (128, 13)])
+@pytest.mark.parametrize("blocks", [20, 64, 150])
+def test_scores_beside_a_rounding_boundary(blocks, d, top_k, dtype, device):
+    """Scores (n + 1/2) steps of the type plus or minus a trace, with B - B added to them: a sum in
+    float32 that keeps 24 bits of its largest term loses the trace for most of the B drawn."""
+    g = torch.Generator().manual_seed(blocks * 7 + d)
+    bits = 8 if dtype == torch.bfloat16 else 11              # significant bits: steps of 2^(1 - bits) in [1, 2)
+    s = blocks * BS - 3
+    ints = lambda lo, hi, *shape: torch.randint(lo, hi + 1, shape, generator=g).double()
+    q = torch.zeros(s, 1, d, dtype=torch.float64)
+    kb = torch.zeros(blocks, 1, d, dtype=torch.float64)
+    q[:, 0, 0] = 2.0 ** ints(0, 10, s)                       # B = q0 k0, -B = q0 k1 and q0 k17 (another step of 16)
+    kb[:, 0, 0] = 1.0
+    near = torch.rand(blocks, generator=g) < 0.5
+    kb[:, 0, 1] = torch.where(near, -1.0, 0.0)
+    kb[:, 0, 17] = torch.where(near, 0.0, -1.0)
+    q[:, 0, 1] = q[:, 0, 17] = q[:, 0, 0]
+    q[:, 0, 2:5] = 1.0
+    kb[:, 0, 2] = 1.0 + ints(0, 3, blocks) * 2.0 ** (1 - bits)
+    kb[:, 0, 3] = 2.0 ** -bits * ints(0, 1, blocks)          # half a step, or none
+    kb[:, 0, 4] = ints(-1, 1, blocks) * 2.0 ** -ints(12, 14, blocks)   # the trace
+    q *= 2.0 ** ints(-1, 1, s)[:, None, None] if dtype == torch.bfloat16 else 1.0
+    q, kb = q.to(dtype).to(device), kb.to(dtype).to(device)
+    check(q, kb, moba.MoBAConfig(BS, top_k, dtype=dtype))
+
+
+@pytest.mark.parametrize("case", ["zero_rows", "tiny", "huge", "same_head"])
+@pytest.mark.parametrize("blocks", [20, 60])
+def test_rows_without_a_finite_bound(blocks, case, device):
+    """zero_rows: query rows of zeros (padding) beside another head whose keys hold an infinity.
+    tiny / huge: squares below / above the range of float32. same_head: the infinity, and a NaN,
+    among the candidates themselves."""
+    dtype, d = torch.bfloat16, 64
+    cfg = moba.MoBAConfig(BS, 6, dtype=dtype)
+    g = torch.Generator().manual_seed(blocks)
+    s = blocks * BS - 7
+    q = torch.randint(-3, 4, (s, 1, d), generator=g).to(dtype).to(device)
+    kb = torch.randint(-1, 2, (blocks, 1, d), generator=g).to(dtype).to(device)
+    if case == "tiny":
+        return check(q * 2.0 ** -80, kb * 2.0 ** 20, cfg)
+    if case == "huge":
+        return check(q * 2.0 ** 80, kb * 2.0 ** -80, cfg)
+    if case == "same_head":
+        kb[blocks // 2, 0, 5] = float("inf")
+        kb[blocks // 3, 0, 6] = float("nan")
+        q[::3] = 0
+        return check(q, kb, cfg, unseen=(blocks // 2, blocks // 3))
+    q[::2] = 0
+    want = selected_by_exact_scores(q, kb, cfg)
+    # two KV heads: the first as drawn, the second with an infinite key at its start
+    k = kb.repeat_interleave(BS, dim=0)[None, :s]
+    k2 = k.clone()
+    k2[0, 3, 0, 0] = float("inf")
+    v = torch.zeros(blocks, 1, d, device=device, dtype=dtype)
+    v[:, 0, :blocks] = torch.eye(blocks, device=device, dtype=dtype)
+    v = v.repeat_interleave(BS, dim=0)[None, :s]
+    out = moba.moba_forward(torch.cat([q[None], q[None]], 2), torch.cat([k, k2], 2), torch.cat([v, v], 2), cfg)
+    assert torch.equal(out[0, :, :1, :blocks] > 0, want)
 
 
 @pytest.mark.parametrize("block", [32, 128], ids=["exact", "plain"])
