@@ -229,6 +229,14 @@ def set_kernel_path(path: int) -> int:
     return old
 
 
+def config_fields(cfg, longest: int) -> tuple:
+    """What a problem record takes from a configuration, for sequences of up to `longest` tokens:
+    (block_size, top_k, slots, take, always_current, num_blocks, gate_window, gate_sinks)."""
+    nb = cfg.num_blocks(longest)
+    return (cfg.block_size, cfg.top_k, cfg.slots_per_query, cfg.past_blocks_selected(nb), int(cfg.always_select_current),
+            nb, int(getattr(cfg, "gate_window", None) or 0), int(getattr(cfg, "gate_sinks", 0)))
+
+
 def make_problem(q_shape, kv_heads: int, dtype: torch.dtype, cfg, cu_seqlens=None,
                  max_seqlen=None, causal: bool = True, part_f32: bool = False,
                  chunk_tiles=None, window=None) -> Problem:
@@ -238,13 +246,12 @@ def make_problem(q_shape, kv_heads: int, dtype: torch.dtype, cfg, cu_seqlens=Non
     packed = cu_seqlens is not None
     n_seq = cu_seqlens.numel() - 1 if packed else b
     longest = max_seqlen if packed else s
-    nb = cfg.num_blocks(longest)
+    block_size, top_k, slots, take, always, nb, gate_window, gate_sinks = config_fields(cfg, longest)
     return Problem(
         dtype=dtype_code(dtype), batch=b, tokens=s, n_seq=n_seq, max_seqlen=longest,
-        q_heads=hq, kv_heads=kv_heads, head_dim=d, block_size=cfg.block_size, top_k=cfg.top_k,
-        slots=cfg.slots_per_query, take=cfg.past_blocks_selected(nb),
-        always_current=int(cfg.always_select_current), num_blocks=nb, causal=int(causal),
+        q_heads=hq, kv_heads=kv_heads, head_dim=d, block_size=block_size, top_k=top_k,
+        slots=slots, take=take, always_current=always, num_blocks=nb, causal=int(causal),
         packed=int(packed), path=_force_path[0], part_f32=int(part_f32),
         chunk_tiles=_chunk_tiles[0] if chunk_tiles is None else int(chunk_tiles),
-        gate_window=int(getattr(cfg, "gate_window", None) or 0), gate_sinks=int(getattr(cfg, "gate_sinks", 0)),
+        gate_window=gate_window, gate_sinks=gate_sinks,
         win_begin=0 if window is None else int(window[0]), win_rows=0 if window is None else int(window[1]))

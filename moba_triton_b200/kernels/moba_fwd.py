@@ -8,6 +8,7 @@ same quantities. `combine_partials` still accepts the reference's triple.
 """
 
 import ctypes
+from operator import index as whole_number
 from typing import Optional
 
 import torch
@@ -70,14 +71,21 @@ _MAX_PLANS = 512
 
 
 def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, partials_dtype=None) -> "_OpPlan":
-    """Validates a call and returns its plan; a call like an earlier one skips both."""
+    """Validates a call and returns its plan; a call like an earlier one skips both. Calls are told
+    apart by values: a `MoBAConfig` is frozen and compares by its fields; of any other configuration
+    object the fields are read on every call, and a `max_seqlen` that is a tensor is read too."""
     on_gpu = q.is_cuda and k.is_cuda and v.is_cuda and (cu_seqlens is None or cu_seqlens.is_cuda)
-    key = (q.shape, k.shape, v.shape, q.dtype, k.dtype, v.dtype, cfg, causal, max_seqlen, partials_dtype,
-           None if cu_seqlens is None else (cu_seqlens.shape, cu_seqlens.dtype),
-           _lib._force_path[0], _lib._chunk_tiles[0])
+    fields = cfg
+    if type(cfg) is not MoBAConfig:
+        _validate(q, k, v, cfg, cu_seqlens, max_seqlen)
+        fields = _lib.config_fields(cfg, q.shape[1] if cu_seqlens is None else max_seqlen)
     try:
+        key = (q.shape, k.shape, v.shape, q.dtype, k.dtype, v.dtype, fields, bool(causal),
+               None if max_seqlen is None else whole_number(max_seqlen), partials_dtype,
+               None if cu_seqlens is None else (cu_seqlens.shape, cu_seqlens.dtype),
+               _lib._force_path[0], _lib._chunk_tiles[0])
         plan = _PLANS.get(key) if on_gpu else None
-    except TypeError:                                        # a foreign configuration object that cannot be hashed
+    except TypeError:                                        # nothing to tell the call by; refused below if it is wrong
         key = None
         plan = None
     if plan is not None:

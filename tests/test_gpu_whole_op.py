@@ -11,6 +11,7 @@ import pytest
 import torch
 
 import moba_triton_b200 as moba
+from moba_triton_b200.kernels.moba_fwd import op_plan
 
 from conftest import make_qkv
 from helpers import max_abs_error
@@ -76,6 +77,34 @@ def test_finer_blocks_with_the_other_options(flags, device):
     for staged, whole in zip(*got):
         assert torch.equal(torch.isnan(staged), torch.isnan(whole))          # no own block: the first rows select nothing
         assert max_abs_error(staged.nan_to_num(), whole.nan_to_num()) <= 2e-2
+
+
+class OpenConfig:
+    """A configuration object of a caller's own: hashable by identity, and mutable."""
+    block_size, top_k, always_select_current = 128, 2, True
+    slots_per_query = property(lambda self: self.top_k)
+
+    def num_blocks(self, n):
+        return -(-n // self.block_size)
+
+    def past_blocks_selected(self, nb):
+        return min(self.top_k - 1, nb)
+
+
+def test_a_call_is_told_from_an_earlier_one_by_values(device):
+    q, k, v = (t.to(device) for t in make_qkv((1, 1000, 2, 64), 2, dtype=torch.bfloat16, seed=63))
+    cfg = OpenConfig()
+    for top_k, block in ((2, 128), (4, 128), (4, 64)):
+        cfg.top_k, cfg.block_size = top_k, block
+        want = moba.moba_forward(q, k, v, moba.MoBAConfig(block, top_k))
+        assert torch.equal(moba.moba_forward(q, k, v, cfg), want)
+        assert torch.equal(moba.moba_attention(q, k, v, cfg), want)
+    # a length that is a tensor, changed in place
+    longest, frozen = torch.tensor(1000, device=device), moba.MoBAConfig(128, 4)
+    for cu in ([0, 300, 1000], [0, 400, 1000]):
+        longest.fill_(max(b - a for a, b in zip(cu[:-1], cu[1:])))
+        cu = torch.tensor(cu, dtype=torch.int32, device=device)
+        assert op_plan(q, k, v, frozen, True, cu, longest).problem.max_seqlen == int(longest)
 
 
 @pytest.mark.parametrize("d,top_k", [(64, 8), (64, 3), (128, 9)])
