@@ -102,9 +102,11 @@ struct Bars {
 
 // AND of a predicate over the threads of a warpgroup (named barrier `id`). Every decision
 // that steers a warpgroup past one of its own barriers is taken through this, so that a wait
-// that gave up in some threads only can never leave the others alone at a barrier.
+// that gave up in some threads only can never leave the others alone at a barrier. The barrier
+// counts warps, whole ones.
 __device__ __forceinline__ bool group_all(bool pred, int id) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"

@@ -190,9 +190,10 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
 
 // AND of a predicate over the threads of a role (named barrier `id`): whoever leaves a role's
 // loop leaves it together, so that a wait that gave up in some threads cannot leave the others
-// alone at a named barrier.
+// alone at a named barrier. The barrier counts warps, whole ones.
 __device__ __forceinline__ bool group_all(bool pred, int id, int threads) {
   uint32_t r;
+  __syncwarp();
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 q, %1, 0;\n\t"
@@ -283,6 +284,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           T* base = (wq == 0 ? dv : dk) + ((size_t)(c.tok0 + c.key0 + r) * p.kv_heads + kvh) * (size_t)D;
           for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(base)[i] = make_uint4(0, 0, 0, 0);
         }
+        __syncwarp();                                  // a block cut short parts the warp, and a named barrier comes next
         continue;
       }
       const int nt = (c.n + kTile - 1) / kTile;

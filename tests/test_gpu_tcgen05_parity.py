@@ -300,3 +300,37 @@ def test_candidate_window_through_the_whole_op(device):
     cfg = moba.MoBAConfig(128, 4, gate_window=3, gate_sinks=1)
     _check_op((1, 2048, 4, 64), 2, torch.bfloat16, cfg, device, seed=63)
     _check_op((1, 1841, 4, 128), 2, torch.bfloat16, cfg, device, cu=[0, 384, 513, 1513, 1641, 1841], seed=64)
+
+
+# ---------------------------------------------------------------------------
+# columns that nobody lists, cut short by the end of their sequence
+# ---------------------------------------------------------------------------
+
+@pytest.mark.parametrize("d,s", [(64, 1201), (128, 1201), (64, 130), (64, 700)])
+def test_an_unlisted_block_cut_short(d, s, device):
+    """Without the own block the last block of a sequence is never selected. Its dK and dV are
+    exact zeros, written by part of a warp where its length is no multiple of 32."""
+    cfg = moba.MoBAConfig(128, 3, always_select_current=False)
+    q, k, v, do = make_qkv((2, s, 4, d), 2, dtype=torch.bfloat16, seed=41, with_do=True)
+    qd, kd, vd, dod = (t.to(device) for t in (q, k, v, do))
+    block_idx = moba.gate_select(qd, moba.pool_blocks(kd, cfg), cfg)
+    t_out, _, t_dq, t_dk, t_dv = oracle_forward(q, k, v, cfg, block_idx, dout=do)
+    got = _grads(qd, kd, vd, cfg, dod)
+    rows = ~torch.isnan(t_out)                                # the first block's queries select nothing
+    assert torch.equal(~torch.isnan(got[0].cpu()), rows)
+    assert max_abs_error(got[0].cpu().double()[rows], t_out[rows]) <= ATOL[torch.bfloat16]
+    for g, t in zip(got[1:], (t_dq, t_dk, t_dv)):
+        assert max_abs_error(g, t) <= ATOL[torch.bfloat16]
+    last = s // 128 * 128
+    assert not got[2][:, last:].any() and not got[3][:, last:].any()
+
+
+@pytest.mark.parametrize("chunk", [400, 333])
+def test_query_windows_of_a_ragged_sequence(chunk, device):
+    """The first windows have no query in the last block, which ends inside a warp's 32 keys."""
+    cfg = moba.MoBAConfig(128, 4)
+    q, k, v, do = (t.to(device) for t in make_qkv((2, 1201, 4, 64), 2, dtype=torch.bfloat16, seed=42, with_do=True))
+    whole, got = _grads(q, k, v, cfg, do), _grads(q, k, v, cfg, do, query_chunk=chunk)
+    assert torch.equal(got[0], whole[0]) and torch.equal(got[1], whole[1])
+    for g, w in zip(got[2:], whole[2:]):
+        assert max_abs_error(g, w) <= ATOL[torch.bfloat16]
