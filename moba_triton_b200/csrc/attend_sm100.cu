@@ -82,7 +82,9 @@ struct RowMeta {                           // of a tile in flight, written by th
 };
 
 struct Bars {
-  uint64_t k_full[2], v_full[2], k_free[2], v_free[2], k_fix, v_fix;
+  uint64_t k_full[2], v_full[2], k_free[2], v_free[2];
+  uint64_t k_fix[2], v_fix[2];             // per K / V buffer: the rows of a block cut short are zeroed (one for
+                                           // both could complete twice before its first phase is looked at)
   uint64_t q_full[4];                      // per buffer: the tile's rows have landed and its row data is written
   uint64_t q_empty[4];                     // the S MMA that read the stage has retired
   uint64_t meta_free[4];                   // the softmax warps have read the row data
@@ -206,10 +208,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       mbar_init(&bars->k_full[i], 1); mbar_init(&bars->v_full[i], 1);
       mbar_init(&bars->k_free[i], 1); mbar_init(&bars->v_free[i], 1);
       mbar_init(&bars->o_staged[i], 4); mbar_init(&bars->stage_free[i], 4); mbar_init(&bars->sp_free[i], 1);
-      mbar_init(&bars->drain[i], 1);
+      mbar_init(&bars->drain[i], 1); mbar_init(&bars->k_fix[i], 1); mbar_init(&bars->v_fix[i], 1);
       bars->stored_end[i] = 0;
     }
-    mbar_init(&bars->k_fix, 1); mbar_init(&bars->v_fix, 1);
     for (int i = 0; i < 4; ++i) {
       mbar_init(&bars->q_full[i], kGatherWarps); mbar_init(&bars->q_empty[i], 1); mbar_init(&bars->meta_free[i], 4);
       mbar_init(&bars->s_full[i], 1); mbar_init(&bars->p_full[i], 4);
@@ -480,7 +481,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         const uint32_t fbits = (fmt << 7) | (fmt << 10);
         const uint32_t aQ = smem_u32(sQ);
         const bool is_s = warp == Cfg::kScoreWarp;
-        uint32_t t = 0, pt = 0;                                   // tiles issued, cut-short columns seen
+        uint32_t t = 0, fixes = 0;                                // tiles issued; bit b: parity of the cut-short columns seen in buffer b
         for (uint32_t it = 0;; ++it) {
           if (!mbar_wait(&bars->col_full[it & 7], (it >> 3) & 1, wc, 20)) break;
           const int n = bars->cols[it & 7].n;
@@ -500,7 +501,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
               if (u >= 1) mbar_wait(D == 128 ? &bars->sp_free[b] : &bars->so_free[b], (u - 1) & 1, wc, 22);
               if (i == 0) {
                 mbar_wait(&bars->k_full[kb], ku & 1, wc, 23);
-                if (partial) mbar_wait(&bars->k_fix, pt & 1, wc, 23);
+                if (partial) mbar_wait(&bars->k_fix[kb], fixes >> kb & 1, wc, 23);
               }
               tc_fence_after();
               const uint32_t qb = aQ + b * Cfg::kOperand;
@@ -519,7 +520,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
               if (D == 128 && u >= 1) mbar_wait(&bars->so_free[b], (u - 1) & 1, wc, 24);   // the O columns have been read out
               if (i == 0) {
                 mbar_wait(&bars->v_full[kb], ku & 1, wc, 25);
-                if (partial) mbar_wait(&bars->v_fix, pt & 1, wc, 25);
+                if (partial) mbar_wait(&bars->v_fix[kb], fixes >> kb & 1, wc, 25);
               }
               tc_fence_after();
               // operand A: P from TMEM, 16 keys (eight columns of 16-bit pairs) per step
@@ -533,7 +534,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
               if (i == nt - 1) umma_commit(&bars->v_free[kb]);
             }
           }
-          if (partial) ++pt;
+          if (partial) fixes ^= 1u << kb;
         }
         // Every MMA of this thread has completed before the CTA lets go of its TMEM, also on
         // the way out of a run that gave up on a wait.
@@ -630,14 +631,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             *reinterpret_cast<uint4*>(bK + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async();
-          mbar_arrive_warp(&bars->k_fix);
+          mbar_arrive_warp(&bars->k_fix[kb]);
           mbar_wait(&bars->v_full[kb], ku & 1, wc, 9);
           for (int i = lane; i < dead * 8 * Cfg::kSubs; i += 32) {
             const int s = i / (dead * 8), rr = c.keys + (i % (dead * 8)) / 8, ch = i % 8;
             *reinterpret_cast<uint4*>(bV + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async();
-          mbar_arrive_warp(&bars->v_fix);
+          mbar_arrive_warp(&bars->v_fix[kb]);
         }
         ++it_cnt;
         c = c_next;

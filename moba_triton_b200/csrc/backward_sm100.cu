@@ -61,7 +61,7 @@ template <int D> struct BwdCfg {
   static constexpr int kSBufs = D == 64 ? 2 : 1;         // S buffers in TMEM
   static constexpr int kDsBytes = 2 * kSub;              // dS tile [keys][queries]; dQ is staged in it too
   static constexpr int kSmemData = 2 * kKvBufs * kOperand + 2 * kStages * kOperand + kDsBytes;
-  static constexpr int kBarBytes = D == 64 ? 5120 : 3072;   // barriers and per-stage row data; 227 KB in all at 128
+  static constexpr int kBarBytes = D == 64 ? 5632 : 3072;   // barriers and per-stage row data; 227 KB in all at 128
   static constexpr int kSmem = kSmemData + kBarBytes;
   static_assert(kSmem <= 232448, "shared memory of an SM");
   static constexpr uint32_t cS = 0, cDP = 128 * kSBufs, cDV = cDP + 128, cDK = cDV + D;
@@ -85,7 +85,9 @@ struct Meta {                                            // of the queries of on
 
 template <int D> struct Bars {
   Meta meta[BwdCfg<D>::kStages];
-  uint64_t k_full[2], v_full[2], k_free[2], v_free[2], k_fix, v_fix;
+  uint64_t k_full[2], v_full[2], k_free[2], v_free[2];
+  uint64_t k_fix[BwdCfg<D>::kKvBufs], v_fix[BwdCfg<D>::kKvBufs];   // per K / V buffer: the rows of a block cut short are zeroed (one for
+                                                         // both could complete twice before its first phase is looked at)
   uint64_t q_full[3], q_empty[3], g_full[3], g_empty[3]; // gather stages of Q (with the row data) and dO
   uint64_t s_full[2], dq_full[2], dq_read[2];   // per S buffer: at head_dim 64 two tiles' dQ can be waiting to be stored
   uint64_t dp_full, p_full, ds_full, p_used, acc_full, acc_read, drain[2];
@@ -239,8 +241,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       mbar_init(&bars->q_full[i], kGatherWarps); mbar_init(&bars->g_full[i], kGatherWarps);
       mbar_init(&bars->q_empty[i], 1); mbar_init(&bars->g_empty[i], 2);      // dK (after S); dP and dV, in either order
     }
+    for (int i = 0; i < NKV; ++i) { mbar_init(&bars->k_fix[i], kGatherWarps); mbar_init(&bars->v_fix[i], kGatherWarps); }
     for (int i = 0; i < 4; ++i) { mbar_init(&bars->col_full[i], 1); mbar_init(&bars->col_free[i], kElemWarps + 2 + kGatherWarps + kStoreWarps); }
-    mbar_init(&bars->k_fix, kGatherWarps); mbar_init(&bars->v_fix, kGatherWarps);
     mbar_init(&bars->dp_full, 1); mbar_init(&bars->p_full, kElemWarps); mbar_init(&bars->ds_full, kElemWarps);
     mbar_init(&bars->acc_full, 1); mbar_init(&bars->acc_read, kElemWarps);
     mbar_init(&bars->p_used, 1); mbar_init(&bars->drain[0], 1); mbar_init(&bars->drain[1], 1);
@@ -486,8 +488,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       const uint32_t fbits = (fmt << 7) | (fmt << 10);
       const uint32_t aS = smem_u32(sS);
       // The CTA's items that have tiles, in order; false at the end of the stream.
-      struct Item { int nt; bool partial; uint32_t kb, ku, pt; };
-      uint32_t it = 0, n_seen = 0, partials = 0, t = 0;
+      struct Item { int nt; bool partial; uint32_t kb, ku, fix; };
+      uint32_t it = 0, n_seen = 0, fixes = 0, t = 0;           // fixes, bit b: parity of the cut-short columns seen in buffer b
       auto next_item = [&](Item& c) -> bool {
         for (;;) {
           if (!sound || !mbar_wait(&bars->col_full[it & 3], (it >> 2) & 1, wc, 20)) return false;
@@ -497,9 +499,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           if (n < 0) return false;
           if (n == 0) continue;
           c.nt = (n + kTile - 1) / kTile; c.partial = keys < kTile;
-          c.kb = n_seen % NKV; c.ku = n_seen / NKV; c.pt = partials;
+          c.kb = n_seen % NKV; c.ku = n_seen / NKV; c.fix = fixes >> c.kb & 1;
           ++n_seen;
-          if (c.partial) ++partials;
+          if (c.partial) fixes ^= 1u << c.kb;
           return true;
         }
       };
@@ -513,7 +515,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             const uint32_t aQ = smem_u32(sQ) + st * Cfg::kOperand, aG = smem_u32(sG) + st * Cfg::kOperand;
             if (i == 0) {
               mbar_wait(&bars->k_full[c.kb], c.ku & 1, wc, 21);
-              if (c.partial) mbar_wait(&bars->k_fix, c.pt & 1, wc, 21);
+              if (c.partial) mbar_wait(&bars->k_fix[c.kb], c.fix, wc, 21);
             }
             mbar_wait(&bars->q_full[st], us & 1, wc, 22);
             // the S buffer: two tiles ago its dQ sat there (64); dV of the tile before has read P (128)
@@ -528,7 +530,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             if (leader) umma_commit(&bars->s_full[t % NS]);
             if (i == 0) {
               mbar_wait(&bars->v_full[c.kb], c.ku & 1, wc, 24);
-              if (c.partial) mbar_wait(&bars->v_fix, c.pt & 1, wc, 24);
+              if (c.partial) mbar_wait(&bars->v_fix[c.kb], c.fix, wc, 24);
             }
             mbar_wait(&bars->g_full[st], us & 1, wc, 24);
             // the dP columns: dK of the tile before has read dS there (64); its dQ has been read out (128)
@@ -714,14 +716,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             *reinterpret_cast<uint4*>(sV + kb * Cfg::kOperand + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async();
-          mbar_arrive_warp(&bars->v_fix);
+          mbar_arrive_warp(&bars->v_fix[kb]);
           mbar_wait(&bars->k_full[kb], ku & 1, wc, 14);
           for (int i = pt; i < dead * 8 * Cfg::kSubs; i += 32 * kGatherWarps) {
             const int s = i / (dead * 8), rr = c.keys + (i % (dead * 8)) / 8, ch = i % 8;
             *reinterpret_cast<uint4*>(sK + kb * Cfg::kOperand + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
           }
           fence_proxy_async();
-          mbar_arrive_warp(&bars->k_fix);
+          mbar_arrive_warp(&bars->k_fix[kb]);
         }
         ++n_seen;
         int i = 0;

@@ -325,6 +325,21 @@ def test_an_unlisted_block_cut_short(d, s, device):
     assert not got[2][:, last:].any() and not got[3][:, last:].any()
 
 
+@pytest.mark.parametrize("d", [64, 128])
+def test_many_short_sequences(d, device):
+    """Sequences of 1 to 200 tokens, far more than CTAs: item after item whose block is cut short."""
+    g = torch.Generator().manual_seed(d)
+    cu = torch.cat([torch.zeros(1, dtype=torch.int64), torch.randint(1, 201, (600,), generator=g).cumsum(0)]).int()
+    cfg, total, longest = moba.MoBAConfig(128, 2), int(cu[-1]), int((cu[1:] - cu[:-1]).max())
+    q, k, v, do = make_qkv((1, total, 4, d), 2, dtype=torch.bfloat16, seed=43, with_do=True)
+    qd, kd, vd, dod = (t.to(device) for t in (q, k, v, do))
+    kw = dict(cu_seqlens=cu.to(device), max_seqlen=longest)
+    block_idx = moba.gate_select(qd, moba.pool_blocks(kd, cfg, **kw), cfg, **kw)
+    t_out, _, t_dq, t_dk, t_dv = oracle_forward(q, k, v, cfg, block_idx, cu=cu, dout=do)
+    for got, want in zip(_grads(qd, kd, vd, cfg, dod, **kw), (t_out, t_dq, t_dk, t_dv)):
+        assert max_abs_error(got, want) <= ATOL[torch.bfloat16]
+
+
 @pytest.mark.parametrize("chunk", [400, 333])
 def test_query_windows_of_a_ragged_sequence(chunk, device):
     """The first windows have no query in the last block, which ends inside a warp's 32 keys."""
