@@ -264,6 +264,23 @@ int moba_b200_op_backward(const moba_b200_problem* p, const void* q, const void*
                           const void* dout, const int32_t* cu_seqlens, const void* keep_ws, void* backward_ws,
                           void* dq, void* dk, void* dv, void* stream);
 
+/* The same from the block ids on, for the query window of the problem record (win_begin, win_rows;
+ * padded batches): host-side chunking along the query axis. block_idx [B,Hq,S,slots] is that of
+ * moba_b200_gate for the whole batch, moba_b200_op_workspace gives the sizes for the window's
+ * record, and a window keeps nothing: the backward builds its index again.
+ *   moba_b200_op_forward_window   the window's rows of out, and of lse [B,Hq,S] (may be NULL)
+ *   moba_b200_op_backward_window  the window's rows of dq, and its contribution to dk and dv; lse as
+ *                                 the forward left it, part_lse [B,Hq,win_rows,slots]: 0 where the
+ *                                 slot names a block, -inf where it does not
+ * O and dQ are the bits of the whole op. The reference planned this chunking and never built it
+ * (docs/deferred-decisions.md:152-220). */
+int moba_b200_op_forward_window(const moba_b200_problem* p, const void* q, const void* k, const void* v,
+                                const int32_t* block_idx, void* keep_ws, void* forward_ws, void* out, float* lse,
+                                void* stream);
+int moba_b200_op_backward_window(const moba_b200_problem* p, const void* q, const void* k, const void* v, const void* out,
+                                 const void* dout, const float* lse, const float* part_lse, const int32_t* block_idx,
+                                 void* keep_ws, void* backward_ws, void* dq, void* dk, void* dv, void* stream);
+
 /* Packed (variable-length) batches, the step either side of the op. A "row" is
  * one token's H*D elements (row_bytes, a multiple of 16), contiguous in the
  * token-major layout.

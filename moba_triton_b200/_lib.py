@@ -30,6 +30,7 @@ EXPORTS = (
     "moba_b200_chunk_tiles", "moba_b200_work_items_per_row", "moba_b200_dkv_scratch_bytes",
     "moba_b200_launch_plan",
     "moba_b200_op_workspace", "moba_b200_op_forward", "moba_b200_op_backward",
+    "moba_b200_op_forward_window", "moba_b200_op_backward_window",
 )
 
 
@@ -90,6 +91,8 @@ def load():
     lib.moba_b200_op_workspace.argtypes = [P, SZ, SZ, SZ]
     lib.moba_b200_op_forward.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, c_int, vp]
     lib.moba_b200_op_backward.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
+    lib.moba_b200_op_forward_window.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, vp, vp]
+    lib.moba_b200_op_backward_window.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     lib.moba_b200_pack_index.argtypes = [vp, c_int, c_int, c_int, vp, vp, vp, vp, vp]
     lib.moba_b200_pack_rows.argtypes = [vp, vp, vp, vp, c_int, c_int, c_size_t, vp]
     lib.moba_b200_unpack_rows.argtypes = [vp, vp, vp, c_int, c_int, c_size_t, vp]

@@ -5,6 +5,10 @@
 // thousand-token training step, 100 of the 150 us of an 8 192-token forward), the passes that
 // only the separate entry points need (the fill of the partial log-sum-exps, the public form of
 // the index) and, for short rows, four of the transpose's five launches.
+//
+// moba_b200_op_forward_window / _backward_window run the second half of each (from the block ids on)
+// for a window of query rows, on the same kernels, so that a call run window by window gives the bits
+// of the whole one whatever its block size.
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -53,17 +57,22 @@ Columns columns_of(const moba_b200_problem& p) {
   return c;
 }
 
-// Byte offsets of the buffers inside the caller's workspaces.
+// Byte offsets of the buffers inside the caller's workspaces. A window call gets block ids and the
+// log-sum-exps from its caller and keeps nothing: its index is built again by the backward.
 struct Layout {
   size_t col_nnz, col_offsets, order, items, entries, part_lse, lse, keep_bytes;      // kept for the backward
   size_t kbar, norms, block_idx, counter, transpose_scratch, part_o, fwd_bytes;              // forward only
-  size_t delta, dq_part, dkv, bwd_bytes;                                              // backward only
+  size_t delta, dq_part, dkv, bwd_transpose_scratch, bwd_bytes;                       // backward only
 };
+inline long long row_capacity(const moba_b200_problem& p) {
+  return (long long)(p.q_heads / p.kv_heads) * window_rows_of_seq(p) * p.slots;
+}
 Layout layout_of(const moba_b200_problem& gate, const moba_b200_problem& p) {
   Layout l;
   const size_t rows = (size_t)p.n_seq * p.kv_heads, nb = p.num_blocks;
-  const size_t pairs = (size_t)p.batch * p.q_heads * p.tokens * p.slots;
-  const size_t capacity = (size_t)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
+  const size_t pairs = (size_t)p.batch * p.q_heads * window_rows(p) * p.slots;
+  const size_t capacity = (size_t)row_capacity(p);
+  const bool window = p.win_rows > 0;
   size_t at = 0;
   auto take = [&](size_t bytes) { const size_t o = at; at = up(at + bytes); return o; };
   l.col_nnz = take(rows * nb * 4);
@@ -72,21 +81,23 @@ Layout layout_of(const moba_b200_problem& gate, const moba_b200_problem& p) {
   l.items = take(rows * (size_t)sched_items_per_row(p) * 16);
   l.entries = take(rows * capacity * 8);
   l.part_lse = take(pairs * 4);
-  l.lse = take((size_t)p.batch * p.q_heads * p.tokens * 4);
+  l.lse = take(window ? 0 : (size_t)p.batch * p.q_heads * p.tokens * 4);
   l.keep_bytes = at;
   at = 0;
   const size_t part_size = p.part_f32 ? 4 : dtype_size(p.dtype);
-  l.kbar = take(rows * gate.num_blocks * p.head_dim * dtype_size(p.dtype));
-  l.norms = take(rows * gate.num_blocks * 4);
-  l.block_idx = take(pairs * 4);
+  const size_t scratch = transpose_small_supported(p) ? 16 : transpose_scratch_bytes(p);
+  l.kbar = take(window ? 0 : rows * gate.num_blocks * p.head_dim * dtype_size(p.dtype));
+  l.norms = take(window ? 0 : rows * gate.num_blocks * 4);
+  l.block_idx = take(window ? 0 : pairs * 4);
   l.counter = take(16);
-  l.transpose_scratch = take(transpose_small_supported(p) ? 16 : transpose_scratch_bytes(p));
+  l.transpose_scratch = take(scratch);
   l.part_o = take(pairs * p.head_dim * part_size);
   l.fwd_bytes = at;
   at = 0;
   l.delta = take((size_t)p.batch * p.q_heads * p.tokens * 4);
   l.dq_part = take(pairs * p.head_dim * dtype_size(p.dtype));
   l.dkv = take(sched_dkv_scratch_bytes(p));
+  l.bwd_transpose_scratch = take(window ? scratch : 0);
   l.bwd_bytes = at;
   return l;
 }
@@ -96,7 +107,7 @@ moba_b200_index index_in(const moba_b200_problem& p, const Layout& l, unsigned c
   ix.col_nnz = reinterpret_cast<int32_t*>(keep + l.col_nnz);
   ix.col_offsets = reinterpret_cast<int32_t*>(keep + l.col_offsets);
   ix.order = reinterpret_cast<int32_t*>(keep + l.order);
-  ix.capacity = (long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots;
+  ix.capacity = row_capacity(p);
   ix.work_items = reinterpret_cast<int32_t*>(keep + l.items);
   ix.items_per_row = (int)sched_items_per_row(p);
   ix.chunk_tiles = sched_chunk_tiles(p);
@@ -104,15 +115,68 @@ moba_b200_index index_in(const moba_b200_problem& p, const Layout& l, unsigned c
   return ix;
 }
 
-int check_op(const moba_b200_problem* p) {
+int check_sizes(const moba_b200_problem* p) {
   MOBA_TRY(check_problem(p));
-  if (p->win_rows > 0) { set_error("the whole-op entry points take no query window"); return MOBA_B200_EUNSUPPORTED; }
   if (p->q_heads >= 1 << 19) { set_error("%d query heads do not fit a packed index entry", p->q_heads); return MOBA_B200_EUNSUPPORTED; }
   if (sched_items_per_row(*p) > 0x7fffffffLL || sched_part_slots(*p) > 0x7fffffffLL) {
     set_error("chunk_tiles %d cuts the problem into too many work items", sched_chunk_tiles(*p));
     return MOBA_B200_EUNSUPPORTED;
   }
   return MOBA_B200_OK;
+}
+int check_op(const moba_b200_problem* p) {
+  MOBA_TRY(check_sizes(p));
+  if (p->win_rows > 0) { set_error("the whole-op entry points take no query window"); return MOBA_B200_EUNSUPPORTED; }
+  return MOBA_B200_OK;
+}
+int check_window(const moba_b200_problem* p) {
+  MOBA_TRY(check_sizes(p));
+  if (p->win_rows == 0) { set_error("a window call needs a query window"); return MOBA_B200_EINVAL; }
+  return MOBA_B200_OK;
+}
+
+int transpose_into(const Columns& c, const moba_b200_index& ix, const int32_t* block_idx, const int32_t* cu, void* scratch,
+                   int32_t* counter, cudaStream_t st) {
+  const moba_b200_problem& p = c.p;
+  int32_t* col_nnz = const_cast<int32_t*>(ix.col_nnz);
+  int32_t* col_offsets = const_cast<int32_t*>(ix.col_offsets);
+  int32_t* order = const_cast<int32_t*>(ix.order);
+  int32_t* items = const_cast<int32_t*>(ix.work_items);
+  int2* entries = reinterpret_cast<int2*>(const_cast<int32_t*>(ix.row_indices));
+  if (transpose_small_supported(p))
+    return launch_transpose_small(p, block_idx, cu, col_nnz, col_offsets, order, entries, c.part_shift, items, counter, st);
+  return launch_transpose(p, block_idx, cu, col_nnz, col_offsets, order, nullptr, nullptr, nullptr, entries, c.part_shift, items,
+                          scratch, transpose_scratch_bytes(p), st);
+}
+
+// From block ids to the output: transpose, attention, merge.
+int attend(const Columns& c, const Layout& l, int fwd_path, const void* q, const void* k, const void* v, const int32_t* block_idx,
+           const int32_t* cu, unsigned char* keep, unsigned char* tmp, void* out, float* lse, cudaStream_t st) {
+  const moba_b200_problem& p = c.p;
+  const moba_b200_index ix = index_in(p, l, keep);
+  float* part_lse = reinterpret_cast<float*>(keep + l.part_lse);
+  void* part_o = tmp + l.part_o;
+  MOBA_TRY(transpose_into(c, ix, block_idx, cu, tmp + l.transpose_scratch, reinterpret_cast<int32_t*>(tmp + l.counter), st));
+  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu, part_o, part_lse, c.part_keys, st));
+  else MOBA_TRY(launch_fwd_portable(p, q, k, v, ix, cu, part_o, part_lse, st));
+  return launch_merge(p, part_o, part_lse, out, lse, st);
+}
+
+// The gradients from an index: delta, dK/dV and dQ partials, reductions.
+int differentiate(const Columns& c, const Layout& l, int path, const void* q, const void* k, const void* v, const void* out,
+                  const void* dout, const float* lse, const float* part_lse, const int32_t* cu, unsigned char* keep,
+                  unsigned char* tmp, void* dq, void* dk, void* dv, cudaStream_t st) {
+  const moba_b200_problem& p = c.p;
+  const moba_b200_index ix = index_in(p, l, keep);
+  float* delta = reinterpret_cast<float*>(tmp + l.delta);
+  void* dq_part = tmp + l.dq_part;
+  bool reduces = false;
+  MOBA_TRY(launch_delta(p, out, dout, delta, st));
+  if (path == MOBA_B200_PATH_TCGEN05)
+    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, c.part_keys, &reduces, st));
+  else
+    MOBA_TRY(launch_bwd_portable(p, q, k, v, dout, lse, delta, ix, cu, dq_part, dk, dv, st));
+  return launch_dq_reduce(p, dq_part, part_lse, dq, reduces, st);
 }
 
 }  // namespace
@@ -123,7 +187,7 @@ using namespace moba;
 extern "C" {
 
 int moba_b200_op_workspace(const moba_b200_problem* p0, size_t* keep_bytes, size_t* forward_bytes, size_t* backward_bytes) {
-  MOBA_TRY(check_op(p0));
+  MOBA_TRY(check_sizes(p0));
   const moba_b200_problem gate = with_cut(*p0);
   const Layout l = layout_of(gate, columns_of(gate).p);
   if (keep_bytes) *keep_bytes = l.keep_bytes;
@@ -148,15 +212,10 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   const Layout l = layout_of(gate, p);
   unsigned char* keep = static_cast<unsigned char*>(keep_ws);
   unsigned char* tmp = static_cast<unsigned char*>(forward_ws);
-  const moba_b200_index ix = index_in(p, l, keep);
   void* kbar = tmp + l.kbar;
   int32_t* block_idx = reinterpret_cast<int32_t*>(tmp + l.block_idx);
   float* part_lse = reinterpret_cast<float*>(keep + l.part_lse);
-  void* part_o = tmp + l.part_o;
   int32_t* counter = reinterpret_cast<int32_t*>(tmp + l.counter);
-  int32_t* col_nnz = const_cast<int32_t*>(ix.col_nnz);
-  int32_t* col_offsets = const_cast<int32_t*>(ix.col_offsets);
-  int32_t* items = const_cast<int32_t*>(ix.work_items);
   // Where the portable gate would run by the library's choice, its selections come from the exact
   // tensor-core gate if that covers the problem.
   const bool exact_gate = gate_path == MOBA_B200_PATH_PORTABLE && gate.path == MOBA_B200_PATH_AUTO && gate_exact_sm100_supported(gate);
@@ -165,16 +224,8 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
   else if (exact_gate) MOBA_TRY(launch_gate_exact_sm100(gate, q, kbar, norms, cu_seqlens, block_idx, part_lse, st));
   else MOBA_TRY(launch_gate_portable(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
-  int2* entries = reinterpret_cast<int2*>(const_cast<int32_t*>(ix.row_indices));
-  int32_t* order = const_cast<int32_t*>(ix.order);
-  if (transpose_small_supported(p))
-    MOBA_TRY(launch_transpose_small(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, entries, columns.part_shift, items, counter, st));
-  else
-    MOBA_TRY(launch_transpose(p, block_idx, cu_seqlens, col_nnz, col_offsets, order, nullptr, nullptr, nullptr, entries, columns.part_shift, items,
-                              tmp + l.transpose_scratch, transpose_scratch_bytes(p), st));
-  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu_seqlens, part_o, part_lse, columns.part_keys, st));
-  else MOBA_TRY(launch_fwd_portable(p, q, k, v, ix, cu_seqlens, part_o, part_lse, st));
-  return launch_merge(p, part_o, part_lse, out, want_lse ? reinterpret_cast<float*>(keep + l.lse) : nullptr, st);
+  return attend(columns, l, fwd_path, q, k, v, block_idx, cu_seqlens, keep, tmp, out,
+                want_lse ? reinterpret_cast<float*>(keep + l.lse) : nullptr, st);
 }
 
 int moba_b200_op_backward(const moba_b200_problem* p0, const void* q, const void* k, const void* v, const void* out,
@@ -194,18 +245,46 @@ int moba_b200_op_backward(const moba_b200_problem* p0, const void* q, const void
   const Layout l = layout_of(gate, p);
   unsigned char* keep = const_cast<unsigned char*>(static_cast<const unsigned char*>(keep_ws));
   unsigned char* tmp = static_cast<unsigned char*>(backward_ws);
-  const moba_b200_index ix = index_in(p, l, keep);
-  const float* part_lse = reinterpret_cast<const float*>(keep + l.part_lse);
-  const float* lse = reinterpret_cast<const float*>(keep + l.lse);
-  float* delta = reinterpret_cast<float*>(tmp + l.delta);
-  void* dq_part = tmp + l.dq_part;
-  bool reduces = false;
-  MOBA_TRY(launch_delta(p, out, dout, delta, st));
-  if (path == MOBA_B200_PATH_TCGEN05)
-    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, columns.part_keys, &reduces, st));
-  else
-    MOBA_TRY(launch_bwd_portable(p, q, k, v, dout, lse, delta, ix, cu_seqlens, dq_part, dk, dv, st));
-  return launch_dq_reduce(p, dq_part, part_lse, dq, reduces, st);
+  return differentiate(columns, l, path, q, k, v, out, dout, reinterpret_cast<const float*>(keep + l.lse),
+                       reinterpret_cast<const float*>(keep + l.part_lse), cu_seqlens, keep, tmp, dq, dk, dv, st);
+}
+
+int moba_b200_op_forward_window(const moba_b200_problem* p0, const void* q, const void* k, const void* v, const int32_t* block_idx,
+                                void* keep_ws, void* forward_ws, void* out, float* lse, void* stream) {
+  MOBA_TRY(check_window(p0));
+  MOBA_TRY(need(q, "q")); MOBA_TRY(need(k, "k")); MOBA_TRY(need(v, "v")); MOBA_TRY(need(out, "out"));
+  MOBA_TRY(need(block_idx, "block_idx")); MOBA_TRY(need(keep_ws, "keep_ws")); MOBA_TRY(need(forward_ws, "forward_ws"));
+  const moba_b200_problem gate = with_cut(*p0);
+  const Columns columns = columns_of(gate);
+  const moba_b200_problem& p = columns.p;
+  const int path = pick(p, fwd_sm100_supported(p), "forward");
+  if (path < 0) return path;
+  cudaStream_t st = (cudaStream_t)stream;
+  const Layout l = layout_of(gate, p);
+  unsigned char* keep = static_cast<unsigned char*>(keep_ws);
+  MOBA_TRY(launch_fill_lse(p, reinterpret_cast<float*>(keep + l.part_lse), st));
+  return attend(columns, l, path, q, k, v, block_idx, nullptr, keep, static_cast<unsigned char*>(forward_ws), out, lse, st);
+}
+
+int moba_b200_op_backward_window(const moba_b200_problem* p0, const void* q, const void* k, const void* v, const void* out,
+                                 const void* dout, const float* lse, const float* part_lse, const int32_t* block_idx, void* keep_ws,
+                                 void* backward_ws, void* dq, void* dk, void* dv, void* stream) {
+  MOBA_TRY(check_window(p0));
+  MOBA_TRY(need(q, "q")); MOBA_TRY(need(k, "k")); MOBA_TRY(need(v, "v")); MOBA_TRY(need(out, "out"));
+  MOBA_TRY(need(dout, "dout")); MOBA_TRY(need(lse, "lse")); MOBA_TRY(need(part_lse, "part_lse"));
+  MOBA_TRY(need(dq, "dq")); MOBA_TRY(need(dk, "dk")); MOBA_TRY(need(dv, "dv"));
+  MOBA_TRY(need(block_idx, "block_idx")); MOBA_TRY(need(keep_ws, "keep_ws")); MOBA_TRY(need(backward_ws, "backward_ws"));
+  const moba_b200_problem gate = with_cut(*p0);
+  const Columns columns = columns_of(gate);
+  const moba_b200_problem& p = columns.p;
+  const int path = pick(p, bwd_sm100_supported(p), "backward");
+  if (path < 0) return path;
+  cudaStream_t st = (cudaStream_t)stream;
+  const Layout l = layout_of(gate, p);
+  unsigned char* keep = static_cast<unsigned char*>(keep_ws);
+  unsigned char* tmp = static_cast<unsigned char*>(backward_ws);
+  MOBA_TRY(transpose_into(columns, index_in(p, l, keep), block_idx, nullptr, tmp + l.bwd_transpose_scratch, nullptr, st));
+  return differentiate(columns, l, path, q, k, v, out, dout, lse, part_lse, nullptr, keep, tmp, dq, dk, dv, st);
 }
 
 }  // extern "C"

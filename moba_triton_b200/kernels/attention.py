@@ -8,8 +8,8 @@ from moba_triton_b200 import _lib
 from moba_triton_b200.config import MoBAConfig
 from moba_triton_b200.kernels.moba_bwd import moba_backward, op_backward
 from moba_triton_b200.kernels.moba_fwd import (_validate, attend_partials, forward_in_query_chunks,
-                                               merge_partials, op_forward, op_plan, query_windows)
-from moba_triton_b200.kernels.routing import CSCIndex, build_csc_from_indices
+                                               merge_partials, op_forward, op_plan, op_workspace, query_windows)
+from moba_triton_b200.kernels.routing import CSCIndex
 
 
 class MoBAAttentionFunction(torch.autograd.Function):
@@ -51,8 +51,8 @@ class MoBAQueryChunkedFunction(torch.autograd.Function):
     """The op run a window of query rows at a time, forward and backward: the partial
     outputs and dQ partials (slots times the size of the output) exist for one window only.
     Saves the gate's block ids instead of an index; the backward rebuilds each window's
-    index from them. O and dQ are the bits of the whole call; dK/dV are summed over the
-    windows in float32 and rounded once."""
+    index from them. O and dQ are the bits of the whole call, whose kernels run; dK/dV are
+    summed over the windows in float32 and rounded once."""
 
     @staticmethod
     def forward(ctx, q, k, v, cfg, causal, query_chunk):
@@ -67,17 +67,22 @@ class MoBAQueryChunkedFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         q, k, v, out, lse, block_idx = ctx.saved_tensors
-        cfg = ctx.cfg
-        nb = cfg.num_blocks(q.shape[1])
-        dq = torch.empty_like(q)
+        cfg, dev = ctx.cfg, q.device
+        dout = dout.to(q.dtype).contiguous()
+        dq, dk_w, dv_w = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dk32 = torch.zeros(k.shape, device=k.device, dtype=torch.float32)
         dv32 = torch.zeros(v.shape, device=v.device, dtype=torch.float32)
         minus_inf = torch.full((), float("-inf"), device=q.device)
         for window in query_windows(q.shape[1], ctx.query_chunk):
-            index = build_csc_from_indices(block_idx, nb, cfg, num_kv_heads=k.shape[2], window=window)
             # which slots of the window's rows were written: those that name a block
             marker = torch.where(block_idx[:, :, window[0]:window[0] + window[1]] >= 0, 0.0, minus_inf).contiguous()
-            _, dk_w, dv_w = moba_backward(dout, q, k, v, out, lse, marker, cfg, index, causal=ctx.causal, dq=dq)
+            prob = _lib.make_problem(tuple(q.shape), k.shape[2], q.dtype, cfg, causal=ctx.causal, window=window)
+            sizes = op_workspace(prob)
+            keep, scratch = (torch.empty((n,), device=dev, dtype=torch.uint8) for n in (sizes[0], sizes[2]))
+            _lib.call("moba_b200_op_backward_window", dev, "moba_backward", prob, _lib.ptr(q), _lib.ptr(k), _lib.ptr(v),
+                      _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(marker), _lib.ptr(block_idx), _lib.ptr(keep),
+                      _lib.ptr(scratch), _lib.ptr(dq), _lib.ptr(dk_w), _lib.ptr(dv_w))
+            del keep, scratch                                # the next window's come from the same memory
             dk32 += dk_w
             dv32 += dv_w
         return dq, dk32.to(k.dtype), dv32.to(v.dtype), None, None, None

@@ -19,7 +19,7 @@ from moba_triton_b200.device import MIN_BLOCK_SIZE, check_gathered_head_dim
 from moba_triton_b200.gqa import head_group_size
 from moba_triton_b200.kernels.gating import gate_select
 from moba_triton_b200.kernels.pooling import pool_blocks
-from moba_triton_b200.kernels.routing import CSCIndex, build_csc_from_indices, build_csc_fused
+from moba_triton_b200.kernels.routing import CSCIndex, build_csc_fused
 from moba_triton_b200.varlen import validate_cu_seqlens
 
 
@@ -53,6 +53,13 @@ def _validate(q, k, v, cfg: MoBAConfig, cu_seqlens=None, max_seqlen=None) -> Non
             "(wording kept from the reference; it is this engine's minimum block too)")
 
 
+def op_workspace(problem) -> tuple:
+    """(keep, forward, backward): bytes of the whole op's workspaces."""
+    sizes = [ctypes.c_size_t() for _ in range(3)]
+    _lib.check(_lib.load().moba_b200_op_workspace(problem, *(ctypes.byref(x) for x in sizes)), "moba_attention")
+    return tuple(x.value for x in sizes)
+
+
 class _OpPlan:
     """What a whole-op call needs beside its tensors: the problem record and the sizes of its
     workspaces. Functions of shapes, dtype and configuration only, kept between calls."""
@@ -60,10 +67,16 @@ class _OpPlan:
 
     def __init__(self, problem):
         self.problem = problem
-        sizes = [ctypes.c_size_t() for _ in range(3)]
-        _lib.check(_lib.load().moba_b200_op_workspace(problem, *(ctypes.byref(x) for x in sizes)), "moba_attention")
-        self.keep_bytes, self.forward_bytes, self.backward_bytes = (x.value for x in sizes)
-        self.native = _lib.autograd().Plan(ctypes.addressof(problem), *(x.value for x in sizes))
+        sizes = op_workspace(problem)
+        self.keep_bytes, self.forward_bytes, self.backward_bytes = sizes
+        self.native = _lib.autograd().Plan(ctypes.addressof(problem), *sizes)
+
+
+def _float32_partials(q, partials_dtype) -> bool:
+    """Whether the partial outputs of a call are wider than its inputs."""
+    if partials_dtype not in (None, q.dtype, torch.float32):
+        raise ValueError(f"partials_dtype must be {q.dtype} or float32, got {partials_dtype}")
+    return partials_dtype == torch.float32 and q.dtype != torch.float32
 
 
 _PLANS = {}
@@ -92,9 +105,7 @@ def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, 
         return plan
     _validate(q, k, v, cfg, cu_seqlens, max_seqlen)
     _lib.require_cuda(q, k, v, cu_seqlens)
-    if partials_dtype not in (None, q.dtype, torch.float32):
-        raise ValueError(f"partials_dtype must be {q.dtype} or float32, got {partials_dtype}")
-    part_f32 = partials_dtype == torch.float32 and q.dtype != torch.float32
+    part_f32 = _float32_partials(q, partials_dtype)
     plan = _OpPlan(_lib.make_problem(tuple(q.shape), k.shape[2], q.dtype, cfg, cu_seqlens, max_seqlen, causal=causal,
                                      part_f32=part_f32))
     if key is not None:
@@ -225,9 +236,9 @@ def query_windows(seq_len: int, query_chunk: int):
 def forward_in_query_chunks(q, k, v, cfg: MoBAConfig, query_chunk: int, causal: bool = True,
                             partials_dtype: Optional[torch.dtype] = None, return_lse: bool = False):
     """The forward run a window of `query_chunk` query rows at a time (padded batches): the
-    gate runs once, then every window gets its own index and reuses one set of partial
-    buffers of `query_chunk` rows. Every (query, block) pair is computed exactly as in the
-    whole call, so the output is the same bit for bit. Returns (out, lse or None, block_idx).
+    gate runs once, then every window gets its own index and partial buffers of `query_chunk`
+    rows. Every (query, block) pair is computed exactly as in the whole call, by the same
+    kernels, so the output is the same bit for bit. Returns (out, lse or None, block_idx).
     The reference planned this host-side chunking and never built it
     (docs/deferred-decisions.md:152-220)."""
     b, s, hq, d = q.shape
@@ -235,15 +246,13 @@ def forward_in_query_chunks(q, k, v, cfg: MoBAConfig, query_chunk: int, causal: 
     block_idx = gate_select(q, kbar, cfg)
     out = torch.empty_like(q)
     lse = torch.empty((b, hq, s), device=q.device, dtype=torch.float32) if return_lse else None
-    partials = None
+    part_f32 = _float32_partials(q, partials_dtype)
     for window in query_windows(s, query_chunk):
-        index = build_csc_from_indices(block_idx, kbar.shape[2], cfg, num_kv_heads=k.shape[2], window=window)
-        if partials is not None and partials[0].shape[2] != window[1]:
-            partials = None                                  # the last window may be shorter
-        part_lse, part_o = attend_partials(q, k, v, cfg, index, causal=causal, partials_dtype=partials_dtype,
-                                           partials=partials)
-        partials = (part_lse, part_o)
-        merge_partials(part_lse, part_o, q.dtype, return_lse=return_lse, out=out, lse=lse, window=window)
+        prob = _lib.make_problem(tuple(q.shape), k.shape[2], q.dtype, cfg, causal=causal, part_f32=part_f32, window=window)
+        keep, scratch = (torch.empty((n,), device=q.device, dtype=torch.uint8) for n in op_workspace(prob)[:2])
+        _lib.call("moba_b200_op_forward_window", q.device, "moba_forward", prob, _lib.ptr(q), _lib.ptr(k), _lib.ptr(v),
+                  _lib.ptr(block_idx), _lib.ptr(keep), _lib.ptr(scratch), _lib.ptr(out), _lib.ptr(lse))
+        del keep, scratch                                    # the next window's come from the same memory
     return out, lse, block_idx
 
 

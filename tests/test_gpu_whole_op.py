@@ -79,6 +79,28 @@ def test_finer_blocks_with_the_other_options(flags, device):
         assert max_abs_error(staged.nan_to_num(), whole.nan_to_num()) <= 2e-2
 
 
+def gradients(q, k, v, do, cfg, **kw):
+    leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+    out = moba.moba_attention(*leaves, cfg, **kw)
+    out.backward(do)
+    return [out.detach()] + [t.grad for t in leaves]
+
+
+@pytest.mark.parametrize("block,top_k,d,dtype", [(64, 4, 64, torch.bfloat16), (32, 6, 128, torch.float16), (16, 3, 64, torch.bfloat16),
+                                                 (128, 12, 64, torch.bfloat16), (48, 4, 64, torch.bfloat16), (64, 4, 64, torch.float32)])
+def test_query_windows_run_the_kernels_of_the_whole_op(block, top_k, d, dtype, device):
+    """O and dQ bit for bit whatever the block size; windows that end inside a block, and one of a row."""
+    cfg = moba.MoBAConfig(block, top_k, dtype=dtype)
+    q, k, v, do = (t.to(device) for t in make_qkv((2, 1201, 4, d), 2, dtype=dtype, seed=64, with_do=True))
+    whole = gradients(q, k, v, do, cfg)
+    for chunk in (400, 333, 5000):
+        got = gradients(q, k, v, do, cfg, query_chunk=chunk)
+        assert torch.equal(got[0], whole[0]) and torch.equal(got[1], whole[1])
+        for a, w in zip(got[2:], whole[2:]):                 # sums over the windows: rounded once more
+            assert max_abs_error(a, w) <= (1e-5 if dtype == torch.float32 else 2e-2)
+        assert torch.equal(moba.moba_forward(q, k, v, cfg, query_chunk=chunk), whole[0])
+
+
 class OpenConfig:
     """A configuration object of a caller's own: hashable by identity, and mutable."""
     block_size, top_k, always_select_current = 128, 2, True
