@@ -19,7 +19,7 @@ from moba_triton_b200.device import MIN_BLOCK_SIZE, check_gathered_head_dim
 from moba_triton_b200.gqa import head_group_size
 from moba_triton_b200.kernels.gating import gate_select
 from moba_triton_b200.kernels.pooling import pool_blocks
-from moba_triton_b200.kernels.routing import CSCIndex, build_csc_fused
+from moba_triton_b200.kernels.routing import CSCIndex
 from moba_triton_b200.varlen import validate_cu_seqlens
 
 
@@ -263,8 +263,8 @@ def moba_forward(q, k, v, cfg: MoBAConfig, index: Optional[CSCIndex] = None, cau
     log-sum-exp kept). Reference: moba_fwd.py:783-835.
 
     `kv_heads_per_pass` (not in the reference) runs that many KV heads at a time,
-    each with its group of query heads, into one set of partial buffers that every
-    pass reuses: same result bit for bit, partial-output memory of one pass.
+    each with its group of query heads, in workspaces of one pass that the next one
+    takes over: same result bit for bit, partial-output memory of one pass.
 
     `query_chunk` (not in the reference either) runs that many query rows at a time instead:
     the partial buffers then hold `query_chunk` rows, whatever the number of heads. Padded
@@ -285,22 +285,12 @@ def moba_forward(q, k, v, cfg: MoBAConfig, index: Optional[CSCIndex] = None, cau
         if kv_heads_per_pass < hkv:
             group = q.shape[2] // hkv
             out = torch.empty_like(q)
-            partials = None
             for h0 in range(0, hkv, kv_heads_per_pass):
                 h1 = min(hkv, h0 + kv_heads_per_pass)
-                qs = q[:, :, h0 * group:h1 * group].contiguous()
-                ks, vs = k[:, :, h0:h1].contiguous(), v[:, :, h0:h1].contiguous()
-                _validate(qs, ks, vs, cfg, cu_seqlens, max_seqlen)
-                _lib.require_cuda(qs, ks, vs, cu_seqlens)
-                idx = build_csc_fused(qs, ks, cfg, cu_seqlens=cu_seqlens, max_seqlen=max_seqlen)
-                if partials is not None and partials[1].shape[1] != qs.shape[2]:
-                    partials = None                          # the last pass may hold fewer heads
-                if partials is None:
-                    partials = empty_partials(qs.shape, idx.max_slots, qs.device,
-                                              partials_dtype if partials_dtype is not None else q.dtype)
-                part_lse, part_o = attend_partials(qs, ks, vs, cfg, idx, causal=causal,
-                                                   partials_dtype=partials_dtype, partials=partials)
-                out[:, :, h0 * group:h1 * group] = merge_partials(part_lse, part_o, q.dtype)
+                heads = slice(h0 * group, h1 * group)
+                qs, ks, vs = q[:, :, heads], k[:, :, h0:h1], v[:, :, h0:h1]
+                plan = op_plan(qs, ks, vs, cfg, causal, cu_seqlens, max_seqlen, partials_dtype)
+                out[:, :, heads] = op_forward(plan, qs.contiguous(), ks.contiguous(), vs.contiguous(), cu_seqlens, False)[0]
             return out
     if index is None:
         plan = op_plan(q, k, v, cfg, causal, cu_seqlens, max_seqlen, partials_dtype)

@@ -101,6 +101,16 @@ def test_query_windows_run_the_kernels_of_the_whole_op(block, top_k, d, dtype, d
         assert torch.equal(moba.moba_forward(q, k, v, cfg, query_chunk=chunk), whole[0])
 
 
+@pytest.mark.parametrize("block,top_k,d,dtype", [(64, 4, 64, torch.bfloat16), (16, 3, 128, torch.float16), (128, 12, 64, torch.bfloat16),
+                                                 (64, 4, 64, torch.float32)])
+def test_passes_over_kv_heads_run_the_kernels_of_the_whole_op(block, top_k, d, dtype, device):
+    cfg = moba.MoBAConfig(block, top_k, dtype=dtype)
+    q, k, v = (t.to(device) for t in make_qkv((2, 1201, 6, d), 3, dtype=dtype, seed=65))
+    whole = moba.moba_forward(q, k, v, cfg)
+    for n in (1, 2):
+        assert torch.equal(moba.moba_forward(q, k, v, cfg, kv_heads_per_pass=n), whole)
+
+
 class OpenConfig:
     """A configuration object of a caller's own: hashable by identity, and mutable."""
     block_size, top_k, always_select_current = 128, 2, True
