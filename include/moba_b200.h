@@ -132,12 +132,17 @@ int moba_b200_profile_read(char* buf, size_t cap);
  * counterpart in the reference. */
 int moba_b200_device_status(unsigned int* word, void* stream);
 
-/* Which kernel family (MOBA_B200_PATH_PORTABLE or _TCGEN05) a stage would run
- * for this problem, or a negative error code. */
+/* Which kernel family (MOBA_B200_PATH_PORTABLE or _TCGEN05) a stage called by itself
+ * (moba_b200_gate, _fwd, _bwd) would run for this problem, or a negative error code.
+ * The whole-op calls have a wider choice: moba_b200_op_launch_plan. */
 int moba_b200_path_for(const moba_b200_problem* p, int stage);
 
 /* The launch table: everything the library decides per problem, looked up in
- * constant time from the problem record (no measurement, no device query).
+ * constant time from the problem record (no measurement, no device query);
+ * moba_b200_launch_plan for the stages called one by one, moba_b200_op_launch_plan
+ * for the whole-op calls. Those run blocks finer than 128 keys as columns of 128
+ * (work items and transpose are then those of the columns), more gates on tensor
+ * cores, and cut small problems finer.
  * The tensor-core kernels have one tile plan per head_dim; the transpose and
  * the scheduler size themselves by sequence length and pair count. Choices
  * never depend on whether the batch is packed, so a packed batch and its
@@ -151,13 +156,14 @@ typedef struct moba_b200_plan {
   int32_t bwd_kv_buffers;                  /* backward: K/V buffers per SM */
   int32_t bwd_gather_stages;               /* backward: stages of gathered Q and dO */
   int32_t gate_slots, gate_step;           /* gate: per-thread buffer slots; scores tested between room checks */
-  int32_t transpose_chunk_rows;            /* transpose: rows per histogram chunk */
+  int32_t transpose_chunk_rows;            /* transpose: rows per histogram chunk (0, as the next two: one launch) */
   int32_t transpose_chunks;                /*            chunks per sequence */
   int32_t scatter_warps;                   /*            runs walked side by side per chunk */
   int32_t chunk_tiles;                     /* scheduler: tiles per work item */
   int32_t work_items_per_row;              /*            table entries per (sequence, kv head) */
 } moba_b200_plan;
 int moba_b200_launch_plan(const moba_b200_problem* p, moba_b200_plan* plan);
+int moba_b200_op_launch_plan(const moba_b200_problem* p, moba_b200_plan* plan);
 
 /* Bytes of scratch moba_b200_transpose needs for this problem. */
 size_t moba_b200_transpose_scratch_bytes(const moba_b200_problem* p);
@@ -169,8 +175,9 @@ size_t moba_b200_transpose_scratch_bytes(const moba_b200_problem* p);
  * the last SMs busy while the others idle. The forward treats each item as a column
  * of its own; in the backward the items of a split column write float32 dK/dV
  * partials into `dkv_scratch`, summed in item order by a reduction pass.
- *   moba_b200_chunk_tiles         the chunk size used for this problem (the policy:
- *                                 total tiles / (4 x 148 SMs), at least 8; or p->chunk_tiles)
+ *   moba_b200_chunk_tiles         the chunk size of an index built by moba_b200_transpose (the policy:
+ *                                 total tiles / (4 x 148 SMs), at least 8; or p->chunk_tiles).
+ *                                 The whole-op calls cut small problems finer
  *   moba_b200_work_items_per_row  entries per (sequence, kv head) of index.work_items
  *   moba_b200_dkv_scratch_bytes   bytes of dkv_scratch moba_b200_bwd needs
  * The reference orders blocks longest first and leaves the rest to the hardware

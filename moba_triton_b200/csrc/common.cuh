@@ -307,6 +307,8 @@ int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const floa
 int check_problem(const moba_b200_problem* p);
 int need(const void* ptr, const char* name);
 int pick(const moba_b200_problem& p, bool fast_ok, const char* stage);
+// The launch table of a problem whose gate runs in family `gate_path` (an error code is passed on).
+int fill_plan(const moba_b200_problem& p, int gate_path, moba_b200_plan* plan);
 
 int launch_pack_index(const void* mask, int mask_bytes, int batch, int seq_len, int32_t* dest, int32_t* lengths,
                       int32_t* cu, int32_t* meta, cudaStream_t st);

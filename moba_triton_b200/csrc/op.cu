@@ -20,9 +20,9 @@ inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 
 // The cut of the work items. The policy of the scheduler has a floor of eight tiles, which is
 // right when the rows fill the GPU; a problem of at most sixteen tiles per SM is mostly tail, and
-// finer items spread it over the SMs (their dK/dV partials then fit the L2). Up to four tiles per
-// SM the size depends on the length of a row only, so that running the KV heads of such a problem
-// in several passes cuts them the same way and gives the same bits.
+// finer items spread it over the SMs (their dK/dV partials then fit the L2). The cut decides in which
+// groups dK and dV are summed: who runs the KV heads of a problem in several passes and wants the
+// bits of the whole gives every pass the whole's chunk_tiles (moba_b200_op_launch_plan).
 moba_b200_problem with_cut(const moba_b200_problem& p0) {
   moba_b200_problem p = p0;
   if (p.chunk_tiles > 0) return p;
@@ -115,6 +115,12 @@ moba_b200_index index_in(const moba_b200_problem& p, const Layout& l, unsigned c
   return ix;
 }
 
+// Which gate the op runs: where the portable one would by the library's choice, its selections come
+// from the exact tensor-core gate if that covers the problem.
+bool runs_exact_gate(const moba_b200_problem& gate, int gate_path) {
+  return gate_path == MOBA_B200_PATH_PORTABLE && gate.path == MOBA_B200_PATH_AUTO && gate_exact_sm100_supported(gate);
+}
+
 int check_sizes(const moba_b200_problem* p) {
   MOBA_TRY(check_problem(p));
   if (p->q_heads >= 1 << 19) { set_error("%d query heads do not fit a packed index entry", p->q_heads); return MOBA_B200_EUNSUPPORTED; }
@@ -196,6 +202,17 @@ int moba_b200_op_workspace(const moba_b200_problem* p0, size_t* keep_bytes, size
   return MOBA_B200_OK;
 }
 
+int moba_b200_op_launch_plan(const moba_b200_problem* p0, moba_b200_plan* plan) {
+  MOBA_TRY(check_sizes(p0));
+  if (plan == nullptr) { set_error("plan is NULL"); return MOBA_B200_EINVAL; }
+  const moba_b200_problem gate = with_cut(*p0);
+  const moba_b200_problem p = columns_of(gate).p;
+  const int gate_path = pick(gate, gate_sm100_supported(gate), "gate");
+  MOBA_TRY(fill_plan(p, gate_path >= 0 && runs_exact_gate(gate, gate_path) ? MOBA_B200_PATH_TCGEN05 : gate_path, plan));
+  if (transpose_small_supported(p)) plan->transpose_chunk_rows = plan->transpose_chunks = plan->scatter_warps = 0;
+  return MOBA_B200_OK;
+}
+
 int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void* k, const void* v,
                          const int32_t* cu_seqlens, void* keep_ws, void* forward_ws, void* out, int want_lse, void* stream) {
   MOBA_TRY(check_op(p0));
@@ -216,9 +233,7 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   int32_t* block_idx = reinterpret_cast<int32_t*>(tmp + l.block_idx);
   float* part_lse = reinterpret_cast<float*>(keep + l.part_lse);
   int32_t* counter = reinterpret_cast<int32_t*>(tmp + l.counter);
-  // Where the portable gate would run by the library's choice, its selections come from the exact
-  // tensor-core gate if that covers the problem.
-  const bool exact_gate = gate_path == MOBA_B200_PATH_PORTABLE && gate.path == MOBA_B200_PATH_AUTO && gate_exact_sm100_supported(gate);
+  const bool exact_gate = runs_exact_gate(gate, gate_path);
   float* norms = reinterpret_cast<float*>(tmp + l.norms);
   MOBA_TRY(launch_pool(gate, k, cu_seqlens, kbar, counter, exact_gate ? norms : nullptr, st));
   if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));

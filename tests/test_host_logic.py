@@ -211,10 +211,11 @@ def test_launch_plan_is_a_table_lookup_on_the_problem_record():
     gqa = launch_plan((1, 524288, 32, 128), 8, torch.bfloat16, cfg)
     assert (gqa["fwd_tiles_in_flight"], gqa["fwd_q_stages"], gqa["bwd_kv_buffers"], gqa["gate_slots"]) == (2, 2, 1, 7)
     assert gqa["scatter_warps"] == 4 and gqa["transpose_chunk_rows"] == 2048
-    # float32 and odd block sizes run the portable kernels; the tile plan is then empty
+    # float32 and odd block sizes run the portable kernels (so do, called as stages, the finer ones); the tile
+    # plan is then empty
     slow = launch_plan((1, 4096, 4, 64), 4, torch.float32, moba.MoBAConfig(128, 8, dtype=torch.float32))
     assert slow["fwd_path"] == "portable" and slow["fwd_tiles_in_flight"] == 0
-    assert launch_plan((1, 4096, 4, 64), 4, torch.bfloat16, moba.MoBAConfig(64, 4))["gate_path"] == "portable"
+    assert launch_plan((1, 4096, 4, 64), 4, torch.bfloat16, moba.MoBAConfig(64, 4), stages=True)["gate_path"] == "portable"
     # packed or padded, the same sequence length gets the same kernels (bitwise packed == alone)
     cu = torch.tensor([0, 1000, 2024], dtype=torch.int32)
     packed = launch_plan((1, 2024, 4, 64), 2, torch.bfloat16, cfg, cu_seqlens=cu, max_seqlen=1024)
@@ -224,6 +225,33 @@ def test_launch_plan_is_a_table_lookup_on_the_problem_record():
         assert packed[key] == alone[key]
     with pytest.raises(ValueError):
         launch_plan((1, 64, 3, 64), 2, torch.bfloat16, cfg)
+
+
+def test_launch_plan_of_the_whole_op_says_what_the_op_runs():
+    """Finer blocks, more ranked blocks and the finer cut of small problems: what only the whole-op calls do."""
+    from moba_triton_b200.tuning import launch_plan
+    shape, bf16 = (2, 8192, 4, 128), torch.bfloat16
+    for block, top_k in ((64, 8), (32, 6), (16, 4), (128, 13)):
+        op = launch_plan(shape, 4, bf16, moba.MoBAConfig(block, top_k))
+        assert op["gate_path"] == op["fwd_path"] == op["bwd_path"] == "tcgen05" and op["gate_slots"] == 7, block
+        staged = launch_plan(shape, 4, bf16, moba.MoBAConfig(block, top_k), stages=True)
+        assert staged["gate_path"] == "portable" and (staged["fwd_path"] == "tcgen05") == (block == 128)
+    for block, top_k, dtype in ((48, 4, bf16), (64, 4, torch.float32)):
+        assert launch_plan(shape, 4, dtype, moba.MoBAConfig(block, top_k))["fwd_path"] == "portable"
+    assert launch_plan(shape, 4, bf16, moba.MoBAConfig(64, 4, gate_window=9))["fwd_path"] == "portable"
+    assert launch_plan((1, 8192, 4, 64), 4, bf16, moba.MoBAConfig(128, 18))["gate_path"] == "portable"
+    # the cut: tiles of the whole problem, 2 and 4 for small ones; work items of columns of 128 keys
+    cfg = moba.MoBAConfig(128, 8)
+    for tokens, heads, cut in ((1024, 4, 2), (4096, 2, 4), (8192, 4, 4), (8192, 5, 8), (131072, 4, 56)):
+        assert launch_plan((1, tokens, heads, 64), heads, bf16, cfg)["chunk_tiles"] == cut
+        assert launch_plan((1, tokens, heads, 64), heads, bf16, cfg, stages=True)["chunk_tiles"] == max(8, cut)
+    finer = launch_plan(shape, 4, bf16, moba.MoBAConfig(64, 8))
+    assert finer["work_items_per_row"] == 64 + 2 * 4 * 8192 * 8 // (128 * finer["chunk_tiles"]) + 1
+    # rows of up to 131072 pairs are transposed in one launch
+    assert launch_plan((1, 16384, 1, 64), 1, bf16, cfg)["transpose_chunks"] == 0
+    assert launch_plan((1, 16512, 1, 64), 1, bf16, cfg)["transpose_chunks"] == 65
+    with pytest.raises(ValueError):
+        launch_plan((1, 64, 3, 64), 2, bf16, cfg)
 
 
 def test_reference_arm_of_the_bench_prints_the_contract_line():
