@@ -88,8 +88,8 @@ class MoBAQueryChunkedFunction(torch.autograd.Function):
         return dq, dk32.to(k.dtype), dv32.to(v.dtype), None, None, None
 
 
-def _attention(q, k, v, cfg, causal, cu_seqlens, max_seqlen):
-    plan = op_plan(q, k, v, cfg, causal, cu_seqlens, max_seqlen)
+def _attention(q, k, v, cfg, causal, cu_seqlens, max_seqlen, chunk_tiles=0):
+    plan = op_plan(q, k, v, cfg, causal, cu_seqlens, max_seqlen, chunk_tiles=chunk_tiles)
     return _lib.autograd().attention(q, k, v, plan.native, cu_seqlens)
 
 
@@ -100,6 +100,19 @@ def _kv_head_passes(q, k, v, kv_heads_per_pass: int):
     for h0 in range(0, hkv, kv_heads_per_pass):
         h1 = min(hkv, h0 + kv_heads_per_pass)
         yield q[:, :, h0 * group:h1 * group], k[:, :, h0:h1], v[:, :, h0:h1]
+
+
+def _cut_of_the_whole(q, k, cfg, causal, cu_seqlens, max_seqlen) -> int:
+    """Tiles per work item that passes over the KV heads of a call take, so that they sum dK and dV
+    in the groups of the whole call; 0 = their own cut. A call of more than 4 736 tiles (32 per SM)
+    has items of a quarter of an SM's share of it, too long for a pass to spread over the SMs."""
+    hkv = k.shape[2]
+    prob = _lib.make_problem((*q.shape[:2], q.shape[2] // hkv * hkv, q.shape[3]), hkv, q.dtype, cfg, cu_seqlens, max_seqlen,
+                             causal=causal)
+    plan = _lib.Plan()
+    if _lib.load().moba_b200_op_launch_plan(prob, plan) < 0:
+        return 0                                              # too large as one call: nothing to equal
+    return plan.chunk_tiles if plan.chunk_tiles <= 8 else 0
 
 
 def moba_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cfg: MoBAConfig,
@@ -119,10 +132,13 @@ def moba_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cfg: MoBAC
     `kv_heads_per_pass` (not in the reference, which planned but never built a
     host-side chunking of the op, docs/deferred-decisions.md:152-220) runs the op
     over that many KV heads at a time, each with its group of query heads. KV
-    heads are independent, so the result is the same bit for bit, while the
+    heads are independent, so O and dQ are the same bit for bit, while the
     per-(query, slot) partial outputs and dQ partials, which are `slots` times the
     size of the output, exist for one pass only: at q [1,524288,32,128] with 8 KV
-    heads that is 4.3 GB per pass instead of 34 GB.
+    heads that is 4.3 GB per pass instead of 34 GB. dK and dV are the same bits too
+    while the whole call has at most 606 208 (query head, query, slot) triples; above,
+    a pass cuts long columns into other pieces than the whole call, and dK and dV are
+    float32 sums of the same products in other groups.
 
     `query_chunk` (the chunking the reference describes there) runs `query_chunk` query
     rows at a time instead, which also bounds the buffers when a GPU holds a single KV
@@ -138,9 +154,10 @@ def moba_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cfg: MoBAC
         if kv_heads_per_pass < 1:
             raise ValueError(f"kv_heads_per_pass must be positive, got {kv_heads_per_pass}")
         if kv_heads_per_pass < k.shape[2]:
-            outs = [_attention(qs, ks, vs, cfg, causal, cu_seqlens, max_seqlen)
-                    for qs, ks, vs in _kv_head_passes(q, k, v, kv_heads_per_pass)]
-            return torch.cat(outs, dim=2)
+            passes = list(_kv_head_passes(q, k, v, kv_heads_per_pass))
+            _validate(*passes[0], cfg, cu_seqlens, max_seqlen)
+            cut = _cut_of_the_whole(q, k, cfg, causal, cu_seqlens, max_seqlen)
+            return torch.cat([_attention(qs, ks, vs, cfg, causal, cu_seqlens, max_seqlen, cut) for qs, ks, vs in passes], dim=2)
     if index is None:
         return _attention(q, k, v, cfg, causal, cu_seqlens, max_seqlen)
     return MoBAAttentionFunction.apply(q, k, v, cfg, index, causal, cu_seqlens, max_seqlen)

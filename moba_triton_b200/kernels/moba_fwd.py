@@ -83,7 +83,7 @@ _PLANS = {}
 _MAX_PLANS = 512
 
 
-def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, partials_dtype=None) -> "_OpPlan":
+def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, partials_dtype=None, chunk_tiles=0) -> "_OpPlan":
     """Validates a call and returns its plan; a call like an earlier one skips both. Calls are told
     apart by values: a `MoBAConfig` is frozen and compares by its fields; of any other configuration
     object the fields are read on every call, and a `max_seqlen` that is a tensor is read too."""
@@ -96,7 +96,7 @@ def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, 
         key = (q.shape, k.shape, v.shape, q.dtype, k.dtype, v.dtype, fields, bool(causal),
                None if max_seqlen is None else whole_number(max_seqlen), partials_dtype,
                None if cu_seqlens is None else (cu_seqlens.shape, cu_seqlens.dtype),
-               _lib._force_path[0], _lib._chunk_tiles[0])
+               _lib._force_path[0], chunk_tiles or _lib._chunk_tiles[0])
         plan = _PLANS.get(key) if on_gpu else None
     except TypeError:                                        # nothing to tell the call by; refused below if it is wrong
         key = None
@@ -107,7 +107,7 @@ def op_plan(q, k, v, cfg: MoBAConfig, causal, cu_seqlens=None, max_seqlen=None, 
     _lib.require_cuda(q, k, v, cu_seqlens)
     part_f32 = _float32_partials(q, partials_dtype)
     plan = _OpPlan(_lib.make_problem(tuple(q.shape), k.shape[2], q.dtype, cfg, cu_seqlens, max_seqlen, causal=causal,
-                                     part_f32=part_f32))
+                                     part_f32=part_f32, chunk_tiles=chunk_tiles or None))
     if key is not None:
         if len(_PLANS) >= _MAX_PLANS:
             _PLANS.clear()

@@ -111,6 +111,18 @@ def test_passes_over_kv_heads_run_the_kernels_of_the_whole_op(block, top_k, d, d
         assert torch.equal(moba.moba_forward(q, k, v, cfg, kv_heads_per_pass=n), whole)
 
 
+@pytest.mark.parametrize("s,hkv,group", [(1024, 16, 1), (2048, 12, 2), (8192, 8, 1)], ids=["cut4", "cut8", "cut8-long"])
+def test_passes_over_kv_heads_cut_columns_like_the_whole_call(s, hkv, group, device):
+    """1 024, 3 072 and 4 096 tiles as a whole, at most half of that in a pass: by itself a pass would
+    cut its columns into finer items and sum dK and dV in other groups."""
+    cfg = moba.MoBAConfig(128, 8)
+    q, k, v, do = (t.to(device) for t in make_qkv((1, s, hkv * group, 64), hkv, dtype=torch.bfloat16, seed=66, with_do=True))
+    whole = gradients(q, k, v, do, cfg)
+    for n in (1, hkv // 2):
+        for a, w in zip(gradients(q, k, v, do, cfg, kv_heads_per_pass=n), whole):
+            assert torch.equal(a, w)
+
+
 class OpenConfig:
     """A configuration object of a caller's own: hashable by identity, and mutable."""
     block_size, top_k, always_select_current = 128, 2, True
