@@ -316,13 +316,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// Same wait, but also names registers of the load it guards as in/out operands, so the compiler
-// cannot schedule their first use above the wait.
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[7]), "+r"(r[8]), "+r"(r[15]), "+r"(r[16]), "+r"(r[23]), "+r"(r[24]), "+r"(r[31])
-               :: "memory");
-}
 
 // ---------------------------------------------------------------------------
 // descriptors

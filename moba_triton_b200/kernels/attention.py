@@ -6,31 +6,26 @@ import torch
 
 from moba_triton_b200 import _lib
 from moba_triton_b200.config import MoBAConfig
-from moba_triton_b200.kernels.moba_bwd import moba_backward, op_backward
+from moba_triton_b200.kernels.moba_bwd import moba_backward
 from moba_triton_b200.kernels.moba_fwd import (_validate, attend_partials, forward_in_query_chunks,
-                                               merge_partials, op_forward, op_plan, op_workspace, query_windows)
-from moba_triton_b200.kernels.routing import CSCIndex
+                                               merge_partials, op_plan, op_workspace, query_windows)
+from moba_triton_b200.kernels.routing import CSCIndex, build_csc_fused
 
 
 class MoBAAttentionFunction(torch.autograd.Function):
-    """Saves q, k, v, out and, when the routing is its own, the workspace that holds the index,
-    the global log2-sum-exp and the per-slot marker; with a given index, the two tensors, and
+    """The op with a given index (built here if it is None; without one `moba_attention` runs the
+    node of csrc/autograd.cpp). Saves q, k, v, out, the global log2-sum-exp and the per-slot marker;
     the index rides on the context. The gate receives no gradient."""
 
     @staticmethod
     def forward(ctx, q, k, v, cfg, index, causal, cu_seqlens, max_seqlen):
-        if index is None:
-            plan = op_plan(q, k, v, cfg, causal, cu_seqlens, max_seqlen)
-            q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-            out, keep = op_forward(plan, q, k, v, cu_seqlens, True)
-            ctx.save_for_backward(q, k, v, out, keep)
-            ctx.plan, ctx.cu_seqlens = plan, cu_seqlens
-            return out
-        ctx.plan = None
-        cu_seqlens, max_seqlen = index.cu_seqlens, index.max_seqlen
+        if index is not None:
+            cu_seqlens, max_seqlen = index.cu_seqlens, index.max_seqlen
         _validate(q, k, v, cfg, cu_seqlens, max_seqlen)
         _lib.require_cuda(q, k, v, cu_seqlens)
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        if index is None:
+            index = build_csc_fused(q, k, cfg, cu_seqlens=cu_seqlens, max_seqlen=max_seqlen)
         part_lse, part_o = attend_partials(q, k, v, cfg, index, causal=causal)
         out, lse = merge_partials(part_lse, part_o, q.dtype, return_lse=True)
         ctx.save_for_backward(q, k, v, out, lse, part_lse)
@@ -39,8 +34,6 @@ class MoBAAttentionFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
-        if ctx.plan is not None:
-            return (*op_backward(ctx.plan, dout, *ctx.saved_tensors, ctx.cu_seqlens), None, None, None, None, None)
         q, k, v, out, lse, part_lse = ctx.saved_tensors
         dq, dk, dv = moba_backward(dout, q, k, v, out, lse, part_lse, ctx.cfg, ctx.index,
                                    causal=ctx.causal)

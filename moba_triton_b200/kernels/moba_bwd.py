@@ -41,17 +41,3 @@ def moba_backward(dout, q, k, v, out, lse, part_lse, cfg: MoBAConfig, index: CSC
               _lib.ptr(part_lse), index.c_struct(), _lib.ptr(index.cu_seqlens), _lib.ptr(delta),
               _lib.ptr(dq_part), _lib.ptr(dkv_scratch), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv))
     return dq, dk, dv
-
-
-def op_backward(plan, dout, q, k, v, out, keep, cu_seqlens):
-    """Gradients of an `op_forward` from the workspace it left: one call, one scratch buffer."""
-    dout = dout.contiguous()
-    if dout.dtype != q.dtype:
-        dout = dout.to(q.dtype)
-    dev = q.device
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    scratch = torch.empty((plan.backward_bytes,), device=dev, dtype=torch.uint8)
-    _lib.call_op("moba_b200_op_backward", dev.index, "moba_backward", plan.problem, q.data_ptr(), k.data_ptr(), v.data_ptr(),
-                 out.data_ptr(), dout.data_ptr(), None if cu_seqlens is None else cu_seqlens.data_ptr(), keep.data_ptr(),
-                 scratch.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr())
-    return dq, dk, dv

@@ -123,6 +123,19 @@ def test_passes_over_kv_heads_cut_columns_like_the_whole_call(s, hkv, group, dev
             assert torch.equal(a, w)
 
 
+def test_the_function_of_a_given_index_builds_one_if_there_is_none(device):
+    cfg = moba.MoBAConfig(128, 4)
+    q, k, v, do = (t.to(device) for t in make_qkv((1, 1000, 4, 64), 2, dtype=torch.bfloat16, seed=67, with_do=True))
+    cu = torch.tensor([0, 300, 1000], dtype=torch.int32, device=device)
+    for kw in ({}, dict(cu_seqlens=cu, max_seqlen=700)):
+        leaves = [t.detach().clone().requires_grad_(True) for t in (q, k, v)]
+        out = moba.MoBAAttentionFunction.apply(*leaves, cfg, None, True, kw.get("cu_seqlens"), kw.get("max_seqlen"))
+        out.backward(do)
+        index = moba.build_csc_fused(q, k, cfg, **kw)
+        for a, w in zip([out] + [t.grad for t in leaves], gradients(q, k, v, do, cfg, index=index)):
+            assert torch.equal(a, w)
+
+
 class OpenConfig:
     """A configuration object of a caller's own: hashable by identity, and mutable."""
     block_size, top_k, always_select_current = 128, 2, True
