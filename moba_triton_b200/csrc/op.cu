@@ -19,18 +19,27 @@ constexpr size_t kAlign = 256;
 inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 
 // The cut of the work items. The policy of the scheduler has a floor of eight tiles, which is
-// right when the rows fill the GPU; a problem of at most sixteen tiles per SM is mostly tail, and
-// finer items spread it over the SMs (their dK/dV partials then fit the L2). The cut decides in which
-// groups dK and dV are summed: who runs the KV heads of a problem in several passes and wants the
-// bits of the whole gives every pass the whole's chunk_tiles (moba_b200_op_launch_plan).
+// right when the rows fill the GPU; a small problem is mostly tail, and finer items spread it over the
+// SMs, at the price of more dK/dV partials to sum. Measured, attention kernels of a step / forward
+// call, us, with items of 2, 4 and 8 tiles (head_dim 64 unless noted):
+//   up to 4 tiles per SM, rows of up to 128 tiles: [1,1000,4->2] 45, 48, 59 /; [1,2048,2] 45, 46, 57 / 29, 30, 33
+//   ... longer rows:                               [1,4096,2] 60, 52, 59 / 37.3, 36.4, 40.5; [1,8192,1] 66, 55, 61 /
+//   4 to 16 per SM, rows of up to 128 tiles:       [1,1024,16] 61, 55, 50 / 38.7, 38.4, 41.5
+//   ... longer rows:                               [1,2048,8->2] of 128 92, 90, 80 / 52.5, 55.2, 55.6;
+//                                                  [1,8192,4] 134, 105, 94 / 59.3, 58.1, 58.1
+//   above:                                         [1,8192,5] 156, 125, 115 / 71.8, 69.5, 70.3
+// The cut decides in which groups dK and dV are summed: who runs the KV heads of a problem in several
+// passes and wants the bits of the whole gives every pass the whole's chunk_tiles
+// (moba_b200_op_launch_plan).
 moba_b200_problem with_cut(const moba_b200_problem& p0) {
   moba_b200_problem p = p0;
   if (p.chunk_tiles > 0) return p;
   p.chunk_tiles = sched_chunk_tiles(p);
   const long long tiles = (sched_pairs_bound(p) + 127) / 128;
   const long long row_tiles = ((long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots + 127) / 128;
-  if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = row_tiles <= 128 ? 2 : 4;
-  else if (tiles <= 16LL * kSchedSMs) p.chunk_tiles = 4;
+  const bool short_rows = row_tiles <= 128;
+  if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = short_rows ? 2 : 4;
+  else if (tiles <= 16LL * kSchedSMs && short_rows) p.chunk_tiles = 4;
   return p;
 }
 

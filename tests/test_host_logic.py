@@ -242,7 +242,7 @@ def test_launch_plan_of_the_whole_op_says_what_the_op_runs():
     assert launch_plan((1, 8192, 4, 64), 4, bf16, moba.MoBAConfig(128, 18))["gate_path"] == "portable"
     # the cut: tiles of the whole problem, 2 and 4 for small ones; work items of columns of 128 keys
     cfg = moba.MoBAConfig(128, 8)
-    for tokens, heads, cut in ((1024, 4, 2), (4096, 2, 4), (8192, 4, 4), (8192, 5, 8), (131072, 4, 56)):
+    for tokens, heads, cut in ((1024, 4, 2), (4096, 2, 4), (1024, 16, 4), (8192, 4, 8), (1024, 40, 8), (131072, 4, 56)):
         assert launch_plan((1, tokens, heads, 64), heads, bf16, cfg)["chunk_tiles"] == cut
         assert launch_plan((1, tokens, heads, 64), heads, bf16, cfg, stages=True)["chunk_tiles"] == max(8, cut)
     finer = launch_plan(shape, 4, bf16, moba.MoBAConfig(64, 8))
