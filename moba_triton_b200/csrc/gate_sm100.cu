@@ -184,8 +184,12 @@ struct Unit {
 // row of block means twice would cost more tensor-core time than the tighter bar saves.
 constexpr int kBoundChunks = 2;
 // So few candidates go through the buffers faster than through a pass of their own (16 sequences
-// of 300 to 9000 tokens, 32 heads: 0.31 ms with a bounding pass for every unit, 0.27 without).
-constexpr int kUnboundedBlocks = 32;
+// of 300 to 9000 tokens, 32 heads: 0.31 ms with a bounding pass for every unit, 0.27 without). Not in
+// the exact gate, where what passes the bar may be scored again in float64: with the pass for every
+// unit 2 x 2048 queries x 4 heads, 32 blocks of 64 46 -> 36 us, 2 x 8192 x 4 of 128 120 -> 113,
+// 65536 x 4, 512 blocks 315 -> 309; for 64 blocks and fewer left out it costs more (207, 324).
+template <bool EXACT> constexpr int kUnboundedBlocks = EXACT ? 0 : 32;
+template <bool EXACT>
 __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_problem& p, const int32_t* cu,
                                           int n_tiles) {
   const int ny = p.n_seq * p.q_heads;
@@ -208,7 +212,7 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
     u.c_hi0 = max(u.n_lo, recent0 / kTile);
   }
   u.n_chunks = u.n_lo + (total - u.c_hi0);
-  u.n_first = u.own_hi > kUnboundedBlocks ? min(u.n_chunks, kBoundChunks) : 0;
+  u.n_first = u.own_hi > kUnboundedBlocks<EXACT> ? min(u.n_chunks, kBoundChunks) : 0;
   return u.row0 < sp.len;
 }
 
@@ -323,7 +327,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
       const int ui = unit_of(round);
       if (ui >= n_units) continue;
       Unit u;
-      if (!load_unit(u, ui, p, cu, n_tiles)) continue;
+      if (!load_unit<EXACT>(u, ui, p, cu, n_tiles)) continue;
       constexpr int NM = L <= 8 ? 8 : 16;                       // column subsets of the bounding pass: at least L
       const int own = EXACT ? min(u.row0 + r, u.len - 1) / p.block_size : u.tile;
       float err = 0.f;                                          // EXACT: bound of |tensor-core sum - exact score|
@@ -523,7 +527,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         const int ui = unit_of(round);
         if (ui >= n_units) continue;
         Unit u;
-        if (!load_unit(u, ui, p, cu, n_tiles) || u.n_chunks == 0) continue;
+        if (!load_unit<EXACT>(u, ui, p, cu, n_tiles) || u.n_chunks == 0) continue;
         mbar_wait(&bars->q_full, nq & 1, wc);
         for (int step = 0; step < u.steps(); ++step, ++gc) {
           const uint32_t st = gc & 1, use = gc >> 1;
@@ -555,7 +559,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         const int ui = unit_of(round);
         if (ui >= n_units) continue;
         Unit u;
-        if (!load_unit(u, ui, p, cu, n_tiles) || u.n_chunks == 0) continue;
+        if (!load_unit<EXACT>(u, ui, p, cu, n_tiles) || u.n_chunks == 0) continue;
         if (*wc.abort) break;                                   // no new loads once a wait gave up
         const size_t b = p.packed ? 0 : (size_t)u.seq;
         const int kv_row = u.seq * p.kv_heads + u.hq / group;
