@@ -184,11 +184,12 @@ struct Unit {
 // row of block means twice would cost more tensor-core time than the tighter bar saves.
 constexpr int kBoundChunks = 2;
 // So few candidates go through the buffers faster than through a pass of their own (16 sequences
-// of 300 to 9000 tokens, 32 heads: 0.31 ms with a bounding pass for every unit, 0.27 without). Not in
-// the exact gate, where what passes the bar may be scored again in float64: with the pass for every
-// unit 2 x 2048 queries x 4 heads, 32 blocks of 64 46 -> 36 us, 2 x 8192 x 4 of 128 120 -> 113,
-// 65536 x 4, 512 blocks 315 -> 309; for 64 blocks and fewer left out it costs more (207, 324).
-template <bool EXACT> constexpr int kUnboundedBlocks = EXACT ? 0 : 32;
+// of 300 to 9000 tokens, 32 heads: 0.31 ms with a bounding pass for every unit, 0.27 without). In the
+// exact gate, where what passes the bar may be scored again in float64, the pass pays as soon as a
+// row has more candidates than it ranks: against a line at 32 blocks 2 x 2048 queries x 4 heads, 32
+// blocks of 64 46 -> 36 us, 2 x 8192 x 4 of 128 120 -> 113, 65536 x 4, 512 blocks 315 -> 309; with
+// the line at 64 207 and 324.
+constexpr int kUnboundedBlocks = 32;
 template <bool EXACT>
 __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_problem& p, const int32_t* cu,
                                           int n_tiles) {
@@ -212,7 +213,7 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
     u.c_hi0 = max(u.n_lo, recent0 / kTile);
   }
   u.n_chunks = u.n_lo + (total - u.c_hi0);
-  u.n_first = u.own_hi > kUnboundedBlocks<EXACT> ? min(u.n_chunks, kBoundChunks) : 0;
+  u.n_first = u.own_hi > (EXACT ? p.take : kUnboundedBlocks) ? min(u.n_chunks, kBoundChunks) : 0;
   return u.row0 < sp.len;
 }
 
