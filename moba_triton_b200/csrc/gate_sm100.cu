@@ -336,6 +336,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
       if constexpr (EXACT) {
         q_row = q + ((size_t)(p.packed ? u.bos : (size_t)u.seq * p.tokens) + min(u.row0 + r, u.len - 1)) * ((size_t)p.q_heads * D) + (size_t)u.hq * D;
         err = score_error<D, T>(q_row, norms + ((size_t)u.seq * p.kv_heads + u.hq / group) * p.num_blocks, u.own_hi, lane);
+        if (u.row0 + r >= u.len) err = 0.f;                     // past the end: nobody reads what it selects
       }
       uint32_t best[L];
 #pragma unroll
