@@ -27,6 +27,7 @@ inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 //   4 to 16 per SM, rows of up to 128 tiles:       [1,1024,16] 61, 55, 50 / 38.7, 38.4, 41.5
 //   ... longer rows:                               [1,2048,8->2] of 128 92, 90, 80 / 52.5, 55.2, 55.6;
 //                                                  [1,8192,4] 134, 105, 94 / 59.3, 58.1, 58.1
+//   ... float32, whose kernel starts a CTA for every tile an item may have: [1,4096,4] / 4: 185, 8: 198
 //   above:                                         [1,8192,5] 156, 125, 115 / 71.8, 69.5, 70.3
 // The cut decides in which groups dK and dV are summed: who runs the KV heads of a problem in several
 // passes and wants the bits of the whole gives every pass the whole's chunk_tiles
@@ -39,7 +40,7 @@ moba_b200_problem with_cut(const moba_b200_problem& p0) {
   const long long row_tiles = ((long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots + 127) / 128;
   const bool short_rows = row_tiles <= 128;
   if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = short_rows ? 2 : 4;
-  else if (tiles <= 16LL * kSchedSMs && short_rows) p.chunk_tiles = 4;
+  else if (tiles <= 16LL * kSchedSMs && (short_rows || p.dtype == MOBA_B200_F32)) p.chunk_tiles = 4;
   return p;
 }
 
