@@ -179,10 +179,12 @@ fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
 // of a work item: S is a 128 x 128 x D product and O a 128 x D x 128 one, each thread holding 8 x 8
 // (8 x D/16) of them in registers and reading operands as 16-byte pieces, so that an FMA costs a
 // sixteenth of a shared-memory load; P takes the place of Q and K between the two. The sums run in
-// the order of the portable kernel (over the head dim, over the keys), in float32 FMAs. It is bound
-// by the FMA pipe: 16 400 clocks of a tile at head_dim 64, of 18 000 to 20 000. The portable kernel,
-// with one CTA per column, a load per FMA and as many as 32 tiles in one CTA, took 1.3 ms for
-// [1,4096,4,64].
+// the order of the portable kernel (over the head dim, over the keys), in float32 FMAs. A tile's FMAs
+// are 16 400 clocks of the SM's pipe at head_dim 64. At [1,4096,4,64] (0.14 ms, about 980 tiles on 296
+// resident CTAs: 3.3 rounds, paid as four) the pipe is 48 % busy, the issue slots 64 %, shared-memory
+// wavefronts 42 % of their peak: two CTAs of eight warps do not fill the gaps of each other's loads and
+// barriers. The portable kernel, with one CTA per column, a load per FMA and as many as 32 tiles in one
+// CTA, took 1.3 ms.
 // ---------------------------------------------------------------------------
 constexpr int kF32Tile = 128;
 template <int D> struct F32Cfg {

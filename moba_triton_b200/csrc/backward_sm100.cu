@@ -23,9 +23,9 @@
 // with every copy, store and exponential and seven eighths of every MMA left out, the hand-overs
 // between the roles and the TMEM loads and stores still take 3 500 of 5 400 at head_dim 64 and
 // 4 400 of 7 200 at 128; the tensor pipe needs 1 900 and 2 560. Measured against the untransposed
-// version with copies through the load-store unit: 11.0 -> 8.9 ms on 262 144 packed tokens, 16
-// heads of 128; 9.1 -> 7.4 ms on [1,131072,32,128] with 8 KV heads; 0.68 -> 0.65 ms on
-// [1,131072,4,64].
+// version with copies through the load-store unit: 11.0 -> 7.4 ms on 262 144 packed tokens, 16
+// heads of 128; 9.1 -> 6.9 ms on [1,131072,32,128] with 8 KV heads. At head_dim 64 it gained nothing
+// that can be told from noise ([1,131072,4,64]: 0.667 ms before, 0.65 to 0.67 now).
 //
 // dQ rows go to the (query, slot) partial buffer; a later pass sums the slots.
 //
