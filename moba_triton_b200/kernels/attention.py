@@ -119,7 +119,8 @@ def moba_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cfg: MoBAC
     q [B,S,Hq,D]; k, v [B,S,Hkv,D] with Hkv dividing Hq (grouped-query heads map
     h -> h // (Hq/Hkv)); packed batches are [1,T,H,D] with `cu_seqlens` (int32,
     on the device) and `max_seqlen`. `index` holds routing fixed and carries its
-    own packing metadata. `causal=False` removes only the mask inside the
+    own packing metadata; such a call runs the staged kernels, which take blocks finer
+    than 128 keys on CUDA cores. `causal=False` removes only the mask inside the
     query's own block. Returns [B,S,Hq,D] in the dtype of q.
 
     `kv_heads_per_pass` (not in the reference, which planned but never built a
