@@ -20,15 +20,18 @@ inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 
 // The cut of the work items. The policy of the scheduler has a floor of eight tiles, which is
 // right when the rows fill the GPU; a small problem is mostly tail, and finer items spread it over the
-// SMs, at the price of more dK/dV partials to sum. Measured, attention kernels of a step / forward
-// call, us, with items of 2, 4 and 8 tiles (head_dim 64 unless noted):
-//   up to 4 tiles per SM, rows of up to 128 tiles: [1,1000,4->2] 45, 48, 59 /; [1,2048,2] 45, 46, 57 / 29, 30, 33
-//   ... longer rows:                               [1,4096,2] 60, 52, 59 / 37.3, 36.4, 40.5; [1,8192,1] 66, 55, 61 /
-//   4 to 16 per SM, rows of up to 128 tiles:       [1,1024,16] 61, 55, 50 / 38.7, 38.4, 41.5
-//   ... longer rows:                               [1,2048,8->2] of 128 92, 90, 80 / 52.5, 55.2, 55.6;
-//                                                  [1,8192,4] 134, 105, 94 / 59.3, 58.1, 58.1
-//   ... float32, whose kernel starts a CTA for every tile an item may have: [1,4096,4] / 4: 185, 8: 198
-//   above:                                         [1,8192,5] 156, 125, 115 / 71.8, 69.5, 70.3
+// SMs, at the price of more dK/dV partials to sum. Measured with items of 2, 4 and 8 tiles, us
+// (head_dim 64 unless noted):          tiles per SM, per row   attention kernels of a step   whole forward call
+//   [1,1000,4 heads on 2], top 4           0.8     63                 45   48   59
+//   [1,2048,2]                             1.7    128                 45   46   57               29   30   33
+//   [1,4096,2]                             3.5    256                 60   52   59               37.3 36.4 40.5
+//   [1,8192,1]                             3.5    512                 66   55   61
+//   [1,1024,16]                            6.9     64                 61   55   50               38.7 38.4 41.5
+//   [1,2048,8 on 2], head_dim 128          6.9    512                 92   90   80               52.5 55.2 55.6
+//   [1,8192,4]                            13.8    512                134  105   94               59.3 58.1 58.1
+//   [1,8192,5]                            17.3    512                156  125  115               71.8 69.5 70.3
+//   [1,4096,4] float32, whose kernel       6.9    256                                               -  185  198
+//     starts a CTA for every tile that an item may have
 // The cut decides in which groups dK and dV are summed: who runs the KV heads of a problem in several
 // passes and wants the bits of the whole gives every pass the whole's chunk_tiles
 // (moba_b200_op_launch_plan).
