@@ -151,7 +151,7 @@ struct TensorCorePlan {
   int head_dim;
   int fwd_tiles_in_flight, fwd_q_stages;
   int bwd_kv_buffers, bwd_gather_stages;
-  int gate_slots, gate_step;
+  int gate_slots, gate_step;      // of a buffer the gate no longer has; the record keeps the fields
 };
 constexpr TensorCorePlan kTensorCorePlans[2] = {
     {64, 4, 4, 2, 2, 16, 8},

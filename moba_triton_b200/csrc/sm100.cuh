@@ -258,6 +258,9 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint6
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// A descriptor `bytes` (a multiple of 16) further on in shared memory.
+__device__ __forceinline__ uint64_t sdesc_at(uint64_t desc, uint32_t bytes) { return desc + (bytes >> 4); }
+
 // D[tmem] (+)= A[tmem] * B[smem]: A is a 128-lane block of TMEM, row m in lane m, 16-bit
 // elements 2 j and 2 j + 1 of the row in the low and high half of column j
 __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
