@@ -58,6 +58,7 @@ template <int D> struct BwdCfg {
   static constexpr int kOperand = kSubs * kSub;          // K, V, one Q stage, one dO stage
   static constexpr int kStages = tensor_core_plan(D).bwd_gather_stages;   // Q / dO gather stages
   static constexpr int kKvBufs = tensor_core_plan(D).bwd_kv_buffers;
+  static_assert(kStages <= 2 && kKvBufs <= 2, "barriers for two");
   static constexpr int kSBufs = D == 64 ? 2 : 1;         // S buffers in TMEM
   static constexpr int kDsBytes = 2 * kSub;              // dS tile [keys][queries]; dQ is staged in it too
   static constexpr int kSmemData = 2 * kKvBufs * kOperand + 2 * kStages * kOperand + kDsBytes;
@@ -88,12 +89,14 @@ template <int D> struct Bars {
   uint64_t k_full[2], v_full[2], k_free[2], v_free[2];
   uint64_t k_fix[BwdCfg<D>::kKvBufs], v_fix[BwdCfg<D>::kKvBufs];   // per K / V buffer: the rows of a block cut short are zeroed (one for
                                                          // both could complete twice before its first phase is looked at)
-  uint64_t q_full[3], q_empty[3], g_full[3], g_empty[3]; // gather stages of Q (with the row data) and dO
+  uint64_t q_full[2], q_empty[2], g_full[2], g_empty[2]; // gather stages of Q (with the row data) and dO
   uint64_t s_full[2], dq_full[2], dq_read[2];   // per S buffer: at head_dim 64 two tiles' dQ can be waiting to be stored
-  uint64_t dp_full, p_full, ds_full, p_used, acc_full, acc_read, drain[2];
+  uint64_t p_full[2];                                    // by tiles in turn: with two S buffers P of the next tile may be complete before
+                                                         // the issuer has looked at this one's, or while a slow warp still owes its part of it
+  uint64_t dp_full, ds_full, p_used, acc_full, acc_read, drain[2];
   uint64_t col_full[4], col_free[4];
   Column cols[4];                                        // ring of item descriptors, published by the loader
-  uint8_t masked[3][4];                                  // stage, gather warp: some query does not attend all 128 keys
+  uint8_t masked[2][4];                                  // stage, gather warp: some query does not attend all 128 keys
   uint32_t tmem_base;
   int abort;
 };
@@ -237,13 +240,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       mbar_init(&bars->k_free[i], 1); mbar_init(&bars->v_free[i], 1);
       mbar_init(&bars->s_full[i], 1); mbar_init(&bars->dq_full[i], 1); mbar_init(&bars->dq_read[i], kStoreWarps);
     }
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars->p_full[i], kElemWarps);
       mbar_init(&bars->q_full[i], kGatherWarps); mbar_init(&bars->g_full[i], kGatherWarps);
       mbar_init(&bars->q_empty[i], 1); mbar_init(&bars->g_empty[i], 2);      // dK (after S); dP and dV, in either order
     }
     for (int i = 0; i < NKV; ++i) { mbar_init(&bars->k_fix[i], kGatherWarps); mbar_init(&bars->v_fix[i], kGatherWarps); }
     for (int i = 0; i < 4; ++i) { mbar_init(&bars->col_full[i], 1); mbar_init(&bars->col_free[i], kElemWarps + 2 + kGatherWarps + kStoreWarps); }
-    mbar_init(&bars->dp_full, 1); mbar_init(&bars->p_full, kElemWarps); mbar_init(&bars->ds_full, kElemWarps);
+    mbar_init(&bars->dp_full, 1); mbar_init(&bars->ds_full, kElemWarps);
     mbar_init(&bars->acc_full, 1); mbar_init(&bars->acc_read, kElemWarps);
     mbar_init(&bars->p_used, 1); mbar_init(&bars->drain[0], 1); mbar_init(&bars->drain[1], 1);
     // The swizzled operands need a base on a 1024-byte boundary. It is one (there is no static
@@ -341,7 +345,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           tmem_st_wait();
         }
         tc_fence_before();
-        mbar_arrive_warp(&bars->p_full);
+        mbar_arrive_warp(&bars->p_full[t & 1]);
         // ---- dS = P (dP - delta) ----
         // The dS tile: dQ of the tile before has read it, and at head_dim 128 dK.
         if (t >= 1) {
@@ -557,7 +561,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             const uint32_t st = t % NST;
             const uint32_t aQ = smem_u32(sQ) + st * Cfg::kOperand, aG = smem_u32(sG) + st * Cfg::kOperand;
             const uint32_t cP = cS + (t % NS) * 128;
-            mbar_wait(&bars->p_full, t & 1, wc, 26);
+            mbar_wait(&bars->p_full[t & 1], (t >> 1) & 1, wc, 26);
             mbar_wait(&bars->g_full[st], (t / NST) & 1, wc, 26);
             if (i == 0 && n_seen >= 2) mbar_wait(&bars->acc_read, (n_seen - 2) & 1, wc, 27);   // the accumulators have been stored
             tc_fence_after();
