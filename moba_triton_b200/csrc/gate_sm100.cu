@@ -30,17 +30,17 @@
 // descriptors do not stay in uniform registers, one took 120. Before, each score that passed was appended to a
 // buffer by predicated stores, five instructions a score whether it passed or not, and the two halves of a row's
 // candidates had lists of their own. us, before and now:
-//   131072 queries x 4 heads of 64, 1024 blocks       218    125       65536 x 4, 512 blocks, 12 each (exact)    319   160
-//   131072 x 32 heads of 128                         2170   1070       2 x 8192 x 4 of 128, blocks of 64 (exact) 117    60
+//   131072 queries x 4 heads of 64, 1024 blocks       218    125       65536 x 4, 512 blocks, 12 each (exact)    319   137
+//   131072 x 32 heads of 128                         2170   1070       2 x 8192 x 4 of 128, blocks of 64 (exact) 117    42
 //   524288 x 32 heads of 128, skewed                27300  12500       16 sequences, 40000 x 32 heads of 128     271   144
 //
 // EXACT: the same kernel where the portable gate used to run (other block sizes that divide 128,
 // more than eight ranked blocks): its selections are those of exact scores, bit for bit. The
 // tensor-core sum is off by at most `err` (a bound from the lengths of the query and of the means of
 // the unit's candidates), so the entry test is loosened by err, the windows keep all 32 bits of a score,
-// and a candidate whose rounding to the input dtype depends on that error is scored again in float64 by
-// its whole warp before it is ranked: about one in forty where scores are large against err, every one
-// near zero. A row without a finite bound (infinities, NaN, squares outside float32) has every candidate
+// and a candidate whose rounding to the input dtype depends on that error is scored again in float64
+// before it is ranked, four by a warp at a time: about one in forty where scores are large against err,
+// every one near zero. A row without a finite bound (infinities, NaN, squares outside float32) has every candidate
 // scored in float64. With blocks finer than the tile a row's candidates end at its own block.
 //
 // Scores are float32 tensor-core sums rounded to the input dtype; the portable
@@ -75,7 +75,9 @@ template <int D, bool EXACT> struct GateCfg {
   // The two windows of a warpgroup also take its Q tile on the way to TMEM.
   static constexpr int kPiece = kTile * 16, kWindow = 8 * kPiece, kQ = kSubs * kSub;
   static_assert(kQ <= 2 * kWindow, "a Q tile fits its warpgroup's windows");
-  static constexpr int kSmem = kTiles * 2 * kWindow + kStages * kKb + 1024 + 512;
+  // Exact: ids of a row's candidates that are to be scored again.
+  static constexpr int kPending = EXACT ? 16 : 0, kPendingBytes = kSelect * kPending * 2;
+  static constexpr int kSmem = kTiles * 2 * kWindow + kStages * kKb + kPendingBytes + 1024 + 512;
   // TMEM columns of a tile: scores [0, 64), queries [64, 64 + D / 2)
   static constexpr int kTileCols = 128, kQCol = kStepBlocks;
 };
@@ -224,16 +226,20 @@ __device__ __forceinline__ bool load_unit(Unit& u, int idx, const moba_b200_prob
   return true;
 }
 
-// Exact score of one (query, block) pair by a whole warp: the products of two 16-bit numbers and
-// their float64 sum carry no error, the result is rounded to float32 as everywhere in the gate.
+// Exact scores of four (query, block) pairs by a warp, eight lanes a pair: the products of two 16-bit numbers
+// and their float64 sum carry no error, the result is rounded to float32 as everywhere in the gate.
 template <int D, typename T>
-__device__ __forceinline__ float exact_score(const T* q_row, const T* kbar_row, int lane) {
+__device__ __forceinline__ float exact_score(const T* q_row, const T* kbar_row, int lane8) {
   double acc = 0.0;
 #pragma unroll
-  for (int i = 0; i < D / 32; ++i)
-    acc = fma((double)Elem<T>::to_f(q_row[i * 32 + lane]), (double)Elem<T>::to_f(kbar_row[i * 32 + lane]), acc);
+  for (int i = 0; i < D / 64; ++i) {
+    const uint4 a = *(reinterpret_cast<const uint4*>(q_row) + i * 8 + lane8), b = __ldg(reinterpret_cast<const uint4*>(kbar_row) + i * 8 + lane8);
+    const T *x = reinterpret_cast<const T*>(&a), *y = reinterpret_cast<const T*>(&b);
 #pragma unroll
-  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int e = 0; e < 8; ++e) acc = fma((double)Elem<T>::to_f(x[e]), (double)Elem<T>::to_f(y[e]), acc);
+  }
+#pragma unroll
+  for (int o = 4; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   return (float)acc;
 }
 
@@ -324,7 +330,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   unsigned char* sWin = smem;                                 // two windows of scores per thread, by warpgroups
   unsigned char* sKb = sWin + NT * 2 * Cfg::kWindow;
-  Bars* bars = reinterpret_cast<Bars*>(sKb + NST * Cfg::kKb);
+  Bars* bars = reinterpret_cast<Bars*>(sKb + NST * Cfg::kKb + Cfg::kPendingBytes);
   static_assert(sizeof(Bars) <= 512, "barrier block outgrew its reservation");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -431,6 +437,49 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
       // Scores that passed and are not ranked yet, a bit per column of a window. `hi` and `lo` are of the
       // window at `at0`, whose first column has id 0xFFFF - id0; `hi1` and `lo1` of the newest.
       uint32_t hi = 0, lo = 0, at0 = win0, id0 = 0, hi1 = 0, lo1 = 0, at1 = win0, id1 = 0;
+      // EXACT: candidates whose rounding depends on the sum's error wait here, by id, and are scored again in
+      // float64 for the whole warp at once, at the end of the unit or when a lane has no room for another. (Scored
+      // as they were popped they were most of the kernel, a memory latency each: 65536 x 4 heads, 12 of 512 blocks,
+      // 163 us, 137 so; 2 x 8192 x 4 of 128, blocks of 64, 60 and 42. Telling those that are in or out whichever way
+      // they round first, so that a sixth is left, costs what it saves: 142 and 40.) The order in which keys get
+      // to the list does not matter.
+      uint32_t pending = 0;
+      const uint32_t pend0 = smem_u32(sKb + NST * Cfg::kKb) + threadIdx.x * 2u;
+      auto resolve = [&]() {
+        while (const unsigned all = __ballot_sync(0xffffffffu, pending != 0u)) {
+          uint32_t id = 0;                                      // of this lane's last
+          if (pending != 0u) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(id) : "r"(pend0 + (pending - 1u) * (Cfg::kSelect * 2u)));
+          float exact = -INFINITY;
+          const size_t kv_row = (size_t)u.seq * p.kv_heads + u.hq / group;
+          for (unsigned open = all; open != 0u;) {              // eight lanes a candidate, two candidates each
+            float got[2];
+            unsigned mine[2] = {0u, 0u};                        // the lanes that the two rounds of four take
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              int who = -1;
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const int next = __ffs((int)open) - 1;
+                if ((lane >> 3) == g) who = next;
+                if (next >= 0) mine[j] |= 1u << next;
+                open &= open - 1u;
+              }
+              const int from = max(who, 0);
+              const uint32_t blk = __shfl_sync(0xffffffffu, id, from);
+              const T* qr = reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(q_row), from));
+              got[j] = exact_score<D, T>(qr, kbar + (kv_row * p.num_blocks + blk) * (size_t)D, lane & 7);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {                       // the n-th lane taken finds its score in the n-th group
+              const float x = __shfl_sync(0xffffffffu, got[j], (__popc(mine[j] & ((1u << lane) - 1u)) & 3) * 8);
+              if (mine[j] >> lane & 1u) exact = x;
+            }
+          }
+          // (a score taken again in float64 may be one that is never selected)
+          list_offer<L>(best, pending != 0u && exact > -INFINITY ? make_key((int)(short)round16<T>(exact), 0xFFFFu - id) : 0u);
+          if (pending != 0u) --pending;
+        }
+      };
       // Every lane offers one of its scores to its list, n times.
       auto pop = [&](uint32_t n) {
         PHASE_CLOCK(fl);
@@ -454,22 +503,15 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             lo = rest;
             float s;
             asm volatile("ld.shared.f32 %0, [%1];" : "=f"(s) : "r"(at0 + (k >> 2) * kPiece + (k & 3u) * 4u));
-            // does the rounding depend on the sum's error?
-            unsigned unsure = __ballot_sync(0xffffffffu, some && (err == INFINITY || round16<T>(s - err) != round16<T>(s + err)));
-            while (unsure) {
-              const int who = __ffs((int)unsure) - 1;
-              unsure &= unsure - 1;
-              const uint32_t blk = 0xFFFFu - __shfl_sync(0xffffffffu, id0 - k, who);
-              const T* qr = reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(q_row), who));
-              const size_t kv_row = (size_t)u.seq * p.kv_heads + u.hq / group;
-              const float exact = exact_score<D, T>(qr, kbar + (kv_row * p.num_blocks + blk) * (size_t)D, lane);
-              if (lane == who) s = exact;
-            }
-            // (a score taken again in float64 may be one that is never selected)
-            key = some && s > -INFINITY ? make_key((int)(short)round16<T>(s), id0 - k) : 0u;
+            const uint32_t pair = pack2<T>(__float_as_uint(s - err), __float_as_uint(s + err));
+            const bool unsure = some && (pair >> 16) != (pair & 0xffffu);
+            if (unsure) asm volatile("st.shared.u16 [%0], %1;" ::"r"(pend0 + pending * (Cfg::kSelect * 2u)), "h"((short)(0xFFFFu - (id0 - k))) : "memory");
+            pending += unsure ? 1u : 0u;
+            key = some && !unsure ? make_key((int)(short)round16<T>(s), id0 - k) : 0u;
           }
           list_offer<L>(best, key);
           if ((hi | lo) == 0u) { hi = hi1; lo = lo1; hi1 = 0u; lo1 = 0u; at0 = at1; id0 = id1; }
+          if (EXACT && __any_sync(0xffffffffu, pending == Cfg::kPending)) resolve();
         }
         if (n != 0u) bar.raise_to_entry(best[L - 1], err);
         PHASE_ADD(wc, 4, fl);                                   // (also counted in its phase)
@@ -605,6 +647,7 @@ gate_sm100_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         PHASE_ADD(wc, 3, ph);                                   // loads, masks, pops
       }
       pop(__reduce_max_sync(0xffffffffu, (uint32_t)(__popc(hi) + __popc(lo))));
+      if constexpr (EXACT) resolve();
       if (row0 + r < u.len) {
         // ---- emit: the best `take` ids plus the own block, ascending, -1 padded ----
         constexpr int NS = L <= 8 ? 8 : 16;
