@@ -11,6 +11,8 @@
 // unnormalised accumulator instead; the merged result is the same quantity).
 #include "common.cuh"
 
+#include <cuda_pipeline.h>
+
 namespace moba {
 
 __global__ void fill_kernel(float* __restrict__ dst, size_t n, float value) {
@@ -180,11 +182,14 @@ fwd_portable_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* _
 // (8 x D/16) of them in registers and reading operands as 16-byte pieces, so that an FMA costs a
 // sixteenth of a shared-memory load; P takes the place of Q and K between the two. The sums run in
 // the order of the portable kernel (over the head dim, over the keys), in float32 FMAs. A tile's FMAs
-// are 16 400 clocks of the SM's pipe at head_dim 64. At [1,4096,4,64] (0.14 ms, about 980 tiles on 296
-// resident CTAs: 3.3 rounds, paid as four) the pipe is 48 % busy, the issue slots 64 %, shared-memory
+// are 16 400 clocks of the SM's pipe at head_dim 64. At [1,4096,4,64] (0.135 ms, about 980 tiles on 296
+// resident CTAs: 3.3 rounds, paid as four) the pipe is half busy, the issue slots two thirds, shared-memory
 // wavefronts 42 % of their peak: two CTAs of eight warps do not fill the gaps of each other's loads and
-// barriers. The portable kernel, with one CTA per column, a load per FMA and as many as 32 tiles in one
-// CTA, took 1.3 ms.
+// barriers. The operands come by asynchronous copies, and V is not waited for before P is there: whole calls of
+// [1,8192,4,128] 825 -> 738 us, of [1,4096,4,64] 180 -> 175. Two queries an FMA instruction (with Q, K and P
+// transposed in shared memory) took 676 and 192: such an instruction takes as long as two, and at head_dim 64
+// the copies it needs twice of an operand cost more than the issue slots it frees. The portable kernel, with one
+// CTA per column, a load per FMA and as many as 32 tiles in one CTA, took 1.3 ms.
 // ---------------------------------------------------------------------------
 constexpr int kF32Tile = 128;
 template <int D> struct F32Cfg {
@@ -219,31 +224,39 @@ fwd_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, const f
   if (n <= 0 || keys <= 0) return;
   const size_t list0 = (size_t)kv_row * ix.capacity + ix.col_offsets[(size_t)kv_row * (p.num_blocks + 1) + w.blk] + w.first +
                        (size_t)blockIdx.y * kF32Tile;
+  // Everything by asynchronous copies, Q and K first; nobody waits for V before P is there.
   constexpr int CPR = D / 4;                                // 16-byte pieces per row
+  auto put = [&](float* to, const float* from, bool there) {
+    if (there) __pipeline_memcpy_async(to, from, 16);
+    else *reinterpret_cast<float4*>(to) = make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+#pragma unroll 4
   for (int i = threadIdx.x; i < kF32Tile * CPR; i += 256) {
     const int j = i / CPR, c = (i % CPR) * 4;
-    float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-    if (j < keys) {
-      const size_t src = ((b * p.tokens + key0 + j) * p.kv_heads + kvh) * (size_t)D + c;
-      kv = __ldg(reinterpret_cast<const float4*>(k + src));
-      vv = __ldg(reinterpret_cast<const float4*>(v + src));
-    }
-    *reinterpret_cast<float4*>(Ks + j * Cfg::kRow + c) = kv;
-    *reinterpret_cast<float4*>(Vs + j * Cfg::kRow + c) = vv;
+    put(Ks + j * Cfg::kRow + c, k + ((b * p.tokens + key0 + j) * p.kv_heads + kvh) * (size_t)D + c, j < keys);
   }
+#pragma unroll 4
   for (int i = threadIdx.x; i < kF32Tile * CPR; i += 256) {
     const int j = i / CPR, c = (i % CPR) * 4;
-    float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* from = q;
     int row = -1, dst = -1;
     if (j < n) {
       const PairEntry e = load_pair(ix, list0 + j);
       row = e.row;
       dst = (int)(part_row(p, b, e.head, e.row) * (size_t)p.slots + e.slot);
-      qv = __ldg(reinterpret_cast<const float4*>(q + ((b * p.tokens + e.row) * p.q_heads + e.head) * (size_t)D + c));
+      from = q + ((b * p.tokens + e.row) * p.q_heads + e.head) * (size_t)D + c;
     }
     if (c == 0) { row_s[j] = row; dst_s[j] = dst; }
-    *reinterpret_cast<float4*>(Qs + j * Cfg::kRow + c) = qv;
+    put(Qs + j * Cfg::kRow + c, from, j < n);
   }
+  __pipeline_commit();
+#pragma unroll 4
+  for (int i = threadIdx.x; i < kF32Tile * CPR; i += 256) {
+    const int j = i / CPR, c = (i % CPR) * 4;
+    put(Vs + j * Cfg::kRow + c, v + ((b * p.tokens + key0 + j) * p.kv_heads + kvh) * (size_t)D + c, j < keys);
+  }
+  __pipeline_commit();
+  __pipeline_wait_prior(1);
   __syncthreads();
 
   // thread (ty, tx): queries ty + 16 i, keys tx + 16 j
@@ -297,6 +310,7 @@ fwd_f32_kernel(const float* __restrict__ q, const float* __restrict__ k, const f
     l[i] = sum;
     if (tx == 0 && row >= 0) part_lse[dst_s[ty + 16 * i]] = m + log2f(sum);
   }
+  __pipeline_wait_prior(0);
   __syncthreads();
 
   // thread (ty, tx): queries ty + 16 i, head-dim columns 4 tx + 64 h

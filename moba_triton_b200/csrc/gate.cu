@@ -18,28 +18,32 @@
 namespace moba {
 
 // ---------------------------------------------------------------------------
-// pool: grid (num_blocks, n_seq * Hkv), 128 threads
+// pool: grid (num_blocks, n_seq * Hkv), 128 or 256 threads
 // ---------------------------------------------------------------------------
+// Threads of a block of keys, and rows in flight per thread. The conversions to float64 bound the 16-bit types
+// (16 a clock and SM), the memory latency float32, which has no second round of loads so: [1,4096,4,64] 14.9 us with
+// 128 and four, 11.2 with 256 and eight; 262144 x 16 heads of 128 in bfloat16 293 and 464.
+template <typename T> constexpr int kPoolThreads = sizeof(T) == 4 ? 256 : 128;
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kPoolThreads<T>)
 pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restrict__ kbar,
             int packed, int tokens, int hkv, int d, int bs, int nb, int* __restrict__ zero_cell, float* __restrict__ norms) {
   pdl_trigger();
   pdl_wait();
   if (zero_cell != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_cell = 0;
-  constexpr int EPV = 16 / sizeof(T);            // elements per 16-byte vector
+  constexpr int EPV = 16 / sizeof(T), NT = kPoolThreads<T>;   // elements per 16-byte vector; threads
   const int blk = (int)(blockIdx.x % nb), kv_row = (int)(blockIdx.x / nb);
   const int seq = kv_row / hkv, h = kv_row % hkv;
   const SeqSpan sp = seq_span(cu, packed, seq, tokens);
   const int vpr = d / EPV;                       // vectors per row
-  const int groups = 128 / vpr;
+  const int groups = NT / vpr;
   const int c = threadIdx.x % vpr, rg = threadIdx.x / vpr;
 
   T* dst = kbar + ((size_t)kv_row * nb + blk) * d;
   const int lo = blk * bs;
   if (lo >= sp.len) {                            // padded slot of a short packed sequence
     if (threadIdx.x < d) dst[threadIdx.x] = Elem<T>::from_f(0.f);
-    for (int i = threadIdx.x + 128; i < d; i += 128) dst[i] = Elem<T>::from_f(0.f);
+    for (int i = threadIdx.x + NT; i < d; i += NT) dst[i] = Elem<T>::from_f(0.f);
     if (norms != nullptr && threadIdx.x == 0) norms[(size_t)kv_row * nb + blk] = 0.f;
     return;
   }
@@ -52,8 +56,7 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
 #pragma unroll
   for (int e = 0; e < EPV; ++e) acc[e] = 0.0;
   if (rg < groups) {
-    // four rows in flight per thread: the loads do not depend on one another
-    constexpr int kAhead = 4;
+    constexpr int kAhead = sizeof(T) == 4 ? 8 : 4;               // the loads do not depend on one another
     for (int r0 = rg; r0 < hi - lo; r0 += groups * kAhead) {
       uint4 raw[kAhead];
 #pragma unroll
@@ -72,16 +75,27 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
     }
   }
   // Sums over the row groups, one output element per thread (float64 sums of these values are
-  // exact, so the order of the additions does not matter).
-  __shared__ double red[128 * EPV];
+  // exact, so the order of the additions does not matter): in float32 first those in a warp, where a row's
+  // vectors fill a part of it, then the warps' (or groups') through shared memory.
+  __shared__ double red[NT * EPV];
+  const bool by_warp = sizeof(T) == 4 && 32 % vpr == 0;
+  int parts = groups, part = rg;
+  if (by_warp) {
+    for (int o = vpr; o < 32; o <<= 1)
 #pragma unroll
-  for (int e = 0; e < EPV; ++e) red[threadIdx.x * EPV + e] = acc[e];
+      for (int e = 0; e < EPV; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    parts = NT / 32; part = threadIdx.x >> 5;
+  }
+  if (by_warp ? (threadIdx.x & 31) < vpr : rg < groups) {
+#pragma unroll
+    for (int e = 0; e < EPV; ++e) red[part * d + c * EPV + e] = acc[e];
+  }
   __syncthreads();
   const float occ = (float)(hi - lo);
   double square = 0.0;                                          // in float64: no square leaves its range
-  for (int i = threadIdx.x; i < d; i += 128) {
+  for (int i = threadIdx.x; i < d; i += NT) {
     double s = 0.0;
-    for (int g = 0; g < groups; ++g) s += red[g * d + i];       // thread g * vpr + i / EPV, element i % EPV
+    for (int g = 0; g < parts; ++g) s += red[g * d + i];
     const float total = Elem<T>::round_f((float)s);
     const T mean = Elem<T>::from_f(__fdiv_rn(total, occ));
     dst[i] = mean;
@@ -89,12 +103,15 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
   }
   if (norms == nullptr) return;
   // the block mean's length, for the error bound of the exact gate
-  __shared__ double part[4];
+  __shared__ double squares[NT / 32];
 #pragma unroll
   for (int o = 16; o; o >>= 1) square += __shfl_xor_sync(0xffffffffu, square, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = square;
+  if ((threadIdx.x & 31) == 0) squares[threadIdx.x >> 5] = square;
   __syncthreads();
-  if (threadIdx.x == 0) norms[(size_t)kv_row * nb + blk] = (float)sqrt(part[0] + part[1] + part[2] + part[3]);
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < NT / 32; ++w) squares[0] += squares[w];
+    norms[(size_t)kv_row * nb + blk] = (float)sqrt(squares[0]);
+  }
 }
 
 // `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from; `norms`
@@ -111,7 +128,7 @@ int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, vo
   if (ctas > 0x7fffffffLL) { set_error("pool: %lld blocks exceed the grid limit", ctas); return MOBA_B200_EUNSUPPORTED; }
   const unsigned grid = (unsigned)ctas;
 #define MOBA_POOL(T)                                                                                   \
-  MOBA_CUDA_OK(launch_chained(pool_kernel<T>, grid, 128, 0, st, (const T*)k, cu, (T*)kbar, p.packed, p.tokens, \
+  MOBA_CUDA_OK(launch_chained(pool_kernel<T>, grid, kPoolThreads<T>, 0, st, (const T*)k, cu, (T*)kbar, p.packed, p.tokens, \
                               p.kv_heads, p.head_dim, p.block_size, p.num_blocks, zero_cell, norms))
   if (p.dtype == MOBA_B200_F32) MOBA_POOL(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_POOL(__nv_bfloat16);
@@ -169,35 +186,34 @@ __device__ __forceinline__ unsigned long long exchange(unsigned long long x, int
   const unsigned long long o = __shfl_xor_sync(0xffffffffu, x, j);
   return (x > o) == keep_larger ? x : o;
 }
-// Bitonic: the warp's 32 keys in descending order over the lanes.
-__device__ __forceinline__ unsigned long long sort_lanes(unsigned long long x, int lane) {
+// Bitonic: the warp's 32 keys of each row in descending order over the lanes. The rows go in step: an exchange
+// waits for its shuffles, and N rows' wait together.
+template <int N>
+__device__ __forceinline__ void sort_lanes(unsigned long long (&x)[N], int lane) {
 #pragma unroll
   for (int k = 2; k <= 32; k <<= 1)
 #pragma unroll
-    for (int j = k >> 1; j >= 1; j >>= 1) x = exchange(x, j, ((lane & j) == 0) == ((lane & k) == 0));
-  return x;
-}
-// The 32 largest of two descending sequences, descending.
-__device__ __forceinline__ unsigned long long merge_sorted(unsigned long long a, unsigned long long b, int lane) {
-  b = __shfl_sync(0xffffffffu, b, 31 - lane);
-  unsigned long long x = a > b ? a : b;
+    for (int j = k >> 1; j >= 1; j >>= 1)
 #pragma unroll
-  for (int j = 16; j >= 1; j >>= 1) x = exchange(x, j, (lane & j) == 0);
-  return x;
+      for (int r = 0; r < N; ++r) x[r] = exchange(x[r], j, ((lane & j) == 0) == ((lane & k) == 0));
 }
-// best[r] for an r that the compiler does not know
+// a: the 32 largest of two descending sequences each, descending.
 template <int N>
-__device__ __forceinline__ unsigned long long sorted_row(const unsigned long long (&best)[N], int r) {
-  unsigned long long x = best[0];
+__device__ __forceinline__ void merge_sorted(unsigned long long (&a)[N], const unsigned long long (&b)[N], int lane) {
 #pragma unroll
-  for (int e = 1; e < N; ++e) if (r == e) x = best[e];
-  return x;
+  for (int r = 0; r < N; ++r) {
+    const unsigned long long o = __shfl_sync(0xffffffffu, b[r], 31 - lane);
+    a[r] = a[r] > o ? a[r] : o;
+  }
+#pragma unroll
+  for (int j = 16; j >= 1; j >>= 1)
+#pragma unroll
+    for (int r = 0; r < N; ++r) a[r] = exchange(a[r], j, (lane & j) == 0);
 }
-
 // SORTED: up to 32 ranked blocks. The row's list lies sorted over the lanes of its warp, and a chunk
 // of 32 candidates is sorted and merged into it in 21 exchanges; offering them one by one, a reduction
 // over the warp and two over the list each, was two thirds of the kernel ([1,4096,4,64] float32,
-// 7 of 32 blocks: 76 us, sorted 29).
+// 7 of 32 blocks: 76 us, sorted 29, with the eight rows of a warp in step and two numbers a load 25).
 template <typename T, bool SORTED>
 __global__ void __launch_bounds__(128)
 gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
@@ -206,9 +222,11 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
   pdl_wait();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int d = p.head_dim, take = p.take, slots = p.slots;
-  double* qs = reinterpret_cast<double*>(smem_raw);                       // [32][d]
-  double* ks = qs + kGateRows * d;                                        // [32][d+1]
-  float* lval = reinterpret_cast<float*>(ks + kGateChunk * (d + 1));      // [32][take]
+  const int qst = (d + 1) / 2 * 2;
+  double* qs = reinterpret_cast<double*>(smem_raw);                       // [32][qst]
+  const int kst = (d + 1) / 2 * 2 + 2;                                    // row stride of ks: lanes on different banks, 16-byte rows
+  double* ks = qs + kGateRows * qst;                                      // [32][kst]
+  float* lval = reinterpret_cast<float*>(ks + kGateChunk * kst);      // [32][take]
   int* lidx = reinterpret_cast<int*>(lval + kGateRows * max(take, 1));    // [32][take]
 
   const int group = p.q_heads / p.kv_heads;
@@ -221,10 +239,10 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // stage the 32 query rows as float64; dead rows are zero
-  for (int i = threadIdx.x; i < kGateRows * d; i += 128) {
-    const int r = i / d, c = i % d;
+  for (int i = threadIdx.x; i < kGateRows * qst; i += 128) {
+    const int r = i / qst, c = i % qst;
     double v = 0.0;
-    if (row0 + r < sp.len)
+    if (c < d && row0 + r < sp.len)
       v = (double)Elem<T>::to_f(q[((batch_base + sp.bos + row0 + r) * p.q_heads + hq) * (size_t)d + c]);
     qs[i] = v;
   }
@@ -244,23 +262,43 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
 
   for (int c0 = 0; take > 0 && c0 < horizon; c0 += kGateChunk) {
     __syncthreads();
-    for (int i = threadIdx.x; i < kGateChunk * d; i += 128) {
-      const int j = i / d, c = i % d;
-      ks[j * (d + 1) + c] = (c0 + j < n_cand) ? (double)Elem<T>::to_f(kb[(size_t)(c0 + j) * d + c]) : 0.0;
+    for (int i = threadIdx.x; i < kGateChunk * qst; i += 128) {
+      const int j = i / qst, c = i % qst;
+      ks[j * kst + c] = (c < d && c0 + j < n_cand) ? (double)Elem<T>::to_f(kb[(size_t)(c0 + j) * d + c]) : 0.0;
     }
     __syncthreads();
 
     double acc[kRowsPerWarp];
 #pragma unroll
     for (int r = 0; r < kRowsPerWarp; ++r) acc[r] = 0.0;
-    const double* krow = ks + lane * (d + 1);
-    const double* qrow = qs + warp * kRowsPerWarp * d;
-    for (int c = 0; c < d; ++c) {
-      const double kv = krow[c];
+    const double* krow = ks + lane * kst;
+    const double* qrow = qs + warp * kRowsPerWarp * qst;
+    for (int c = 0; c < qst; c += 2) {                             // (past d: zeros)
+      const double2 kv = *reinterpret_cast<const double2*>(krow + c);
 #pragma unroll
-      for (int r = 0; r < kRowsPerWarp; ++r) acc[r] = fma(qrow[r * d + c], kv, acc[r]);
+      for (int r = 0; r < kRowsPerWarp; ++r) {
+        const double2 qv = *reinterpret_cast<const double2*>(qrow + r * qst + c);
+        acc[r] = fma(qv.y, kv.y, fma(qv.x, kv.x, acc[r]));
+      }
     }
     const int blk = c0 + lane;
+    if constexpr (SORTED) {
+      unsigned long long key[kRowsPerWarp];
+      bool enters = false;
+#pragma unroll
+      for (int r = 0; r < kRowsPerWarp; ++r) {
+        const int row = row0 + warp * kRowsPerWarp + r;
+        const bool candidate = gate_candidate(p, blk, row / p.block_size) && blk < n_cand && row < sp.len;
+        key[r] = candidate ? rank_key(Elem<T>::round_f((float)acc[r]), blk) : 0ull;
+        const unsigned long long bar = __shfl_sync(0xffffffffu, best[r], take - 1);   // (by all lanes)
+        enters |= key[r] > bar;
+      }
+      if (__any_sync(0xffffffffu, enters)) {
+        sort_lanes(key, lane);
+        merge_sorted(best, key, lane);
+      }
+      continue;
+    }
 #pragma unroll
     for (int r = 0; r < kRowsPerWarp; ++r) {
       const int lrow = warp * kRowsPerWarp + r;
@@ -268,12 +306,6 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
       const int own = row / p.block_size;
       float s = Elem<T>::round_f((float)acc[r]);
       if (!(gate_candidate(p, blk, own) && blk < n_cand && row < sp.len)) s = -INFINITY;
-      if constexpr (SORTED) {
-        const unsigned long long key = rank_key(s, blk);
-        if (__any_sync(0xffffffffu, key > __shfl_sync(0xffffffffu, best[r], take - 1)))
-          best[r] = merge_sorted(best[r], sort_lanes(key, lane), lane);
-        continue;
-      }
       float* lv = lval + lrow * take;
       int* li = lidx + lrow * take;
       // offer the chunk's candidates in (score desc, id asc) order while they clear the bar
@@ -306,7 +338,7 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
   __syncwarp();
 
   // emit ascending ids: rank every kept entry (and the own block) by id
-#pragma unroll 1
+#pragma unroll
   for (int r = 0; r < kRowsPerWarp; ++r) {
     const int lrow = warp * kRowsPerWarp + r;
     const int row = row0 + lrow;
@@ -317,7 +349,7 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
     const size_t out_at = ((b * p.q_heads + hq) * p.tokens + sp.bos + row) * (size_t)slots;
     int32_t* out = block_idx + out_at;
     if constexpr (SORTED) {
-      const unsigned long long key = sorted_row(best, r);
+      const unsigned long long key = best[r];
       const bool have = lane < take && key != 0ull;
       const int id = have ? (int)(0xffffffffu - (unsigned)key) : kEmptyIdx;
       int rank = 0;
@@ -360,7 +392,8 @@ int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* 
                          const int32_t* cu, int32_t* block_idx, float* lse_fill, cudaStream_t st) {
   KernelTimer timer__("gate_portable_kernel", st);
   const int d = p.head_dim;
-  const size_t smem = sizeof(double) * (kGateRows * d + kGateChunk * (d + 1)) +
+  const int qst = (d + 1) / 2 * 2;
+  const size_t smem = sizeof(double) * (kGateRows * qst + kGateChunk * (qst + 2)) +
                       (size_t)kGateRows * (p.take > 0 ? p.take : 1) * 8;
   if (smem > 200 * 1024) {
     set_error("gate: head_dim %d / top_k %d need %zu bytes of shared memory", d, p.top_k, smem);
