@@ -32,10 +32,20 @@ inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 //   [1,8192,5]                            17.3    512                156  125  115               71.8 69.5 70.3
 //   [1,4096,4] float32, whose kernel       6.9    256                                               -  185  198
 //     starts a CTA for every tile that an item may have
+// Between 24 and 64 tiles per SM the partials are what a finer cut costs: eight tiles on top of a quarter of an
+// SM's share. us, attention kernels and sums of a training step (head_dim 128 unless noted), with items of
+//                                     tiles per SM   a quarter, at least 8     12    16    24    32
+//   [2,8192,4], blocks of 64                27.7     250   (8)             245   238   243   259
+//   [1,16384,4], head_dim 64                27.7     158   (8)             152   149   154   161
+//   [1,32768,4]                             55       389  (14)             393   391   375   390
+//   [1,8192,16 on 4]                        55       340  (14)             345   335   325   329
+//   [1,32768,8 on 2], head_dim 64          111       462  (28)             487   475   462   452 (447 with 36)
+//   [1,65536,4], head_dim 64               111       493  (28)             525   515   496   493 (503 with 36)
+// A forward alone has no partials and keeps the finer items, the better spread (2 % of its kernel).
 // The cut decides in which groups dK and dV are summed: who runs the KV heads of a problem in several
 // passes and wants the bits of the whole gives every pass the whole's chunk_tiles
 // (moba_b200_op_launch_plan).
-moba_b200_problem with_cut(const moba_b200_problem& p0) {
+moba_b200_problem with_cut(const moba_b200_problem& p0, bool training = true) {
   moba_b200_problem p = p0;
   if (p.chunk_tiles > 0) return p;
   p.chunk_tiles = sched_chunk_tiles(p);
@@ -44,6 +54,8 @@ moba_b200_problem with_cut(const moba_b200_problem& p0) {
   const bool short_rows = row_tiles <= 128;
   if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = short_rows ? 2 : 4;
   else if (tiles <= 16LL * kSchedSMs && (short_rows || p.dtype == MOBA_B200_F32)) p.chunk_tiles = 4;
+  else if (training && p.dtype != MOBA_B200_F32 && tiles >= 24LL * kSchedSMs && tiles <= 64LL * kSchedSMs)
+    p.chunk_tiles = (int)((tiles + kSchedSplit * kSchedSMs - 1) / (kSchedSplit * kSchedSMs)) + kMinChunkTiles;
   return p;
 }
 
@@ -91,7 +103,9 @@ Layout layout_of(const moba_b200_problem& gate, const moba_b200_problem& p) {
   l.col_nnz = take(rows * nb * 4);
   l.col_offsets = take(rows * (nb + 1) * 4);
   l.order = take(rows * nb * 4);
-  l.items = take(rows * (size_t)sched_items_per_row(p) * 16);
+  moba_b200_problem alone = p;                               // a forward alone may have finer items, and more
+  if (p.chunk_tiles > kMinChunkTiles) { alone.chunk_tiles = 0; alone.chunk_tiles = sched_chunk_tiles(alone); }
+  l.items = take(rows * (size_t)(sched_items_per_row(alone) > sched_items_per_row(p) ? sched_items_per_row(alone) : sched_items_per_row(p)) * 16);
   l.entries = take(rows * capacity * 8);
   l.part_lse = take(pairs * 4);
   l.lse = take(window ? 0 : (size_t)p.batch * p.q_heads * p.tokens * 4);
@@ -248,11 +262,13 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   int32_t* counter = reinterpret_cast<int32_t*>(tmp + l.counter);
   const bool exact_gate = runs_exact_gate(gate, gate_path);
   float* norms = reinterpret_cast<float*>(tmp + l.norms);
+  Columns cut = columns;                                     // the layout holds either cut's table
+  if (!want_lse) cut.p.chunk_tiles = with_cut(*p0, false).chunk_tiles;
   MOBA_TRY(launch_pool(gate, k, cu_seqlens, kbar, counter, exact_gate ? norms : nullptr, st));
   if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
   else if (exact_gate) MOBA_TRY(launch_gate_exact_sm100(gate, q, kbar, norms, cu_seqlens, block_idx, part_lse, st));
   else MOBA_TRY(launch_gate_portable(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
-  return attend(columns, l, fwd_path, q, k, v, block_idx, cu_seqlens, keep, tmp, out,
+  return attend(cut, l, fwd_path, q, k, v, block_idx, cu_seqlens, keep, tmp, out,
                 want_lse ? reinterpret_cast<float*>(keep + l.lse) : nullptr, st);
 }
 

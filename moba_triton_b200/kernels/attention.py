@@ -98,14 +98,14 @@ def _kv_head_passes(q, k, v, kv_heads_per_pass: int):
 def _cut_of_the_whole(q, k, cfg, causal, cu_seqlens, max_seqlen) -> int:
     """Tiles per work item that passes over the KV heads of a call take, so that they sum dK and dV
     in the groups of the whole call; 0 = their own cut. A call of more than 4 736 tiles (32 per SM)
-    has items of a quarter of an SM's share of it, too long for a pass to spread over the SMs."""
+    has items of more than 16, too long for a pass to spread over the SMs."""
     hkv = k.shape[2]
     prob = _lib.make_problem((*q.shape[:2], q.shape[2] // hkv * hkv, q.shape[3]), hkv, q.dtype, cfg, cu_seqlens, max_seqlen,
                              causal=causal)
     plan = _lib.Plan()
     if _lib.load().moba_b200_op_launch_plan(prob, plan) < 0:
         return 0                                              # too large as one call: nothing to equal
-    return plan.chunk_tiles if plan.chunk_tiles <= 8 else 0
+    return plan.chunk_tiles if plan.chunk_tiles <= 16 else 0
 
 
 def moba_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cfg: MoBAConfig,
