@@ -322,7 +322,7 @@ int moba_b200_fwd(const moba_b200_problem* p, const void* q, const void* k, cons
   cudaStream_t st = (cudaStream_t)stream;
   MOBA_TRY(launch_fill_lse(*p, part_lse, st));
   if (path == MOBA_B200_PATH_TCGEN05)
-    return launch_fwd_sm100(*p, q, k, v, *index, cu_seqlens, part_o, part_lse, kBlockKeys, st);
+    return launch_fwd_sm100(*p, q, k, v, *index, cu_seqlens, part_o, part_lse, kBlockKeys, nullptr, st);
   return launch_fwd_portable(*p, q, k, v, *index, cu_seqlens, part_o, part_lse, st);
 }
 
@@ -348,10 +348,10 @@ int moba_b200_bwd(const moba_b200_problem* p, const void* q, const void* k, cons
   if (path < 0) return path;
   cudaStream_t st = (cudaStream_t)stream;
   bool reduces = false;
-  MOBA_TRY(launch_delta(*p, out, dout, delta, st));
+  MOBA_TRY(launch_delta(*p, out, dout, delta, nullptr, st));
   if (path == MOBA_B200_PATH_TCGEN05)
     MOBA_TRY(launch_bwd_sm100(*p, q, k, v, dout, lse, delta, *index, cu_seqlens, dq_part,
-                              static_cast<float*>(dkv_scratch), dk, dv, kBlockKeys, &reduces, st));
+                              static_cast<float*>(dkv_scratch), dk, dv, kBlockKeys, nullptr, &reduces, st));
   else
     MOBA_TRY(launch_bwd_portable(*p, q, k, v, dout, lse, delta, *index, cu_seqlens, dq_part, dk, dv, st));
   return launch_dq_reduce(*p, dq_part, part_lse, dq, reduces, st);

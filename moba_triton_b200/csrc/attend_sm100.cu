@@ -124,13 +124,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-// Work item `item` of the launch: the items of the (sequence, kv head) rows interleaved, each
-// row's in its dispatch order (heaviest first); false for padding.
-__device__ __forceinline__ bool load_column(Column& c, int item, const moba_b200_index& ix,
-                                            const moba_b200_problem& p, const int32_t* cu, int n_kv_rows) {
-  c.kv_row = item % n_kv_rows;
+// Work item `j` of a (sequence, kv head) row, in its dispatch order (heaviest first); false for padding.
+__device__ __forceinline__ bool load_column(Column& c, int kv_row, int j, const moba_b200_index& ix,
+                                            const moba_b200_problem& p, const int32_t* cu) {
+  c.kv_row = kv_row;
   WorkItem w;
-  if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, item / n_kv_rows)) return false;
+  if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, j)) return false;
   c.blk = w.blk;
   c.n = w.n;
   c.lo = ix.col_offsets[(size_t)c.kv_row * (p.num_blocks + 1) + c.blk] + w.first;
@@ -179,7 +178,7 @@ __global__ void __launch_bounds__(FwdCfg<D>::kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                  const __grid_constant__ CUtensorMap q_map, moba_b200_index ix, const int32_t* __restrict__ cu,
                  TP* __restrict__ part_o, float* __restrict__ part_lse, moba_b200_problem p, int part_keys, int n_items,
-                 unsigned* error_word) {
+                 ClaimOrder order, unsigned* error_word) {
   using Cfg = FwdCfg<D>;
   constexpr int NB = Cfg::kBufs, NKV = Cfg::kKvBufs;
   constexpr bool kStaged = sizeof(TP) == 2;
@@ -574,22 +573,45 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       Column mine;
       unsigned found = 0;
       int round0 = 0;
-      auto next = [&](Column& c) {
-        while (found == 0) {
-          if ((long long)round0 * G >= n_items) return false;
-          const int round = round0 + lane;
-          const long long item = (long long)round * G + ((round & 1) ? (G - 1 - (int)blockIdx.x) : (int)blockIdx.x);
-          found = __ballot_sync(0xffffffffu, item < n_items && load_column(mine, (int)item, ix, p, cu, n_kv_rows));
-          round0 += 32;
-        }
-        const int src = __ffs(found) - 1;
-        found &= found - 1;
+      auto take = [&](Column& c, int src) {
         c.kv_row = __shfl_sync(0xffffffffu, mine.kv_row, src); c.blk = __shfl_sync(0xffffffffu, mine.blk, src);
         c.n = __shfl_sync(0xffffffffu, mine.n, src); c.lo = __shfl_sync(0xffffffffu, mine.lo, src);
         c.key0 = __shfl_sync(0xffffffffu, mine.key0, src); c.keys = __shfl_sync(0xffffffffu, mine.keys, src);
         c.bos = __shfl_sync(0xffffffffu, mine.bos, src); c.tok0 = __shfl_sync(0xffffffffu, mine.tok0, src);
         return true;
       };
+      auto dealt = [&](Column& c) {
+        while (found == 0) {
+          if ((long long)round0 * G >= n_items) return false;
+          const int round = round0 + lane;
+          const long long item = (long long)round * G + ((round & 1) ? (G - 1 - (int)blockIdx.x) : (int)blockIdx.x);
+          found = __ballot_sync(0xffffffffu, item < n_items && load_column(mine, (int)(item % n_kv_rows), (int)(item / n_kv_rows), ix, p, cu));
+          round0 += 32;
+        }
+        const int src = __ffs(found) - 1;
+        found &= found - 1;
+        return take(c, src);
+      };
+      // The next item by a claim. Padding ends every row of the table: when 32 entries from the claimed one on,
+      // which reach every row of the group, name nothing, the group is done.
+      auto claim = [&](Column& c) {
+        for (;;) {
+          int g = 0;
+          if (lane == 0) g = atomicAdd(order.next, 1);
+          g = __shfl_sync(0xffffffffu, g, 0);
+          if (g >= n_items) return false;
+          const int end = claimed_item(g, n_kv_rows, ix.items_per_row, order.rows).group_end;
+          bool there = false;
+          if (g + lane < end) {
+            const ClaimedItem at = claimed_item(g + lane, n_kv_rows, ix.items_per_row, order.rows);
+            there = load_column(mine, at.kv_row, at.j, ix, p, cu);
+          }
+          const unsigned some = __ballot_sync(0xffffffffu, there);
+          if (some & 1u) return take(c, 0);
+          if (some == 0u && lane == 0) atomicMax(order.next, end);
+        }
+      };
+      auto next = [&](Column& c) { return order.next != nullptr ? claim(c) : dealt(c); };
       auto publish = [&](const Column& c, uint32_t n) {
         if (n >= 8) mbar_wait(&bars->col_free[n & 7], ((n >> 3) - 1) & 1, wc, 6);
         __syncwarp();
@@ -665,14 +687,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
 template <int D, typename T, typename TP>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensorMap& vm, const CUtensorMap& qm,
                const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse, int part_keys, int n_items,
-               unsigned* err, cudaStream_t st) {
+               const ClaimOrder& order, unsigned* err, cudaStream_t st) {
   auto kern = fwd_sm100_kernel<D, T, TP>;
   static SmemLimit limit;
   if (int rc = raise_smem_limit(limit, (const void*)kern, FwdCfg<D>::kSmem)) return rc;
   const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
   MOBA_CUDA_OK(launch_chained(kern, grid, FwdCfg<D>::kThreads, FwdCfg<D>::kSmem, st, km, vm, qm, ix, cu,
-                              (TP*)part_o, part_lse, p, part_keys, n_items, err));
+                              (TP*)part_o, part_lse, p, part_keys, n_items, order, err));
   return MOBA_B200_OK;
 }
 
@@ -686,7 +708,7 @@ bool fwd_sm100_supported(const moba_b200_problem& p) {
 
 int launch_fwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse,
-                     int part_keys, cudaStream_t st) {
+                     int part_keys, int* claims, cudaStream_t st) {
   KernelTimer timer__("fwd_sm100_kernel", st);
   unsigned* err = device_error_word();
   if (err == nullptr) { set_error("forward: no device error word"); return MOBA_B200_ECUDA; }
@@ -706,8 +728,10 @@ int launch_fwd_sm100(const moba_b200_problem& p, const void* q, const void* k, c
   const long long n_items_ll = (long long)ix.items_per_row * p.n_seq * p.kv_heads;
   if (n_items_ll > 0x7fffffffLL) { set_error("forward: too many work items"); return MOBA_B200_EUNSUPPORTED; }
   const int n_items = (int)n_items_ll;
+  const int rows_claimed = claims != nullptr ? claim_rows(p, p.head_dim == 64 ? 192 : 48) : 0;
+  const ClaimOrder order{rows_claimed > 0 ? claims : nullptr, rows_claimed};
   const bool bf = p.dtype == MOBA_B200_BF16;
-#define GO(D, T, TP) return launch_one<D, T, TP>(p, km, vm, qm, ix, cu, part_o, part_lse, part_keys, n_items, err, st)
+#define GO(D, T, TP) return launch_one<D, T, TP>(p, km, vm, qm, ix, cu, part_o, part_lse, part_keys, n_items, order, err, st)
   if (p.head_dim == 64) {
     if (bf) { if (p.part_f32) GO(64, __nv_bfloat16, float); else GO(64, __nv_bfloat16, __nv_bfloat16); }
     else { if (p.part_f32) GO(64, __half, float); else GO(64, __half, __half); }

@@ -23,9 +23,11 @@ namespace moba {
 template <typename T>
 __global__ void __launch_bounds__(256)
 delta_kernel(const T* __restrict__ out, const T* __restrict__ dout, float* __restrict__ delta,
-             unsigned rows_per_batch, int tokens, int q_heads, int d, unsigned long long heads_recip, int heads_shift) {
+             unsigned rows_per_batch, int tokens, int q_heads, int d, unsigned long long heads_recip, int heads_shift,
+             int* __restrict__ zero_cell) {
   pdl_trigger();
   pdl_wait();
+  if (zero_cell != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *zero_cell = 0;
   constexpr int EPV = 16 / sizeof(T);
   const int tpr = d / EPV;                        // threads per row: power of two, <= 32
   const unsigned gid = blockIdx.x * 256u + threadIdx.x;
@@ -50,7 +52,8 @@ delta_kernel(const T* __restrict__ out, const T* __restrict__ dout, float* __res
   }
 }
 
-int launch_delta(const moba_b200_problem& p, const void* out, const void* dout, float* delta,
+// `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from.
+int launch_delta(const moba_b200_problem& p, const void* out, const void* dout, float* delta, int* zero_cell,
                  cudaStream_t st) {
   KernelTimer timer__("delta_kernel", st);
   const int epv = 16 / (int)dtype_size(p.dtype);
@@ -73,7 +76,7 @@ int launch_delta(const moba_b200_problem& p, const void* out, const void* dout, 
   const dim3 grid((unsigned)((rows_per_batch * tpr + 255) / 256), (unsigned)p.batch);
 #define MOBA_DELTA(T) \
   MOBA_CUDA_OK(launch_chained(delta_kernel<T>, grid, 256, 0, st, (const T*)out, (const T*)dout, delta, (unsigned)rows_per_batch, \
-                              p.tokens, p.q_heads, p.head_dim, recip, shift))
+                              p.tokens, p.q_heads, p.head_dim, recip, shift, zero_cell))
   if (p.dtype == MOBA_B200_F32) MOBA_DELTA(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_DELTA(__nv_bfloat16);
   else MOBA_DELTA(__half);

@@ -102,13 +102,12 @@ template <int D> struct Bars {
 };
 static_assert(sizeof(Bars<64>) <= BwdCfg<64>::kBarBytes && sizeof(Bars<128>) <= BwdCfg<128>::kBarBytes, "barrier block outgrew its reservation");
 
-// Work item `item` of the launch: the items of the (sequence, kv head) rows interleaved, each
-// row's in its dispatch order (heaviest first); false for padding.
-__device__ __forceinline__ bool load_column(Column& c, int item, const moba_b200_index& ix,
-                                            const moba_b200_problem& p, const int32_t* cu, int n_kv_rows) {
-  c.kv_row = item % n_kv_rows;
+// Work item `j` of a (sequence, kv head) row, in its dispatch order (heaviest first); false for padding.
+__device__ __forceinline__ bool load_column(Column& c, int kv_row, int j, const moba_b200_index& ix,
+                                            const moba_b200_problem& p, const int32_t* cu) {
+  c.kv_row = kv_row;
   WorkItem w;
-  if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, item / n_kv_rows)) return false;
+  if (!load_work_item(w, ix, ix.col_nnz + (size_t)c.kv_row * p.num_blocks, c.kv_row, j)) return false;
   const int seq = c.kv_row / p.kv_heads;
   const SeqSpan sp = seq_span(cu, p.packed, seq, p.tokens);
   c.blk = w.blk;
@@ -214,7 +213,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
                  const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap g_map, const float* __restrict__ lse,
                  const float* __restrict__ delta, moba_b200_index ix, const int32_t* __restrict__ cu,
                  T* __restrict__ dq_part, float* __restrict__ dkv_scratch, T* __restrict__ dk, T* __restrict__ dv,
-                 moba_b200_problem p, int part_keys, int n_items, unsigned* error_word) {
+                 moba_b200_problem p, int part_keys, int n_items, ClaimOrder order, unsigned* error_word) {
   using Cfg = BwdCfg<D>;
   constexpr int NST = Cfg::kStages, NKV = Cfg::kKvBufs, NS = Cfg::kSBufs;
   constexpr uint32_t cS = Cfg::cS, cDP = Cfg::cDP, cDV = Cfg::cDV, cDK = Cfg::cDK;
@@ -619,21 +618,44 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         Column mine;
         unsigned found = 0;
         int round0 = 0;
-        auto next = [&](Column& c) {
-          while (found == 0) {
-            if ((long long)round0 * gridDim.x >= n_items) return false;
-            const long long item = snake_item(round0 + lane);
-            found = __ballot_sync(0xffffffffu, item < n_items && load_column(mine, (int)item, ix, p, cu, n_kv_rows));
-            round0 += 32;
-          }
-          const int src = __ffs(found) - 1;
-          found &= found - 1;
+        auto take = [&](Column& c, int src) {
           c.kv_row = __shfl_sync(0xffffffffu, mine.kv_row, src); c.blk = __shfl_sync(0xffffffffu, mine.blk, src);
           c.n = __shfl_sync(0xffffffffu, mine.n, src); c.lo = __shfl_sync(0xffffffffu, mine.lo, src);
           c.keys = __shfl_sync(0xffffffffu, mine.keys, src); c.key0 = __shfl_sync(0xffffffffu, mine.key0, src);
           c.slot = __shfl_sync(0xffffffffu, mine.slot, src); c.tok0 = __shfl_sync(0xffffffffu, mine.tok0, src);
           return true;
         };
+        auto dealt = [&](Column& c) {
+          while (found == 0) {
+            if ((long long)round0 * gridDim.x >= n_items) return false;
+            const long long item = snake_item(round0 + lane);
+            found = __ballot_sync(0xffffffffu, item < n_items && load_column(mine, (int)(item % n_kv_rows), (int)(item / n_kv_rows), ix, p, cu));
+            round0 += 32;
+          }
+          const int src = __ffs(found) - 1;
+          found &= found - 1;
+          return take(c, src);
+        };
+        // The next item by a claim. Padding ends every row of the table: when 32 entries from the claimed one on,
+        // which reach every row of the group, name nothing, the group is done.
+        auto claim = [&](Column& c) {
+          for (;;) {
+            int g = 0;
+            if (lane == 0) g = atomicAdd(order.next, 1);
+            g = __shfl_sync(0xffffffffu, g, 0);
+            if (g >= n_items) return false;
+            const int end = claimed_item(g, n_kv_rows, ix.items_per_row, order.rows).group_end;
+            bool there = false;
+            if (g + lane < end) {
+              const ClaimedItem at = claimed_item(g + lane, n_kv_rows, ix.items_per_row, order.rows);
+              there = load_column(mine, at.kv_row, at.j, ix, p, cu);
+            }
+            const unsigned some = __ballot_sync(0xffffffffu, there);
+            if (some & 1u) return take(c, 0);
+            if (some == 0u && lane == 0) atomicMax(order.next, end);
+          }
+        };
+        auto next = [&](Column& c) { return order.next != nullptr ? claim(c) : dealt(c); };
         // The index entries of a column are read a tile at a time; asking the L2 for them, and for
         // its K and V blocks, a column ahead saves a DRAM round trip per tile and item.
         auto prefetch = [&](const Column& c) {
@@ -888,7 +910,7 @@ dkv_reduce_kernel(const float* __restrict__ dkv_scratch, moba_b200_index ix, con
 template <int D, typename T>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensorMap& vm, const CUtensorMap& qm,
                const CUtensorMap& gm, const float* lse, const float* delta, const moba_b200_index& ix,
-               const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, bool* reduces, int n_items, unsigned* err,
+               const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, bool* reduces, int n_items, const ClaimOrder& order, unsigned* err,
                cudaStream_t st) {
   const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
@@ -898,7 +920,7 @@ int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensor
     static SmemLimit limit;
     if (int rc = raise_smem_limit(limit, (const void*)kern, BwdCfg<D>::kSmem)) return rc;
     MOBA_CUDA_OK(launch_chained(kern, grid, kThreads, BwdCfg<D>::kSmem, st, km, vm, qm, gm, lse, delta,
-                                ix, cu, (T*)dq_part, dkv_scratch, (T*)dk, (T*)dv, p, part_keys, n_items, err));
+                                ix, cu, (T*)dq_part, dkv_scratch, (T*)dk, (T*)dv, p, part_keys, n_items, order, err));
   }
   // No column can be long enough to be cut: nothing to sum.
   // (a query lists a column once per block in it)
@@ -928,7 +950,7 @@ bool bwd_sm100_supported(const moba_b200_problem& p) {
 
 int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const void* dout, const float* lse, const float* delta, const moba_b200_index& ix,
-                     const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, bool* reduces,
+                     const int32_t* cu, void* dq_part, float* dkv_scratch, void* dk, void* dv, int part_keys, int* claims, bool* reduces,
                      cudaStream_t st) {
   *reduces = false;
   unsigned* err = device_error_word();
@@ -952,13 +974,15 @@ int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, c
   const long long n_items_ll = (long long)ix.items_per_row * p.n_seq * p.kv_heads;
   if (n_items_ll > 0x7fffffffLL) { set_error("backward: too many work items"); return MOBA_B200_EUNSUPPORTED; }
   const int n_items = (int)n_items_ll;
+  const int rows_claimed = claims != nullptr ? claim_rows(p, p.head_dim == 64 ? 192 : 96) : 0;
+  const ClaimOrder order{rows_claimed > 0 ? claims : nullptr, rows_claimed};
   const bool bf = p.dtype == MOBA_B200_BF16;
   if (p.head_dim == 64) {
-    if (bf) return launch_one<64, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
-    return launch_one<64, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
+    if (bf) return launch_one<64, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, order, err, st);
+    return launch_one<64, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, order, err, st);
   }
-  if (bf) return launch_one<128, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
-  return launch_one<128, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, err, st);
+  if (bf) return launch_one<128, __nv_bfloat16>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, order, err, st);
+  return launch_one<128, __half>(p, km, vm, qm, gm, lse, delta, ix, cu, dq_part, dkv_scratch, dk, dv, part_keys, reduces, n_items, order, err, st);
 }
 
 }  // namespace moba

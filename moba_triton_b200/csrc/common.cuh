@@ -249,6 +249,45 @@ __device__ __forceinline__ bool load_work_item(WorkItem& w, const moba_b200_inde
   return true;
 }
 
+// ---- claimed items: which item a CTA takes next, by a counter instead of a fixed deal ----
+// The items of `rows` neighbouring (sequence, kv head) rows are interleaved, each row's heaviest first, one
+// group of rows after the other.
+struct ClaimOrder {
+  int* next;                 // counter of claims, zero before the launch; NULL: the fixed deal
+  int rows;                  // of a group, at most 32
+};
+struct ClaimedItem { int kv_row, j, group_end; };
+__device__ __forceinline__ ClaimedItem claimed_item(int g, int n_rows, int items_per_row, int rows) {
+  const int span = rows * items_per_row, group = g / span, first = group * rows, size = min(rows, n_rows - first), rem = g - group * span;
+  return ClaimedItem{first + rem % size, rem / size, group * span + size * items_per_row};
+}
+// Rows of a group, 0 for the fixed deal.
+// A CTA claims its next item when it begins one, and may then hold it while others have none: a problem needs
+// `tiles_per_sm` tiles per SM for claims to pay (192 at head_dim 64; 48 in the forward and 96 in the backward at
+// 128). us, forward and backward kernel, dealt and claimed:
+//   22211 tokens in 4 sequences x 4 heads of 64      38 tiles per SM     63   74     119  136
+//   62153 in 16 x 4 on 2 of 64                      105                 149  162
+//   131072 x 4 of 64                                221                 294  286     645  618
+//   45440 x 2 x 4 on 1 of 128                        38                 102  101     178  183
+//   31468 in 8 x 4 of 128                            80                 166  162     299  309
+//   89558 in 8 x 4 on 2 of 128                       76                 197  179
+//   70465 in 8 x 8 on 2 of 128                      179                 489  390     827  707
+//   524288 x 32 on 8 of 128, skewed                7000               19300 18540  29300 28370
+// (Claiming one further ahead, to hide the claim's latency, was 2 to 10 % slower than that.)
+// As a rule all rows are one group: its last items are its smallest. Where the queries of all rows are far more than
+// the L2 and those of a few are not, groups of 48 MB keep them there while their columns gather them once per
+// selected block: 262144 tokens in 32 sequences, 16 heads of 128, 4114 -> 3776, 7963 -> 7437. The items of the last
+// group are then not small, and there have to be many more than they hold: 40000 in 16 sequences, 32 heads on 8,
+// 978 -> 1026 in groups (540 tiles per SM, columns of 32).
+static inline int claim_rows(const moba_b200_problem& p, int tiles_per_sm) {
+  const long long tiles = (sched_pairs_bound(p) + 127) / 128;
+  if (tiles < (long long)tiles_per_sm * kSchedSMs) return 0;
+  const long long n_rows = (long long)p.n_seq * p.kv_heads, column = (long long)(p.q_heads / p.kv_heads) * p.slots;
+  const double bytes = 2.0 * p.batch * p.tokens * p.q_heads * p.head_dim, row = bytes / (double)n_rows;
+  if (bytes > 96e6 && 48e6 / row >= 2.0 && tiles >= 32LL * column * kSchedSMs) return (int)(48e6 / row < 32.0 ? 48e6 / row : 32.0);
+  return n_rows <= 32 ? (int)n_rows : 0;                  // (the end of the list is told from 32 entries of it)
+}
+
 // ---- stage launchers (defined one per .cu file) -----------------------------
 int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell, float* norms,
                 cudaStream_t st);
@@ -283,12 +322,12 @@ int launch_fwd_portable(const moba_b200_problem& p, const void* q, const void* k
                         float* part_lse, cudaStream_t st);
 int launch_fwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const moba_b200_index& ix, const int32_t* cu, void* part_o,
-                     float* part_lse, int part_keys, cudaStream_t st);
+                     float* part_lse, int part_keys, int* claims, cudaStream_t st);
 bool fwd_sm100_supported(const moba_b200_problem& p);
 int launch_merge(const moba_b200_problem& p, const void* part_o, const float* part_lse,
                  void* out, float* lse, cudaStream_t st);
 
-int launch_delta(const moba_b200_problem& p, const void* out, const void* dout, float* delta,
+int launch_delta(const moba_b200_problem& p, const void* out, const void* dout, float* delta, int* zero_cell,
                  cudaStream_t st);
 int launch_bwd_portable(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                         const void* dout, const float* lse, const float* delta,
@@ -297,7 +336,7 @@ int launch_bwd_portable(const moba_b200_problem& p, const void* q, const void* k
 int launch_bwd_sm100(const moba_b200_problem& p, const void* q, const void* k, const void* v,
                      const void* dout, const float* lse, const float* delta,
                      const moba_b200_index& ix, const int32_t* cu, void* dq_part, float* dkv_scratch,
-                     void* dk, void* dv, int part_keys, bool* reduces, cudaStream_t st);
+                     void* dk, void* dv, int part_keys, int* claims, bool* reduces, cudaStream_t st);
 bool bwd_sm100_supported(const moba_b200_problem& p);
 // `beside`: the kernel before is the dK/dV reduction, which this one does not depend on.
 int launch_dq_reduce(const moba_b200_problem& p, const void* dq_part, const float* part_lse,

@@ -30,7 +30,7 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
             int packed, int tokens, int hkv, int d, int bs, int nb, int* __restrict__ zero_cell, float* __restrict__ norms) {
   pdl_trigger();
   pdl_wait();
-  if (zero_cell != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *zero_cell = 0;
+  if (zero_cell != nullptr && blockIdx.x == 0 && threadIdx.x == 0) zero_cell[0] = zero_cell[1] = 0;
   constexpr int EPV = 16 / sizeof(T), NT = kPoolThreads<T>;   // elements per 16-byte vector; threads
   const int blk = (int)(blockIdx.x % nb), kv_row = (int)(blockIdx.x / nb);
   const int seq = kv_row / hkv, h = kv_row % hkv;
@@ -114,7 +114,7 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
   }
 }
 
-// `zero_cell` (may be NULL): a counter that a later kernel of the same op claims from; `norms`
+// `zero_cell` (may be NULL): two counters that later kernels of the same op claim from; `norms`
 // (may be NULL): the length of every block mean, [n_seq, Hkv, num_blocks].
 int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, void* kbar, int* zero_cell, float* norms,
                 cudaStream_t st) {

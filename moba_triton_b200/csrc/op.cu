@@ -87,7 +87,7 @@ Columns columns_of(const moba_b200_problem& p) {
 struct Layout {
   size_t col_nnz, col_offsets, order, items, entries, part_lse, lse, keep_bytes;      // kept for the backward
   size_t kbar, norms, block_idx, counter, transpose_scratch, part_o, fwd_bytes;              // forward only
-  size_t delta, dq_part, dkv, bwd_transpose_scratch, bwd_bytes;                       // backward only
+  size_t delta, claims, dq_part, dkv, bwd_transpose_scratch, bwd_bytes;                       // backward only
 };
 inline long long row_capacity(const moba_b200_problem& p) {
   return (long long)(p.q_heads / p.kv_heads) * window_rows_of_seq(p) * p.slots;
@@ -122,6 +122,7 @@ Layout layout_of(const moba_b200_problem& gate, const moba_b200_problem& p) {
   l.fwd_bytes = at;
   at = 0;
   l.delta = take((size_t)p.batch * p.q_heads * p.tokens * 4);
+  l.claims = take(16);
   l.dq_part = take(pairs * p.head_dim * dtype_size(p.dtype));
   l.dkv = take(sched_dkv_scratch_bytes(p));
   l.bwd_transpose_scratch = take(window ? scratch : 0);
@@ -182,15 +183,15 @@ int transpose_into(const Columns& c, const moba_b200_index& ix, const int32_t* b
                           scratch, transpose_scratch_bytes(p), st);
 }
 
-// From block ids to the output: transpose, attention, merge.
+// From block ids to the output: transpose, attention, merge. `claims`: a counter that is zero by then, or NULL.
 int attend(const Columns& c, const Layout& l, int fwd_path, const void* q, const void* k, const void* v, const int32_t* block_idx,
-           const int32_t* cu, unsigned char* keep, unsigned char* tmp, void* out, float* lse, cudaStream_t st) {
+           const int32_t* cu, unsigned char* keep, unsigned char* tmp, int* claims, void* out, float* lse, cudaStream_t st) {
   const moba_b200_problem& p = c.p;
   const moba_b200_index ix = index_in(p, l, keep);
   float* part_lse = reinterpret_cast<float*>(keep + l.part_lse);
   void* part_o = tmp + l.part_o;
   MOBA_TRY(transpose_into(c, ix, block_idx, cu, tmp + l.transpose_scratch, reinterpret_cast<int32_t*>(tmp + l.counter), st));
-  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu, part_o, part_lse, c.part_keys, st));
+  if (fwd_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_fwd_sm100(p, q, k, v, ix, cu, part_o, part_lse, c.part_keys, claims, st));
   else MOBA_TRY(launch_fwd_portable(p, q, k, v, ix, cu, part_o, part_lse, st));
   return launch_merge(p, part_o, part_lse, out, lse, st);
 }
@@ -204,9 +205,10 @@ int differentiate(const Columns& c, const Layout& l, int path, const void* q, co
   float* delta = reinterpret_cast<float*>(tmp + l.delta);
   void* dq_part = tmp + l.dq_part;
   bool reduces = false;
-  MOBA_TRY(launch_delta(p, out, dout, delta, st));
+  int* claims = reinterpret_cast<int*>(tmp + l.claims);
+  MOBA_TRY(launch_delta(p, out, dout, delta, claims, st));
   if (path == MOBA_B200_PATH_TCGEN05)
-    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, c.part_keys, &reduces, st));
+    MOBA_TRY(launch_bwd_sm100(p, q, k, v, dout, lse, delta, ix, cu, dq_part, reinterpret_cast<float*>(tmp + l.dkv), dk, dv, c.part_keys, claims, &reduces, st));
   else
     MOBA_TRY(launch_bwd_portable(p, q, k, v, dout, lse, delta, ix, cu, dq_part, dk, dv, st));
   return launch_dq_reduce(p, dq_part, part_lse, dq, reduces, st);
@@ -268,7 +270,7 @@ int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void*
   if (gate_path == MOBA_B200_PATH_TCGEN05) MOBA_TRY(launch_gate_sm100(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
   else if (exact_gate) MOBA_TRY(launch_gate_exact_sm100(gate, q, kbar, norms, cu_seqlens, block_idx, part_lse, st));
   else MOBA_TRY(launch_gate_portable(gate, q, kbar, cu_seqlens, block_idx, part_lse, st));
-  return attend(cut, l, fwd_path, q, k, v, block_idx, cu_seqlens, keep, tmp, out,
+  return attend(cut, l, fwd_path, q, k, v, block_idx, cu_seqlens, keep, tmp, counter + 1, out,
                 want_lse ? reinterpret_cast<float*>(keep + l.lse) : nullptr, st);
 }
 
@@ -307,7 +309,7 @@ int moba_b200_op_forward_window(const moba_b200_problem* p0, const void* q, cons
   const Layout l = layout_of(gate, p);
   unsigned char* keep = static_cast<unsigned char*>(keep_ws);
   MOBA_TRY(launch_fill_lse(p, reinterpret_cast<float*>(keep + l.part_lse), st));
-  return attend(columns, l, path, q, k, v, block_idx, nullptr, keep, static_cast<unsigned char*>(forward_ws), out, lse, st);
+  return attend(columns, l, path, q, k, v, block_idx, nullptr, keep, static_cast<unsigned char*>(forward_ws), nullptr, out, lse, st);
 }
 
 int moba_b200_op_backward_window(const moba_b200_problem* p0, const void* q, const void* k, const void* v, const void* out,
