@@ -49,9 +49,12 @@ constexpr int kGatherWarp0 = kElemWarps + 4, kGatherWarps = 4;
 constexpr int kStoreWarp0 = kGatherWarp0 + kGatherWarps, kStoreWarps = 4;
 constexpr int kThreads = (kStoreWarp0 + kStoreWarps) * 32;   // warp 19 only completes its warpgroup
 // Registers: 896 threads are launched with 72 each (64 512). 512 elementwise threads take 80, 128
-// storing threads 104 (a whole dQ row each), the other 256 give down to 40: 64 512 again.
-constexpr int kLaunchRegs = 72, kElemRegs = 80, kStoreRegs = 104, kOtherRegs = 40;
-static_assert(kElemWarps * 32 * kElemRegs + kStoreWarps * 32 * kStoreRegs + 256 * kOtherRegs <= kThreads * kLaunchRegs, "register split");
+// storing threads what a dQ row needs, the other 256 give down to the rest: 64 512 again.
+constexpr int kLaunchRegs = 72, kElemRegs = 80;
+template <int D> constexpr int kStoreRegs = D == 64 ? 88 : 104;
+template <int D> constexpr int kOtherRegs = D == 64 ? 48 : 40;
+template <int D> constexpr bool kRegsFit = kElemWarps * 32 * kElemRegs + kStoreWarps * 32 * kStoreRegs<D> + 256 * kOtherRegs<D> <= kThreads * kLaunchRegs;
+static_assert(kRegsFit<64> && kRegsFit<128>, "register split");
 
 template <int D> struct BwdCfg {
   static constexpr int kSubs = D / 64;
@@ -432,7 +435,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
       // four so that four neighbouring lanes write 64 contiguous bytes of a row (one row per lane
       // would touch 32 lines per instruction). Kept off the elementwise warps, whose two phases
       // bound the tile, and off shared memory, which has no room for another tile at 128.
-      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kStoreRegs));
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kStoreRegs<D>));
       const int grp = warp & 3, r = grp * 32 + lane;
       const uint32_t lane_off = (uint32_t)(grp * 32) << 16;
       constexpr int CH = D / 8;                            // 16-byte pieces per row
@@ -481,7 +484,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         }
       }
     } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs<D>));
     if (warp == kScoreWarp || warp == kGradWarp) {
       // ============================== MMA issuers ==============================
       // Two warps feed the tensor core, so that neither waits for what the other's next MMA
