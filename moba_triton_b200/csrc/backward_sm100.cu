@@ -25,7 +25,8 @@
 // 4 400 of 7 200 at 128; the tensor pipe needs 1 900 and 2 560. Measured against the untransposed
 // version with copies through the load-store unit: 11.0 -> 7.4 ms on 262 144 packed tokens, 16
 // heads of 128; 9.1 -> 6.9 ms on [1,131072,32,128] with 8 KV heads. At head_dim 64 it gained nothing
-// that can be told from noise ([1,131072,4,64]: 0.667 ms before, 0.65 to 0.67 now).
+// that can be told from noise ([1,131072,4,64]: 0.667 ms before, 0.65 to 0.67 after); claimed items
+// and the register split below make that 0.61.
 //
 // dQ rows go to the (query, slot) partial buffer; a later pass sums the slots.
 //
@@ -49,7 +50,8 @@ constexpr int kGatherWarp0 = kElemWarps + 4, kGatherWarps = 4;
 constexpr int kStoreWarp0 = kGatherWarp0 + kGatherWarps, kStoreWarps = 4;
 constexpr int kThreads = (kStoreWarp0 + kStoreWarps) * 32;   // warp 19 only completes its warpgroup
 // Registers: 896 threads are launched with 72 each (64 512). 512 elementwise threads take 80, 128
-// storing threads what a dQ row needs, the other 256 give down to the rest: 64 512 again.
+// storing threads what a dQ row needs, the other 256 give down to the rest: 64 512 again. At head_dim 64
+// a dQ row needs 88; with 104 the other 256 had 40 and spilled 148 bytes (32 now): 624 -> 612 us at [1,131072,4,64].
 constexpr int kLaunchRegs = 72, kElemRegs = 80;
 template <int D> constexpr int kStoreRegs = D == 64 ? 88 : 104;
 template <int D> constexpr int kOtherRegs = D == 64 ? 48 : 40;
