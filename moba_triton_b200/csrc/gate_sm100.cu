@@ -24,7 +24,8 @@
 //          A key is the score rounded to the input dtype and made monotone in the high half and
 //          0xFFFF - block id in the low half, so "score descending, ties to the lower id" is plain
 //          integer order.
-// The ALU pipe bounds it: 2.5 of a score's 5.7 instructions run there, at half rate. An SM's tensor pipe takes
+// The ALU pipe bounds it (58 % of its peak): 2.5 of the 5.7 instructions that one more score costs run there, at
+// half rate. An SM's tensor pipe takes
 // 90 clocks for an M128 N64 K16 instruction with both operands in shared memory and half of that with A in
 // TMEM, which at head_dim 128 would bound the kernel otherwise; and issued from a branch of one lane, where
 // descriptors do not stay in uniform registers, one took 120. Before, each score that passed was appended to a
