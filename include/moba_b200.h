@@ -140,7 +140,9 @@ int moba_b200_path_for(const moba_b200_problem* p, int stage);
 /* The launch table: everything the library decides per problem, looked up in
  * constant time from the problem record (no measurement, no device query);
  * moba_b200_launch_plan for the stages called one by one, moba_b200_op_launch_plan
- * for the whole-op calls. Those run blocks finer than 128 keys as columns of 128
+ * for a training step of the whole-op calls, moba_b200_op_forward_launch_plan for
+ * moba_b200_op_forward with want_lse == 0, whose items are shorter than those of a
+ * step of medium size. The whole-op calls run blocks finer than 128 keys as columns of 128
  * (work items and transpose are then those of the columns), more gates on tensor
  * cores, and cut small problems finer.
  * The tensor-core kernels have one tile plan per head_dim; the transpose and
@@ -164,6 +166,7 @@ typedef struct moba_b200_plan {
 } moba_b200_plan;
 int moba_b200_launch_plan(const moba_b200_problem* p, moba_b200_plan* plan);
 int moba_b200_op_launch_plan(const moba_b200_problem* p, moba_b200_plan* plan);
+int moba_b200_op_forward_launch_plan(const moba_b200_problem* p, moba_b200_plan* plan);
 
 /* Bytes of scratch moba_b200_transpose needs for this problem. */
 size_t moba_b200_transpose_scratch_bytes(const moba_b200_problem* p);

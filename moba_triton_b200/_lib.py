@@ -28,7 +28,7 @@ EXPORTS = (
     "moba_b200_device_status", "moba_b200_transpose_noalloc",
     "moba_b200_pack_index", "moba_b200_pack_rows", "moba_b200_unpack_rows", "moba_b200_seq_meta",
     "moba_b200_chunk_tiles", "moba_b200_work_items_per_row", "moba_b200_dkv_scratch_bytes",
-    "moba_b200_launch_plan", "moba_b200_op_launch_plan",
+    "moba_b200_launch_plan", "moba_b200_op_launch_plan", "moba_b200_op_forward_launch_plan",
     "moba_b200_op_workspace", "moba_b200_op_forward", "moba_b200_op_backward",
     "moba_b200_op_forward_window", "moba_b200_op_backward_window",
 )
@@ -79,7 +79,8 @@ def load():
     lib.moba_b200_gate.argtypes = [P, vp, vp, vp, vp, vp]
     lib.moba_b200_transpose.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, c_size_t, vp]
     lib.moba_b200_transpose_noalloc.argtypes = [P, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
-    lib.moba_b200_launch_plan.argtypes = lib.moba_b200_op_launch_plan.argtypes = [P, POINTER(Plan)]
+    for plan in (lib.moba_b200_launch_plan, lib.moba_b200_op_launch_plan, lib.moba_b200_op_forward_launch_plan):
+        plan.argtypes = [P, POINTER(Plan)]
     lib.moba_b200_chunk_tiles.argtypes = [P]
     lib.moba_b200_work_items_per_row.argtypes = [P]
     lib.moba_b200_dkv_scratch_bytes.argtypes = [P]

@@ -214,6 +214,19 @@ int differentiate(const Columns& c, const Layout& l, int path, const void* q, co
   return launch_dq_reduce(p, dq_part, part_lse, dq, reduces, st);
 }
 
+// What a whole-op call runs; `training`: a forward that keeps its log-sum-exps, and its backward.
+int op_plan(const moba_b200_problem* p0, bool training, moba_b200_plan* plan) {
+  MOBA_TRY(check_sizes(p0));
+  if (plan == nullptr) { set_error("plan is NULL"); return MOBA_B200_EINVAL; }
+  const moba_b200_problem gate = with_cut(*p0);
+  moba_b200_problem p = columns_of(gate).p;
+  if (!training && p0->win_rows == 0) p.chunk_tiles = with_cut(*p0, false).chunk_tiles;   // (a window's forward takes the cut of its backward)
+  const int gate_path = pick(gate, gate_sm100_supported(gate), "gate");
+  MOBA_TRY(fill_plan(p, gate_path >= 0 && runs_exact_gate(gate, gate_path) ? MOBA_B200_PATH_TCGEN05 : gate_path, plan));
+  if (transpose_small_supported(p)) plan->transpose_chunk_rows = plan->transpose_chunks = plan->scatter_warps = 0;
+  return MOBA_B200_OK;
+}
+
 }  // namespace
 }  // namespace moba
 
@@ -231,16 +244,8 @@ int moba_b200_op_workspace(const moba_b200_problem* p0, size_t* keep_bytes, size
   return MOBA_B200_OK;
 }
 
-int moba_b200_op_launch_plan(const moba_b200_problem* p0, moba_b200_plan* plan) {
-  MOBA_TRY(check_sizes(p0));
-  if (plan == nullptr) { set_error("plan is NULL"); return MOBA_B200_EINVAL; }
-  const moba_b200_problem gate = with_cut(*p0);
-  const moba_b200_problem p = columns_of(gate).p;
-  const int gate_path = pick(gate, gate_sm100_supported(gate), "gate");
-  MOBA_TRY(fill_plan(p, gate_path >= 0 && runs_exact_gate(gate, gate_path) ? MOBA_B200_PATH_TCGEN05 : gate_path, plan));
-  if (transpose_small_supported(p)) plan->transpose_chunk_rows = plan->transpose_chunks = plan->scatter_warps = 0;
-  return MOBA_B200_OK;
-}
+int moba_b200_op_launch_plan(const moba_b200_problem* p0, moba_b200_plan* plan) { return op_plan(p0, true, plan); }
+int moba_b200_op_forward_launch_plan(const moba_b200_problem* p0, moba_b200_plan* plan) { return op_plan(p0, false, plan); }
 
 int moba_b200_op_forward(const moba_b200_problem* p0, const void* q, const void* k, const void* v,
                          const int32_t* cu_seqlens, void* keep_ws, void* forward_ws, void* out, int want_lse, void* stream) {

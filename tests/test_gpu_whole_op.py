@@ -11,7 +11,9 @@ import pytest
 import torch
 
 import moba_triton_b200 as moba
+from moba_triton_b200 import _lib
 from moba_triton_b200.kernels.moba_fwd import op_plan
+from moba_triton_b200.tuning import launch_plan
 
 from conftest import make_qkv
 from helpers import max_abs_error
@@ -121,6 +123,31 @@ def test_passes_over_kv_heads_cut_columns_like_the_whole_call(s, hkv, group, dev
     for n in (1, hkv // 2):
         for a, w in zip(gradients(q, k, v, do, cfg, kv_heads_per_pass=n), whole):
             assert torch.equal(a, w)
+
+
+@pytest.mark.parametrize("s,hkv,group,d,block,cuts", [(14208, 4, 1, 64, 128, (14, 8)), (18944, 2, 2, 64, 128, (16, 8)),
+                                                      (37888, 4, 1, 128, 128, (24, 16)), (14300, 2, 2, 64, 32, (15, 8))],
+                         ids=["shortest", "passes", "longest", "finer"])
+def test_a_forward_alone_is_cut_finer_than_the_forward_of_a_step(s, hkv, group, d, block, cuts, device):
+    """24 to 64 tiles per SM: one workspace holds either table of work items. O is the same bits for both, all
+    four results are those of staged calls with the step's cut, and (up to 32 tiles per SM) of passes."""
+    cfg = moba.MoBAConfig(block, 8)
+    q, k, v, do = (t.to(device) for t in make_qkv((1, s, hkv * group, d), hkv, dtype=torch.bfloat16, seed=68, with_do=True))
+    step, alone = (launch_plan(q.shape, hkv, q.dtype, cfg, gradients=g) for g in (True, False))
+    assert (step["chunk_tiles"], alone["chunk_tiles"]) == cuts
+    assert step["work_items_per_row"] < alone["work_items_per_row"]
+    whole = gradients(q, k, v, do, cfg)
+    assert torch.equal(moba.moba_forward(q, k, v, cfg), whole[0])
+    if block == 128:
+        old = _lib.set_chunk_tiles(step["chunk_tiles"])
+        try:
+            staged = gradients(q, k, v, do, cfg, index=moba.build_csc_fused(q, k, cfg))
+        finally:
+            _lib.set_chunk_tiles(old)
+        for a, w in zip(staged, whole):
+            assert torch.equal(a, w)
+    for a, w in zip(gradients(q, k, v, do, cfg, kv_heads_per_pass=1), whole if cuts[0] <= 16 else whole[:2]):
+        assert torch.equal(a, w)
 
 
 def test_the_function_of_a_given_index_builds_one_if_there_is_none(device):

@@ -254,6 +254,21 @@ def test_launch_plan_of_the_whole_op_says_what_the_op_runs():
         launch_plan((1, 64, 3, 64), 2, bf16, cfg)
 
 
+@pytest.mark.parametrize("tokens,forward,step", [(14204, 8, 8), (14208, 8, 14), (16384, 8, 15), (37888, 16, 24), (37889, 17, 17)])
+def test_launch_plan_tells_a_forward_from_a_training_step(tokens, forward, step):
+    """Both ends of the range (24 to 64 tiles per SM) in which a training step has longer work items than a
+    forward alone, and the first sizes outside it; float32 has one cut."""
+    from moba_triton_b200.tuning import launch_plan
+    for dtype, cuts in ((torch.bfloat16, (forward, step)), (torch.float32, (forward, forward))):
+        cfg = moba.MoBAConfig(128, 8, dtype=dtype)
+        for gradients, cut in zip((False, True), cuts):
+            plan = launch_plan((1, tokens, 4, 64), 4, dtype, cfg, gradients=gradients)
+            assert plan["chunk_tiles"] == cut
+            assert plan["work_items_per_row"] == -(-tokens // 128) + tokens * 4 * 8 // (128 * cut) + 1
+        assert launch_plan((1, tokens, 4, 64), 4, dtype, cfg)["chunk_tiles"] == cuts[1]
+        assert launch_plan((1, tokens, 4, 64), 4, dtype, cfg, stages=True)["chunk_tiles"] == forward
+
+
 def test_reference_arm_of_the_bench_prints_the_contract_line():
     """`bench.py --impl reference` needs no GPU: it times the oracle on the host cores and
     prints one JSON line whose `config` is the object our arm prints for the same workload."""
