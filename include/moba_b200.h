@@ -100,7 +100,8 @@ typedef struct moba_b200_index {
   const int32_t* slot_of_pair;
   int64_t capacity;       /* entries per (sequence, kv head) in the three pair arrays */
   const int32_t* work_items; /* [n_seq, Hkv, items_per_row, 4]: {block, first tile, tiles, dK/dV partial
-                                slot or -1 (whole column) or -2 (padding)}, in dispatch order; written
+                                slot or -1 (whole column) or -2 (padding, whose second word is the
+                                number of full pieces in the row)}, in dispatch order; written
                                 by moba_b200_transpose. NULL: the tensor-core kernels refuse the index */
   int32_t items_per_row;  /* moba_b200_work_items_per_row() of the problem the index was built for */
   int32_t chunk_tiles;    /* the chunk size the items were cut with */

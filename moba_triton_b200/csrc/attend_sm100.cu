@@ -175,7 +175,7 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) 
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int D, typename T, typename TP>
+template <int D, typename T, typename TP, bool CLAIM>
 __global__ void __launch_bounds__(FwdCfg<D>::kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
                  const __grid_constant__ CUtensorMap q_map, moba_b200_index ix, const int32_t* __restrict__ cu,
@@ -595,26 +595,15 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
         found &= found - 1;
         return take(c, src);
       };
-      // The next item by a claim. Padding ends every row of the table: when 32 entries from the claimed one on,
-      // which reach every row of the group, name nothing, the group is done.
-      auto claim = [&](Column& c) {
-        for (;;) {
-          int g = 0;
-          if (lane == 0) g = atomicAdd(order.next, 1);
-          g = __shfl_sync(0xffffffffu, g, 0);
-          if (g >= n_items) return false;
-          const int end = claimed_item(g, n_kv_rows, ix.items_per_row, order.rows).group_end;
-          bool there = false;
-          if (g + lane < end) {
-            const ClaimedItem at = claimed_item(g + lane, n_kv_rows, ix.items_per_row, order.rows);
-            there = load_column(mine, at.kv_row, at.j, ix, p, cu);
-          }
-          const unsigned some = __ballot_sync(0xffffffffu, there);
-          if (some & 1u) return take(c, 0);
-          if (some == 0u && lane == 0) atomicMax(order.next, end);
-        }
+      ClaimWalk walk{0, 0};
+      auto claimed = [&](Column& c) {
+        int kv_row, j;
+        do {                                                    // (an item without pairs is nothing to the forward)
+          if (!claim_item(walk, order, ix, p, cu, n_kv_rows, kv_row, j)) return false;
+        } while (!load_column(c, kv_row, j, ix, p, cu));
+        return true;
       };
-      auto next = [&](Column& c) { return order.next != nullptr ? claim(c) : dealt(c); };
+      auto next = [&](Column& c) { if constexpr (CLAIM) return claimed(c); else return dealt(c); };
       auto publish = [&](const Column& c, uint32_t n) {
         if (n >= 8) mbar_wait(&bars->col_free[n & 7], ((n >> 3) - 1) & 1, wc, 6);
         __syncwarp();
@@ -623,49 +612,52 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           mbar_arrive(&bars->col_full[n & 7]);
         }
       };
+      // One call of `next`: each turn takes an item and loads the one taken before.
       Column c, c_next;
-      bool more = next(c);
-      if (more) { prefetch_entries(c); publish(c, 0); }
-      while (more) {
+      uint32_t published = 0;
+      c.n = 0;
+      for (;;) {
         // The gather warps run ahead of the MMAs: at the last tiles of an item they are at tiles of
         // the next one, so its descriptor (and, in the L2, its index entries) must be there before
         // this item's K and V are even loaded.
-        more = next(c_next);
-        if (more) { prefetch_entries(c_next); publish(c_next, it_cnt + 1); }
+        const bool more = next(c_next);
+        if (more) { prefetch_entries(c_next); publish(c_next, published++); }
         if (__any_sync(0xffffffffu, *wc.abort)) break;        // no new loads once a wait gave up
-        const int kvh = c.kv_row % p.kv_heads;
-        const int tok = c.tok0 + c.key0;
-        const uint32_t kb = it_cnt % NKV, ku = it_cnt / NKV;     // buffer of this item, its earlier uses
-        unsigned char* bK = sK + kb * Cfg::kOperand;
-        unsigned char* bV = sV + kb * Cfg::kOperand;
-        if (ku >= 1) mbar_wait(&bars->k_free[kb], (ku - 1) & 1, wc, 7);
-        if (lane == 0) {
-          mbar_expect_tx(&bars->k_full[kb], Cfg::kOperand);
-          for (int s = 0; s < Cfg::kSubs; ++s) tma_load_3d_hint(bK + s * kSub, &k_map, &bars->k_full[kb], s * 64, kvh, tok, keep);
-        }
-        if (ku >= 1) mbar_wait(&bars->v_free[kb], (ku - 1) & 1, wc, 8);
-        if (lane == 0) {
-          mbar_expect_tx(&bars->v_full[kb], Cfg::kOperand);
-          for (int s = 0; s < Cfg::kSubs; ++s) tma_load_3d_hint(bV + s * kSub, &v_map, &bars->v_full[kb], s * 64, kvh, tok, keep);
-        }
-        if (c.keys < kTile) {
-          const int dead = kTile - c.keys;
-          mbar_wait(&bars->k_full[kb], ku & 1, wc, 9);
-          for (int i = lane; i < dead * 8 * Cfg::kSubs; i += 32) {
-            const int s = i / (dead * 8), rr = c.keys + (i % (dead * 8)) / 8, ch = i % 8;
-            *reinterpret_cast<uint4*>(bK + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
+        if (c.n > 0) {
+          const int kvh = c.kv_row % p.kv_heads, tok = c.tok0 + c.key0;
+          const uint32_t kb = it_cnt % NKV, ku = it_cnt / NKV;     // buffer of this item, its earlier uses
+          unsigned char* bK = sK + kb * Cfg::kOperand;
+          unsigned char* bV = sV + kb * Cfg::kOperand;
+          if (ku >= 1) mbar_wait(&bars->k_free[kb], (ku - 1) & 1, wc, 7);
+          if (lane == 0) {
+            mbar_expect_tx(&bars->k_full[kb], Cfg::kOperand);
+            for (int s = 0; s < Cfg::kSubs; ++s) tma_load_3d_hint(bK + s * kSub, &k_map, &bars->k_full[kb], s * 64, kvh, tok, keep);
           }
-          fence_proxy_async();
-          mbar_arrive_warp(&bars->k_fix[kb]);
-          mbar_wait(&bars->v_full[kb], ku & 1, wc, 9);
-          for (int i = lane; i < dead * 8 * Cfg::kSubs; i += 32) {
-            const int s = i / (dead * 8), rr = c.keys + (i % (dead * 8)) / 8, ch = i % 8;
-            *reinterpret_cast<uint4*>(bV + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
+          if (ku >= 1) mbar_wait(&bars->v_free[kb], (ku - 1) & 1, wc, 8);
+          if (lane == 0) {
+            mbar_expect_tx(&bars->v_full[kb], Cfg::kOperand);
+            for (int s = 0; s < Cfg::kSubs; ++s) tma_load_3d_hint(bV + s * kSub, &v_map, &bars->v_full[kb], s * 64, kvh, tok, keep);
           }
-          fence_proxy_async();
-          mbar_arrive_warp(&bars->v_fix[kb]);
+          if (c.keys < kTile) {
+            const int dead = kTile - c.keys;
+            mbar_wait(&bars->k_full[kb], ku & 1, wc, 9);
+            for (int i = lane; i < dead * 8 * Cfg::kSubs; i += 32) {
+              const int s = i / (dead * 8), rr = c.keys + (i % (dead * 8)) / 8, ch = i % 8;
+              *reinterpret_cast<uint4*>(bK + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
+            }
+            fence_proxy_async();
+            mbar_arrive_warp(&bars->k_fix[kb]);
+            mbar_wait(&bars->v_full[kb], ku & 1, wc, 9);
+            for (int i = lane; i < dead * 8 * Cfg::kSubs; i += 32) {
+              const int s = i / (dead * 8), rr = c.keys + (i % (dead * 8)) / 8, ch = i % 8;
+              *reinterpret_cast<uint4*>(bV + s * kSub + rr * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
+            }
+            fence_proxy_async();
+            mbar_arrive_warp(&bars->v_fix[kb]);
+          }
+          ++it_cnt;
         }
-        ++it_cnt;
+        if (!more) break;
         c = c_next;
       }
       c.n = -1;                                                 // end of the stream
@@ -691,9 +683,10 @@ template <int D, typename T, typename TP>
 int launch_one(const moba_b200_problem& p, const CUtensorMap& km, const CUtensorMap& vm, const CUtensorMap& qm,
                const moba_b200_index& ix, const int32_t* cu, void* part_o, float* part_lse, int part_keys, int n_items,
                const ClaimOrder& order, unsigned* err, cudaStream_t st) {
-  auto kern = fwd_sm100_kernel<D, T, TP>;
-  static SmemLimit limit;
-  if (int rc = raise_smem_limit(limit, (const void*)kern, FwdCfg<D>::kSmem)) return rc;
+  const bool claimed = order.next != nullptr;
+  auto kern = claimed ? fwd_sm100_kernel<D, T, TP, true> : fwd_sm100_kernel<D, T, TP, false>;
+  static SmemLimit limits[2];
+  if (int rc = raise_smem_limit(limits[claimed], (const void*)kern, FwdCfg<D>::kSmem)) return rc;
   const int sms = sm_count();
   const int grid = n_items < sms ? n_items : sms;
   MOBA_CUDA_OK(launch_chained(kern, grid, FwdCfg<D>::kThreads, FwdCfg<D>::kSmem, st, km, vm, qm, ix, cu,

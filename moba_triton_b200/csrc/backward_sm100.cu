@@ -644,26 +644,15 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
           found &= found - 1;
           return take(c, src);
         };
-        // The next item by a claim. Padding ends every row of the table: when 32 entries from the claimed one on,
-        // which reach every row of the group, name nothing, the group is done.
-        auto claim = [&](Column& c) {
-          for (;;) {
-            int g = 0;
-            if (lane == 0) g = atomicAdd(order.next, 1);
-            g = __shfl_sync(0xffffffffu, g, 0);
-            if (g >= n_items) return false;
-            const int end = claimed_item(g, n_kv_rows, ix.items_per_row, order.rows).group_end;
-            bool there = false;
-            if (g + lane < end) {
-              const ClaimedItem at = claimed_item(g + lane, n_kv_rows, ix.items_per_row, order.rows);
-              there = load_column(mine, at.kv_row, at.j, ix, p, cu);
-            }
-            const unsigned some = __ballot_sync(0xffffffffu, there);
-            if (some & 1u) return take(c, 0);
-            if (some == 0u && lane == 0) atomicMax(order.next, end);
-          }
+        ClaimWalk walk{0, 0};
+        auto claimed = [&](Column& c) {
+          int kv_row, j;
+          do {
+            if (!claim_item(walk, order, ix, p, cu, n_kv_rows, kv_row, j)) return false;
+          } while (!load_column(c, kv_row, j, ix, p, cu));
+          return true;
         };
-        auto next = [&](Column& c) { return order.next != nullptr ? claim(c) : dealt(c); };
+        auto next = [&](Column& c) { return order.next != nullptr ? claimed(c) : dealt(c); };
         // The index entries of a column are read a tile at a time; asking the L2 for them, and for
         // its K and V blocks, a column ahead saves a DRAM round trip per tile and item.
         auto prefetch = [&](const Column& c) {
@@ -681,12 +670,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             tma_prefetch_3d(&v_map, s * 64, c.kv_row % p.kv_heads, c.tok0 + c.key0);
           }
         };
+        // One call of `next` (its code twice costs the other roles of this register share spills): each turn takes
+        // an item and loads the one taken before.
         Column c, c_next;
-        bool more = next(c);
-        if (more) prefetch(c);
-        while (more) {
-          publish(c);
-          more = next(c_next);
+        c.n = 0;
+        for (;;) {
+          const bool more = next(c_next);
           if (more) prefetch(c_next);
           if (__any_sync(0xffffffffu, *wc.abort)) break;   // no new loads once a wait gave up
           if (c.n > 0) {
@@ -706,7 +695,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constan
             }
             ++n_seen;
           }
+          if (!more) break;
           c = c_next;
+          publish(c);
         }
         c.n = -1;
         publish(c);

@@ -251,15 +251,51 @@ __device__ __forceinline__ bool load_work_item(WorkItem& w, const moba_b200_inde
 
 // ---- claimed items: which item a CTA takes next, by a counter instead of a fixed deal ----
 // The items of `rows` neighbouring (sequence, kv head) rows are interleaved, each row's heaviest first, one
-// group of rows after the other.
+// group of rows after the other. What is claimed are items, not entries of the table: sequences of unequal
+// lengths have several entries of padding to an item, and each that a claim met cost a round trip to the counter
+// and to the table (4 heads of 64 over 4 sequences, forward dealt and claimed: 200 tiles per SM 1.13 -> 1.01,
+// 300 1.11 -> 0.97; over one sequence nothing changed).
 struct ClaimOrder {
   int* next;                 // counter of claims, zero before the launch; NULL: the fixed deal
   int rows;                  // of a group, at most 32
 };
-struct ClaimedItem { int kv_row, j, group_end; };
-__device__ __forceinline__ ClaimedItem claimed_item(int g, int n_rows, int items_per_row, int rows) {
-  const int span = rows * items_per_row, group = g / span, first = group * rows, size = min(rows, n_rows - first), rem = g - group * span;
-  return ClaimedItem{first + rem % size, rem / size, group * span + size * items_per_row};
+// The group of rows a warp claims from: its first row, and how many items the groups before it have.
+struct ClaimWalk { int first, before; };
+// Claims the next item for the warp: row and place of it in its row; false when there are no more.
+__device__ __forceinline__ bool claim_item(ClaimWalk& w, const ClaimOrder& order, const moba_b200_index& ix,
+                                           const moba_b200_problem& p, const int32_t* cu, int n_rows, int& kv_row, int& j) {
+  const int lane = threadIdx.x & 31;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(order.next, 1);
+  // Items of the lane's row: its full pieces, which the padding at its end counts, and one for each block of its
+  // sequence. (Read again with every claim, beside the counter: kept in registers they cost the backward spills.)
+  int mine = 0, all;
+  for (;;) {
+    const int row = w.first + lane;
+    if (lane < order.rows && row < n_rows) {
+      const int pieces = __ldg(ix.work_items + ((size_t)(row + 1) * ix.items_per_row - 1) * 4 + 1);
+      mine = pieces + (seq_span(cu, p.packed, row / p.kv_heads, p.tokens).len + kBlockKeys - 1) / kBlockKeys;
+    }
+    all = __reduce_add_sync(0xffffffffu, mine);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (at < w.before + all) break;
+    if (w.first + order.rows >= n_rows) return false;
+    w.before += all;
+    w.first += order.rows;
+    mine = 0;
+  }
+  // The last place j with no more than `at` items before it: every row has min(mine, j) of those.
+  at -= w.before;
+  int hi = __reduce_max_sync(0xffffffffu, mine);
+  j = 0;
+  while (hi - j > 1) {
+    const int mid = (j + hi) >> 1;
+    if ((int)__reduce_add_sync(0xffffffffu, min(mine, mid)) <= at) j = mid; else hi = mid;
+  }
+  at -= __reduce_add_sync(0xffffffffu, min(mine, j));
+  const unsigned there = __ballot_sync(0xffffffffu, mine > j);
+  kv_row = w.first + __ffs((int)__ballot_sync(0xffffffffu, mine > j && __popc(there & ((1u << lane) - 1u)) == at)) - 1;
+  return true;
 }
 // Rows of a group, 0 for the fixed deal.
 // A CTA claims its next item when it begins one, and may then hold it while others have none: a problem needs
@@ -285,7 +321,7 @@ static inline int claim_rows(const moba_b200_problem& p, int tiles_per_sm) {
   const long long n_rows = (long long)p.n_seq * p.kv_heads, column = (long long)(p.q_heads / p.kv_heads) * p.slots;
   const double bytes = 2.0 * p.batch * p.tokens * p.q_heads * p.head_dim, row = bytes / (double)n_rows;
   if (bytes > 96e6 && 48e6 / row >= 2.0 && tiles >= 32LL * column * kSchedSMs) return (int)(48e6 / row < 32.0 ? 48e6 / row : 32.0);
-  return n_rows <= 32 ? (int)n_rows : 0;                  // (the end of the list is told from 32 entries of it)
+  return n_rows <= 32 ? (int)n_rows : 0;                  // (a lane per row)
 }
 
 // ---- stage launchers (defined one per .cu file) -----------------------------

@@ -200,7 +200,9 @@ offsets_order_kernel(const int32_t* __restrict__ col_nnz, int32_t* __restrict__ 
 // eight items. The slots of a row are consecutive and claimed from a counter, so rows may
 // claim in any order: slot numbers name scratch memory, results do not depend on them, nor on
 // the order of the list. A row with more than kMaxCut cut columns keeps its columns' pieces
-// side by side, in column order (it has items enough for the order not to matter).
+// side by side, in column order (it has items enough for the order not to matter). Every row ends
+// in at least one entry of padding (sched_extra_items); it says how many full pieces the row has
+// (its items less one per block): who claims items, and not entries, reads it there.
 constexpr int kMaxCut = 2048;
 // The row's work items, by all 1024 threads of a CTA. `nnz` and `ord` are the row's column
 // totals and dispatch order (global or shared memory), `out` its stretch of the item table.
@@ -318,7 +320,7 @@ __device__ void write_work_items(const int32_t* nnz, const int32_t* ord, int4* o
       }
       put(n_full + (r - n_cut) + lo, make_int4(blk, 0, tiles, -1));
     }
-    for (int j = n_full + nb + threadIdx.x; j < items_per_row; j += 1024) out[j] = make_int4(0, 0, 0, -2);   // padding
+    for (int j = n_full + nb + threadIdx.x; j < items_per_row; j += 1024) out[j] = make_int4(0, n_full, 0, -2);   // padding, which tells how many pieces lead the row
     return;
   }
 
@@ -339,7 +341,7 @@ __device__ void write_work_items(const int32_t* nnz, const int32_t* ord, int4* o
     __syncthreads();
   }
   const int used = (int)(carry_s & 0xffffffffLL);
-  for (int j = used + threadIdx.x; j < items_per_row; j += 1024) out[j] = make_int4(0, 0, 0, -2);   // padding
+  for (int j = used + threadIdx.x; j < items_per_row; j += 1024) out[j] = make_int4(0, used - nb, 0, -2);   // padding, which tells how many pieces lead the row
 }
 
 __global__ void __launch_bounds__(1024)
@@ -737,7 +739,7 @@ transpose_small_kernel(const int32_t* __restrict__ block_idx, const int32_t* __r
       if (full0 + i < items_per_row) out[full0 + i] = make_int4(col, i * tc, tc, slot_or_none(i));
     if (n_full + by_piece < items_per_row) out[n_full + by_piece] = make_int4(col, (pieces - 1) * tc, last_tiles, slot_or_none(pieces - 1));
   }
-  for (int j = n_full + nb + threadIdx.x; j < items_per_row; j += kSmallThreads) out[j] = make_int4(0, 0, 0, -2);   // padding
+  for (int j = n_full + nb + threadIdx.x; j < items_per_row; j += kSmallThreads) out[j] = make_int4(0, n_full, 0, -2);   // padding, which tells how many pieces lead the row
 }
 
 // Entries of a warp's run: at most this many per lane.
