@@ -298,28 +298,34 @@ __device__ __forceinline__ bool claim_item(ClaimWalk& w, const ClaimOrder& order
   return true;
 }
 // Rows of a group, 0 for the fixed deal.
-// A CTA claims its next item when it begins one, and may then hold it while others have none: a problem needs
+// A CTA claims its next item when it begins one, and may then hold it while others have none. So a problem needs
 // `tiles_per_sm` tiles per SM for claims to pay (192 at head_dim 64; 48 in the forward and 96 in the backward at
-// 128). us, forward and backward kernel, dealt and claimed:
-//   22211 tokens in 4 sequences x 4 heads of 64      38 tiles per SM     63   74     119  136
-//   62153 in 16 x 4 on 2 of 64                      105                 149  162
-//   131072 x 4 of 64                                221                 294  286     645  618
-//   45440 x 2 x 4 on 1 of 128                        38                 102  101     178  183
-//   31468 in 8 x 4 of 128                            80                 166  162     299  309
-//   89558 in 8 x 4 on 2 of 128                       76                 197  179
-//   70465 in 8 x 8 on 2 of 128                      179                 489  390     827  707
-//   524288 x 32 on 8 of 128, skewed                7000               19300 18540  29300 28370
+// 128), and six times those of a column, the size of the items that are left at the end. Kernel time, claimed over
+// dealt, forward and backward, of one padded sequence by its tiles per SM (q heads on kv heads):
+//                          60         75         110        160        220        300        440
+//   head_dim 128   4 on 4  1.00 0.96  1.00 0.96  0.99 0.94  0.98 0.92  0.99 0.93  0.96 0.88  0.99 0.95
+//                  4 on 1  1.13 1.07  1.09 1.03  1.04 1.01  1.00 1.00  1.01 1.00  0.99 0.94  0.99 0.96
+//                 16 on 1  1.02 0.99  1.01 0.99  1.04 1.02  1.14 1.07  1.07 1.04  1.11 1.03  1.04 1.06
+//   head_dim 64    4 on 4  1.03 1.01             1.03 0.96  1.00 0.96  0.98 0.95  0.96 0.95  0.99 0.96
+//                  4 on 1  1.13 1.10             1.08 1.04  1.03 1.02  1.01 1.00  1.00 0.97  1.01 0.99
+//                 16 on 1  0.99 1.01             1.05 1.04  1.09 1.07  1.08 1.09  1.05 1.06  1.06 1.05
+// (524288 x 32 on 8 of 128, skewed, 7000 tiles per SM: 0.96 0.97.) The deal is even where all rows are equally
+// long. Over a batch of unequal sequences it is off by a tenth to a half whatever the column, and the second
+// condition does not apply: 16 on 1 of 128 over 8 sequences, 60 to 440 tiles per SM, 0.43 to 0.98; 8 on 2 of 64 over
+// 4 or 8, 200 to 480, 0.56 to 1.05. Two sequences are nearer to one: 16 on 2, 110 to 300, 0.99 to 1.15.
 // (Claiming one further ahead, to hide the claim's latency, was 2 to 10 % slower than that.)
 // As a rule all rows are one group: its last items are its smallest. Where the queries of all rows are far more than
 // the L2 and those of a few are not, groups of 48 MB keep them there while their columns gather them once per
-// selected block: 262144 tokens in 32 sequences, 16 heads of 128, 4114 -> 3776, 7963 -> 7437. The items of the last
-// group are then not small, and there have to be many more than they hold: 40000 in 16 sequences, 32 heads on 8,
+// selected block: 262144 tokens in 32 sequences, 16 heads of 128, 4114 -> 3776, 7963 -> 7437 us. The items of the
+// last group are then not small, and there have to be many more than they hold: 40000 in 16 sequences, 32 heads on 8,
 // 978 -> 1026 in groups (540 tiles per SM, columns of 32).
+// A query window counts with its own rows, in tiles and in bytes.
 static inline int claim_rows(const moba_b200_problem& p, int tiles_per_sm) {
-  const long long tiles = (sched_pairs_bound(p) + 127) / 128;
-  if (tiles < (long long)tiles_per_sm * kSchedSMs) return 0;
-  const long long n_rows = (long long)p.n_seq * p.kv_heads, column = (long long)(p.q_heads / p.kv_heads) * p.slots;
-  const double bytes = 2.0 * p.batch * p.tokens * p.q_heads * p.head_dim, row = bytes / (double)n_rows;
+  const long long tiles = (sched_pairs_bound(p) + 127) / 128, column = (long long)(p.q_heads / p.kv_heads) * p.slots;
+  const bool even = !p.packed || p.n_seq <= 2;
+  if (tiles < (even && 6 * column > tiles_per_sm ? 6 * column : (long long)tiles_per_sm) * kSchedSMs) return 0;
+  const long long n_rows = (long long)p.n_seq * p.kv_heads;
+  const double bytes = 2.0 * p.batch * window_rows(p) * p.q_heads * p.head_dim, row = bytes / (double)n_rows;
   if (bytes > 96e6 && 48e6 / row >= 2.0 && tiles >= 32LL * column * kSchedSMs) return (int)(48e6 / row < 32.0 ? 48e6 / row : 32.0);
   return n_rows <= 32 ? (int)n_rows : 0;                  // (a lane per row)
 }
