@@ -131,3 +131,67 @@ def test_a_negative_zero_ties_with_zero(block, rows, device):
     if rows == "zero":
         q[::2] = 0
     check(q, kb, cfg)
+
+
+def selected_by_the_packed_op(qs, kbs, cfg):
+    """As `selected_by_the_op`, for sequences packed into one call: a list of [S_i, H, blocks_i]."""
+    d, lens = qs[0].shape[2], [q.shape[0] for q in qs]
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device=qs[0].device)
+    keys = lambda rows: torch.cat([r.repeat_interleave(cfg.block_size, dim=0)[:n] for r, n in zip(rows, lens)])[None]
+    out = [[] for _ in qs]
+    for b0 in range(0, max(kb.shape[0] for kb in kbs), d):
+        v = [torch.eye(kb.shape[0], device=kb.device, dtype=kb.dtype)[:, b0:b0 + d] for kb in kbs]
+        v = [torch.nn.functional.pad(x, (0, d - x.shape[1]))[:, None] for x in v]
+        got = moba.moba_forward(torch.cat(qs)[None], keys(kbs), keys(v), cfg, cu_seqlens=cu, max_seqlen=max(lens))
+        for i, o in enumerate(got[0].split(lens)):
+            out[i].append(o)
+    return [torch.cat(o, -1)[..., :kb.shape[0]] for o, kb in zip(out, kbs)]
+
+
+def ladder(blocks, rows, d, dtype, tiles, g):
+    """Queries and block means whose every score lies on the middle between two values of the type, or a trace
+    beside it: any of them is unsure, and passes or not by its whole part, of which the rows have five kinds. They
+    are spread over the rows by tiles of 128, so that all of a warp's lists fill up together, or row by row."""
+    ids = torch.arange(blocks)
+    half, span = (0.5, 128) if dtype == torch.bfloat16 else (0.0625, 64)       # half a step of the type in [128, 256)
+    whole = torch.stack([ids % span,                          # rising: all enter the list
+                         span - 1 - ids % span,               # falling: none after the first
+                         torch.full_like(ids, 7),             # equal: the trace and the id decide
+                         torch.where(ids < 256, ids % 3, span // 2 + ids % 5),   # high past the first 256, which bound
+                         torch.randint(0, span, (blocks,), generator=g)])
+    kb = torch.zeros(blocks, 1, d, dtype=torch.float64)
+    q = torch.zeros(rows, 2, d, dtype=torch.float64)
+    for h in range(2):
+        kind = (torch.arange(rows) // (128 if tiles else 1) + h) % 5
+        q[:, h] = torch.nn.functional.one_hot(3 * kind, d) + torch.nn.functional.one_hot(3 * kind + 1, d) + torch.nn.functional.one_hot(3 * kind + 2, d)
+    for p in range(5):
+        kb[:, 0, 3 * p] = 128.0 + whole[p]
+        kb[:, 0, 3 * p + 1] = half
+        kb[:, 0, 3 * p + 2] = torch.randint(-1, 2, (blocks,), generator=g) * 2.0 ** -10
+    return q.to(dtype), kb.to(dtype)
+
+
+@pytest.mark.parametrize("tiles", [True, False], ids=["by-tiles", "by-rows"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
+@pytest.mark.parametrize("d,top_k", [(64, 4), (64, 12), (64, 17), (128, 13)])
+@pytest.mark.parametrize("blocks", [255, 256, 257, 321, 577])
+def test_unsure_scores_past_the_bounding_pass(blocks, d, top_k, dtype, tiles, device):
+    """More candidates than the first 256 that bound the rest; every score is taken again in float64, so the
+    lists of those that wait fill up in the middle of a window, with lanes that lag a window behind."""
+    g = torch.Generator().manual_seed(blocks + d + top_k)
+    q, kb = ladder(blocks, blocks * BS - 11, d, dtype, tiles, g)
+    check(q.to(device), kb.to(device), moba.MoBAConfig(BS, top_k, dtype=dtype))
+
+
+@pytest.mark.parametrize("block,d,top_k", [(32, 64, 12), (64, 128, 5), (128, 64, 17), (128, 128, 13)])
+def test_unsure_scores_in_packed_sequences(block, d, top_k, device):
+    """Odd and even numbers of query tiles, sequences of one row and of less than a block, starts anywhere."""
+    g = torch.Generator().manual_seed(block + d)
+    cfg = moba.MoBAConfig(block, top_k)
+    qs, kbs = [], []
+    for n in (1, 300 * block - 5, 127, 3 * 128, 40 * block + 1, 2 * 128 - 1, 259 * block, 17):
+        q, kb = ladder(-(-n // block), n, d, torch.bfloat16, n % 2 == 0, g)
+        qs.append(q.to(device))
+        kbs.append(kb.to(device))
+    for q, kb, got in zip(qs, kbs, selected_by_the_packed_op(qs, kbs, cfg)):
+        assert torch.equal(got > 0, selected_by_exact_scores(q, kb, cfg))
