@@ -48,12 +48,15 @@ KernelTimer::~KernelTimer() {
   g_timed.push_back(TimedLaunch{name_, start_, stop});
 }
 
+// Also below the 48 KB that need no permission: those are for a kernel's static and dynamic memory together.
 int raise_smem_limit(SmemLimit& done, const void* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return MOBA_B200_OK;
   int dev = 0;
   MOBA_CUDA_OK(cudaGetDevice(&dev));
-  int* have = dev >= 0 && dev < 64 ? &done.bytes[dev] : nullptr;      // racing callers set the same limit twice, harmlessly
+  int* have = dev >= 0 && dev < 64 ? &done.bytes[dev] : nullptr;
   if (have != nullptr && __atomic_load_n(have, __ATOMIC_RELAXED) >= (int)bytes) return MOBA_B200_OK;
+  static std::mutex mu;                                      // a call that needs less must not set the limit back
+  std::lock_guard<std::mutex> lock(mu);
+  if (have != nullptr && *have >= (int)bytes) return MOBA_B200_OK;
   MOBA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   if (have != nullptr) __atomic_store_n(have, (int)bytes, __ATOMIC_RELAXED);
   return MOBA_B200_OK;

@@ -31,6 +31,8 @@ CASES = [
     (1, 5000, 5, 5, 64, 128, 4, torch.bfloat16, None),           # five rows: clusters of eight
     (1, 8192, 2, 2, 64, 16, 2, torch.bfloat16, None),            # 512 columns
     (1, 8208, 2, 2, 64, 16, 2, torch.bfloat16, None),            # 513
+    (1, 6144, 5, 5, 64, 16, 3, torch.float32, None),             # 384 columns: 48 KB of counters beside static memory
+    (1, 45000, 1, 1, 64, 128, 2, torch.bfloat16, None),          # 352
     (1, 1500, 4, 2, 64, 128, 4, torch.bfloat16, [0, 1, 130, 700, 1500]),
     (1, 700, 2, 2, 64, 32, 5, torch.float32, [0, 333, 700]),
     (2, 1000, 4, 2, 128, 64, 8, torch.bfloat16, None),           # a column's second block cut short
