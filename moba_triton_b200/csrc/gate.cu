@@ -20,18 +20,20 @@ namespace moba {
 // ---------------------------------------------------------------------------
 // pool: grid (num_blocks, n_seq * Hkv), 128 or 256 threads
 // ---------------------------------------------------------------------------
-// Threads of a block of keys, and rows in flight per thread. The conversions to float64 bound the 16-bit types
-// (16 a clock and SM), the memory latency float32, which has no second round of loads so: [1,4096,4,64] 14.9 us with
-// 128 and four, 11.2 with 256 and eight; 262144 x 16 heads of 128 in bfloat16 293 and 464.
-template <typename T> constexpr int kPoolThreads = sizeof(T) == 4 ? 256 : 128;
-template <typename T>
-__global__ void __launch_bounds__(kPoolThreads<T>)
+// NT threads of a block of keys, four rows in flight per thread. The conversions to float64 bound the 16-bit types (16
+// a clock and SM), the memory latency float32, which takes 256 threads where a block has rows for them. us in
+// float32, with 128 threads, 256, and 256 with eight rows in flight and sums over the lanes of a warp first:
+//   8192 x 4 heads of 64       16.1  12.3  12.2         131072 x 4 of 64                     55  57   92
+//   16384 x 2 of 128           24.4  16.2  16.3         16384 x 4 of 64, blocks of 16        14  20   35
+// (The third kept so much in registers that a large call had too few CTAs on an SM.)
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT)
 pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restrict__ kbar,
             int packed, int tokens, int hkv, int d, int bs, int nb, int* __restrict__ zero_cell, float* __restrict__ norms) {
   pdl_trigger();
   pdl_wait();
   if (zero_cell != nullptr && blockIdx.x == 0 && threadIdx.x == 0) zero_cell[0] = zero_cell[1] = 0;
-  constexpr int EPV = 16 / sizeof(T), NT = kPoolThreads<T>;   // elements per 16-byte vector; threads
+  constexpr int EPV = 16 / sizeof(T);            // elements per 16-byte vector
   const int blk = (int)(blockIdx.x % nb), kv_row = (int)(blockIdx.x / nb);
   const int seq = kv_row / hkv, h = kv_row % hkv;
   const SeqSpan sp = seq_span(cu, packed, seq, tokens);
@@ -56,7 +58,7 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
 #pragma unroll
   for (int e = 0; e < EPV; ++e) acc[e] = 0.0;
   if (rg < groups) {
-    constexpr int kAhead = sizeof(T) == 4 ? 8 : 4;               // the loads do not depend on one another
+    constexpr int kAhead = 4;                                    // the loads do not depend on one another
     for (int r0 = rg; r0 < hi - lo; r0 += groups * kAhead) {
       uint4 raw[kAhead];
 #pragma unroll
@@ -75,27 +77,16 @@ pool_kernel(const T* __restrict__ k, const int32_t* __restrict__ cu, T* __restri
     }
   }
   // Sums over the row groups, one output element per thread (float64 sums of these values are
-  // exact, so the order of the additions does not matter): in float32 first those in a warp, where a row's
-  // vectors fill a part of it, then the warps' (or groups') through shared memory.
+  // exact, so the order of the additions does not matter).
   __shared__ double red[NT * EPV];
-  const bool by_warp = sizeof(T) == 4 && 32 % vpr == 0;
-  int parts = groups, part = rg;
-  if (by_warp) {
-    for (int o = vpr; o < 32; o <<= 1)
 #pragma unroll
-      for (int e = 0; e < EPV; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-    parts = NT / 32; part = threadIdx.x >> 5;
-  }
-  if (by_warp ? (threadIdx.x & 31) < vpr : rg < groups) {
-#pragma unroll
-    for (int e = 0; e < EPV; ++e) red[part * d + c * EPV + e] = acc[e];
-  }
+  for (int e = 0; e < EPV; ++e) red[threadIdx.x * EPV + e] = acc[e];
   __syncthreads();
   const float occ = (float)(hi - lo);
   double square = 0.0;                                          // in float64: no square leaves its range
   for (int i = threadIdx.x; i < d; i += NT) {
     double s = 0.0;
-    for (int g = 0; g < parts; ++g) s += red[g * d + i];
+    for (int g = 0; g < groups; ++g) s += red[g * d + i];       // thread g * vpr + i / EPV, element i % EPV
     const float total = Elem<T>::round_f((float)s);
     const T mean = Elem<T>::from_f(__fdiv_rn(total, occ));
     dst[i] = mean;
@@ -127,12 +118,14 @@ int launch_pool(const moba_b200_problem& p, const void* k, const int32_t* cu, vo
   const long long ctas = (long long)p.num_blocks * p.n_seq * p.kv_heads;
   if (ctas > 0x7fffffffLL) { set_error("pool: %lld blocks exceed the grid limit", ctas); return MOBA_B200_EUNSUPPORTED; }
   const unsigned grid = (unsigned)ctas;
-#define MOBA_POOL(T)                                                                                   \
-  MOBA_CUDA_OK(launch_chained(pool_kernel<T>, grid, kPoolThreads<T>, 0, st, (const T*)k, cu, (T*)kbar, p.packed, p.tokens, \
+#define MOBA_POOL(T, NT)                                                                               \
+  MOBA_CUDA_OK(launch_chained(pool_kernel<T, NT>, grid, NT, 0, st, (const T*)k, cu, (T*)kbar, p.packed, p.tokens, \
                               p.kv_heads, p.head_dim, p.block_size, p.num_blocks, zero_cell, norms))
-  if (p.dtype == MOBA_B200_F32) MOBA_POOL(float);
-  else if (p.dtype == MOBA_B200_BF16) MOBA_POOL(__nv_bfloat16);
-  else MOBA_POOL(__half);
+  // (by the block size alone: the sums of a sequence do not depend on what else is in the call)
+  if (p.dtype == MOBA_B200_F32 && p.block_size >= 64) MOBA_POOL(float, 256);
+  else if (p.dtype == MOBA_B200_F32) MOBA_POOL(float, 128);
+  else if (p.dtype == MOBA_B200_BF16) MOBA_POOL(__nv_bfloat16, 128);
+  else MOBA_POOL(__half, 128);
 #undef MOBA_POOL
   return MOBA_B200_OK;
 }
