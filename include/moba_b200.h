@@ -158,7 +158,7 @@ typedef struct moba_b200_plan {
   int32_t fwd_q_stages;                    /* forward: shared-memory stages of gathered Q */
   int32_t bwd_kv_buffers;                  /* backward: K/V buffers per SM */
   int32_t bwd_gather_stages;               /* backward: stages of gathered Q and dO */
-  int32_t gate_slots, gate_step;           /* of a buffer the gate no longer has; fixed values */
+  int32_t gate_slots, gate_step;           /* nothing a kernel has: fixed by head_dim, kept for the layout */
   int32_t transpose_chunk_rows;            /* transpose: rows per histogram chunk (0, as the next two: one launch) */
   int32_t transpose_chunks;                /*            chunks per sequence */
   int32_t scatter_warps;                   /*            runs walked side by side per chunk */

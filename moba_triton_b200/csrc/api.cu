@@ -145,7 +145,8 @@ int fill_plan(const moba_b200_problem& p, int gate_path, moba_b200_plan* plan) {
   const TensorCorePlan& t = tensor_core_plan(p.head_dim);
   if (plan->fwd_path == MOBA_B200_PATH_TCGEN05) { plan->fwd_tiles_in_flight = t.fwd_tiles_in_flight; plan->fwd_q_stages = t.fwd_q_stages; }
   if (plan->bwd_path == MOBA_B200_PATH_TCGEN05) { plan->bwd_kv_buffers = t.bwd_kv_buffers; plan->bwd_gather_stages = t.bwd_gather_stages; }
-  if (plan->gate_path == MOBA_B200_PATH_TCGEN05) { plan->gate_slots = t.gate_slots; plan->gate_step = t.gate_step; }
+  // No kernel has these any more; whoever reads the record finds the values that it has always had.
+  if (plan->gate_path == MOBA_B200_PATH_TCGEN05) { plan->gate_slots = p.head_dim == 64 ? 16 : 7; plan->gate_step = p.head_dim == 64 ? 8 : 4; }
   transpose_plan(p, &plan->transpose_chunk_rows, &plan->transpose_chunks, &plan->scatter_warps);
   plan->chunk_tiles = sched_chunk_tiles(p);
   const long long per_row = sched_items_per_row(p);

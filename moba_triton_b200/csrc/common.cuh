@@ -151,11 +151,10 @@ struct TensorCorePlan {
   int head_dim;
   int fwd_tiles_in_flight, fwd_q_stages;
   int bwd_kv_buffers, bwd_gather_stages;
-  int gate_slots, gate_step;      // of a buffer the gate no longer has; the record keeps the fields
 };
 constexpr TensorCorePlan kTensorCorePlans[2] = {
-    {64, 4, 4, 2, 2, 16, 8},
-    {128, 2, 2, 1, 2, 7, 4},
+    {64, 4, 4, 2, 2},
+    {128, 2, 2, 1, 2},
 };
 constexpr const TensorCorePlan& tensor_core_plan(int head_dim) { return kTensorCorePlans[head_dim == 64 ? 0 : 1]; }
 

@@ -1,5 +1,5 @@
-// Gate scorer on tcgen05 tensor cores (bf16/f16, block_size 128, head_dim
-// 64/128, at most 8 ranked blocks per query).
+// Gate scorer on tcgen05 tensor cores (bf16/f16, head_dim 64/128): block_size 128 and at most 8 ranked
+// blocks per query; EXACT (below) for the other block sizes and up to 16.
 //
 // Persistent CTAs (two per SM) walk units of two neighbouring 128-query tiles of one (sequence, query
 // head), heaviest first, in alternating direction per round. With 128-token blocks a tile is exactly one
@@ -820,8 +820,9 @@ int launch_gate_sm100(const moba_b200_problem& p, const void* q, const void* kba
 #undef GO
 }
 
-// Block sizes that divide the tile of 128 queries; as many ranked blocks as the per-thread buffers
-// can exchange; a candidate window keeps the portable kernel.
+// Block sizes that divide the tile of 128 queries. The list of a row lies in registers: up to 16 ranked blocks at
+// head_dim 64 (104 bytes of spills), 12 at 128 (120 in float16; a list of 16 spills 216 there and is not built, 13
+// to 16 ranked blocks keep the portable kernel). A candidate window keeps it too.
 bool gate_exact_sm100_supported(const moba_b200_problem& p) {
   return (p.dtype == MOBA_B200_BF16 || p.dtype == MOBA_B200_F16) && p.block_size >= 16 && kTile % p.block_size == 0 &&
          (p.head_dim == 64 || p.head_dim == 128) && p.take <= (p.head_dim == 64 ? 16 : 12) && p.gate_window == 0 &&
