@@ -207,8 +207,15 @@ __device__ __forceinline__ void merge_sorted(unsigned long long (&a)[N], const u
 // of 32 candidates is sorted and merged into it in 21 exchanges; offering them one by one, a reduction
 // over the warp and two over the list each, was two thirds of the kernel ([1,4096,4,64] float32,
 // 7 of 32 blocks: 76 us, sorted 29, with the eight rows of a warp in step and two numbers a load 25).
-template <typename T, bool SORTED>
-__global__ void __launch_bounds__(128)
+// IN_STEP: the exchanges of the eight rows of a warp wait together, in every chunk that enters a list of theirs.
+// That takes 128 registers, four CTAs an SM, where six fit the shared memory of head_dim 64, and the further a row
+// goes the fewer of its chunks enter its list. Row by row, in 80 registers, long rows are the faster there (2 heads
+// of 64 in float32, us in step and row by row: 2 of blocks of 16, 256 blocks 60 and 78, 1024 388 and 371, 4096 4240
+// and 3861; 7 of blocks of 128, 512 666 and 711, 1024 2385 and 2326, 2048 8979 and 8087; 31 of blocks of 16, 2048
+// 1385 and 1534). From head_dim 128 on the shared memory holds three CTAs whatever the registers (4096 blocks 7600
+// and 8540).
+template <typename T, bool SORTED, bool IN_STEP>
+__global__ void __launch_bounds__(128, SORTED && !IN_STEP ? 6 : 1)
 gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
                      const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx,
                      float* __restrict__ lse_fill, moba_b200_problem p) {
@@ -276,19 +283,34 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
     }
     const int blk = c0 + lane;
     if constexpr (SORTED) {
-      unsigned long long key[kRowsPerWarp];
-      bool enters = false;
-#pragma unroll
-      for (int r = 0; r < kRowsPerWarp; ++r) {
+      auto key_of = [&](int r) {
         const int row = row0 + warp * kRowsPerWarp + r;
         const bool candidate = gate_candidate(p, blk, row / p.block_size) && blk < n_cand && row < sp.len;
-        key[r] = candidate ? rank_key(Elem<T>::round_f((float)acc[r]), blk) : 0ull;
-        const unsigned long long bar = __shfl_sync(0xffffffffu, best[r], take - 1);   // (by all lanes)
-        enters |= key[r] > bar;
-      }
-      if (__any_sync(0xffffffffu, enters)) {
-        sort_lanes(key, lane);
-        merge_sorted(best, key, lane);
+        return candidate ? rank_key(Elem<T>::round_f((float)acc[r]), blk) : 0ull;
+      };
+      auto bar_of = [&](int r) { return __shfl_sync(0xffffffffu, best[r], take - 1); };   // (by all lanes)
+      if constexpr (IN_STEP) {
+        unsigned long long key[kRowsPerWarp];
+        bool enters = false;
+#pragma unroll
+        for (int r = 0; r < kRowsPerWarp; ++r) {
+          key[r] = key_of(r);
+          const unsigned long long bar = bar_of(r);
+          enters |= key[r] > bar;
+        }
+        if (__any_sync(0xffffffffu, enters)) {
+          sort_lanes(key, lane);
+          merge_sorted(best, key, lane);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < kRowsPerWarp; ++r) {
+          unsigned long long key[1] = {key_of(r)}, list[1] = {best[r]};
+          if (!__any_sync(0xffffffffu, key[0] > bar_of(r))) continue;
+          sort_lanes(key, lane);
+          merge_sorted(list, key, lane);
+          best[r] = list[0];
+        }
       }
       continue;
     }
@@ -397,13 +419,19 @@ int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* 
     return MOBA_B200_EUNSUPPORTED;
   }
   dim3 grid((p.max_seqlen + kGateRows - 1) / kGateRows, p.n_seq * p.q_heads);
-#define MOBA_GATE(T, SORTED)                                                                  \
+  const bool in_step = d >= 128 || p.num_blocks <= 768 + 32 * p.take;
+#define MOBA_GATE(T, SORTED, IN_STEP)                                                         \
   do {                                                                                        \
     static SmemLimit limit;                                                                   \
-    if (int rc = raise_smem_limit(limit, (const void*)gate_portable_kernel<T, SORTED>, smem)) return rc; \
-    MOBA_CUDA_OK(launch_chained(gate_portable_kernel<T, SORTED>, grid, 128, smem, st, (const T*)q, (const T*)kbar, cu, block_idx, lse_fill, p)); \
+    if (int rc = raise_smem_limit(limit, (const void*)gate_portable_kernel<T, SORTED, IN_STEP>, smem)) return rc; \
+    MOBA_CUDA_OK(launch_chained(gate_portable_kernel<T, SORTED, IN_STEP>, grid, 128, smem, st, (const T*)q, (const T*)kbar, cu, block_idx, lse_fill, p)); \
   } while (0)
-#define MOBA_GATE_T(T) do { if (p.take <= 32) MOBA_GATE(T, true); else MOBA_GATE(T, false); } while (0)
+#define MOBA_GATE_T(T)                                                                        \
+  do {                                                                                        \
+    if (p.take > 32) MOBA_GATE(T, false, false);                                              \
+    else if (in_step) MOBA_GATE(T, true, true);                                               \
+    else MOBA_GATE(T, true, false);                                                           \
+  } while (0)
   if (p.dtype == MOBA_B200_F32) MOBA_GATE_T(float);
   else if (p.dtype == MOBA_B200_BF16) MOBA_GATE_T(__nv_bfloat16);
   else MOBA_GATE_T(__half);

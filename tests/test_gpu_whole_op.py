@@ -237,3 +237,21 @@ def test_portable_gate_lists(blocks, top_k, device):
     want = torch.cat([want, own[None, :, None].expand(2, -1, 1)], -1).sort(-1).values
     have = torch.where(got < 0, blocks, got.long()).sort(-1).values[..., :want.shape[-1]]
     assert torch.equal(have, want)
+
+
+@pytest.mark.parametrize("blocks,top_k,d", [(800, 2, 64), (801, 2, 64), (1024, 9, 64), (1025, 9, 64), (1792, 33, 64), (1793, 33, 64), (1100, 5, 128)])
+def test_portable_gate_lists_of_long_rows(blocks, top_k, d, device):
+    """Either side of the line between the rows of a warp sorted in step and row by row; the last rows, with ties."""
+    cfg = moba.MoBAConfig(16, top_k, dtype=torch.float32)
+    s, n = blocks * 16 - 3, 500
+    g = torch.Generator().manual_seed(blocks)
+    q = torch.randint(-2, 3, (1, s, 1, d), generator=g).float().to(device)
+    kbar = torch.randint(-2, 3, (1, 1, blocks, d), generator=g).float().to(device)
+    got = moba.gate_select(q, kbar, cfg).reshape(s, -1)[-n:]
+    scores = q[0, -n:, 0].double() @ kbar.reshape(blocks, d).double().t()
+    own = torch.arange(s - n, s, device=device) // 16
+    ids = torch.arange(blocks, device=device)
+    key = scores * 4096 - ids
+    key[ids[None, :] >= own[:, None]] = -float("inf")
+    want = torch.cat([key.topk(top_k - 1, dim=-1).indices, own[:, None]], -1).sort(-1).values
+    assert torch.equal(got.long(), want)
