@@ -5,8 +5,8 @@
 // head), heaviest first, in alternating direction per round. With 128-token blocks a tile is exactly one
 // block, so every row of a tile has the same candidates: the blocks before the tile's own. Roles:
 //   loader (1 thread)  TMA: block means, 64 blocks a step; the unit's queries into the L2
-//   mma    (1 warp)    S = Q Kbar^T (M128 N64 K=D) with Q as operand A from TMEM, tile by tile, for the
-//                      first steps of the unit (bounding pass) and then for all (ranking pass)
+//   mma    (1 warp)    S = Q Kbar^T (M128 N64 K=D) with Q as operand A from TMEM, tile by tile, for a
+//                      few steps of the unit (bounding pass) and then for all (ranking pass)
 //   select (4 warps per tile) bring the tile's queries into TMEM, then one row per thread; no two
 //          threads share a word:
 //          1. The bounding pass only keeps, per row, the maxima of sixteen interleaved subsets of
@@ -185,17 +185,24 @@ struct Unit {
   int n_first;              // steps the bounding pass scores before the ranking pass scores all
   // 64 blocks of the Kbar row that a step of the unit scores
   __device__ __forceinline__ int blocks_of(int step) const {
-    const int s = step < n_first ? step : step - n_first;
+    const int s = step >= n_first ? step - n_first : step < n_first / 2 ? step : step + max(0, n_steps - 1 - n_first);
     return (s < n_lo ? s : s_hi0 + (s - n_lo)) * kStepBlocks;
   }
   // a unit takes n_first + n_steps steps: the bounding pass, then the ranking pass
   __device__ __forceinline__ int steps() const { return n_first + n_steps; }
   __device__ __forceinline__ bool has(int w) const { return w < tiles && tile0 + w >= 0; }
 };
-// The bounding pass looks at the first 256 candidates only: they give a bar that few scores of a later
+// The bounding pass looks at 256 candidates only: they give a bar that few scores of another
 // step pass, and scoring a long row of block means twice would cost more tensor-core time than the
 // tighter bar saves: us for 1024 and 4096 blocks, head_dim 128: 2 steps 1070 and 337, 4 steps 1068 and 332, 6 1088
-// and 342, 8 1141 and 383.
+// and 342, 8 1141 and 383. Two steps are the first and two the last that a unit fills: scores that rise with
+// the position pass a bar of the first blocks one and all. us with all four at the front, and so (the last step itself,
+// half empty, makes a worse bar of independent scores), for scores of deviation 0.7 (1.4 in blocks of 32) that rise
+// over the sequence by                                               0            6            32
+//   131072 queries x 4 heads of 64, 1024 blocks                   126  129     263  127     427  136
+//   262144 x 4 of 64, 2048 blocks                                 371  379     674  359    1957  363
+//   65536 x 4 of 64, 512 blocks, 12 each (exact)                  133  135     303  189     432  216
+//   16384 x 4 of 64, 512 blocks of 32 (exact)                      33   34      54   42     159   78
 constexpr int kBoundSteps = 4;
 // So few candidates are ranked faster than a pass of their own takes: 8192 x 4, 64 blocks 12.8 us with the line at
 // 32, 11.1 at 16, 10.9 at 8; 16 sequences of 300 to 9000 tokens 149, 144, 144.

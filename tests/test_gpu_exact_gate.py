@@ -157,7 +157,7 @@ def ladder(blocks, rows, d, dtype, tiles, g):
     whole = torch.stack([ids % span,                          # rising: all enter the list
                          span - 1 - ids % span,               # falling: none after the first
                          torch.full_like(ids, 7),             # equal: the trace and the id decide
-                         torch.where(ids < 256, ids % 3, span // 2 + ids % 5),   # high past the first 256, which bound
+                         torch.where(ids < 256, ids % 3, span // 2 + ids % 5),   # high past the first 256
                          torch.randint(0, span, (blocks,), generator=g)])
     kb = torch.zeros(blocks, 1, d, dtype=torch.float64)
     q = torch.zeros(rows, 2, d, dtype=torch.float64)
@@ -176,7 +176,7 @@ def ladder(blocks, rows, d, dtype, tiles, g):
 @pytest.mark.parametrize("d,top_k", [(64, 4), (64, 12), (64, 17), (128, 13)])
 @pytest.mark.parametrize("blocks", [255, 256, 257, 321, 577])
 def test_unsure_scores_past_the_bounding_pass(blocks, d, top_k, dtype, tiles, device):
-    """More candidates than the first 256 that bound the rest; every score is taken again in float64, so the
+    """More candidates than the 256 that bound the rest; every score is taken again in float64, so the
     lists of those that wait fill up in the middle of a window, with lanes that lag a window behind."""
     g = torch.Generator().manual_seed(blocks + d + top_k)
     q, kb = ladder(blocks, blocks * BS - 11, d, dtype, tiles, g)

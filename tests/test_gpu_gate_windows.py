@@ -1,5 +1,5 @@
 """The tensor-core gate where its bookkeeping has edges: candidate counts around a window of 64 scores,
-around the bounding pass (more than 16 candidates; the first 256 bound) and odd numbers of query tiles,
+around the bounding pass (more than 16 candidates; 128 at either end bound) and odd numbers of query tiles,
 with score patterns that let every candidate pass its bar, or none after the first.
 
 Scores are whole numbers that both 16-bit types hold, so the rule decides alone: score descending,
@@ -30,7 +30,7 @@ def patterns(blocks, d, g):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "f16"])
 @pytest.mark.parametrize("d,top_k", [(64, 8), (64, 3), (128, 8), (128, 9)])
-@pytest.mark.parametrize("blocks", [1, 2, 17, 18, 33, 64, 65, 66, 129, 257, 258, 321])
+@pytest.mark.parametrize("blocks", [1, 2, 17, 18, 33, 64, 65, 66, 129, 257, 258, 321, 386, 449, 641])
 def test_selection_is_the_rule(blocks, d, top_k, dtype, device):
     g = torch.Generator().manual_seed(blocks * 3 + d)
     kb = patterns(blocks, d, g)
