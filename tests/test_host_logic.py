@@ -205,7 +205,7 @@ def test_launch_plan_is_a_table_lookup_on_the_problem_record():
     assert target["gate_path"] == target["fwd_path"] == target["bwd_path"] == "tcgen05"
     assert (target["fwd_tiles_in_flight"], target["fwd_q_stages"]) == (4, 4)
     assert (target["bwd_kv_buffers"], target["bwd_gather_stages"]) == (2, 2)
-    assert (target["gate_slots"], target["gate_step"]) == (16, 8)                   # fixed: fields that no kernel has a use for
+    assert (target["gate_slots"], target["gate_step"]) == (16, 8)
     assert (target["transpose_chunk_rows"], target["transpose_chunks"], target["scatter_warps"]) == (512, 256, 8)
     assert target["chunk_tiles"] == -(-(131072 * 4 * 8 // 128) // (4 * 148))
     gqa = launch_plan((1, 524288, 32, 128), 8, torch.bfloat16, cfg)
