@@ -209,13 +209,18 @@ __device__ __forceinline__ void merge_sorted(unsigned long long (&a)[N], const u
 // 7 of 32 blocks: 76 us, sorted 29, with the eight rows of a warp in step and two numbers a load 25).
 // IN_STEP: the exchanges of the eight rows of a warp wait together, in every chunk that enters a list of theirs.
 // That takes 128 registers, four CTAs an SM, where six fit the shared memory of head_dim 64, and the further a row
-// goes the fewer of its chunks enter its list. Row by row, in 80 registers, long rows are the faster there (2 heads
-// of 64 in float32, us in step and row by row: 2 of blocks of 16, 256 blocks 60 and 78, 1024 388 and 371, 4096 4240
-// and 3861; 7 of blocks of 128, 512 666 and 711, 1024 2385 and 2326, 2048 8979 and 8087; 31 of blocks of 16, 2048
-// 1385 and 1534). From head_dim 128 on the shared memory holds three CTAs whatever the registers (4096 blocks 7600
-// and 8540).
+// goes the fewer of its chunks enter its list; the longer the list, the more do. Row by row, in 80 registers, the
+// time is, of that in step (2 heads of 64 in float32, blocks of 16 unless noted, by ranked and all blocks):
+//    1   500 1.06    700 0.98    850 0.98              9  1100 1.12   1500 1.01   2000 0.98
+//    2   700 1.02    850 1.00   1024 0.97   4096 0.92  12  1500 1.03   2000 1.00   3000 0.96
+//    4   800 1.10   1024 1.02                         16  1500 1.05   2000 1.03   3000 0.98   4096 0.95
+//    7  1100 1.09   1500 0.99   2000 0.96             21  3000 1.04   4096 1.02
+//    7 (of 128)  800 1.01   1000 0.98   1400 0.94     31  2500 1.12   4096 1.06   8000 0.97
+// From head_dim 128 on the shared memory holds three CTAs whatever the registers (7 of 1024 blocks 1.20). (A minimum
+// of 0 CTAs leaves the registers to the compiler, 128 and, without SORTED, 96; a minimum of one let it take 201,
+// and [1,4096,4,64] 35 us.)
 template <typename T, bool SORTED, bool IN_STEP>
-__global__ void __launch_bounds__(128, SORTED && !IN_STEP ? 6 : 1)
+__global__ void __launch_bounds__(128, SORTED && !IN_STEP ? 6 : 0)
 gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
                      const int32_t* __restrict__ cu, int32_t* __restrict__ block_idx,
                      float* __restrict__ lse_fill, moba_b200_problem p) {
@@ -283,19 +288,15 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
     }
     const int blk = c0 + lane;
     if constexpr (SORTED) {
-      auto key_of = [&](int r) {
-        const int row = row0 + warp * kRowsPerWarp + r;
-        const bool candidate = gate_candidate(p, blk, row / p.block_size) && blk < n_cand && row < sp.len;
-        return candidate ? rank_key(Elem<T>::round_f((float)acc[r]), blk) : 0ull;
-      };
-      auto bar_of = [&](int r) { return __shfl_sync(0xffffffffu, best[r], take - 1); };   // (by all lanes)
       if constexpr (IN_STEP) {
         unsigned long long key[kRowsPerWarp];
         bool enters = false;
 #pragma unroll
         for (int r = 0; r < kRowsPerWarp; ++r) {
-          key[r] = key_of(r);
-          const unsigned long long bar = bar_of(r);
+          const int row = row0 + warp * kRowsPerWarp + r;
+          const bool candidate = gate_candidate(p, blk, row / p.block_size) && blk < n_cand && row < sp.len;
+          key[r] = candidate ? rank_key(Elem<T>::round_f((float)acc[r]), blk) : 0ull;
+          const unsigned long long bar = __shfl_sync(0xffffffffu, best[r], take - 1);   // (by all lanes)
           enters |= key[r] > bar;
         }
         if (__any_sync(0xffffffffu, enters)) {
@@ -305,8 +306,10 @@ gate_portable_kernel(const T* __restrict__ q, const T* __restrict__ kbar,
       } else {
 #pragma unroll
         for (int r = 0; r < kRowsPerWarp; ++r) {
-          unsigned long long key[1] = {key_of(r)}, list[1] = {best[r]};
-          if (!__any_sync(0xffffffffu, key[0] > bar_of(r))) continue;
+          const int row = row0 + warp * kRowsPerWarp + r;
+          const bool candidate = gate_candidate(p, blk, row / p.block_size) && blk < n_cand && row < sp.len;
+          unsigned long long key[1] = {candidate ? rank_key(Elem<T>::round_f((float)acc[r]), blk) : 0ull}, list[1] = {best[r]};
+          if (!__any_sync(0xffffffffu, key[0] > __shfl_sync(0xffffffffu, best[r], take - 1))) continue;
           sort_lanes(key, lane);
           merge_sorted(list, key, lane);
           best[r] = list[0];
@@ -419,7 +422,7 @@ int launch_gate_portable(const moba_b200_problem& p, const void* q, const void* 
     return MOBA_B200_EUNSUPPORTED;
   }
   dim3 grid((p.max_seqlen + kGateRows - 1) / kGateRows, p.n_seq * p.q_heads);
-  const bool in_step = d >= 128 || p.num_blocks <= 768 + 32 * p.take;
+  const bool in_step = d >= 128 || p.take > 16 || p.num_blocks <= 768 + 128 * p.take;
 #define MOBA_GATE(T, SORTED, IN_STEP)                                                         \
   do {                                                                                        \
     static SmemLimit limit;                                                                   \

@@ -239,7 +239,7 @@ def test_portable_gate_lists(blocks, top_k, device):
     assert torch.equal(have, want)
 
 
-@pytest.mark.parametrize("blocks,top_k,d", [(800, 2, 64), (801, 2, 64), (1024, 9, 64), (1025, 9, 64), (1792, 33, 64), (1793, 33, 64), (1100, 5, 128)])
+@pytest.mark.parametrize("blocks,top_k,d", [(896, 2, 64), (897, 2, 64), (1792, 9, 64), (1793, 9, 64), (2816, 17, 64), (2817, 17, 64), (2945, 18, 64), (1100, 5, 128)])
 def test_portable_gate_lists_of_long_rows(blocks, top_k, d, device):
     """Either side of the line between the rows of a warp sorted in step and row by row; the last rows, with ties."""
     cfg = moba.MoBAConfig(16, top_k, dtype=torch.float32)
