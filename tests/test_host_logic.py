@@ -254,7 +254,7 @@ def test_launch_plan_of_the_whole_op_says_what_the_op_runs():
         launch_plan((1, 64, 3, 64), 2, bf16, cfg)
 
 
-@pytest.mark.parametrize("tokens,forward,step", [(14204, 8, 8), (14208, 8, 14), (16384, 8, 15), (37888, 16, 24), (37889, 17, 17)])
+@pytest.mark.parametrize("tokens,forward,step", [(14204, 8, 8), (14208, 8, 12), (16384, 8, 13), (18940, 8, 14), (18944, 8, 16), (37888, 16, 24), (37889, 17, 17)])
 def test_launch_plan_tells_a_forward_from_a_training_step(tokens, forward, step):
     """Both ends of the range (24 to 64 tiles per SM) in which a training step has longer work items than a
     forward alone, and the first sizes outside it; float32 has one cut."""
