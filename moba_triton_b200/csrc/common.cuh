@@ -316,8 +316,15 @@ __device__ __forceinline__ bool claim_item(ClaimWalk& w, const ClaimOrder& order
 // As a rule all rows are one group: its last items are its smallest. Where the queries of all rows are far more than
 // the L2 and those of a few are not, groups of 48 MB keep them there while their columns gather them once per
 // selected block: 262144 tokens in 32 sequences, 16 heads of 128, 4114 -> 3776, 7963 -> 7437 us. The items of the
-// last group are then not small, and there have to be many more than they hold: 40000 in 16 sequences, 32 heads on 8,
-// 978 -> 1026 in groups (540 tiles per SM, columns of 32).
+// last group are then not small, and there have to be many more than they hold. Time in groups over that without
+// (dealt, or claimed over all rows), least and most of packed batches of 12000 to 180000 tokens in 8, 16 and 32
+// sequences, 16 to 64 heads, by tiles per SM over the tiles of a column:
+//                      below 8      8 to 12     12 to 20    20 to 24    24 to 32    32 to 64    above
+//   64   forward      0.92 1.23   0.86 1.16   0.96 1.12   0.81 0.99   0.91 0.97   0.90 0.96   0.83 0.89
+//        backward     0.91 1.24   0.87 1.13   0.96 1.16   0.83 1.02   0.93 1.03   0.89 0.99   0.92 0.95
+//   128  forward      0.81 1.14   0.84 1.12   0.88 1.14   0.73 0.98   0.78 1.00   0.78 0.96   0.90 0.92
+//        backward     0.81 1.23   0.86 1.13   0.91 1.15   0.85 1.00   0.91 1.04   0.92 0.98   0.92 0.95
+// The line is at 32, above which all of these 25 gained.
 // A query window counts with its own rows, in tiles and in bytes.
 static inline int claim_rows(const moba_b200_problem& p, int tiles_per_sm) {
   const long long tiles = (sched_pairs_bound(p) + 127) / 128, column = (long long)(p.q_heads / p.kv_heads) * p.slots;
