@@ -51,10 +51,10 @@ constexpr int kStoreWarp0 = kGatherWarp0 + kGatherWarps, kStoreWarps = 4;
 constexpr int kThreads = (kStoreWarp0 + kStoreWarps) * 32;   // warp 19 only completes its warpgroup
 // Registers: 896 threads are launched with 72 each (64 512). 512 elementwise threads take 80, 128
 // storing threads what a dQ row needs, the other 256 give down to the rest: 64 512 again. At head_dim 64
-// a dQ row needs 88; with 104 the other 256 had 40 and spilled 148 bytes (32 now): 624 -> 612 us at [1,131072,4,64].
-// At 128 the other 256 spill some 130 bytes (with a 64-bit division in the walk over the items 180, and the deal
-// took 1 to 3 % longer). Splits that spill less cost more elsewhere: 72, 104 and 56 registers (56 bytes) 5 %, 80, 88
-// and 48 up to 13 %, on dealt and on claimed items.
+// a dQ row needs 88; with 104 the other 256 had 40 and spilled 148 bytes (48 now): 624 -> 612 us at [1,131072,4,64].
+// At 128 the other 256 spill 84 bytes (180 with a 64-bit division in the walk over the items, and the next item
+// taken in two places of the code: the deal took 1 to 3 % longer). Splits that spill less cost more elsewhere: 72,
+// 104 and 56 registers (56 bytes) 5 %, 80, 88 and 48 up to 13 %, on dealt and on claimed items.
 constexpr int kLaunchRegs = 72, kElemRegs = 80;
 template <int D> constexpr int kStoreRegs = D == 64 ? 88 : 104;
 template <int D> constexpr int kOtherRegs = D == 64 ? 48 : 40;
