@@ -192,9 +192,9 @@ def base_config(wl, total_tokens):
 # captures of one launch at [1,65536,4,64] (2 082 816 pairs). The traffic of these kernels is
 # per-pair partial rows, so a launch's traffic is this figure times the pairs it processes.
 DRAM_BYTES_PER_PAIR = {
-    "bwd_sm100_kernel": (362.2e6 + 302.2e6) / 2082816,
-    "fwd_sm100_kernel": (168.5e6 + 224.8e6) / 2082816,
-    "gate_sm100_kernel": 33.8e6 / 2082816,
+    "bwd_sm100_kernel": (365.5e6 + 303.9e6) / 2082816,
+    "fwd_sm100_kernel": (168.1e6 + 227.2e6) / 2082816,
+    "gate_sm100_kernel": 33.9e6 / 2082816,
 }
 
 
