@@ -31,6 +31,159 @@
 // descriptors do not stay in uniform registers, one took 120. Before, each score that passed was appended to a
 // buffer by predicated stores, five instructions a score whether it passed or not, and the two halves of a row's
 // candidates had lists of their own. us, before and now:
+//   131072 queries x 4 heads of 64, 1024 blocks       218    125       65536 x 4, 512 blocks, 12 each (exact)    319   137
+//   131072 x 32 heads of 128                         2170   1070       2 x 8192 x 4 of 128, blocks of 64 (exact) 117    42
+//   524288 x 32 heads of 128, skewed                27300  12500       16 sequences, 40000 x 32 heads of 128     271   144
+//
+// EXACT: the same kernel where the portable gate used to run (other block sizes that divide 128,
+// more than eight ranked blocks): its selections are those of exact scores, bit for bit. The
+// tensor-core sum is off by at most `err` (a bound from the lengths of the query and of the means of
+// the unit's candidates), so the entry test is loosened by err, the windows keep all 32 bits of a score,
+// and a candidate whose rounding to the input dtype depends on that error is scored again in float64
+// before it is ranked, four by a warp at a time: about one in forty where scores are large against err,
+// every one near zero. A row without a finite bound (infinities, NaN, squares outside float32) has every candidate
+// scored in float64. With blocks finer than the tile a row's candidates end at its own block.
+//
+// Scores are float32 tensor-core sums rounded to the input dtype; the portable
+// gate rounds the exact sum. The two differ only when a float32 partial sum
+// straddles a rounding boundary of the input dtype.
+//
+// Stands in for gate_kernel of the reference (src/moba/kernels/gating.py:92-335).
+#include "common.cuh"
+#include "sm100.cuh"
+
+#include <type_traits>
+
+namespace moba {
+using namespace sm100;
+
+namespace {
+
+constexpr int kTile = 128;
+constexpr int kSub = kTile * 128;
+constexpr int kStepBlocks = 64;            // blocks scored per step
+constexpr int kMaxTake = 8;
+constexpr int kSubsets = 16;               // column subsets of the bounding pass: at least L
+
+// Two tiles to a CTA and two CTAs to an SM, so that one's hand-over between units falls into the other's work.
+template <int D, bool EXACT> struct GateCfg {
+  static constexpr int kTiles = 2, kCtas = 2;
+  static constexpr int kSubs = D / 64;
+  static constexpr int kKb = kSubs * kStepBlocks * 128, kStages = D == 64 ? 4 : 2;   // block means: bytes of a step, stages
+  static constexpr int kSelect = kTiles * kTile, kThreads = kSelect + 64;
+  static constexpr int kMmaWarp = kSelect / 32, kLoadWarp = kMmaWarp + 1;
+  // A thread's window of scores: 64 columns of two bytes (exact: 32 of four), in eight pieces of 16 bytes.
+  // The two windows of a warpgroup also take its Q tile on the way to TMEM.
+  static constexpr int kPiece = kTile * 16, kWindow = 8 * kPiece, kQ = kSubs * kSub;
+  static_assert(kQ <= 2 * kWindow, "a Q tile fits its warpgroup's windows");
+  // Exact: ids of a row's candidates that are to be scored again.
+  static constexpr int kPending = EXACT ? 16 : 0, kPendingBytes = kSelect * kPending * 2;
+  static constexpr int kSmem = kTiles * 2 * kWindow + kStages * kKb + kPendingBytes + 1024 + 512;
+  // TMEM columns of a tile: scores [0, 64), queries [64, 64 + D / 2)
+  static constexpr int kTileCols = 128, kQCol = kStepBlocks;
+};
+
+struct Bars {
+  uint64_t q_here[2], q_full[2], kb_full[4], kb_empty[4], s_full[2], s_free[2], drain;
+  uint32_t tmem_base;
+  int abort;
+};
+
+// Sorted (descending) register list of the L best keys seen so far, t[0, L).
+template <int L, int N>
+__device__ __forceinline__ void list_offer(uint32_t (&t)[N], uint32_t x) {
+#pragma unroll
+  for (int i = 0; i < L; ++i) {
+    const uint32_t hi = max(t[i], x);
+    x = min(t[i], x);
+    t[i] = hi;
+  }
+}
+
+// Batcher's odd-even merge sort, descending; N a power of two.
+template <int N, typename V>
+__device__ __forceinline__ void sort_descending(V (&a)[N]) {
+#pragma unroll
+  for (int p = 1; p < N; p <<= 1)
+#pragma unroll
+    for (int k = p; k >= 1; k >>= 1)
+#pragma unroll
+      for (int j = k % p; j + k < N; j += 2 * k)
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+          if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+            const V x = a[i + j], y = a[i + j + k];
+            a[i + j] = max(x, y);
+            a[i + j + k] = min(x, y);
+          }
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+template <typename T> __device__ __forceinline__ uint32_t round16(float a);
+template <> __device__ __forceinline__ uint32_t round16<__nv_bfloat16>(float a) {
+  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a));
+}
+template <> __device__ __forceinline__ uint32_t round16<__half>(float a) {
+  return (uint32_t)__half_as_ushort(__float2half_rn(a));
+}
+template <typename T> __device__ __forceinline__ float widen16(uint32_t bits);
+template <> __device__ __forceinline__ float widen16<__nv_bfloat16>(uint32_t bits) { return __uint_as_float(bits << 16); }
+template <> __device__ __forceinline__ float widen16<__half>(uint32_t bits) {
+  return __half2float(__ushort_as_half((unsigned short)bits));
+}
+
+// Bits of a score rounded to T, sign-extended, and the low half -> sortable key; never 0 for a real
+// candidate (the low half is 0xFFFF - id with id <= 0xFFFE). The high half counts the steps of T from
+// zero, which both zeros are, with 0x8000 added.
+__device__ __forceinline__ uint32_t make_key(int b, uint32_t low) {
+  const uint32_t mono = b < 0 ? (uint32_t)-b : (uint32_t)b + 0x8000u;
+  return (mono << 16) | low;
+}
+// The other way, from the high half of a key (at least that of -infinity) to the bits of T.
+__device__ __forceinline__ uint32_t bits_of(uint32_t mono) { return mono & 0x8000u ? mono & 0x7FFFu : 0x10000u - mono; }
+template <typename T> constexpr uint32_t kLowest = std::is_same<T, __nv_bfloat16>::value ? 0x80u : 0x400u;   // of -infinity
+
+// What a score has to exceed to be ranked. The plain gate compares scores rounded to T, two at a time,
+// with a number of T; the exact one float32 scores with a bar that err has been taken off.
+template <typename T, bool EXACT> struct Bar;
+template <typename T> struct Bar<T, false> {
+  uint32_t mono = kLowest<T>, pair = 0x10001u * bits_of(kLowest<T>);
+  __device__ __forceinline__ void raise(uint32_t m) { mono = max(mono, m); pair = 0x10001u * bits_of(mono); }
+  // to a score that the list's last entry has, or to the step below one that L candidates reach
+  __device__ __forceinline__ void raise_to_entry(uint32_t key, float) { raise(key >> 16); }
+  __device__ __forceinline__ void raise_below(float reached, float) { raise((make_key((int)(short)round16<T>(reached), 0u) >> 16) - 1u); }
+};
+template <typename T> struct Bar<T, true> {
+  float bar = -INFINITY;
+  __device__ __forceinline__ void raise(uint32_t mono, float err) { bar = fmaxf(bar, widen16<T>(bits_of(max(mono, kLowest<T>))) - err); }
+  __device__ __forceinline__ void raise_to_entry(uint32_t key, float err) { raise(key >> 16, err); }
+  __device__ __forceinline__ void raise_below(float reached, float err) { raise((make_key((int)(short)round16<T>(reached - err), 0u) >> 16) - 1u, err); }
+};
+
+// Which unit a CTA takes in its `round`-th turn: heaviest units first, alternating
+// direction, so that no CTA collects the heaviest unit of every round.
+__device__ __forceinline__ int unit_of(int round) {
+  const int g = (int)gridDim.x, c = (int)blockIdx.x;
+  return round * g + ((round & 1) ? (g - 1 - c) : c);
+}
+
+// Blocks are 128 keys, or (exact) a power of two that divides 128.
+template <bool EXACT> __device__ __forceinline__ int block_of(int row, const moba_b200_problem& p) {
+  return EXACT ? row >> (31 - __clz(p.block_size)) : row / kTile;
+}
+
+// The bounding pass looks at 256 candidates only: they give a bar that few scores of another
+// step pass, and scoring a long row of block means twice would cost more tensor-core time than the
+// tighter bar saves: us for 1024 and 4096 blocks, head_dim 128: 2 steps 1070 and 337, 4 steps 1068 and 332, 6 1088
+// and 342, 8 1141 and 383. Two steps are the first and two the last that a unit fills: scores that rise with
+// the position pass a bar of the first blocks one and all. us with all four at the front, and so (the last step itself,
+// half empty, makes a worse bar of independent scores), for scores of deviation 0.7 (1.4 in blocks of 32) that rise
+// over the sequence by                                               0            6            32
 //   131072 queries x 4 heads of 64, 1024 blocks                   125  126     250  122     425  136
 //   262144 x 4 of 64, 2048 blocks                                 370  372     625  343    1938  359
 //   65536 x 4 of 64, 512 blocks, 12 each (exact)                  132  133     213  144     272  154
