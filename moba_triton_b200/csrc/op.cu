@@ -33,24 +33,31 @@ inline size_t up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
 //   [1,4096,4] float32, whose kernel       6.9    256                                               -  185  198
 //     starts a CTA for every tile that an item may have
 // Between 24 and 64 tiles per SM the partials are what a finer cut costs: eight tiles on top of a quarter of an
-// SM's share, or six below 32, where columns longer than the items make about two items to an SM and two of eight
-// more are longer than its share. Training step, its time over that with items of a quarter (at least 8), by tiles
-// per SM (8 selected blocks; q heads on kv heads):
-//                   quarter + 8:  24    26    28    30    40    50    58    64    72    84   100     + 6:  24    26    28    30
-//   head_dim 64    4 on 4        0.96              0.96  0.96  0.98  0.97  0.98  0.98  0.99  1.01
-//                  4 on 1        0.99              0.96  0.97  0.98  1.00  1.00  0.99  1.00  1.00
-//                  8 on 2        0.99              0.92  0.95  0.95  0.97  0.96  0.97  0.96  0.99
-//                 16 on 4        1.06  1.04  0.96  0.95                                                   0.95  0.99  0.92  0.91
-//                 32 on 8        0.98  1.01  1.04  1.04                                                   1.00  0.98  0.98  0.98
-//   head_dim 128   4 on 4        0.97  0.98  0.96  0.97  0.98  0.98  0.99  1.00  0.99  1.01  1.00         0.97  0.98  0.96  0.97
-//                  4 on 1        1.04  0.97  0.94  0.96                                                   0.98  0.95  0.97  0.99
-//                  8 on 2        1.04  0.98  0.94  0.94                                                   0.95  0.93  0.94  0.94
-//                 16 on 4        1.05  1.02  0.97  0.97  0.96  0.98  0.99  0.99  0.99  0.98  0.99         0.96  0.97  0.93  0.93
-//                 32 on 8        0.99  1.02  1.04  1.03                                                   0.99  1.00  0.98  0.97
-//                  8 on 2 of 12  1.04  1.02  0.98  0.95                                                   0.97  0.98  0.94  0.91
-//                  4 on 4 of 4   1.04  1.01  0.99  0.98                                                   1.03  1.01  0.98  0.98
+// SM's share. Below 32 that makes about two items to an SM where columns are longer than the items, more than
+// its share: with columns of more than 16 tiles six on top. Columns of four tiles or less are hardly cut, the longest
+// of them alone, and begin at 27. Training step, its time over that with items of a quarter (at least 8), by tiles
+// per SM (q heads on kv heads of selected blocks):
+//                   quarter + 8:  24    27    30    32    40    50    58    64    72    84   100     + 6:  24    27    30    32
+//   head_dim 64    4 on 4 of 8   0.96        0.96        0.96  0.98  0.97  0.98  0.98  0.99  1.01
+//                  4 on 1 of 8   0.99        0.96        0.97  0.98  1.00  1.00  0.99  1.00  1.00
+//                  8 on 2 of 8   0.99        0.92        0.95  0.95  0.97  0.96  0.97  0.96  0.99
+//                  4 on 4 of 4   1.04  1.00  0.98  1.00                                                   1.03  0.99  0.98  0.99
+//                  4 on 4 of 12  0.97  0.93  0.96  0.95                                                   0.98  0.97  0.98  0.96
+//                  4 on 2 of 8   0.92  0.91  0.92  0.94                                                   0.94  0.94  0.94  0.95
+//                 16 on 4 of 8   1.06  1.00  0.95  0.94                                                   0.95  0.94  0.91  0.94
+//                 32 on 8 of 8   0.98  1.02  1.04  0.99                                                   1.00  0.98  0.98  0.94
+//   head_dim 128   4 on 4 of 8   0.97  0.96  0.97  0.97  0.98  0.98  0.99  1.00  0.99  1.01  1.00         0.97  0.96  0.97  0.96
+//                  4 on 1 of 8   1.04  0.96  0.96  0.97                                                   0.98  0.96  0.99  1.01
+//                  8 on 2 of 8   1.04  0.95  0.94  0.94                                                   0.95  0.94  0.94  0.99
+//                 16 on 4 of 8   1.05  1.00  0.97  0.94  0.96  0.98  0.99  0.99  0.99  0.98  0.99         0.96  0.94  0.93  0.96
+//                 32 on 8 of 8   0.99  1.03  1.03  0.99                                                   0.99  0.98  0.97  0.94
+//                  4 on 2 of 6   0.95  0.94  0.96  0.95                                                   0.97  0.98  0.97  0.96
+//                 16 on 4 of 6   1.04  0.97  0.95  0.94                                                   0.98  0.94  0.95  0.96
+//                  8 on 2 of 12  1.04  0.98  0.95  0.94                                                   0.97  0.95  0.91  0.94
+//                 16 on 16 of 4  1.04  0.98  0.98  0.99                                                   1.04  0.98  0.99  1.00
+//                  4 on 4 of 2   1.00  1.00  1.01  0.98                                                   1.00  1.00  1.01  0.98
 // (Below, at 18 and 21, a longer item is 0.95 to 1.06 of the time. Passes of one KV head of such a call take the
-// call's cut, for its bits; at head_dim 128 they were faster with items of 8: [1,16384,4] 884 us, 948.)
+// call's cut, for its bits; at head_dim 128 they were faster with items of 8: [1,16384,4] 884 us, 982 with 15.)
 // A forward alone has no partials and keeps the finer items, the better spread (2 % of its kernel).
 // The cut decides in which groups dK and dV are summed: who runs the KV heads of a problem in several
 // passes and wants the bits of the whole gives every pass the whole's chunk_tiles
@@ -61,12 +68,13 @@ moba_b200_problem with_cut(const moba_b200_problem& p0, bool training = true) {
   p.chunk_tiles = sched_chunk_tiles(p);
   const long long tiles = (sched_pairs_bound(p) + 127) / 128;
   const long long row_tiles = ((long long)(p.q_heads / p.kv_heads) * p.max_seqlen * p.slots + 127) / 128;
+  const int column = p.q_heads / p.kv_heads * p.slots;       // tiles, on average
   const bool short_rows = row_tiles <= 128;
   if (tiles <= 4LL * kSchedSMs) p.chunk_tiles = short_rows ? 2 : 4;
   else if (tiles <= 16LL * kSchedSMs && (short_rows || p.dtype == MOBA_B200_F32)) p.chunk_tiles = 4;
-  else if (training && p.dtype != MOBA_B200_F32 && tiles >= 24LL * kSchedSMs && tiles <= 64LL * kSchedSMs)
+  else if (training && p.dtype != MOBA_B200_F32 && tiles >= (column <= 4 ? 27LL : 24LL) * kSchedSMs && tiles <= 64LL * kSchedSMs)
     p.chunk_tiles = (int)((tiles + kSchedSplit * kSchedSMs - 1) / (kSchedSplit * kSchedSMs)) +
-                    (tiles < 32LL * kSchedSMs ? 6 : kMinChunkTiles);
+                    (column > 16 && tiles < 32LL * kSchedSMs ? 6 : 8);
   return p;
 }
 

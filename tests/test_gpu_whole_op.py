@@ -127,9 +127,9 @@ def test_passes_over_kv_heads_cut_columns_like_the_whole_call(s, hkv, group, dev
             assert torch.equal(a, w)
 
 
-@pytest.mark.parametrize("s,hkv,group,d,block,cuts", [(14208, 4, 1, 64, 128, (12, 8)), (18944, 2, 2, 64, 128, (16, 8)),
-                                                      (37888, 4, 1, 128, 128, (24, 16)), (14300, 2, 2, 64, 32, (13, 8))],
-                         ids=["shortest", "passes", "longest", "finer"])
+@pytest.mark.parametrize("s,hkv,group,d,block,cuts", [(14208, 4, 1, 64, 128, (14, 8)), (18944, 2, 2, 64, 128, (16, 8)),
+                                                      (37888, 4, 1, 128, 128, (24, 16)), (14300, 2, 2, 64, 32, (15, 8)), (7104, 2, 4, 64, 128, (12, 8))],
+                         ids=["shortest", "passes", "longest", "finer", "long-columns"])
 def test_a_forward_alone_is_cut_finer_than_the_forward_of_a_step(s, hkv, group, d, block, cuts, device):
     """24 to 64 tiles per SM: one workspace holds either table of work items. O is the same bits for both, all
     four results are those of staged calls with the step's cut, and (up to 32 tiles per SM) of passes."""

@@ -254,7 +254,7 @@ def test_launch_plan_of_the_whole_op_says_what_the_op_runs():
         launch_plan((1, 64, 3, 64), 2, bf16, cfg)
 
 
-@pytest.mark.parametrize("tokens,forward,step", [(14204, 8, 8), (14208, 8, 12), (16384, 8, 13), (18940, 8, 14), (18944, 8, 16), (37888, 16, 24), (37889, 17, 17)])
+@pytest.mark.parametrize("tokens,forward,step", [(14204, 8, 8), (14208, 8, 14), (16384, 8, 15), (37888, 16, 24), (37889, 17, 17)])
 def test_launch_plan_tells_a_forward_from_a_training_step(tokens, forward, step):
     """Both ends of the range (24 to 64 tiles per SM) in which a training step has longer work items than a
     forward alone, and the first sizes outside it; float32 has one cut."""
@@ -267,6 +267,15 @@ def test_launch_plan_tells_a_forward_from_a_training_step(tokens, forward, step)
             assert plan["work_items_per_row"] == -(-tokens // 128) + tokens * 4 * 8 // (128 * cut) + 1
         assert launch_plan((1, tokens, 4, 64), 4, dtype, cfg)["chunk_tiles"] == cuts[1]
         assert launch_plan((1, tokens, 4, 64), 4, dtype, cfg, stages=True)["chunk_tiles"] == forward
+
+
+@pytest.mark.parametrize("tokens,hkv,top_k,step", [(14208, 1, 8, 12), (16384, 1, 8, 13), (18940, 1, 8, 14), (18944, 1, 8, 16), (14208, 2, 8, 14),
+                                                   (28416, 4, 4, 8), (31960, 4, 4, 8), (31968, 4, 4, 15), (22732, 4, 5, 14)])
+def test_the_cut_of_a_training_step_follows_the_size_of_its_columns(tokens, hkv, top_k, step):
+    """Four query heads: columns of 32, 16, 4 and 5 tiles on either side of 24, 27 and 32 tiles per SM."""
+    from moba_triton_b200.tuning import launch_plan
+    cfg = moba.MoBAConfig(128, top_k, dtype=torch.bfloat16)
+    assert launch_plan((1, tokens, 4, 64), hkv, torch.bfloat16, cfg)["chunk_tiles"] == step
 
 
 def test_reference_arm_of_the_bench_prints_the_contract_line():
